@@ -166,7 +166,8 @@ def _model(c, seed):
         m.p["embed"].copy_(embed)
         nxt = _successor(cfg.vocab, seed)
         head = rows(0.35 / math.sqrt(cfg.d_model))
-        head[nxt] += embed * (7.0 / cfg.d_model)
+        # the favourite's logit is about 7: a layer adds about 2.6 to the mean square of a stream that starts at 1
+        head[nxt] += embed * (7.0 * math.sqrt(1 + 2.6 * cfg.n_layers) / cfg.d_model)
         m.p["lm_head"].copy_(head)
         return m, nxt
     cfg = _served_config(c)
@@ -196,7 +197,8 @@ def _prompts(c, vocab, seed):
 
 
 def _rollout(c, vocab, seed):
-    """Finished rollouts of a policy whose log-probs lie near -ln(vocab): dictionary of tensors, padded to the longest."""
+    """Finished rollouts of a policy whose log-probs lie near -ln(vocab), a little above the reference's: dictionary of tensors, padded to
+    the longest."""
     g, lens = _rng(seed, 5), _train_lens(c)
     n, s, t = len(lens), max(p for p, _ in lens), max(r for _, r in lens)
     f32 = dict(generator=g, device=DEVICE)
@@ -204,7 +206,7 @@ def _rollout(c, vocab, seed):
     mask = (torch.arange(t, device=DEVICE)[None, :] < r_len[:, None]).float()
     scores = torch.randn(n, **f32)
     return dict(prompt_ids=torch.randint(3, vocab, (n, s), dtype=torch.int32, **f32), resp_ids=torch.randint(3, vocab, (n, t), dtype=torch.int32, **f32),
-                old_logp=(-math.log(vocab) + 0.01 * torch.randn((n, t), **f32)) * mask, ref_logp=(-math.log(vocab) + 0.01 * torch.randn((n, t), **f32)) * mask,
+                old_logp=(-math.log(vocab) + 0.01 * torch.randn((n, t), **f32)) * mask, ref_logp=(-math.log(vocab) - 0.05 + 0.01 * torch.randn((n, t), **f32)) * mask,
                 mask=mask, adv=((scores + 0.5)[:, None] * mask).contiguous())
 
 
