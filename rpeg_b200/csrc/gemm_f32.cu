@@ -3,14 +3,16 @@
 // plain; grouped: rows of A and C form segments, segment s is multiplied by rows [s * N, s * N + N) of B (the experts of a
 // mixture, see moe.cu for the segment layout and the activations); or batched: the same product for every head, at fixed
 // strides, with B either [N, K] or [K, N].
-// 64 x 64 tile per CTA, 16-deep K slices in shared memory, 4 x 4 outputs per thread.
+//
+// Two kernels. gemm_f32_kernel: 64 x 64 tiles, bound by the FMA rate once M fills them. gemm_f32_rows_kernel: up to SR_MAX rows
+// (decode), bound by streaming B once from memory.
 #include "act_io.cuh"
 #include "moe_segments.cuh"
 #include "rpeg_kernels.h"
 
 namespace rpeg {
 
-constexpr int SG_T = 64, SG_K = 16;
+constexpr int SG_T = 64;
 
 struct GemmF32 {
   const float *A, *X, *B;
@@ -23,18 +25,23 @@ struct GemmF32 {
 
 enum { SG_PLAIN = 0, SG_GROUPED = 1, SG_GATED = 2, SG_BATCHED = 3, SG_BATCHED_KN = 4 };   // KN: B is stored [K, N]
 
-template <int MODE>
+// 64 x 64 outputs per CTA, 4 x 4 per thread, K slices in two shared-memory buffers: the next slice is in registers while this one is
+// multiplied, one barrier a slice. A slice is 32 deep, long enough to cover a memory access (16 where two tiles of B leave no room).
+// VEC: rows of A and B are read as float4 (16-byte aligned operands, K and pitches multiples of 4). Every output is one fp32 sum in the
+// order of k. 282 rows, N = K = 2048: 221 -> 151 us; N = 32000: 1542 -> 1230 us (one scalar slice at a time before).
+template <int MODE, bool VEC>
 __global__ void __launch_bounds__(256)
 gemm_f32_kernel(const GemmF32 p) {
   constexpr bool GATED = MODE == SG_GATED;
-  __shared__ float as[SG_K][SG_T + 4], bs[GATED ? 2 : 1][SG_K][SG_T + 4];
+  constexpr int NB = GATED ? 2 : 1, SK = GATED ? 16 : 32, NV = SK / 16;
+  __shared__ __align__(16) float as[2][SK][SG_T + 4], bs[2][NB][SK][SG_T + 4];
   int M = p.M;
   const float *a = p.A, *B = p.B;
   float* C = p.C;
   if constexpr (MODE == SG_GROUPED || GATED) {
     const MoeSegment sg = moe_segment(p.seg_off, p.n_routed, p.seg_rows, blockIdx.z);
     M = sg.rows;
-    B += static_cast<size_t>(blockIdx.z) * p.N * (GATED ? 2 : 1) * p.ldb;
+    B += static_cast<size_t>(blockIdx.z) * p.N * NB * p.ldb;
     a = p.X != nullptr && static_cast<int>(blockIdx.z) >= p.n_routed ? p.X : p.A + static_cast<size_t>(sg.row0) * p.lda;
     C += static_cast<size_t>(sg.row0) * p.ldc;
   }
@@ -46,38 +53,70 @@ gemm_f32_kernel(const GemmF32 p) {
   const int m0 = blockIdx.y * SG_T, n0 = blockIdx.x * SG_T;
   if (m0 >= M) return;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  float acc[GATED ? 2 : 1][4][4] = {};
-  for (int k0 = 0; k0 < p.K; k0 += SG_K) {
+  // what this thread carries of a slice: of row lr, columns lk + 16 v .. + 3 of A and B; of B stored [K, N], columns 4 (tid % 16) .. of the
+  // rows tid / 16 + 16 v
+  const int lr = tid >> 2, lk = (tid & 3) * 4;
+  float ra[NV][4], rb[NB][NV][4];
+  auto row4 = [&](const float* base, bool live, int k, float (&v)[4]) {
+    if constexpr (VEC) {
+      const float4 t = live && k < p.K ? load4(base + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int e = tid + i * 256, k = e & 15, r = e >> 4;
-      as[k][r] = (m0 + r < M && k0 + k < p.K) ? a[static_cast<size_t>(m0 + r) * p.lda + k0 + k] : 0.f;
+      for (int i = 0; i < 4; ++i) v[i] = live && k + i < p.K ? base[k + i] : 0.f;
+    }
+  };
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      row4(a + static_cast<size_t>(m0 + lr) * p.lda, m0 + lr < M, k0 + lk + 16 * v, ra[v]);
       if constexpr (MODE == SG_BATCHED_KN) {
-        const int n = e & 63, kk = e >> 6;
-        bs[0][kk][n] = (n0 + n < p.N && k0 + kk < p.K) ? B[static_cast<size_t>(k0 + kk) * p.ldb + n0 + n] : 0.f;
+        const int n = n0 + tx * 4, k = k0 + ty + 16 * v;
+        const float* src = B + static_cast<size_t>(k) * p.ldb;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) rb[0][v][i] = n + i < p.N && k < p.K ? src[n + i] : 0.f;
       } else {
 #pragma unroll
-        for (int g = 0; g < (GATED ? 2 : 1); ++g)
-          bs[g][k][r] = (n0 + r < p.N && k0 + k < p.K) ? B[(static_cast<size_t>(g) * p.N + n0 + r) * p.ldb + k0 + k] : 0.f;
+        for (int g = 0; g < NB; ++g) row4(B + (static_cast<size_t>(g) * p.N + n0 + lr) * p.ldb, n0 + lr < p.N, k0 + lk + 16 * v, rb[g][v]);
       }
     }
-    __syncthreads();
+  };
+  auto stash = [&](int buf) {
 #pragma unroll
-    for (int k = 0; k < SG_K; ++k) {
-      float x[4];
+    for (int v = 0; v < NV; ++v)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) x[i] = as[k][ty * 4 + i];
+      for (int i = 0; i < 4; ++i) {
+        as[buf][lk + 16 * v + i][lr] = ra[v][i];
 #pragma unroll
-      for (int g = 0; g < (GATED ? 2 : 1); ++g) {
-        float y[4];
+        for (int g = 0; g < NB; ++g) {
+          if constexpr (MODE == SG_BATCHED_KN) bs[buf][g][ty + 16 * v][tx * 4 + i] = rb[g][v][i];
+          else bs[buf][g][lk + 16 * v + i][lr] = rb[g][v][i];
+        }
+      }
+  };
+  float acc[NB][4][4] = {};
+  fetch(0);
+  stash(0);
+  __syncthreads();
+  int buf = 0;
+  for (int k0 = 0; k0 < p.K; k0 += SK, buf ^= 1) {
+    const bool more = k0 + SK < p.K;
+    if (more) fetch(k0 + SK);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) y[j] = bs[g][k][tx * 4 + j];
+    for (int k = 0; k < SK; ++k) {
+      const float4 x4 = load4(&as[buf][k][ty * 4]);
+      const float x[4] = {x4.x, x4.y, x4.z, x4.w};
+#pragma unroll
+      for (int g = 0; g < NB; ++g) {
+        const float4 y4 = load4(&bs[buf][g][k][tx * 4]);
+        const float y[4] = {y4.x, y4.y, y4.z, y4.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
           for (int j = 0; j < 4; ++j) acc[g][i][j] = fmaf(x[i], y[j], acc[g][i][j]);
       }
     }
+    if (more) stash(buf ^ 1);      // last read before the previous barrier
     __syncthreads();
   }
 #pragma unroll
@@ -96,11 +135,175 @@ gemm_f32_kernel(const GemmF32 p) {
   }
 }
 
+// ---------------------------------------------------------------------------------- few rows
+constexpr int SR_MAX = 16;      // rows of A per pass over B
+constexpr int SR_ROWS = 32;     // most rows of A
+constexpr int SR_WARPS = 4, SR_N = 4;   // a warp's rows of B
+
+__device__ __forceinline__ float4 stream4(const float* p) {   // read once: leaves the L1 to A
+  float4 v;
+  asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+
+// Sums NV values over the 32 lanes: every step halves the lanes that share a value and the values a lane holds. Afterwards a lane holds
+// NV / 32 sums (one if NV < 32) from index `first` on.
+template <int NV>
+__device__ __forceinline__ void spread_sum(float (&v)[NV], int lane, int& first) {
+  first = 0;
+  int n = NV;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    if (n > 1) {
+      n >>= 1;
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < NV / 2; ++i)
+        if (i < n) {
+          const float keep = up ? v[i + n] : v[i], send = up ? v[i] : v[i + n];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+      if (up) first += n;
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  }
+}
+
+// The outputs of MR rows of A against one warp's SR_N rows of B over the K slices that are this warp's. `sums`: [SR_N * MR] of this warp.
+template <int MR>
+__device__ __forceinline__ void rows_dot(const float* a, int lda, int M, const float* const (&b)[SR_N], int K, int ks, int slice, int lane,
+                                         float* sums) {
+  constexpr int U = MR <= 4 ? 4 : 2;      // float4 of each B row in flight
+  float acc[SR_N * MR] = {};
+  const int k4 = K >> 2, step = 32 * ks;
+  auto fold = [&](int f, const float4 (&w)[SR_N]) {
+#pragma unroll
+    for (int m = 0; m < MR; ++m) {
+      const float4 x = load4(a + static_cast<size_t>(m < M ? m : M - 1) * lda + static_cast<size_t>(f) * 4);
+#pragma unroll
+      for (int r = 0; r < SR_N; ++r) {
+        float& s = acc[r * MR + m];
+        s = fmaf(x.x, w[r].x, s); s = fmaf(x.y, w[r].y, s); s = fmaf(x.z, w[r].z, s); s = fmaf(x.w, w[r].w, s);
+      }
+    }
+  };
+  int f = slice * 32 + lane;
+  for (; f + (U - 1) * step < k4; f += U * step) {
+    float4 w[U][SR_N];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int r = 0; r < SR_N; ++r) w[u][r] = stream4(b[r] + static_cast<size_t>(f + u * step) * 4);
+#pragma unroll
+    for (int u = 0; u < U; ++u) fold(f + u * step, w[u]);
+  }
+  for (; f < k4; f += step) {
+    float4 w[SR_N];
+#pragma unroll
+    for (int r = 0; r < SR_N; ++r) w[r] = stream4(b[r] + static_cast<size_t>(f) * 4);
+    fold(f, w);
+  }
+  int first;
+  spread_sum<SR_N * MR>(acc, lane, first);
+  constexpr int NV = SR_N * MR, PER = NV > 32 ? NV / 32 : 1;
+#pragma unroll
+  for (int i = 0; i < PER; ++i)
+    if (NV >= 32 || (lane & (32 / NV - 1)) == 0) sums[first + i] = acc[i];
+}
+
+// Up to SR_ROWS rows of A (per segment), SR_MAX per pass: a warp streams SR_N rows of B, lanes side by side along K, every element of B read once and
+// multiplied with all rows of A (which stay in the L1); `ks` warps share the K range of the same rows of B when N alone gives too few
+// warps to keep memory busy. Bound by the bytes of B: at 4 rows, N = 32000, K = 2048 (262 MB) the 64 x 64 tiles took 331 us, this
+// 51 us (5.2 TB/s); 33 experts of 1024 x 2048, 4 rows of which each takes a few: 342 -> 20 us.
 template <int MODE>
-static int launch_gemm_f32(const GemmF32& p, int rows, int batch, void* stream) {
+__global__ void __launch_bounds__(SR_WARPS * 32)
+gemm_f32_rows_kernel(const GemmF32 p, int ks) {
+  constexpr bool GATED = MODE == SG_GATED;
+  __shared__ float sums[SR_WARPS][SR_N * SR_MAX];
+  griddep_launch();
+  griddep_wait();
+  int M = p.M;
+  const float *a = p.A, *B = p.B;
+  float* C = p.C;
+  if constexpr (MODE == SG_GROUPED || GATED) {
+    const MoeSegment sg = moe_segment(p.seg_off, p.n_routed, p.seg_rows, blockIdx.z);
+    M = sg.rows;
+    if (M <= 0) return;
+    B += static_cast<size_t>(blockIdx.z) * p.N * (GATED ? 2 : 1) * p.ldb;
+    a = p.X != nullptr && static_cast<int>(blockIdx.z) >= p.n_routed ? p.X : p.A + static_cast<size_t>(sg.row0) * p.lda;
+    C += static_cast<size_t>(sg.row0) * p.ldc;
+  }
+  if constexpr (MODE == SG_BATCHED) {
+    a += blockIdx.z * p.a_stride;
+    B += blockIdx.z * p.b_stride;
+    C += blockIdx.z * p.c_stride;
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int group = warp / ks, slice = warp - group * ks, groups = SR_WARPS / ks;
+  constexpr int COLS = GATED ? SR_N / 2 : SR_N;           // outputs of a warp per row of A
+  const int n0 = (blockIdx.x * groups + group) * COLS;
+  const float* b[SR_N];
+#pragma unroll
+  for (int r = 0; r < SR_N; ++r) {
+    const int n = min(n0 + (GATED ? r >> 1 : r), p.N - 1);    // gated: gate and up row of a column side by side
+    b[r] = B + static_cast<size_t>(GATED && (r & 1) ? p.N + n : n) * p.ldb;
+  }
+  for (int m0 = 0; m0 < M; m0 += SR_MAX, a += static_cast<size_t>(SR_MAX) * p.lda, C += static_cast<size_t>(SR_MAX) * p.ldc) {
+    const int left = M - m0;
+    int mr = SR_MAX;
+    if (left <= 1) { mr = 1; rows_dot<1>(a, p.lda, left, b, p.K, ks, slice, lane, sums[warp]); }
+    else if (left <= 2) { mr = 2; rows_dot<2>(a, p.lda, left, b, p.K, ks, slice, lane, sums[warp]); }
+    else if (left <= 4) { mr = 4; rows_dot<4>(a, p.lda, left, b, p.K, ks, slice, lane, sums[warp]); }
+    else if (left <= 8) { mr = 8; rows_dot<8>(a, p.lda, left, b, p.K, ks, slice, lane, sums[warp]); }
+    else rows_dot<SR_MAX>(a, p.lda, left, b, p.K, ks, slice, lane, sums[warp]);
+    __syncthreads();
+    for (int i = threadIdx.x; i < groups * COLS * mr; i += SR_WARPS * 32) {
+      const int g = i / (COLS * mr), c = (i / mr) % COLS, m = i % mr, n = (blockIdx.x * groups + g) * COLS + c;
+      if (m >= left || n >= p.N) continue;
+      float v[2] = {0.f, 0.f};
+#pragma unroll
+      for (int t = 0; t < (GATED ? 2 : 1); ++t)
+        for (int s = 0; s < ks; ++s) v[t] += sums[g * ks + s][(GATED ? 2 * c + t : c) * mr + m];
+      float o = v[0];
+      if constexpr (GATED) o = silu_mul(v[0], v[1]);
+      if constexpr (MODE == SG_GROUPED) o = p.act == FF_GELU ? ff_act<FF_GELU>(o) : (p.act == FF_RELU2 ? ff_act<FF_RELU2>(o) : o);
+      C[static_cast<size_t>(m) * p.ldc + n] = o;
+    }
+    __syncthreads();          // the sums are read
+  }
+}
+
+// float4 reads of A's and B's rows: aligned bases, pitches, K and (where they move the base) strides.
+template <int MODE>
+static bool vector_rows(const GemmF32& p) {
+  const uintptr_t base = reinterpret_cast<uintptr_t>(p.A) | reinterpret_cast<uintptr_t>(p.X) | reinterpret_cast<uintptr_t>(p.B);
+  if ((base & 15) || ((p.lda | p.ldb | p.K) & 3)) return false;
+  return MODE != SG_BATCHED || ((p.a_stride | p.b_stride) & 3) == 0;
+}
+
+template <int MODE>
+static int launch_gemm_f32(const GemmF32& p, int rows, int batch, void* stream_v) {
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
   const dim3 grid((p.N + SG_T - 1) / SG_T, (rows + SG_T - 1) / SG_T, batch);
   if (grid.y > 65535u || grid.z > 65535u) return -2;
-  gemm_f32_kernel<MODE><<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(p);
+  if constexpr (MODE != SG_BATCHED_KN) {
+    if (vector_rows<MODE>(p)) {
+      // Up to 32 rows (an upper bound of a segment's): 16 rows, N = 32000, K = 2048 take 114 us here and 310 in 64 x 64 tiles, 32 rows (two
+      // passes) 222 and 313; N = 2048: 17 and 29 against 144 us. Four passes would lose at large N (64 rows: 320 us in tiles).
+      if (rows <= SR_ROWS) {
+        const int cols = MODE == SG_GATED ? SR_N / 2 : SR_N;
+        int ks = 1;
+        while (ks < SR_WARPS && static_cast<long long>((p.N + cols * SR_WARPS - 1) / (cols * SR_WARPS)) * batch * ks < 4 * 148) ks *= 2;
+        const int per = cols * SR_WARPS / ks;
+        return launch_pdl(gemm_f32_rows_kernel<MODE>, dim3((p.N + per - 1) / per, 1, batch), dim3(SR_WARPS * 32), 0, stream, p, ks) == cudaSuccess
+                   ? 0 : -21;
+      }
+      gemm_f32_kernel<MODE, true><<<grid, 256, 0, stream>>>(p);
+      return cudaGetLastError() == cudaSuccess ? 0 : -21;
+    }
+  }
+  gemm_f32_kernel<MODE, false><<<grid, 256, 0, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 

@@ -1,0 +1,55 @@
+"""GPU tests of single kernels at the sizes where a branch of a dispatch, a tile edge or a remainder can go wrong, against fp64 or fp32
+PyTorch."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from rpeg_b200.ops import kernels as K  # noqa: E402
+
+
+@pytest.fixture(autouse=True)
+def _status():
+    yield
+    K.check_status()
+
+
+def _rel(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-300))
+
+
+# fp32 sums of n products: the error of a sum in any order is below n * 2^-24 of the sum of magnitudes; random signs leave about its root
+F32 = 2e-6
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 7, 8, 9, 16, 17, 65])
+@pytest.mark.parametrize("n,k", [(1, 4), (5, 132), (130, 512), (700, 2052), (64, 65)])
+def test_gemm_f32_rows(cuda_device, m, n, k):
+    g = torch.Generator(device=cuda_device).manual_seed(m * 1000 + n)
+    a, b = (torch.randn(r, k, generator=g, device=cuda_device) for r in (m, n))
+    assert _rel(K.gemm_f32(a, b), a.double() @ b.double().T) < F32
+    wide = torch.randn(m, k + 8, generator=g, device=cuda_device)        # strided rows; one float off: no 16-byte alignment
+    for c0 in (4, 1):
+        assert _rel(K.gemm_f32(wide[:, c0:c0 + k], b), wide[:, c0:c0 + k].double() @ b.double().T) < F32
+
+
+@pytest.mark.parametrize("t,top,shared", [(1, 2, 0), (5, 3, 2), (16, 4, 1), (17, 4, 1)])
+@pytest.mark.parametrize("act", ["none", "gelu", "relu2", "swiglu"])
+def test_moe_gemm_f32_rows(cuda_device, t, top, shared, act):
+    e, n, k, dev = 6, 36, 200, cuda_device
+    g = torch.Generator(device=dev).manual_seed(t)
+    x = torch.randn(t, k, generator=g, device=dev)
+    w = torch.randn(e + shared, n * (2 if act == "swiglu" else 1), k, generator=g, device=dev) / k ** 0.5
+    counts = torch.zeros(e, dtype=torch.int32, device=dev)
+    ids, wts, ticket = K.moe_route(torch.randn(t, e, generator=g, device=dev), e, top, counts)
+    r = K.moe_dispatch(x, ids, wts, ticket, counts, e)
+    got = K.moe_gemm(r.x_sorted, w, r, e, shared, shared_x=x if shared else None, act=act)
+    f = {"none": lambda z: z, "gelu": torch.nn.functional.gelu, "relu2": lambda z: torch.relu(z) ** 2,
+         "swiglu": lambda z: torch.nn.functional.silu(z[:, :n]) * z[:, n:]}[act]
+    want = torch.zeros_like(got, dtype=torch.float64)
+    for i in range(t):
+        for j in range(top):
+            want[int(r.row_of[i, j])] = f(x[i:i + 1].double() @ w[int(ids[i, j])].double().T)[0]
+        for s in range(shared):
+            want[t * top + s * t + i] = f(x[i:i + 1].double() @ w[e + s].double().T)[0]
+    assert _rel(got, want) < F32 * 2
