@@ -381,13 +381,6 @@ constexpr int FB_STAGE_ROW = 64 + 4;                       // floats per staged 
 constexpr int FB_STAGE_BYTES = 128 * FB_STAGE_ROW * 4;     // (rows 272 bytes apart: conflict-free float4 stores)
 constexpr int FB_SMEM = FA_TILE_BYTES * 5 + FB_STAGE_BYTES + 1024 + 1024 + 256;
 
-// global[0 .. bytes) += shared[0 .. bytes) as fp32, one bulk operation in the current bulk group
-__device__ __forceinline__ void bulk_reduce_add_f32(float* gdst, const float* ssrc, uint32_t bytes) {
-  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(gdst), "r"(smem_u32(ssrc)),
-               "r"(bytes)
-               : "memory");
-}
-
 __global__ void attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
                                      float* __restrict__ dvec, int T, int H) {
   // one warp per (token, head): D[h, t] = sum_d dO * O

@@ -53,3 +53,22 @@ def test_moe_gemm_f32_rows(cuda_device, t, top, shared, act):
         for s in range(shared):
             want[t * top + s * t + i] = f(x[i:i + 1].double() @ w[e + s].double().T)[0]
     assert _rel(got, want) < F32 * 2
+
+
+@pytest.mark.parametrize("rows,d", [(1, 8), (3, 264), (149, 4096), (700, 4104), (67, 8192), (33, 8200)])
+@pytest.mark.parametrize("residual,shift", [(True, 0), (False, 1)])
+def test_rmsnorm_bwd_rows(cuda_device, rows, d, residual, shift):
+    """Register-resident rows (up to 8192 columns) and the general kernel; ``shift``: a weight gradient without 16-byte alignment."""
+    g = torch.Generator(device=cuda_device).manual_seed(d)
+    bf = dict(generator=g, device=cuda_device)
+    x, dy, res = (torch.randn(rows, d, **bf).bfloat16() for _ in range(3))
+    w = (1 + 0.1 * torch.randn(d, **bf)).bfloat16()
+    _, rstd, _ = K.rmsnorm_fwd(x, w, 1e-5)
+    dw0 = torch.randn(d, **bf)
+    dw = torch.empty(d + shift, device=cuda_device)[shift:].copy_(dw0)
+    dx = K.rmsnorm_bwd(dy, x, w, rstd, dw, dres_in=res if residual else None)
+    xd, wd = x.double().requires_grad_(), w.double().requires_grad_()
+    y = xd * torch.rsqrt((xd * xd).mean(-1, keepdim=True) + 1e-5) * wd
+    y.backward(dy.double())
+    assert _rel(dx, xd.grad + (res.double() if residual else 0)) < 3e-3      # one rounding to bf16: at most 2^-9 of an element
+    assert _rel(dw, dw0.double() + wd.grad) < 1e-5
