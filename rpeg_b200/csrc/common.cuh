@@ -296,6 +296,12 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r
       : "memory");
 }
 
+__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+
 // Shared-memory matrix descriptor for tcgen05.mma with the 128-byte swizzle.
 //  K-major operand  (rows of 64 bf16 = 128 B, 8-row groups 1024 B apart): sbo = 1024, lbo unused.
 //  MN-major operand (64 contiguous MN elements = 128 B per K row, 8 K rows per 1024 B group):

@@ -164,7 +164,7 @@ int rpeg_flash_attn_fwd(const void* qkv, int ld, int q_col0, int k_col0, int v_c
 
 int rpeg_flash_attn_bwd(const void* qkv, int ld, int q_col0, int k_col0, int v_col0, const void* out,
                         const void* dout, const float* lse, const int* cu_seqlens, int B, int max_seqlen, int T,
-                        int H, int Hkv, int hd, float scale, float* dvec, float* dq_acc, void* dqkv, int ld_dqkv,
+                        int H, int Hkv, int hd, float scale, float* dvec, void* dqkv, int ld_dqkv,
                         int* status, void* stream);
 
 // ---- residual_norm.cu: norms around an fp32 residual stream (`kind`: 0 activation, 1 split-K partials, 2 expert outputs,

@@ -104,7 +104,7 @@ _SIGNATURES = {
     "rpeg_latent_prefill": [P, I, I, P, P, LL, I, I, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, P, P],
     "rpeg_head_gemm": [P, P, P, I, I, I, I, I, I, I, I, I, P, P],
     "rpeg_flash_attn_fwd": [P, I, I, I, I, P, I, I, I, I, I, I, F, P, P, P, P],
-    "rpeg_flash_attn_bwd": [P, I, I, I, I, P, P, P, P, I, I, I, I, I, I, F, P, P, P, I, P, P],
+    "rpeg_flash_attn_bwd": [P, I, I, I, I, P, P, P, P, I, I, I, I, I, I, F, P, P, I, P, P],
 }
 
 

@@ -595,11 +595,10 @@ def flash_attn_bwd(qkv, q_col0, k_col0, v_col0, out, dout, lse, cu_seqlens, max_
     if dqkv is None:
         dqkv = torch.empty_like(qkv)
     dvec = torch.empty((n_heads, T), dtype=torch.float32, device=qkv.device)
-    dq_acc = torch.empty((T, n_heads * head_dim), dtype=torch.float32, device=qkv.device)
     check(lib().rpeg_flash_attn_bwd(qkv.data_ptr(), qkv.stride(0), q_col0, k_col0, v_col0, out.data_ptr(),
                                     dout.data_ptr(), lse.data_ptr(), cu_seqlens.data_ptr(), cu_seqlens.numel() - 1,
                                     max_seqlen, T, n_heads, n_kv_heads, head_dim, scale, dvec.data_ptr(),
-                                    dq_acc.data_ptr(), dqkv.data_ptr(), dqkv.stride(0),
+                                    dqkv.data_ptr(), dqkv.stride(0),
                                     status_word(qkv.device).data_ptr(), _stream()), "rpeg_flash_attn_bwd")
     return dqkv
 

@@ -72,3 +72,31 @@ def test_rmsnorm_bwd_rows(cuda_device, rows, d, residual, shift):
     y.backward(dy.double())
     assert _rel(dx, xd.grad + (res.double() if residual else 0)) < 3e-3      # one rounding to bf16: at most 2^-9 of an element
     assert _rel(dw, dw0.double() + wd.grad) < 1e-5
+
+
+@pytest.mark.parametrize("lens", [[1], [64], [65, 2], [63, 128, 129], [191, 1, 320], [700]])
+@pytest.mark.parametrize("H,Hkv", [(2, 2), (4, 1), (6, 2)])
+def test_flash_attn_bwd_tiles(cuda_device, lens, H, Hkv):
+    """Sub-tiles of 64 streamed rows, tiles of 128 kept ones, heads that share keys: one sub-tile, odd numbers of them, ragged ends."""
+    hd, T, dev = 128, sum(lens), cuda_device
+    g = torch.Generator(device=dev).manual_seed(T * 10 + H)
+    kc, vc, width = H * hd, (H + Hkv) * hd, (H + 2 * Hkv) * hd
+    qkv = torch.randn(T, width, generator=g, device=dev).bfloat16()
+    dout = torch.randn(T, H * hd, generator=g, device=dev).bfloat16()
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), device=dev, dtype=torch.int32)
+    out, lse = K.flash_attn_fwd(qkv, 0, kc, vc, cu, max(lens), H, Hkv, hd)
+    got = K.flash_attn_bwd(qkv, 0, kc, vc, out, dout, lse, cu, max(lens), H, Hkv, hd)
+    x = qkv.double().requires_grad_()
+    off = 0
+    for l in lens:
+        q, k, v = (x[off:off + l, a:b].view(l, -1, hd).transpose(0, 1) for a, b in ((0, kc), (kc, vc), (vc, width)))
+        k, v = k.repeat_interleave(H // Hkv, 0), v.repeat_interleave(H // Hkv, 0)
+        s = (q @ k.transpose(1, 2) * hd ** -0.5).masked_fill(torch.ones(l, l, device=dev).triu(1).bool(), float("-inf"))
+        o = (torch.softmax(s, -1) @ v).transpose(0, 1).reshape(l, -1)
+        o.backward(dout[off:off + l].double())
+        off += l
+    # P, dS, the saved output and the result are each rounded to bf16 (2^-9 of an element at most): four independent roundings. Where a
+    # query sees one key dP - D is zero and the fp32 sums of 128 products leave up to 128 * 2^-23 of |dO| |V| ~ 130, times scale |K| ~ 1
+    for lo, hi in ((0, kc), (kc, vc), (vc, width)):
+        want = x.grad[:, lo:hi]
+        assert float((got[:, lo:hi].double() - want).norm()) < 1e-2 * float(want.norm()) + 2e-3
