@@ -1,0 +1,384 @@
+// bf16 GEMM of full-size shapes for sm_100a: two CTAs work on one 256-row tile (tcgen05 cta_group::2).
+//
+//   C[M,N] = op(A)[M,K] * op(B)[N,K]^T        (fp32 accumulate in TMEM; operand majors as in gemm.cu)
+//
+// Why pairs. With one CTA per 128 x 256 tile every SM reads 48 KB of operands from shared memory per 64-deep K block; a pair shares
+// B (each CTA holds its 128 rows of A and half of B's columns), so an SM stages and reads 32 KB for the same products, the ring is
+// six blocks deep instead of four, and half as much comes through L2. The accumulator (rows 0..127 in the even CTA, 128..255 in the odd
+// one) is double buffered, 2 x 256 TMEM columns.
+//
+// Roles per CTA (192 threads): warp 0 loads this CTA's halves; warp 1 of the even CTA issues the MMAs of both; warps 2..5 carry a
+// 32-row quadrant each through a swizzled 4 KB staging buffer (two per warp) and a TMA store, so that memory sees whole 128-byte
+// lines. Gradients are added by the TMA reduction (fp32 add in L2): nothing is read back into the SM.
+#include "common.cuh"
+#include "rpeg_kernels.h"
+
+namespace rpeg {
+
+// gemm.cu
+int make_tmap_bf16_2d(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner, uint32_t box_outer);
+int make_tmap_f32_2d(CUtensorMap* out, void* ptr, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner, uint32_t box_outer);
+
+constexpr int PG_BM = 128;              // rows per CTA; the pair's tile has 256
+constexpr int PG_BK = 64;
+constexpr int PG_THREADS = 192;
+constexpr int PG_STAGING = 4 * 2 * 4096;
+
+template <int BN>
+struct PairCfg {
+  static constexpr int A_BYTES = PG_BM * PG_BK * 2;
+  static constexpr int B_BYTES = (BN / 2) * PG_BK * 2;
+  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int STAGES = BN == 256 ? 6 : 8;
+  static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + PG_STAGING + 512;
+};
+static_assert(PairCfg<256>::SMEM_BYTES <= 227 * 1024 && PairCfg<128>::SMEM_BYTES <= 227 * 1024, "shared memory");
+
+enum { PG_BF16 = 0, PG_F32 = 1, PG_F32_ADD = 2, PG_SWIGLU = 3 };
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The same shared-memory word in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+// Load into this CTA's shared memory; the bytes are counted on `bar`, which may be the other CTA's.
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m, uint32_t bar, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
+                   smem_u32(dst)),
+               "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(y)
+               : "memory");
+}
+__device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* m, const void* smem_src, int x, int y) {
+  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(reinterpret_cast<uint64_t>(m)),
+               "r"(smem_u32(smem_src)), "r"(x), "r"(y)
+               : "memory");
+}
+__device__ __forceinline__ void umma_bf16_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// The barrier at this offset in both CTAs arrives once every MMA issued so far by this thread has completed.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+  const uint16_t both = 3;
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+               "h"(both)
+               : "memory");
+}
+
+template <int BN, int EPI, bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(PG_THREADS, 1) __cluster_dims__(2, 1, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                 const __grid_constant__ CUtensorMap tmap_c, int M, int N, int K, int group_m, int* status) {
+  using Cfg = PairCfg<BN>;
+  constexpr int STAGES = Cfg::STAGES;
+  constexpr int TN = EPI == PG_SWIGLU ? BN / 2 : BN;       // output columns per tile
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* staging = smem + STAGES * Cfg::STAGE_BYTES;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(staging + PG_STAGING);     // even CTA: both CTAs' bytes of a stage
+  uint64_t* empty_bar = full_bar + STAGES;                                    // each CTA: the pair's MMAs have read the stage
+  uint64_t* tfull_bar = empty_bar + STAGES;                                   // each CTA: accumulator complete
+  uint64_t* tempty_bar = tfull_bar + 2;                                       // even CTA: all eight epilogue warps have read it
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = uniform_warp();
+  const int lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
+  const int m_tiles = (M + 2 * PG_BM - 1) / (2 * PG_BM);
+  const int n_tiles = (N + TN - 1) / TN;
+  const int num_tiles = m_tiles * n_tiles;
+  const int num_kb = (K + PG_BK - 1) / PG_BK;
+  const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&tfull_bar[b], 1);
+      mbar_init(&tempty_bar[b], 8);
+    }
+    *abort_flag = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tmap_a);
+    tma_prefetch_desc(&tmap_b);
+    tma_prefetch_desc(&tmap_c);
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2 * BN) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();                   // the other CTA's barriers exist before anything is counted on them
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  griddep_launch();
+  griddep_wait();                       // returns at once unless this grid was launched as a programmatic dependent
+
+  // Tile order: groups of `group_m` row tiles sweep N together, so that their rows of A stay in L2.
+  auto tile_coords = [&](int t, int& tm, int& tn) {
+    const int per_group = group_m * n_tiles;
+    const int g = t / per_group;
+    const int first_m = g * group_m;
+    const int gsize = min(m_tiles - first_m, group_m);
+    const int r = t - g * per_group;
+    tm = first_m + (r % gsize);
+    tn = r / gsize;
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int w = first; w < num_tiles; w += step) {
+        int tm, tn;
+        tile_coords(w, tm, tn);
+        const int m0 = tm * 2 * PG_BM + static_cast<int>(rank) * PG_BM;
+        // swiglu: the even CTA holds the gate rows of the tile's columns, the odd one the up rows (N = f rows further on)
+        const int n0 = EPI == PG_SWIGLU ? tn * TN + static_cast<int>(rank) * N : tn * TN + static_cast<int>(rank) * (BN / 2);
+        for (int kb = 0; kb < num_kb; ++kb) {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, status, 160)) goto producer_done;
+          uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
+          uint8_t* sb = sa + Cfg::A_BYTES;
+          if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * Cfg::STAGE_BYTES);
+          const uint32_t bar = cluster_addr(&full_bar[stage], 0);
+          if constexpr (!A_MN) {
+            tma_load_2d_pair(sa, &tmap_a, bar, kb * PG_BK, m0);
+          } else {
+#pragma unroll
+            for (int c = 0; c < PG_BM / 64; ++c) tma_load_2d_pair(sa + c * (64 * PG_BK * 2), &tmap_a, bar, m0 + c * 64, kb * PG_BK);
+          }
+          if constexpr (!B_MN) {
+            tma_load_2d_pair(sb, &tmap_b, bar, kb * PG_BK, n0);
+          } else {
+#pragma unroll
+            for (int c = 0; c < BN / 128; ++c) tma_load_2d_pair(sb + c * (64 * PG_BK * 2), &tmap_b, bar, n0 + c * 64, kb * PG_BK);
+          }
+          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+        }
+      }
+    producer_done:;
+    }
+  } else if (warp == 1) {
+    if (rank == 0) {
+      constexpr uint32_t idesc = make_idesc_bf16(2 * PG_BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      const uint32_t s0 = smem_u32(smem);
+      const uint64_t da0 = A_MN ? make_smem_desc_sw128(s0, 64 * PG_BK * 2, 1024) : make_smem_desc_sw128(s0, 16, 1024);
+      const uint64_t db0 = B_MN ? make_smem_desc_sw128(s0 + Cfg::A_BYTES, 64 * PG_BK * 2, 1024) : make_smem_desc_sw128(s0 + Cfg::A_BYTES, 16, 1024);
+      int stage = 0, buf = 0;
+      uint32_t phase = 0, acc_phase = 0;
+      bool ok = true;
+      for (int w = first; w < num_tiles && ok; w += step) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&tempty_bar[buf], acc_phase ^ 1u, abort_flag, status, 260));
+        if (!ok) break;
+        tc_fence_after_sync();
+        const uint32_t tacc = tmem_base + static_cast<uint32_t>(buf * BN);
+        for (int kb = 0; kb < num_kb; ++kb) {
+          ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, abort_flag, status, 261));
+          if (!ok) break;
+          tc_fence_after_sync();
+          const uint64_t da = smem_desc_at(da0, stage * Cfg::STAGE_BYTES), db = smem_desc_at(db0, stage * Cfg::STAGE_BYTES);
+          if (elect_one()) {
+#pragma unroll
+            for (int k = 0; k < PG_BK / 16; ++k)
+              umma_bf16_ss_pair(tacc, smem_desc_at(da, k * (A_MN ? 2048 : 32)), smem_desc_at(db, k * (B_MN ? 2048 : 32)), idesc,
+                                (kb != 0 || k != 0) ? 1u : 0u);
+            umma_commit_pair(&empty_bar[stage]);
+            if (kb == num_kb - 1) umma_commit_pair(&tfull_bar[buf]);
+          }
+          __syncwarp();
+          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+        }
+        if (++buf == 2) { buf = 0; acc_phase ^= 1u; }
+      }
+    }
+  } else {
+    const int quad = warp & 3;          // TMEM lane quadrant this warp may read
+    uint8_t* mine = staging + (warp - 2) * 8192;
+    constexpr bool WIDE = EPI == PG_F32 || EPI == PG_F32_ADD;
+    constexpr int CW = WIDE ? 32 : 64;  // columns per 128-byte line of the staging buffer
+    const uint32_t swz = static_cast<uint32_t>(lane & 7);
+    int buf = 0, sbuf = 0;
+    uint32_t acc_phase = 0;
+    for (int w = first; w < num_tiles; w += step) {
+      int tm, tn;
+      tile_coords(w, tm, tn);
+      const int row0 = tm * 2 * PG_BM + static_cast<int>(rank) * PG_BM + quad * 32, n0 = tn * TN;
+      if (!__all_sync(0xffffffffu, mbar_wait(&tfull_bar[buf], acc_phase, abort_flag, status, 360))) break;
+      tc_fence_after_sync();
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(buf * BN);
+#pragma unroll 1
+      for (int c = 0; c < TN / CW; ++c) {
+        uint4 line[8];
+        if constexpr (EPI == PG_SWIGLU) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t gv[32], uv[32];
+            tmem_ld_32x32(taddr + c * 64 + h * 32, gv);
+            tmem_ld_32x32(taddr + TN + c * 64 + h * 32, uv);
+            tmem_wait_ld();
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              uint32_t o[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float g0 = __uint_as_float(gv[v * 8 + 2 * e]), g1 = __uint_as_float(gv[v * 8 + 2 * e + 1]);
+                o[e] = pack_bf16x2(g0 / (1.f + __expf(-g0)) * __uint_as_float(uv[v * 8 + 2 * e]),
+                                   g1 / (1.f + __expf(-g1)) * __uint_as_float(uv[v * 8 + 2 * e + 1]));
+              }
+              line[h * 4 + v] = make_uint4(o[0], o[1], o[2], o[3]);
+            }
+          }
+        } else if constexpr (EPI == PG_BF16) {
+          uint32_t r0[32], r1[32];
+          tmem_ld_32x32(taddr + c * 64, r0);
+          tmem_ld_32x32(taddr + c * 64 + 32, r1);
+          tmem_wait_ld();
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            uint32_t o[4], q[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              o[e] = pack_bf16x2(__uint_as_float(r0[v * 8 + 2 * e]), __uint_as_float(r0[v * 8 + 2 * e + 1]));
+              q[e] = pack_bf16x2(__uint_as_float(r1[v * 8 + 2 * e]), __uint_as_float(r1[v * 8 + 2 * e + 1]));
+            }
+            line[v] = make_uint4(o[0], o[1], o[2], o[3]);
+            line[4 + v] = make_uint4(q[0], q[1], q[2], q[3]);
+          }
+        } else {
+          uint32_t r[32];
+          tmem_ld_32x32(taddr + c * 32, r);
+          tmem_wait_ld();
+#pragma unroll
+          for (int v = 0; v < 8; ++v) line[v] = make_uint4(r[v * 4], r[v * 4 + 1], r[v * 4 + 2], r[v * 4 + 3]);
+        }
+        if (c == TN / CW - 1) {         // the accumulator has been read: the next but one tile may overwrite it
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(cluster_addr(&tempty_bar[buf], 0));
+        }
+        const int col0 = n0 + c * CW;
+        if (row0 >= M || col0 >= N) continue;              // the same for the whole warp
+        uint8_t* line0 = mine + sbuf * 4096;
+        if (lane == 0) tma_store_wait_read<1>();            // the store before the last one has left this buffer
+        __syncwarp();
+#pragma unroll
+        for (uint32_t v = 0; v < 8; ++v) *reinterpret_cast<uint4*>(line0 + lane * 128 + ((v ^ swz) << 4)) = line[v];
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {                // rows and columns past the edges are clipped by the tensor map
+          if constexpr (EPI == PG_F32_ADD) tma_reduce_add_2d(&tmap_c, line0, col0, row0);
+          else tma_store_2d(&tmap_c, line0, col0, row0);
+          tma_store_commit();
+        }
+        sbuf ^= 1;
+      }
+      if (++buf == 2) { buf = 0; acc_phase ^= 1u; }
+    }
+    if (lane == 0) tma_store_wait<0>();
+  }
+
+  // Teardown. After an aborted wait there may be bulk copies in flight; give them time to land before either CTA exits.
+  __syncwarp();
+  if (*abort_flag) __nanosleep(200000);
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();
+  if (warp == 1) {
+    tc_fence_after_sync();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * BN) : "memory");
+  }
+}
+
+template <int BN, int EPI, bool A_MN, bool B_MN>
+static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, int M, int N, int K, int num_sms, int pdl,
+                       int* status, cudaStream_t stream) {
+  using Cfg = PairCfg<BN>;
+  auto kern = gemm_pair_kernel<BN, EPI, A_MN, B_MN>;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) != cudaSuccess) return -20;
+    configured = true;
+  }
+  constexpr int TN = EPI == PG_SWIGLU ? BN / 2 : BN;
+  const int m_tiles = (M + 255) / 256, n_tiles = (N + TN - 1) / TN;
+  const long long tiles = static_cast<long long>(m_tiles) * n_tiles;
+  const int pairs = tiles < num_sms / 2 ? static_cast<int>(tiles) : num_sms / 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * pairs);
+  cfg.blockDim = dim3(PG_THREADS);
+  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, M, N, K, 8, status) == cudaSuccess ? 0 : -21;
+}
+
+template <int BN, int EPI>
+static int pair_major(int transA, int transB, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, int M, int N, int K,
+                      int num_sms, int pdl, int* status, cudaStream_t stream) {
+  if (!transA && !transB) return launch_pair<BN, EPI, false, false>(ta, tb, tc, M, N, K, num_sms, pdl, status, stream);
+  if (transA && !transB) return launch_pair<BN, EPI, true, false>(ta, tb, tc, M, N, K, num_sms, pdl, status, stream);
+  if (!transA) return launch_pair<BN, EPI, false, true>(ta, tb, tc, M, N, K, num_sms, pdl, status, stream);
+  return launch_pair<BN, EPI, true, true>(ta, tb, tc, M, N, K, num_sms, pdl, status, stream);
+}
+
+// Tensor map of the output for stores of 32-row, 128-byte-wide boxes.
+static int make_tmap_out(CUtensorMap* out, void* C, int M, int N, int ldc, bool f32) {
+  if (!f32) return make_tmap_bf16_2d(out, C, N, M, ldc, 64, 32);
+  return make_tmap_f32_2d(out, C, N, M, ldc, 32, 32);
+}
+
+// Arguments are those of rpeg_gemm_bf16, checked there.
+int gemm_pair(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int transA, int transB, int out_fp32,
+              int accumulate, int bn, int num_sms, int pdl, int* status, cudaStream_t stream) {
+  CUtensorMap ta, tb, tc;
+  int rc = transA ? make_tmap_bf16_2d(&ta, A, M, K, lda, 64, PG_BK) : make_tmap_bf16_2d(&ta, A, K, M, lda, PG_BK, PG_BM);
+  if (rc) return rc;
+  rc = transB ? make_tmap_bf16_2d(&tb, B, N, K, ldb, 64, PG_BK) : make_tmap_bf16_2d(&tb, B, K, N, ldb, PG_BK, bn / 2);
+  if (rc) return rc - 100;
+  rc = make_tmap_out(&tc, C, M, N, ldc, out_fp32 != 0);
+  if (rc) return rc - 200;
+#define RPEG_PAIR(BN_)                                                                                                             \
+  (!out_fp32 ? pair_major<BN_, PG_BF16>(transA, transB, ta, tb, tc, M, N, K, num_sms, pdl, status, stream)                         \
+   : accumulate ? pair_major<BN_, PG_F32_ADD>(transA, transB, ta, tb, tc, M, N, K, num_sms, pdl, status, stream)                   \
+                : pair_major<BN_, PG_F32>(transA, transB, ta, tb, tc, M, N, K, num_sms, pdl, status, stream))
+  return bn == 256 ? RPEG_PAIR(256) : RPEG_PAIR(128);
+#undef RPEG_PAIR
+}
+
+int gemm_pair_swiglu(const void* A, const void* W, void* C, int M, int f, int K, int lda, int ldw, int ldc, int num_sms, int* status,
+                     cudaStream_t stream) {
+  CUtensorMap ta, tb, tc;
+  int rc = make_tmap_bf16_2d(&ta, A, K, M, lda, PG_BK, PG_BM);
+  if (rc) return rc;
+  rc = make_tmap_bf16_2d(&tb, W, K, 2ull * f, ldw, PG_BK, 128);
+  if (rc) return rc - 100;
+  rc = make_tmap_out(&tc, C, M, f, ldc, false);
+  if (rc) return rc - 200;
+  return launch_pair<256, PG_SWIGLU, false, false>(ta, tb, tc, M, f, K, num_sms, 0, status, stream);
+}
+
+}  // namespace rpeg

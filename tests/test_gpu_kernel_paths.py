@@ -100,3 +100,31 @@ def test_flash_attn_bwd_tiles(cuda_device, lens, H, Hkv):
     for lo, hi in ((0, kc), (kc, vc), (vc, width)):
         want = x.grad[:, lo:hi]
         assert float((got[:, lo:hi].double() - want).norm()) < 1e-2 * float(want.norm()) + 2e-3
+
+
+# bf16 operands are exact in fp32, so an fp32 result is off by sums alone; a bf16 result by half a unit in its last place (2^-9) at most
+@pytest.mark.parametrize("m,n,k", [(1, 8, 1024), (129, 136, 1032), (257, 264, 1096), (300, 4096, 1024), (1000, 5000, 520), (2304, 8200, 72), (5000, 1288, 64)])
+@pytest.mark.parametrize("trans_a,trans_b", [(False, False), (True, False), (False, True), (True, True)])
+def test_gemm_pair_tiles(cuda_device, m, n, k, trans_a, trans_b):
+    if trans_a:
+        m = (m + 7) // 8 * 8
+    g = torch.Generator(device=cuda_device).manual_seed(m + n)
+    a = torch.randn((k, m) if trans_a else (m, k), generator=g, device=cuda_device).bfloat16()
+    b = torch.randn((k, n) if trans_b else (n, k), generator=g, device=cuda_device).bfloat16()
+    want = (a.T if trans_a else a).double() @ (b if trans_b else b.T).double()
+    wide = torch.full((m, n + 16), 7.0, dtype=torch.bfloat16, device=cuda_device)       # columns beside the output stay as they are
+    K.gemm(a, b, trans_a=trans_a, trans_b=trans_b, out=wide[:, 8:8 + n])
+    assert _rel(wide[:, 8:8 + n], want) < 2 ** -9 and bool((wide[:, :8] == 7).all()) and bool((wide[:, 8 + n:] == 7).all())
+    acc = torch.randn(m, n, generator=g, device=cuda_device)
+    start = acc.double()
+    K.gemm(a, b, trans_a=trans_a, trans_b=trans_b, out=acc, accumulate=True)
+    assert _rel(acc, start + want) < F32
+    assert _rel(K.gemm(a, b, trans_a=trans_a, trans_b=trans_b, out_dtype=torch.float32), want) < F32
+
+
+@pytest.mark.parametrize("m,f,k", [(128, 256, 72), (129, 128, 64), (700, 1408, 520)])
+def test_gemm_swiglu_pair_tiles(cuda_device, m, f, k):
+    g = torch.Generator(device=cuda_device).manual_seed(m)
+    x, w = (torch.randn(r, k, generator=g, device=cuda_device).bfloat16() for r in (m, 2 * f))
+    gate, up = (x.double() @ w.double().T).chunk(2, 1)
+    assert _rel(K.gemm_swiglu(x, w), torch.nn.functional.silu(gate) * up) < 2 ** -8
