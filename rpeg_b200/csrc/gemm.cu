@@ -379,15 +379,17 @@ int make_tmap_bf16_2d(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_
   return r == CUDA_SUCCESS ? 0 : -11;
 }
 
-// 2-D fp32 tensor map of an output, 128-byte swizzle: boxes of `box_inner` (32: one swizzle row) columns.
-int make_tmap_f32_2d(CUtensorMap* out, void* ptr, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner, uint32_t box_outer) {
+// fp32 tensor map of an output, 128-byte swizzle: d0 contiguous elements, d1 rows of `ld1` elements and, if rank is 3, d2 slabs of `ld2`; boxes
+// of b0 (32: one swizzle row) x b1 (x 1) elements.
+int make_tmap_f32_3d(CUtensorMap* out, void* ptr, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t ld1, uint64_t ld2, uint32_t b0, uint32_t b1,
+                     int rank) {
   EncodeTiledFn fn = get_encode_fn();
   if (fn == nullptr) return -10;
-  cuuint64_t dims[2] = {inner, outer};
-  cuuint64_t strides[1] = {ld * 4};
-  cuuint32_t box[2] = {box_inner, box_outer};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  cuuint64_t dims[3] = {d0, d1, d2};
+  cuuint64_t strides[2] = {ld1 * 4, ld2 * 4};
+  cuuint32_t box[3] = {b0, b1, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, static_cast<cuuint32_t>(rank), ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -11;
 }
@@ -457,8 +459,12 @@ static int dispatch_major(int transA, int transB, const CUtensorMap& ta, const C
 static int g_num_sms = 0;
 
 // gemm_pair.cu
+struct PairPlan {
+  int bn, splits, kb_per;
+};
 int gemm_pair(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int transA, int transB, int out_fp32,
-              int accumulate, int bn, int num_sms, int pdl, int* status, cudaStream_t stream);
+              int accumulate, PairPlan plan, int num_sms, int pdl, int* status, cudaStream_t stream);
+PairPlan pair_plan(int M, int N, int K, int transB, bool f32, long long slab_elems, int num_sms);
 int gemm_pair_swiglu(const void* A, const void* W, void* C, int M, int f, int K, int lda, int ldw, int ldc, int num_sms, int* status,
                      cudaStream_t stream);
 
@@ -524,19 +530,21 @@ static int gemm_impl(const void* A, const void* B, void* C, int M, int N, int K,
   // bit 0x1000 of the tile-width hint: the caller chains this GEMM into a decode step (see `pdl` below)
   const bool chain = (bn_hint & 0x1000) != 0;
   bn_hint &= 0xfff;
-  // Two CTAs per tile (gemm_pair.cu) for everything that does not run split-K, unless the product is small: short K loops over few
-  // tiles do not repay the pair's set-up (256 x 256 x 256: 8 us here, 10 us there; 1024 x 512 columns, 700 rows: 10 and 12 us), long ones
-  // do at any M (16 x 12288 x 4096: 47 and 33 us; 637 x 4096 x 11008: 115 and 66 us; 8192 x 22016 x 4096: 1233 and 1003 us). Added
-  // gradients always go there: this kernel reads and writes them a row per thread (4096 x 4096, 637 tokens: 132 and 48 us).
-  if (bn_hint == 0 && gate.flags == nullptr && (workspace == nullptr || out_fp32 || accumulate || M > 2 * BM)) {
-    const int pairs = g_num_sms / 2, m256 = (M + 255) / 256;
-    const int wide = m256 * ((N + 255) / 256);
-    if ((out_fp32 && accumulate) || K >= 1024 || wide >= pairs / 2) {
-      // the narrow tile re-reads A twice as often; it pays while all its tiles are resident at once (320 x 4096 x 4096: 25 us against
-      // 31 us; 637 rows, more tiles than pairs: 39 us against 31 us)
-      const int narrow = m256 * ((N + 127) / 128);
-      return gemm_pair(A, B, C, M, N, K, lda, ldb, ldc, transA, transB, out_fp32, accumulate, narrow <= pairs ? 128 : 256, g_num_sms,
-                       chain ? pdl_enabled() : 0, status, stream);
+  // Two CTAs per tile (gemm_pair.cu), unless the product is small: short K loops over few tiles do not repay the pair's set-up
+  // (256 x 256 x 256: 8 us here, 10 us there; 1024 x 512 columns, 700 rows: 10 and 12 us), long ones do at any M (16 x 12288 x 4096: 47
+  // and 33 us; 637 x 4096 x 11008: 115 and 66 us; 8192 x 22016 x 4096: 1233 and 1003 us). Added gradients always go there: this kernel
+  // reads and writes them a row per thread (4096 x 4096, 637 tokens: 132 and 48 us). With a workspace (decode) up to 128 rows stay
+  // here, where split K keeps every SM on the weights; beyond, a second row tile would stream them twice (256 x 22016 x 4096: 77 and 50 us).
+  const bool split_k = workspace != nullptr && !out_fp32 && !accumulate && M <= 2 * BM;
+  if (bn_hint == 0 && gate.flags == nullptr && (!split_k || M > BM)) {
+    const int wide = ((M + 255) / 256) * ((N + 255) / 256);
+    if ((out_fp32 && accumulate) || K >= 1024 || wide >= g_num_sms / 4) {
+      const PairPlan plan = pair_plan(M, N, K, transB, out_fp32 != 0, split_k ? workspace_elems : 0, g_num_sms);
+      const int pdl = (split_k || chain) ? pdl_enabled() : 0;
+      if (plan.splits == 1)
+        return gemm_pair(A, B, C, M, N, K, lda, ldb, ldc, transA, transB, out_fp32, accumulate, plan, g_num_sms, pdl, status, stream);
+      const int rc = gemm_pair(A, B, workspace, M, N, K, lda, ldb, N, transA, transB, 1, 0, plan, g_num_sms, pdl, status, stream);
+      return rc != 0 ? rc : rpeg_splitk_reduce(workspace, C, M, N, ldc, plan.splits, stream_v);
     }
   }
   int bn = bn_hint;
@@ -673,6 +681,11 @@ extern "C" int rpeg_gemm_bf16_partials(const void* A, const void* B, int M, int 
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+  if (M > BM) {                                            // two row tiles: pairs read the weights once (see gemm_impl)
+    const PairPlan plan = pair_plan(M, N, K, 0, true, workspace_elems, g_num_sms);
+    *k_splits_out = plan.splits;
+    return gemm_pair(A, B, workspace, M, N, K, lda, ldb, N, 0, 0, 1, 0, plan, g_num_sms, pdl_enabled(), status, stream);
   }
   const int bn = N >= 256 ? 256 : (N >= 128 ? 128 : (N >= 64 ? 64 : 32));
   const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);

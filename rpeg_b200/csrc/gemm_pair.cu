@@ -17,22 +17,28 @@ namespace rpeg {
 
 // gemm.cu
 int make_tmap_bf16_2d(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner, uint32_t box_outer);
-int make_tmap_f32_2d(CUtensorMap* out, void* ptr, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner, uint32_t box_outer);
+int make_tmap_f32_3d(CUtensorMap* out, void* ptr, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t ld1, uint64_t ld2, uint32_t b0, uint32_t b1,
+                     int rank);
 
 constexpr int PG_BM = 128;              // rows per CTA; the pair's tile has 256
 constexpr int PG_BK = 64;
 constexpr int PG_THREADS = 192;
 constexpr int PG_STAGING = 4 * 2 * 4096;
 
-template <int BN>
-struct PairCfg {
-  static constexpr int A_BYTES = PG_BM * PG_BK * 2;
-  static constexpr int B_BYTES = (BN / 2) * PG_BK * 2;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = BN == 256 ? 6 : 8;
-  static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + PG_STAGING + 512;
+constexpr int PG_A_BYTES = PG_BM * PG_BK * 2;
+constexpr int PG_STAGE_BYTES = PG_A_BYTES + 128 * PG_BK * 2;     // up to 128 columns of B per CTA
+constexpr int PG_STAGES = 6;
+constexpr int PG_SMEM = 1024 + PG_STAGES * PG_STAGE_BYTES + PG_STAGING + 512;
+static_assert(PG_SMEM <= 227 * 1024, "shared memory");
+
+struct PairPlan {                       // of pair_plan() below
+  int bn, splits, kb_per;
 };
-static_assert(PairCfg<256>::SMEM_BYTES <= 227 * 1024 && PairCfg<128>::SMEM_BYTES <= 227 * 1024, "shared memory");
+// Work of a launch: tiles of 256 rows x `bn` accumulator columns, each cut into `splits` pieces of `kb_per` K blocks (splits > 1: every piece
+// stores its own sums, `PG_F32` only).
+struct PairWork {
+  int M, N, K, bn, splits, kb_per;
+};
 
 enum { PG_BF16 = 0, PG_F32 = 1, PG_F32_ADD = 2, PG_SWIGLU = 3 };
 
@@ -65,6 +71,11 @@ __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* m, const vo
                "r"(smem_u32(smem_src)), "r"(x), "r"(y)
                : "memory");
 }
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* m, const void* smem_src, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(reinterpret_cast<uint64_t>(m)),
+               "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
+               : "memory");
+}
 __device__ __forceinline__ void umma_bf16_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
@@ -81,16 +92,16 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
                : "memory");
 }
 
-template <int BN, int EPI, bool A_MN, bool B_MN>
+template <int EPI, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(PG_THREADS, 1) __cluster_dims__(2, 1, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                 const __grid_constant__ CUtensorMap tmap_c, int M, int N, int K, int group_m, int* status) {
-  using Cfg = PairCfg<BN>;
-  constexpr int STAGES = Cfg::STAGES;
-  constexpr int TN = EPI == PG_SWIGLU ? BN / 2 : BN;       // output columns per tile
+                 const __grid_constant__ CUtensorMap tmap_c, const PairWork pw, int* status) {
+  constexpr int STAGES = PG_STAGES;
+  const int M = pw.M, N = pw.N, BN = pw.bn;
+  const int TN = EPI == PG_SWIGLU ? BN / 2 : BN;           // output columns per tile
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* staging = smem + STAGES * Cfg::STAGE_BYTES;
+  uint8_t* staging = smem + STAGES * PG_STAGE_BYTES;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(staging + PG_STAGING);     // even CTA: both CTAs' bytes of a stage
   uint64_t* empty_bar = full_bar + STAGES;                                    // each CTA: the pair's MMAs have read the stage
   uint64_t* tfull_bar = empty_bar + STAGES;                                   // each CTA: accumulator complete
@@ -103,8 +114,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   const uint32_t rank = cluster_rank();
   const int m_tiles = (M + 2 * PG_BM - 1) / (2 * PG_BM);
   const int n_tiles = (N + TN - 1) / TN;
-  const int num_tiles = m_tiles * n_tiles;
-  const int num_kb = (K + PG_BK - 1) / PG_BK;
+  const int num_items = m_tiles * n_tiles * pw.splits;
+  const int num_kb = (pw.K + PG_BK - 1) / PG_BK;
+  const uint32_t stage_tx = 2u * static_cast<uint32_t>(PG_A_BYTES + (B_MN ? (BN / 2 + 63) / 64 * 64 : BN / 2) * PG_BK * 2);   // both CTAs
   const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
@@ -123,7 +135,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     tma_prefetch_desc(&tmap_c);
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2 * BN) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before_sync();
@@ -134,32 +146,33 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   griddep_launch();
   griddep_wait();                       // returns at once unless this grid was launched as a programmatic dependent
 
-  // Tile order: groups of `group_m` row tiles sweep N together, so that their rows of A stay in L2.
-  auto tile_coords = [&](int t, int& tm, int& tn) {
-    const int per_group = group_m * n_tiles;
+  // Item order: groups of eight row tiles sweep N together, so that their rows of A stay in L2; the pieces of a tile follow each other.
+  struct Item { int tm, tn, split, kb0, kb1; };
+  auto item = [&](int w) -> Item {
+    constexpr int GROUP_M = 8;
+    const int t = w / pw.splits, split = w - t * pw.splits;
+    const int per_group = GROUP_M * n_tiles;
     const int g = t / per_group;
-    const int first_m = g * group_m;
-    const int gsize = min(m_tiles - first_m, group_m);
+    const int first_m = g * GROUP_M;
+    const int gsize = min(m_tiles - first_m, GROUP_M);
     const int r = t - g * per_group;
-    tm = first_m + (r % gsize);
-    tn = r / gsize;
+    return {first_m + (r % gsize), r / gsize, split, split * pw.kb_per, min(num_kb, (split + 1) * pw.kb_per)};
   };
 
   if (warp == 0) {
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
-      for (int w = first; w < num_tiles; w += step) {
-        int tm, tn;
-        tile_coords(w, tm, tn);
-        const int m0 = tm * 2 * PG_BM + static_cast<int>(rank) * PG_BM;
+      for (int w = first; w < num_items; w += step) {
+        const Item it = item(w);
+        const int m0 = it.tm * 2 * PG_BM + static_cast<int>(rank) * PG_BM;
         // swiglu: the even CTA holds the gate rows of the tile's columns, the odd one the up rows (N = f rows further on)
-        const int n0 = EPI == PG_SWIGLU ? tn * TN + static_cast<int>(rank) * N : tn * TN + static_cast<int>(rank) * (BN / 2);
-        for (int kb = 0; kb < num_kb; ++kb) {
+        const int n0 = EPI == PG_SWIGLU ? it.tn * TN + static_cast<int>(rank) * N : it.tn * TN + static_cast<int>(rank) * (BN / 2);
+        for (int kb = it.kb0; kb < it.kb1; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, status, 160)) goto producer_done;
-          uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
-          uint8_t* sb = sa + Cfg::A_BYTES;
-          if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * Cfg::STAGE_BYTES);
+          uint8_t* sa = smem + stage * PG_STAGE_BYTES;
+          uint8_t* sb = sa + PG_A_BYTES;
+          if (rank == 0) mbar_expect_tx(&full_bar[stage], stage_tx);
           const uint32_t bar = cluster_addr(&full_bar[stage], 0);
           if constexpr (!A_MN) {
             tma_load_2d_pair(sa, &tmap_a, bar, kb * PG_BK, m0);
@@ -170,8 +183,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           if constexpr (!B_MN) {
             tma_load_2d_pair(sb, &tmap_b, bar, kb * PG_BK, n0);
           } else {
-#pragma unroll
-            for (int c = 0; c < BN / 128; ++c) tma_load_2d_pair(sb + c * (64 * PG_BK * 2), &tmap_b, bar, n0 + c * 64, kb * PG_BK);
+            for (int c = 0; c * 64 < BN / 2; ++c) tma_load_2d_pair(sb + c * (64 * PG_BK * 2), &tmap_b, bar, n0 + c * 64, kb * PG_BK);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
@@ -180,30 +192,31 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else if (warp == 1) {
     if (rank == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(2 * PG_BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      const uint32_t idesc = make_idesc_bf16(2 * PG_BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
       const uint32_t s0 = smem_u32(smem);
       const uint64_t da0 = A_MN ? make_smem_desc_sw128(s0, 64 * PG_BK * 2, 1024) : make_smem_desc_sw128(s0, 16, 1024);
-      const uint64_t db0 = B_MN ? make_smem_desc_sw128(s0 + Cfg::A_BYTES, 64 * PG_BK * 2, 1024) : make_smem_desc_sw128(s0 + Cfg::A_BYTES, 16, 1024);
+      const uint64_t db0 = B_MN ? make_smem_desc_sw128(s0 + PG_A_BYTES, 64 * PG_BK * 2, 1024) : make_smem_desc_sw128(s0 + PG_A_BYTES, 16, 1024);
       int stage = 0, buf = 0;
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
-      for (int w = first; w < num_tiles && ok; w += step) {
+      for (int w = first; w < num_items && ok; w += step) {
+        const Item it = item(w);
         ok = __all_sync(0xffffffffu, mbar_wait(&tempty_bar[buf], acc_phase ^ 1u, abort_flag, status, 260));
         if (!ok) break;
         tc_fence_after_sync();
-        const uint32_t tacc = tmem_base + static_cast<uint32_t>(buf * BN);
-        for (int kb = 0; kb < num_kb; ++kb) {
+        const uint32_t tacc = tmem_base + static_cast<uint32_t>(buf * 256);
+        for (int kb = it.kb0; kb < it.kb1; ++kb) {
           ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, abort_flag, status, 261));
           if (!ok) break;
           tc_fence_after_sync();
-          const uint64_t da = smem_desc_at(da0, stage * Cfg::STAGE_BYTES), db = smem_desc_at(db0, stage * Cfg::STAGE_BYTES);
+          const uint64_t da = smem_desc_at(da0, stage * PG_STAGE_BYTES), db = smem_desc_at(db0, stage * PG_STAGE_BYTES);
           if (elect_one()) {
 #pragma unroll
             for (int k = 0; k < PG_BK / 16; ++k)
               umma_bf16_ss_pair(tacc, smem_desc_at(da, k * (A_MN ? 2048 : 32)), smem_desc_at(db, k * (B_MN ? 2048 : 32)), idesc,
-                                (kb != 0 || k != 0) ? 1u : 0u);
+                                (kb != it.kb0 || k != 0) ? 1u : 0u);
             umma_commit_pair(&empty_bar[stage]);
-            if (kb == num_kb - 1) umma_commit_pair(&tfull_bar[buf]);
+            if (kb == it.kb1 - 1) umma_commit_pair(&tfull_bar[buf]);
           }
           __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
@@ -219,13 +232,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     const uint32_t swz = static_cast<uint32_t>(lane & 7);
     int buf = 0, sbuf = 0;
     uint32_t acc_phase = 0;
-    for (int w = first; w < num_tiles; w += step) {
-      int tm, tn;
-      tile_coords(w, tm, tn);
-      const int row0 = tm * 2 * PG_BM + static_cast<int>(rank) * PG_BM + quad * 32, n0 = tn * TN;
+    for (int w = first; w < num_items; w += step) {
+      const Item it = item(w);
+      const int row0 = it.tm * 2 * PG_BM + static_cast<int>(rank) * PG_BM + quad * 32, n0 = it.tn * TN;
       if (!__all_sync(0xffffffffu, mbar_wait(&tfull_bar[buf], acc_phase, abort_flag, status, 360))) break;
       tc_fence_after_sync();
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(buf * BN);
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(buf * 256);
 #pragma unroll 1
       for (int c = 0; c < TN / CW; ++c) {
         uint4 line[8];
@@ -287,6 +299,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         __syncwarp();
         if (lane == 0) {                // rows and columns past the edges are clipped by the tensor map
           if constexpr (EPI == PG_F32_ADD) tma_reduce_add_2d(&tmap_c, line0, col0, row0);
+          else if constexpr (EPI == PG_F32) tma_store_3d(&tmap_c, line0, col0, row0, it.split);
           else tma_store_2d(&tmap_c, line0, col0, row0);
           tma_store_commit();
         }
@@ -305,68 +318,89 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   cluster_sync_all();
   if (warp == 1) {
     tc_fence_after_sync();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * BN) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
   }
 }
 
-template <int BN, int EPI, bool A_MN, bool B_MN>
-static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, int M, int N, int K, int num_sms, int pdl,
-                       int* status, cudaStream_t stream) {
-  using Cfg = PairCfg<BN>;
-  auto kern = gemm_pair_kernel<BN, EPI, A_MN, B_MN>;
+template <int EPI, bool A_MN, bool B_MN>
+static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const PairWork& pw, int num_sms, int pdl, int* status,
+                       cudaStream_t stream) {
+  auto kern = gemm_pair_kernel<EPI, A_MN, B_MN>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) != cudaSuccess) return -20;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PG_SMEM) != cudaSuccess) return -20;
     configured = true;
   }
-  constexpr int TN = EPI == PG_SWIGLU ? BN / 2 : BN;
-  const int m_tiles = (M + 255) / 256, n_tiles = (N + TN - 1) / TN;
-  const long long tiles = static_cast<long long>(m_tiles) * n_tiles;
-  const int pairs = tiles < num_sms / 2 ? static_cast<int>(tiles) : num_sms / 2;
+  const int tn = EPI == PG_SWIGLU ? pw.bn / 2 : pw.bn;
+  const long long items = static_cast<long long>((pw.M + 255) / 256) * ((pw.N + tn - 1) / tn) * pw.splits;
+  const int pairs = items < num_sms / 2 ? static_cast<int>(items) : num_sms / 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs);
   cfg.blockDim = dim3(PG_THREADS);
-  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+  cfg.dynamicSmemBytes = PG_SMEM;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, M, N, K, 8, status) == cudaSuccess ? 0 : -21;
+  return cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, pw, status) == cudaSuccess ? 0 : -21;
 }
 
-template <int BN, int EPI>
-static int pair_major(int transA, int transB, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, int M, int N, int K,
-                      int num_sms, int pdl, int* status, cudaStream_t stream) {
-  if (!transA && !transB) return launch_pair<BN, EPI, false, false>(ta, tb, tc, M, N, K, num_sms, pdl, status, stream);
-  if (transA && !transB) return launch_pair<BN, EPI, true, false>(ta, tb, tc, M, N, K, num_sms, pdl, status, stream);
-  if (!transA) return launch_pair<BN, EPI, false, true>(ta, tb, tc, M, N, K, num_sms, pdl, status, stream);
-  return launch_pair<BN, EPI, true, true>(ta, tb, tc, M, N, K, num_sms, pdl, status, stream);
+template <int EPI>
+static int pair_major(int transA, int transB, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const PairWork& pw, int num_sms,
+                      int pdl, int* status, cudaStream_t stream) {
+  if (!transA && !transB) return launch_pair<EPI, false, false>(ta, tb, tc, pw, num_sms, pdl, status, stream);
+  if (transA && !transB) return launch_pair<EPI, true, false>(ta, tb, tc, pw, num_sms, pdl, status, stream);
+  if (!transA) return launch_pair<EPI, false, true>(ta, tb, tc, pw, num_sms, pdl, status, stream);
+  return launch_pair<EPI, true, true>(ta, tb, tc, pw, num_sms, pdl, status, stream);
 }
 
-// Tensor map of the output for stores of 32-row, 128-byte-wide boxes.
-static int make_tmap_out(CUtensorMap* out, void* C, int M, int N, int ldc, bool f32) {
-  if (!f32) return make_tmap_bf16_2d(out, C, N, M, ldc, 64, 32);
-  return make_tmap_f32_2d(out, C, N, M, ldc, 32, 32);
+// Accumulator columns of a tile (`bn`) and K pieces (`splits` of `kb_per` 64-deep blocks; slab_elems: fp32 words for their sums, 0: one piece).
+// What a K block of a tile costs, in that of 256 columns, measured over whole waves of tiles (8192 x 4096 x 4096: 26.2 us a wave of 256,
+// 20.0 of 192, 18.9 of 128, 18.0 of 64): narrow tiles read A as often for less work, so they are for sizes whose wide tiles leave the
+// last wave nearly empty (700 x 4096 x 4096: 33 us at 256, 27 us at 192; 5900 rows: 135 and 139 us). An item starts and ends in about four
+// blocks' time, and every slab is written and read once more (256 x 12288 x 4096: 1 us each).
+PairPlan pair_plan(int M, int N, int K, int transB, bool f32, long long slab_elems, int num_sms) {
+  static const struct { int bn; double cost; bool any_b, any_out; } widths[] = {      // B stored [K, N] comes in boxes of 64 columns a CTA;
+      {256, 1.0, true, true}, {224, 0.88, false, false}, {192, 0.77, false, true},    // a bf16 line of the output has 64 columns
+      {160, 0.75, false, false}, {128, 0.72, true, true}, {64, 0.69, false, true}};
+  const int pairs = num_sms / 2, num_kb = (K + PG_BK - 1) / PG_BK;
+  const long long m_tiles = (M + 255) / 256, slab = static_cast<long long>(M) * N;
+  const double slab_cost = static_cast<double>(slab) * 8.0 / 2.4e6 * 0.25;
+  PairPlan best{256, 1, num_kb};
+  double least = 1e300;
+  for (const auto& w : widths) {
+    if ((transB && !w.any_b) || (!f32 && slab_elems == 0 && !w.any_out)) continue;
+    const long long tiles = m_tiles * ((N + w.bn - 1) / w.bn);
+    for (int sp = 1; sp <= 16 && (sp == 1 || (num_kb / sp >= 4 && sp * slab <= slab_elems)); ++sp) {
+      const int kb_per = (num_kb + sp - 1) / sp;
+      if ((num_kb + kb_per - 1) / kb_per != sp) continue;
+      if (sp == 1 && !f32 && !w.any_out) continue;
+      const double cost = static_cast<double>((tiles * sp + pairs - 1) / pairs) * (kb_per * w.cost + 4.0) + (sp > 1 || slab_elems > 0 ? sp * slab_cost : 0.0);
+      if (cost < least * 0.999) { least = cost; best = PairPlan{w.bn, sp, kb_per}; }
+    }
+  }
+  return best;
 }
 
-// Arguments are those of rpeg_gemm_bf16, checked there.
+// Arguments are those of rpeg_gemm_bf16, checked there. splits > 1: C is fp32 [splits][M][ldc], every piece's sums in a slab of its own.
 int gemm_pair(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int transA, int transB, int out_fp32,
-              int accumulate, int bn, int num_sms, int pdl, int* status, cudaStream_t stream) {
+              int accumulate, PairPlan plan, int num_sms, int pdl, int* status, cudaStream_t stream) {
+  const int bn = plan.bn, splits = plan.splits;
   CUtensorMap ta, tb, tc;
   int rc = transA ? make_tmap_bf16_2d(&ta, A, M, K, lda, 64, PG_BK) : make_tmap_bf16_2d(&ta, A, K, M, lda, PG_BK, PG_BM);
   if (rc) return rc;
   rc = transB ? make_tmap_bf16_2d(&tb, B, N, K, ldb, 64, PG_BK) : make_tmap_bf16_2d(&tb, B, K, N, ldb, PG_BK, bn / 2);
   if (rc) return rc - 100;
-  rc = make_tmap_out(&tc, C, M, N, ldc, out_fp32 != 0);
+  // stores of 32 rows, 128 bytes wide
+  rc = out_fp32 ? make_tmap_f32_3d(&tc, C, N, M, splits, ldc, static_cast<uint64_t>(M) * ldc, 32, 32, accumulate ? 2 : 3)
+                : make_tmap_bf16_2d(&tc, C, N, M, ldc, 64, 32);
   if (rc) return rc - 200;
-#define RPEG_PAIR(BN_)                                                                                                             \
-  (!out_fp32 ? pair_major<BN_, PG_BF16>(transA, transB, ta, tb, tc, M, N, K, num_sms, pdl, status, stream)                         \
-   : accumulate ? pair_major<BN_, PG_F32_ADD>(transA, transB, ta, tb, tc, M, N, K, num_sms, pdl, status, stream)                   \
-                : pair_major<BN_, PG_F32>(transA, transB, ta, tb, tc, M, N, K, num_sms, pdl, status, stream))
-  return bn == 256 ? RPEG_PAIR(256) : RPEG_PAIR(128);
-#undef RPEG_PAIR
+  const PairWork pw{M, N, K, bn, splits, plan.kb_per};
+  if (!out_fp32) return pair_major<PG_BF16>(transA, transB, ta, tb, tc, pw, num_sms, pdl, status, stream);
+  if (accumulate) return pair_major<PG_F32_ADD>(transA, transB, ta, tb, tc, pw, num_sms, pdl, status, stream);
+  return pair_major<PG_F32>(transA, transB, ta, tb, tc, pw, num_sms, pdl, status, stream);
 }
 
 int gemm_pair_swiglu(const void* A, const void* W, void* C, int M, int f, int K, int lda, int ldw, int ldc, int num_sms, int* status,
@@ -376,9 +410,9 @@ int gemm_pair_swiglu(const void* A, const void* W, void* C, int M, int f, int K,
   if (rc) return rc;
   rc = make_tmap_bf16_2d(&tb, W, K, 2ull * f, ldw, PG_BK, 128);
   if (rc) return rc - 100;
-  rc = make_tmap_out(&tc, C, M, f, ldc, false);
+  rc = make_tmap_bf16_2d(&tc, C, f, M, ldc, 64, 32);
   if (rc) return rc - 200;
-  return launch_pair<256, PG_SWIGLU, false, false>(ta, tb, tc, M, f, K, num_sms, 0, status, stream);
+  return launch_pair<PG_SWIGLU, false, false>(ta, tb, tc, PairWork{M, f, K, 256, 1, (K + PG_BK - 1) / PG_BK}, num_sms, 0, status, stream);
 }
 
 }  // namespace rpeg

@@ -128,3 +128,15 @@ def test_gemm_swiglu_pair_tiles(cuda_device, m, f, k):
     x, w = (torch.randn(r, k, generator=g, device=cuda_device).bfloat16() for r in (m, 2 * f))
     gate, up = (x.double() @ w.double().T).chunk(2, 1)
     assert _rel(K.gemm_swiglu(x, w), torch.nn.functional.silu(gate) * up) < 2 ** -8
+
+
+@pytest.mark.parametrize("m", [129, 200, 256])
+@pytest.mark.parametrize("n,k", [(136, 264), (1288, 4096), (12288, 1032)])
+def test_gemm_partials_of_two_row_tiles(cuda_device, m, n, k):
+    g = torch.Generator(device=cuda_device).manual_seed(m)
+    a, b = (torch.randn(r, k, generator=g, device=cuda_device).bfloat16() for r in (m, n))
+    want = a.double() @ b.double().T
+    ws = torch.full((32 * 1024 * 1024,), float("nan"), device=cuda_device)
+    p = K.gemm_partials(a, b, ws)
+    assert _rel(p.buf[: p.splits * m * n].view(p.splits, m, n).sum(0), want) < F32
+    assert _rel(K.gemm(a, b, workspace=ws), want) < 2 ** -9
