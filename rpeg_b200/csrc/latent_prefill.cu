@@ -13,7 +13,7 @@
 //   * A query / key row is KA atoms of 64 columns (unrotated ones, then rotated ones), a value row VA atoms. The TMA unit pads narrower ones.
 //   * Key and value atoms (128 rows x 128 bytes) share one ring, freed atom by atom: with 192-wide keys and 128-wide values two key
 //     tiles and a value tile are in flight.
-//   * A value atom is a matrix product of its own (64 output columns), so atoms need not be neighbours in the ring.
+//   * Value atoms that are neighbours in the ring are one matrix product of 128 output columns, others one of 64 each.
 #include "prefill_softmax.cuh"
 #include "rpeg_kernels.h"
 
@@ -87,7 +87,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int s = 0; s < SLOTS; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -133,74 +133,92 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk = make_idesc_bf16(128, 128, 0, 0);
-      constexpr uint32_t idesc_pv = make_idesc_bf16(128, 64, 0, 1);
-      auto active = [&](int u, int j) -> bool { return u == 0 ? j >= u0.jb && j < u0.je : has1 && j >= u1.jb && j < u1.je; };
-      auto wait_atoms = [&](int i0, int n) -> bool {
-        for (int i = i0; i < i0 + n; ++i)
-          if (!mbar_wait(&full[slot_of(i)], parity_of(i), abort_flag, a.status, 1210)) return false;
-        tc_fence_after_sync();
-        return true;
-      };
-      // Q K^T of unit u over tile j; the tile's key atoms are free again once the last unit has used them
-      auto issue_qk = [&](int u, int j) {
-        if (active(u, j)) {
-          uint32_t acc = 0u;
+    // All lanes run the loop, one issues: in a branch of one lane the operands' way into uniform registers bounds the issue rate.
+    const bool leader = elect_one();
+    constexpr uint32_t idesc_qk = make_idesc_bf16(128, 128, 0, 0);
+    constexpr uint32_t idesc_pv = make_idesc_bf16(128, 64, 0, 1), idesc_pv2 = make_idesc_bf16(128, 128, 0, 1);
+    const uint64_t qd = make_smem_desc_sw128(smem_u32(q_sm), 16, 1024), kd = make_smem_desc_sw128(smem_u32(ring), 16, 1024);
+    const uint64_t vd = make_smem_desc_sw128(smem_u32(ring), LP_ATOM, 1024);
+    auto wait = [&](uint64_t* bar, uint32_t parity, int where) -> bool {
+      return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, a.status, where));
+    };
+    auto active = [&](int u, int j) -> bool { return u == 0 ? j >= u0.jb && j < u0.je : has1 && j >= u1.jb && j < u1.je; };
+    auto wait_atoms = [&](int i0, int n) -> bool {
+      for (int i = i0; i < i0 + n; ++i)
+        if (!wait(&full[slot_of(i)], parity_of(i), 1210)) return false;
+      tc_fence_after_sync();
+      return true;
+    };
+    // Q K^T of unit u over tile j; the tile's key atoms are free again once the last unit has used them
+    auto issue_qk = [&](int u, int j) {
+      if (active(u, j)) {
 #pragma unroll
-          for (int c = 0; c < KA; ++c) {
-            const uint32_t qa = smem_u32(q_sm + (u * KA + c) * LP_ATOM), ka = smem_u32(ring + slot_of(j * TA + c) * LP_ATOM);
-            const int steps = c == a.nope_atoms - 1 ? a.nope_steps : (c == KA - 1 ? a.rot_steps : 4);
+        for (int c = 0; c < KA; ++c) {
+          const uint64_t qa = smem_desc_at(qd, (u * KA + c) * LP_ATOM), ka = smem_desc_at(kd, slot_of(j * TA + c) * LP_ATOM);
+          const int steps = c == a.nope_atoms - 1 ? a.nope_steps : (c == KA - 1 ? a.rot_steps : 4);
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-              if (k < steps) {
-                umma_bf16_ss(tmem_base + u * 128, make_smem_desc_sw128(qa + k * 32, 16, 1024), make_smem_desc_sw128(ka + k * 32, 16, 1024), idesc_qk, acc);
-                acc = 1u;
-              }
-          }
-          umma_commit(&s_full[u]);
+          for (int k = 0; k < 4; ++k)
+            if (leader && k < steps) umma_bf16_ss(tmem_base + u * 128, smem_desc_at(qa, k * 32), smem_desc_at(ka, k * 32), idesc_qk, (c | k) != 0 ? 1u : 0u);
         }
-        if (u == 1)
+        if (leader) umma_commit(&s_full[u]);
+      }
+      if (u == 1)
 #pragma unroll
-          for (int c = 0; c < KA; ++c) umma_commit(&empty[slot_of(j * TA + c)]);
-      };
-      bool ok = mbar_wait(q_full, 0, abort_flag, a.status, 1211) && wait_atoms(0, KA);
-      if (ok) {
-        issue_qk(0, 0);
-        issue_qk(1, 0);
-        for (int j = 0; j < n_tiles && ok; ++j) {
-          if (!wait_atoms(j * TA + KA, VA)) break;
-          if (j + 1 < n_tiles && !wait_atoms((j + 1) * TA, KA)) break;
+        for (int c = 0; c < KA; ++c)
+          if (leader) umma_commit(&empty[slot_of(j * TA + c)]);
+    };
+    bool ok = wait(q_full, 0, 1211) && wait_atoms(0, KA);
+    if (ok) {
+      issue_qk(0, 0);
+      issue_qk(1, 0);
+      for (int j = 0; j < n_tiles && ok; ++j) {
+        if (!wait_atoms(j * TA + KA, VA)) break;
+        if (j + 1 < n_tiles && !wait_atoms((j + 1) * TA, KA)) break;
+        const int v0 = slot_of(j * TA + KA), v1 = slot_of(j * TA + KA + VA - 1);
+        const uint64_t vd0 = smem_desc_at(vd, v0 * LP_ATOM);
+        const bool joined = VA == 2 && v1 == v0 + 1;         // neighbouring atoms are one product of 128 columns
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            if (active(u, j)) {
-              const int n = j - (u ? u1.jb : u0.jb);         // tiles of this unit before this one
-              const uint32_t tp = tmem_base + u * 128, to = tmem_base + 256 + u * 128;
+        for (int u = 0; u < 2; ++u) {
+          if (active(u, j)) {
+            const int n = j - (u ? u1.jb : u0.jb);           // tiles of this unit before this one
+            const uint32_t tp = tmem_base + u * 128, to = tmem_base + 256 + u * 128;
 #pragma unroll
-              for (int half = 0; half < 2 && ok; ++half) {   // the first keys are multiplied while the last ones are exponentiated
-                ok = mbar_wait(half ? &p_full[u] : &p_half[u], static_cast<uint32_t>(n) & 1u, abort_flag, a.status, 1213 + half);
-                if (!ok) break;
-                tc_fence_after_sync();
+            for (int half = 0; half < 2 && ok; ++half) {     // the first keys are multiplied while the last ones are exponentiated
+              ok = wait(half ? &p_full[u] : &p_half[u], static_cast<uint32_t>(n) & 1u, 1213 + half);
+              if (!ok) break;
+              tc_fence_after_sync();
+              // 16 keys a step: 8 packed columns of P, 16 rows (2 KiB) of the value atoms
+              if (joined) {
+#pragma unroll
+                for (int part = 0; part < 2; ++part)
+#pragma unroll
+                  for (int k = half * 4; k < half * 4 + 4; ++k)
+                    if (leader)
+                      umma_bf16_ts(to, tp + (k >> 1) * 32 + part * 16 + (k & 1) * 8, smem_desc_at(vd0, k * 2048), idesc_pv2,
+                                   (n | half | part | (k & 3)) != 0 ? 1u : 0u);
+              } else {
 #pragma unroll
                 for (int va = 0; va < VA; ++va) {
-                  const uint32_t v_addr = smem_u32(ring + slot_of(j * TA + KA + va) * LP_ATOM);
+                  const uint64_t vda = smem_desc_at(vd, (va ? v1 : v0) * LP_ATOM);
 #pragma unroll
                   for (int part = 0; part < 2; ++part)
 #pragma unroll
-                    for (int k = half * 4; k < half * 4 + 4; ++k)   // 16 keys: 8 packed columns of P, 16 rows (2 KiB) of the value atom
-                      umma_bf16_ts(to + va * 64, tp + (k >> 1) * 32 + part * 16 + (k & 1) * 8, make_smem_desc_sw128(v_addr + k * 2048, LP_ATOM, 1024),
-                                   idesc_pv, (n | half | part | (k & 3)) != 0 ? 1u : 0u);
+                    for (int k = half * 4; k < half * 4 + 4; ++k)
+                      if (leader)
+                        umma_bf16_ts(to + va * 64, tp + (k >> 1) * 32 + part * 16 + (k & 1) * 8, smem_desc_at(vda, k * 2048), idesc_pv,
+                                     (n | half | part | (k & 3)) != 0 ? 1u : 0u);
                 }
               }
-              if (!ok) break;
-              if (j + 1 == (u ? u1.je : u0.je)) umma_commit(&o_full[u]);
             }
-            if (u == 1)
-#pragma unroll
-              for (int va = 0; va < VA; ++va) umma_commit(&empty[slot_of(j * TA + KA + va)]);
-            tc_fence_after_sync();
-            if (j + 1 < n_tiles) issue_qk(u, j + 1);
+            if (!ok) break;
+            if (leader && j + 1 == (u ? u1.je : u0.je)) umma_commit(&o_full[u]);
           }
+          if (u == 1)
+#pragma unroll
+            for (int va = 0; va < VA; ++va)
+              if (leader) umma_commit(&empty[va ? v1 : v0]);
+          tc_fence_after_sync();
+          if (j + 1 < n_tiles) issue_qk(u, j + 1);
         }
       }
     }

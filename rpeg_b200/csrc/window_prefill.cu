@@ -98,7 +98,7 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int s = 0; s < WP_STAGES; ++s) {
@@ -152,61 +152,64 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk = make_idesc_bf16(128, 128, 0, 0);
-      constexpr uint32_t idesc_pv = make_idesc_bf16(128, HDT, 0, 1);
-      auto active = [&](int u, int j) -> bool { return u == 0 ? j >= u0.jb && j < u0.je : has1 && j >= u1.jb && j < u1.je; };
-      // Q K^T of unit u over tile j; the tile's K buffer is free again once the last unit has used it
-      auto issue_qk = [&](int u, int j) {
-        const int st = j % WP_STAGES;
-        if (active(u, j)) {
-          const uint32_t q_addr = smem_u32(q_sm + u * TILE), k_addr = smem_u32(k_sm + st * TILE);
+    // All lanes run the loop, one issues: in a branch of one lane the operands' way into uniform registers bounds the issue rate.
+    const bool leader = elect_one();
+    constexpr uint32_t idesc_qk = make_idesc_bf16(128, 128, 0, 0);
+    constexpr uint32_t idesc_pv = make_idesc_bf16(128, HDT, 0, 1);
+    const uint64_t qd = make_smem_desc_sw128(smem_u32(q_sm), 16, 1024), kd = make_smem_desc_sw128(smem_u32(k_sm), 16, 1024);
+    const uint64_t vd = make_smem_desc_sw128(smem_u32(v_sm), 16384, 1024);
+    auto wait = [&](uint64_t* bar, uint32_t parity, int where) -> bool {
+      return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, a.status, where));
+    };
+    auto active = [&](int u, int j) -> bool { return u == 0 ? j >= u0.jb && j < u0.je : has1 && j >= u1.jb && j < u1.je; };
+    // Q K^T of unit u over tile j; the tile's K buffer is free again once the last unit has used it
+    auto issue_qk = [&](int u, int j) {
+      const int st = j % WP_STAGES;
+      if (active(u, j)) {
+        const uint64_t qa = smem_desc_at(qd, u * TILE), ka = smem_desc_at(kd, st * TILE);
 #pragma unroll
-          for (int k = 0; k < HDT / 16; ++k) {
-            const uint32_t off = static_cast<uint32_t>((k >> 2) * 16384 + (k & 3) * 32);
-            umma_bf16_ss(tmem_base + u * 128, make_smem_desc_sw128(q_addr + off, 16, 1024), make_smem_desc_sw128(k_addr + off, 16, 1024),
-                         idesc_qk, k != 0 ? 1u : 0u);
-          }
-          umma_commit(&s_full[u]);
+        for (int k = 0; k < HDT / 16; ++k) {
+          const uint32_t off = static_cast<uint32_t>((k >> 2) * 16384 + (k & 3) * 32);
+          if (leader) umma_bf16_ss(tmem_base + u * 128, smem_desc_at(qa, off), smem_desc_at(ka, off), idesc_qk, k != 0 ? 1u : 0u);
         }
-        if (u == 1) umma_commit(&k_empty[st]);
-      };
-      bool ok = mbar_wait(q_full, 0, abort_flag, a.status, 910);
-      if (ok) ok = mbar_wait(&k_full[0], 0, abort_flag, a.status, 911);
-      if (ok) {
-        tc_fence_after_sync();
-        issue_qk(0, 0);
-        issue_qk(1, 0);
-        for (int j = 0; j < n_tiles && ok; ++j) {
-          const int st = j % WP_STAGES, st1 = (j + 1) % WP_STAGES;
-          if (!mbar_wait(&v_full[st], static_cast<uint32_t>(j / WP_STAGES) & 1u, abort_flag, a.status, 915)) break;
-          if (j + 1 < n_tiles &&
-              !mbar_wait(&k_full[st1], static_cast<uint32_t>((j + 1) / WP_STAGES) & 1u, abort_flag, a.status, 912)) break;
-          const uint32_t v_addr = smem_u32(v_sm + st * TILE);
+        if (leader) umma_commit(&s_full[u]);
+      }
+      if (leader && u == 1) umma_commit(&k_empty[st]);
+    };
+    bool ok = wait(q_full, 0, 910) && wait(&k_full[0], 0, 911);
+    if (ok) {
+      tc_fence_after_sync();
+      issue_qk(0, 0);
+      issue_qk(1, 0);
+      for (int j = 0; j < n_tiles && ok; ++j) {
+        const int st = j % WP_STAGES, st1 = (j + 1) % WP_STAGES;
+        if (!wait(&v_full[st], static_cast<uint32_t>(j / WP_STAGES) & 1u, 915)) break;
+        if (j + 1 < n_tiles && !wait(&k_full[st1], static_cast<uint32_t>((j + 1) / WP_STAGES) & 1u, 912)) break;
+        const uint64_t va = smem_desc_at(vd, st * TILE);
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            if (active(u, j)) {
-              const int n = j - (u ? u1.jb : u0.jb);         // tiles of this unit before this one
-              const uint32_t tp = tmem_base + u * 128, to = tmem_base + 256 + u * 128;
+        for (int u = 0; u < 2; ++u) {
+          if (active(u, j)) {
+            const int n = j - (u ? u1.jb : u0.jb);           // tiles of this unit before this one
+            const uint32_t tp = tmem_base + u * 128, to = tmem_base + 256 + u * 128;
 #pragma unroll
-              for (int half = 0; half < 2 && ok; ++half) {   // the first keys are multiplied while the last ones are exponentiated
-                ok = mbar_wait(half ? &p_full[u] : &p_half[u], static_cast<uint32_t>(n) & 1u, abort_flag, a.status, 913 + half);
-                if (!ok) break;
-                tc_fence_after_sync();
-#pragma unroll
-                for (int part = 0; part < 2; ++part)
-#pragma unroll
-                  for (int k = half * 4; k < half * 4 + 4; ++k)   // 16 keys: 8 packed columns of P, 16 rows (2 KiB) of the V tile
-                    umma_bf16_ts(to, tp + (k >> 1) * 32 + part * 16 + (k & 1) * 8, make_smem_desc_sw128(v_addr + k * 2048, 16384, 1024), idesc_pv,
-                                 (n | half | part | (k & 3)) != 0 ? 1u : 0u);
-              }
+            for (int half = 0; half < 2 && ok; ++half) {     // the first keys are multiplied while the last ones are exponentiated
+              ok = wait(half ? &p_full[u] : &p_half[u], static_cast<uint32_t>(n) & 1u, 913 + half);
               if (!ok) break;
-              if (j + 1 == (u ? u1.je : u0.je)) umma_commit(&o_full[u]);
+              tc_fence_after_sync();
+#pragma unroll
+              for (int part = 0; part < 2; ++part)
+#pragma unroll
+                for (int k = half * 4; k < half * 4 + 4; ++k)     // 16 keys: 8 packed columns of P, 16 rows (2 KiB) of the V tile
+                  if (leader)
+                    umma_bf16_ts(to, tp + (k >> 1) * 32 + part * 16 + (k & 1) * 8, smem_desc_at(va, k * 2048), idesc_pv,
+                                 (n | half | part | (k & 3)) != 0 ? 1u : 0u);
             }
-            if (u == 1) umma_commit(&v_empty[st]);
-            tc_fence_after_sync();
-            if (j + 1 < n_tiles) issue_qk(u, j + 1);
+            if (!ok) break;
+            if (leader && j + 1 == (u ? u1.je : u0.je)) umma_commit(&o_full[u]);
           }
+          if (leader && u == 1) umma_commit(&v_empty[st]);
+          tc_fence_after_sync();
+          if (j + 1 < n_tiles) issue_qk(u, j + 1);
         }
       }
     }
