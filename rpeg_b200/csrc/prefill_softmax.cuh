@@ -72,4 +72,30 @@ __device__ __forceinline__ float wp_exp_row(const WpRow& row, uint32_t ts, float
   return (s0.x + s0.y) + (s1.x + s1.y);
 }
 
+// The same with plain bf16 weights: P over the first 64 columns of S, 16 columns a chunk.
+__device__ __forceinline__ float wp_exp_row_bf16(const WpRow& row, uint32_t ts, float scale_log2, float m_ref, uint64_t* half_bar) {
+  const uint64_t scale2 = pack2(scale_log2, scale_log2), shift2 = pack2(-m_ref, -m_ref);
+  uint64_t sum2[2] = {0ull, 0ull};
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t w[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float2 t = unpack2(fma2(pack2(__uint_as_float(row.s[c][2 * i]), __uint_as_float(row.s[c][2 * i + 1])), scale2, shift2));
+      const float p0 = exp2f(t.x), p1 = exp2f(t.y);
+      sum2[i & 1] = add2(sum2[i & 1], pack2(p0, p1));
+      w[i] = pack_bf16x2(p0, p1);
+    }
+    tmem_st_32x16(ts + c * 16, w);
+    if (c == 1) {
+      tmem_wait_st();
+      tc_fence_before_sync();
+      __syncwarp();
+      if ((threadIdx.x & 31) == 0) mbar_arrive(half_bar);
+    }
+  }
+  const float2 s0 = unpack2(sum2[0]), s1 = unpack2(sum2[1]);
+  return (s0.x + s0.y) + (s1.x + s1.y);
+}
+
 }  // namespace rpeg

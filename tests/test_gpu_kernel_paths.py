@@ -140,3 +140,22 @@ def test_gemm_partials_of_two_row_tiles(cuda_device, m, n, k):
     p = K.gemm_partials(a, b, ws)
     assert _rel(p.buf[: p.splits * m * n].view(p.splits, m, n).sum(0), want) < F32
     assert _rel(K.gemm(a, b, workspace=ws), want) < 2 ** -9
+
+
+@pytest.mark.parametrize("h,hkv", [(2, 2), (8, 2)])
+def test_flash_attn_fwd_units(cuda_device, h, hkv):
+    hd, lens = 128, [1, 127, 129, 255, 256, 257, 385, 640]          # one unit, two, and a last tile that only the second one sees
+    g = torch.Generator(device=cuda_device).manual_seed(h)
+    qkv = torch.randn(sum(lens), (h + 2 * hkv) * hd, generator=g, device=cuda_device).bfloat16()
+    qkv[400:] *= 3                                                   # scores that grow by more than 2^8 between tiles: O is rescaled
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), device=cuda_device, dtype=torch.int32)
+    out, lse = K.flash_attn_fwd(qkv, 0, h * hd, (h + hkv) * hd, cu, max(lens), h, hkv, hd)
+    at = 0
+    for n in lens:
+        q, k, v = qkv[at:at + n].double().view(n, -1, hd).split([h, hkv, hkv], 1)
+        s = torch.einsum("qhd,khd->hqk", q, k.repeat_interleave(h // hkv, 1)) * hd ** -0.5
+        s = s.masked_fill(torch.ones(n, n, device=cuda_device, dtype=torch.bool).triu(1), float("-inf"))
+        want = torch.einsum("hqk,khd->qhd", s.softmax(-1), v.repeat_interleave(h // hkv, 1)).reshape(n, -1)
+        assert _rel(out[at:at + n], want) < 2 ** -8                  # weights and output rounded to bf16
+        assert float((lse[:, at:at + n] - s.logsumexp(-1)).abs().max()) < 1e-4
+        at += n
