@@ -24,8 +24,9 @@ the length cap; outputs are returned per original row index, right padded, with 
 from __future__ import annotations
 
 from dataclasses import dataclass, field
-from typing import Dict, List, Optional
+from typing import Dict, List, Optional, Sequence
 
+import numpy as np
 import torch
 
 from ..models.llama import LlamaModel
@@ -224,16 +225,33 @@ class Generator:
         _lib.add_launches(self._graph_launches[key])
 
     # ------------------------------------------------------------------ prefill of admitted rows
+    def _upload(self, arrays: Sequence[np.ndarray]) -> List[torch.Tensor]:
+        """int32 arrays on the device, in one copy (every one starts on a 16-byte boundary)."""
+        at, total = [], 0
+        for a in arrays:
+            at.append(total)
+            total += (a.size + 3) // 4 * 4
+        buf = np.zeros(total, dtype=np.int32)
+        for o, a in zip(at, arrays):
+            buf[o:o + a.size] = a
+        dev = torch.from_numpy(buf).to(self.dev)
+        return [dev[o:o + a.size] for o, a in zip(at, arrays)]
+
     def prefill_hidden(self, pieces: List[torch.Tensor], slots: List[int], starts: Optional[List[int]] = None):
         """Run one piece of tokens per slot through the model, each continuing at position ``starts[i]`` (0 without it),
         and store the K/V through the slots' page-table rows. Returns the hidden rows of all pieces and their offsets."""
-        cfg, dev = self.cfg, self.dev
+        cfg = self.cfg
         lens = [int(p.numel()) for p in pieces]
         starts = [0] * len(lens) if starts is None else starts
-        tokens = torch.cat(pieces).to(device=dev, dtype=torch.int32)
-        pos = torch.cat([torch.arange(s, s + l, dtype=torch.int32) for s, l in zip(starts, lens)]).to(dev)
-        seq_id = torch.cat([torch.full((l,), s, dtype=torch.int32) for l, s in zip(lens, slots)]).to(dev)
-        cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=dev)
+        n = sum(lens)
+        host = all(not p.is_cuda for p in pieces)
+        # one upload for everything the host knows (each costs tens of microseconds before the first kernel)
+        up = [np.concatenate([np.arange(s, s + l, dtype=np.int32) for s, l in zip(starts, lens)]), np.repeat(np.asarray(slots, dtype=np.int32), lens),
+              np.concatenate([np.zeros(1, dtype=np.int32), np.cumsum(lens, dtype=np.int32)])]
+        if host:
+            up.append(torch.cat(pieces).to(torch.int32).numpy())
+        pos, seq_id, cu, *rest = self._upload(up)
+        tokens = rest[0] if host else torch.cat([p.to(self.dev) for p in pieces]).to(torch.int32)
         if self.cached_prefill:
             kw = {"spans": (starts, lens)} if getattr(self.model, "prefill_spans", False) else {}
             return self.model.prefill(tokens, pos, cu, max(lens), seq_id, self.page_table, self.kcache, self.vcache, **kw), cu
@@ -275,9 +293,8 @@ class Generator:
         """Sample the first token of every admitted row from its prompt's last-position logits (one row of ``logits``
         per slot) and initialise the slot state for decoding."""
         dev = self.dev
-        sl = torch.tensor(slots, dtype=torch.long, device=dev)
-        lens_t = torch.tensor(lens, dtype=torch.int32, device=dev)
-        f_len = torch.tensor(forced if forced is not None else [0] * len(slots), dtype=torch.int32, device=dev)
+        sl, lens_t, f_len = self._upload([np.asarray(v, dtype=np.int32) for v in (slots, lens, forced if forced is not None else [0] * len(slots))])
+        sl = sl.long()
         first_forced = torch.where(f_len == 1, torch.full_like(f_len, self.eos_id), torch.full_like(f_len, -1))
         tok, lp = K.sample(logits, temperature, greedy, seed ^ 0x5DEECE66D, forced=first_forced, seed_offset=self.step_counter,
                            top_k=top_k, top_p=top_p)
@@ -449,17 +466,19 @@ class Generator:
             if idx:
                 self.page_table.view(-1)[torch.tensor(idx, dtype=torch.long, device=dev)] = 0
 
-        def copy_page(src: int, dst: List[int]) -> None:
-            """Copy one KV page (all layers, K and V) onto the pages ``dst``."""
-            d = torch.tensor(dst, dtype=torch.long, device=dev)
-            if len(set(self.geometry)) > 1 or self.geometry[0][1] != self.geometry[0][2]:
-                for c in (*self.kcache, *self.vcache):
-                    if c.numel():                        # a layer may keep no values, or nothing of its own
-                        c[d] = c[src].clone()
-                return
-            pages = self.kcache[0].shape[0]              # layers of one shape: a single strided copy
-            flat = self.kv_storage.view(2 * self.cfg.n_layers, pages, -1)
-            flat[:, d] = flat[:, src].unsqueeze(1)
+        def copy_pages(src: List[int], dst: List[int]) -> None:
+            """Copy KV pages (all layers, K and V): page ``src[i]`` onto ``dst[i]``, a few at a time (the copy passes through a buffer)."""
+            for i in range(0, len(src), 16):
+                s_idx, d_idx = self._upload([np.asarray(v[i:i + 16], dtype=np.int32) for v in (src, dst)])
+                s_idx, d_idx = s_idx.long(), d_idx.long()
+                if len(set(self.geometry)) > 1 or self.geometry[0][1] != self.geometry[0][2]:
+                    for c in (*self.kcache, *self.vcache):
+                        if c.numel():                    # a layer may keep no values, or nothing of its own
+                            c[d_idx] = c[s_idx]
+                else:
+                    pages = self.kcache[0].shape[0]      # layers of one shape: a single strided copy
+                    flat = self.kv_storage.view(2 * self.cfg.n_layers, pages, -1)
+                    flat[:, d_idx] = flat[:, s_idx]
 
         while retired < N:
             free = [s for s in range(n) if slot_row[s] < 0]
@@ -486,7 +505,7 @@ class Generator:
                     new_rows.append(queue.pop(0))
                     new_slots.append(s)
                 if new_rows:
-                    table = torch.zeros((len(new_rows), self.pages_per_row), dtype=torch.int32)
+                    table = np.zeros((len(new_rows), self.pages_per_row), dtype=np.int32)
                     prefill_rows, prefill_slots = [], []
                     for j, (r, s) in enumerate(zip(new_rows, new_slots)):
                         plen = int(rows[r].numel())
@@ -507,27 +526,40 @@ class Generator:
                         counters["kv_pages_taken"] += len(own)
                         slot_pages[s], slot_row[s], slot_prompt[s], slot_bound[s], slot_shared[s] = own, r, plen, plen + 1, sh
                         if sh:
-                            table[j, :sh] = torch.tensor(groups[g]["pages"], dtype=torch.int32)
-                        table[j, sh:sh + len(own)] = torch.tensor(own, dtype=torch.int32)
-                    self.page_table[torch.tensor(new_slots, dtype=torch.long, device=dev)] = table.to(dev)
+                            table[j, :sh] = groups[g]["pages"]
+                        table[j, sh:sh + len(own)] = own
+                    slot_idx, flat_table = self._upload([np.asarray(new_slots, dtype=np.int32), table.reshape(-1)])
+                    self.page_table[slot_idx.long()] = flat_table.view(len(new_rows), -1)
                     if prefill_rows:
                         logits = self._prefill([rows[r] for r in prefill_rows], prefill_slots)
                         counters["prefill_calls"] += 1
                         counters["prompts_prefilled"] += len(prefill_rows)
                         counters["prefill_tokens"] += sum(int(rows[r].numel()) for r in prefill_rows)
                     if G > 1:
+                        src, dst = [], []
+                        at = {r: j for j, r in enumerate(prefill_rows)}
+                        fresh = {}                          # groups whose prompt was prefilled just now: their row of `logits`
                         for j, (r, s) in enumerate(zip(prefill_rows, prefill_slots)):
                             g = groups.get(r // G)
                             if g is not None and g["logits"] is None:
                                 g["logits"] = logits[j].clone()
+                                fresh[r // G] = j
                                 if g["tail"]:               # keep the prompt's ragged tail for the rows that come later
-                                    copy_page(slot_pages[s][0], [g["tail"]])
+                                    src.append(slot_pages[s][0])
+                                    dst.append(g["tail"])
+                        copy_pages(src, dst)
+                        src, dst = [], []
                         for r, s in zip(new_rows, new_slots):   # rows that alias an already prefilled prompt need its tail
                             g = groups.get(r // G)
-                            if g is not None and g["tail"] and not (r in prefill_rows):
-                                copy_page(g["tail"], [slot_pages[s][0]])
-                        row_logits = torch.stack([groups[r // G]["logits"] if (r // G) in groups else logits[prefill_rows.index(r)]
-                                                  for r in new_rows])
+                            if g is not None and g["tail"] and r not in at:
+                                src.append(g["tail"])
+                                dst.append(slot_pages[s][0])
+                        copy_pages(src, dst)
+                        place = [fresh.get(r // G, -1) if (r // G) in groups else at[r] for r in new_rows]
+                        if min(place) >= 0:
+                            row_logits = logits[self._upload([np.asarray(place, dtype=np.int32)])[0].long()]
+                        else:
+                            row_logits = torch.stack([groups[r // G]["logits"] if (r // G) in groups else logits[at[r]] for r in new_rows])
                     else:
                         row_logits = logits
                     self._start_rows(row_logits, [int(rows[r].numel()) for r in new_rows], new_slots,

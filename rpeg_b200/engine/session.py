@@ -7,9 +7,11 @@ the decode step, everything else through the prefill, each continuing from what 
 """
 from __future__ import annotations
 
+from array import array
 from dataclasses import dataclass, field
 from typing import Dict, Hashable, List, Optional, Sequence, Tuple
 
+import numpy as np
 import torch
 
 from ..ops import kernels as K
@@ -37,14 +39,22 @@ class Session:
         self.rows = torch.arange(gen.max_slots, dtype=torch.int32, device=gen.dev)
 
     # ------------------------------------------------------------------ pages
-    def _reserve(self, q: _Request, n: int) -> None:
-        """Pages for ``n`` more tokens of the request."""
-        have = q.gone + len(q.pages)
-        need = -(-(q.length + n) // PAGE) - have
-        if need > 0:
-            new = self.gen.pool.take(need)
-            q.pages.extend(new)
-            self.gen.page_table[q.slot, have:have + need] = torch.tensor(new, dtype=torch.int32, device=self.gen.dev)
+    def _reserve(self, reqs: Sequence[_Request], more: Sequence[int]) -> None:
+        """Pages for ``more[i]`` more tokens of request ``i``, entered in the table with one upload."""
+        place, page = [], []
+        try:
+            for q, n in zip(reqs, more):
+                have = q.gone + len(q.pages)
+                need = -(-(q.length + n) // PAGE) - have
+                if need > 0:
+                    new = self.gen.pool.take(need)
+                    q.pages.extend(new)
+                    place.extend(range(q.slot * self.gen.pages_per_row + have, q.slot * self.gen.pages_per_row + have + need))
+                    page.extend(new)
+        finally:                                            # the pool may run dry half way: what was taken is in the table
+            if place:
+                at, new = self.gen._upload([np.asarray(v, dtype=np.int32) for v in (place, page)])
+                self.gen.page_table.view(-1).index_copy_(0, at.long(), new)
 
     def _drop_passed(self, q: _Request) -> None:
         """Give back the pages no later token of the request reads."""
@@ -80,10 +90,18 @@ class Session:
         g = self.gen
         if len({rid for rid, _, _ in entries}) != len(entries):
             raise ValueError("a request may appear once per step")
+        arrays: List[np.ndarray] = []
         for rid, tokens, want in entries:
             if not len(tokens):
                 raise ValueError(f"request {rid!r} brings no tokens")
-            if min(tokens) < 0 or max(tokens) >= g.cfg.vocab:
+            try:
+                ids = np.frombuffer(array("i", list(tokens)), dtype=np.int32)
+                low, high = int(ids.min()), int(ids.max())
+            except (TypeError, OverflowError):              # not plain 32-bit integers
+                low, high = min(tokens), max(tokens)
+                ids = np.asarray(list(tokens)).astype(np.int32) if 0 <= low and high < g.cfg.vocab else np.zeros(0, np.int32)
+            arrays.append(ids)
+            if low < 0 or high >= g.cfg.vocab:
                 raise ValueError(f"request {rid!r} brings a token outside the vocabulary")
             if len(want) and (min(want) < 0 or max(want) >= len(tokens)):
                 raise ValueError(f"request {rid!r} wants a place outside its tokens")
@@ -96,8 +114,7 @@ class Session:
         for rid in new:
             self.requests[rid] = _Request(self.free_slots.pop())
         reqs = [self.requests[rid] for rid, _, _ in entries]
-        for q, (_, tokens, _) in zip(reqs, entries):
-            self._reserve(q, len(tokens))
+        self._reserve(reqs, [len(tokens) for _, tokens, _ in entries])
         out: List[Optional[torch.Tensor]] = [None] * len(entries)
         single = [i for i, q in enumerate(reqs) if q.length > 0 and len(entries[i][1]) == 1]
         many = [i for i in range(len(entries)) if i not in set(single)]
@@ -111,9 +128,11 @@ class Session:
         serial = [i for i in many if reqs[i].length > 0 and not g.cached_prefill]      # no prefill behind a cached prefix
         packed = [i for i in many if i not in set(serial)]
         if packed:
-            hidden, cu = g.prefill_hidden([torch.tensor(list(entries[i][1]), dtype=torch.int32) for i in packed], [reqs[i].slot for i in packed],
-                                          [reqs[i].length for i in packed])
-            offs = cu.tolist()
+            hidden, cu = g.prefill_hidden([torch.from_numpy(arrays[i]) for i in packed], [reqs[i].slot for i in packed],
+                                         [reqs[i].length for i in packed])
+            offs = [0]
+            for i in packed:
+                offs.append(offs[-1] + len(arrays[i]))
             rows = [offs[j] + int(w) for j, i in enumerate(packed) for w in entries[i][2]]
             if rows:
                 logits = g.model.lm_logits(K.gather_rows(hidden, torch.tensor(rows, dtype=torch.int32, device=g.dev)))
