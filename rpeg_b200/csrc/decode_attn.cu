@@ -6,13 +6,14 @@
 // their pages back to the allocator, so no compaction copy is ever needed.
 //
 // Decode attention is bandwidth bound (one query row per head): each CTA owns (head, sequence,
-// split), its 4 warps stride over 32-key blocks, 16 lanes per key row so every load is a coalesced
+// split), its 4 warps stride over 16-key blocks, 16 lanes per key row so every load is a coalesced
 // 256-byte line, keeping an online-softmax state per warp that is merged in shared memory.
 // With nsplit > 1 the partial (m, l, o) of every split goes to a scratch buffer and a second
 // kernel merges them.
 //
 // Replaces the reference's static-KV decode: Megatron StaticInferenceContext plus per-layer
 // index_select/copy compaction (RPEG/runtime/workers/megatron_worker.py:2585-2598, 2667-2811).
+#include <cmath>
 #include "common.cuh"
 #include "rpeg_kernels.h"
 
@@ -171,6 +172,21 @@ __device__ __forceinline__ float transpose_reduce16(float (&v)[16], int lane) {
   return keep + __shfl_xor_sync(0xffffffffu, send, 1);
 }
 
+// 8 per-lane partial dot products (one per key) -> the full dot product of key `lane & 7` in every lane of a 16-lane group: at each level
+// half of the values go to the partner.
+__device__ __forceinline__ float transpose_reduce8(float (&v)[8], int lane) {
+#pragma unroll
+  for (int w = 4; w > 0; w >>= 1)
+#pragma unroll
+    for (int i = 0; i < w; ++i) {
+      const bool up = lane & w;
+      const float send = up ? v[i] : v[i + w];
+      const float keep = up ? v[i + w] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+    }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 8);
+}
+
 __device__ __forceinline__ float dot8(const uint4& kv, const float (&q)[8]) {
   const float2 a = unpack_bf16x2(kv.x), b = unpack_bf16x2(kv.y), c = unpack_bf16x2(kv.z), d = unpack_bf16x2(kv.w);
   return a.x * q[0] + a.y * q[1] + b.x * q[2] + b.y * q[3] + c.x * q[4] + c.y * q[5] + d.x * q[6] + d.y * q[7];
@@ -185,13 +201,18 @@ __device__ __forceinline__ void axpy8(float (&acc)[8], float p, const uint4& vv)
 // q: [B, ldq] with head h at column q_col0 + h*HD. out: [B, H*HD] bf16.
 // partial (when nsplit > 1): [B, H, nsplit, HD + 2] fp32 = {o[HD], m, l}.
 //
-// Work split inside a warp: the 32 lanes form two groups of 16; a group reads one 256-byte K (or
-// V) row per load instruction, lane c of the group owning the 16-byte chunk c (head dims 8c..8c+7),
-// so every global load is fully coalesced and a lane keeps 8 independent 16-byte loads in flight.
-// Group g takes keys g*16..g*16+15 of a 32-key block; the 16 partial dot products of a lane are
-// summed across the group by a transposing butterfly that leaves the score of key `lane` in lane
-// `lane`, which is the layout the online softmax wants. For PV each lane accumulates its 8 head
-// dims over the group's keys; the two groups are added at the end.
+// Bound by streaming the cache: a block of 16 keys (4 KB of K and of V) comes into a warp's own shared memory as one bulk copy each, the
+// next K as soon as this one's scores are taken, so 24 warps an SM keep up to 192 KB in flight whatever their registers allow (loads to
+// registers waited four times per 32 keys: 16 rows of 280 keys, 32 heads 31 -> 23 us, 256 rows of 540 410 -> 323 us, 7.0 TB/s;
+// 256 rows in groups of eight over 512 shared keys 256 -> 199 us).
+// Work split inside a warp: the 32 lanes form two groups of 16; a group reads one 256-byte K (or V) row per load instruction, lane c of the
+// group owning the 16-byte chunk c (head dims 8c..8c+7). Group g takes keys g*8..g*8+7 of a block; the 8 partial dot products of a lane are
+// summed across the group by a transposing butterfly that leaves the score of key `lane & 7` in two lanes. For PV each lane
+// accumulates its 8 head dims over the group's keys; the two groups are added at the end.
+constexpr int DA_KEYS = 16;                          // keys of a block, a divisor of the page
+constexpr int DA_BLOCK_BYTES = DA_KEYS * HD * 2;
+constexpr int DA_SMEM = 4 * 2 * DA_BLOCK_BYTES;      // per warp: a block of K and of V
+
 __global__ void __launch_bounds__(128)
 paged_decode_attn_kernel(const __nv_bfloat16* __restrict__ q, int ldq, int q_col0,
                          const __nv_bfloat16* __restrict__ kcache, const __nv_bfloat16* __restrict__ vcache,
@@ -201,19 +222,25 @@ paged_decode_attn_kernel(const __nv_bfloat16* __restrict__ q, int ldq, int q_col
                          int* __restrict__ arrive) {
   griddep_launch();
   griddep_wait();   // may have been scheduled under the previous kernel's tail: nothing is read or written before this
+  extern __shared__ __align__(128) uint8_t kv_sm[];
+  __shared__ uint64_t kv_bar[4][2];
+  __shared__ int abort_word;
   __shared__ float red_m[4], red_l[4];
   __shared__ int is_last;
   __shared__ __align__(16) float red_o[4][HD];
   const int h = blockIdx.x, b = blockIdx.y, split = blockIdx.z;
   const int hk = h / (H / Hkv);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint8_t* const k_sm = kv_sm + warp * 2 * DA_BLOCK_BYTES;
+  uint8_t* const v_sm = k_sm + DA_BLOCK_BYTES;
+  uint64_t* const bar = kv_bar[warp];
   const int grp = lane >> 4, c = lane & 15;
   const int L = seq_lens[b];
-  const int nblk = (L + 31) / 32;                  // 32-key blocks
+  const int nblk = (L + DA_KEYS - 1) / DA_KEYS;
   // keys before row_key0[b] (a multiple of 64: whole shared prompt pages) are covered by the group kernel below,
   // which leaves its result in partial slot 0; this kernel then fills slots slot_base .. slot_base + nsplit - 1
   const int key0 = row_key0 != nullptr ? min(row_key0[b], L) : 0;
-  const int blk_first = key0 / 32;
+  const int blk_first = key0 / DA_KEYS;
   const int blk_per_split = (max(nblk - blk_first, 0) + nsplit - 1) / nsplit;
   const int blk0 = blk_first + split * blk_per_split;
   const int blk1 = min(nblk, blk0 + blk_per_split);
@@ -231,57 +258,77 @@ paged_decode_attn_kernel(const __nv_bfloat16* __restrict__ q, int ldq, int q_col
 #pragma unroll
   for (int k = 0; k < 8; ++k) acc[k] = 0.f;
   const int* pt = page_table + static_cast<size_t>(b) * max_pages;
-  for (int blk = blk0 + warp; blk < blk1; blk += 4) {
-    const int page = pt[(blk * 32) / PAGE];
-    // first row of this group's 16 keys, this lane's 16-byte chunk
-    const size_t base = ((static_cast<size_t>(page) * Hkv + hk) * PAGE + ((blk * 32) % PAGE) + grp * 16) * HD + c * 8;
-    const int nk = min(32, L - blk * 32) - grp * 16;   // valid keys of this group (may be <= 0)
-    const uint4* kp = reinterpret_cast<const uint4*>(kcache + base);
-    const uint4* vp = reinterpret_cast<const uint4*>(vcache + base);
-    float part[16];
-    if (nk >= 16) {
+  const int first = blk0 + warp;
+  int page = first < blk1 ? pt[(first * DA_KEYS) / PAGE] : 0;
+  auto fetch = [&](int blk, int pg, const __nv_bfloat16* cache, uint8_t* dst, uint64_t* done) {     // one lane
+    const uint32_t bytes = min(DA_KEYS, L - blk * DA_KEYS) * (HD * 2);
+    mbar_expect_tx(done, bytes);
+    bulk_load(dst, cache + ((static_cast<size_t>(pg) * Hkv + hk) * PAGE + (blk * DA_KEYS) % PAGE) * HD, bytes, done);
+  };
+  if (lane == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    if (warp == 0) abort_word = 0;
+    fence_mbar_init();
+    if (first < blk1) {
+      fetch(first, page, kcache, k_sm, &bar[0]);
+      fetch(first, page, vcache, v_sm, &bar[1]);
+    }
+  }
+  __syncthreads();
+  uint32_t phase = 0;
+  for (int blk = first; blk < blk1; blk += 4, phase ^= 1u) {
+    const int next = blk + 4;
+    const int next_page = next < blk1 ? pt[(next * DA_KEYS) / PAGE] : 0;
+    const int nk = min(DA_KEYS, L - blk * DA_KEYS) - grp * 8;   // valid keys of this group (may be <= 0)
+    const uint4* kp = reinterpret_cast<const uint4*>(k_sm) + grp * 8 * (HD / 8) + c;      // this lane's chunk of the group's rows
+    const uint4* vp = reinterpret_cast<const uint4*>(v_sm) + grp * 8 * (HD / 8) + c;
+    if (!__all_sync(0xffffffffu, mbar_wait(&bar[0], phase, &abort_word, nullptr, 0))) break;
+    float part[8];
+    if (nk >= 8) {
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint4 kv[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) kv[j] = kp[(half * 8 + j) * (HD / 8)];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) part[half * 8 + j] = dot8(kv[j], qr);
-      }
+      for (int j = 0; j < 8; ++j) part[j] = dot8(kp[j * (HD / 8)], qr);
     } else {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
+      for (int j = 0; j < 8; ++j) {
         part[j] = 0.f;
         if (j < nk) part[j] = dot8(kp[j * (HD / 8)], qr);
       }
     }
-    float s = transpose_reduce16(part, lane);       // score of key (blk*32 + lane)
-    if (c >= nk) s = -INFINITY;
-    const float bm = warp_max(s);
-    const float nm = fmaxf(m, bm);
+    __syncwarp();
+    if (lane == 0 && next < blk1) fetch(next, next_page, kcache, k_sm, &bar[0]);
+    const int key = lane & 7;
+    float s = transpose_reduce8(part, lane);        // score of key `key` of the group, in two lanes
+    if (key >= nk) s = -INFINITY;
+    const float nm = fmaxf(m, warp_max(s));
     const float alpha = exp2f(m - nm);              // m = -inf on the first block gives 0
-    const float p = (c < nk) ? exp2f(s - nm) : 0.f;
-    l = l * alpha + warp_sum(p);
+    const float p = (key < nk) ? exp2f(s - nm) : 0.f;
+    l = l * alpha + ((lane & 8) ? 0.f : p);         // this lane's share, added up at the end
 #pragma unroll
     for (int k = 0; k < 8; ++k) acc[k] *= alpha;
     m = nm;
-    if (nk >= 16) {
+    if (!__all_sync(0xffffffffu, mbar_wait(&bar[1], phase, &abort_word, nullptr, 0))) break;
+    if (nk >= 8) {
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint4 vv[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) vv[j] = vp[(half * 8 + j) * (HD / 8)];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) axpy8(acc, __shfl_sync(0xffffffffu, p, grp * 16 + half * 8 + j), vv[j]);
-      }
+      for (int j = 0; j < 8; ++j) axpy8(acc, __shfl_sync(0xffffffffu, p, grp * 16 + j), vp[j * (HD / 8)]);
     } else {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
+      for (int j = 0; j < 8; ++j) {
         const float pj = __shfl_sync(0xffffffffu, p, grp * 16 + j);
         if (j < nk) axpy8(acc, pj, vp[j * (HD / 8)]);
       }
     }
+    __syncwarp();
+    if (lane == 0 && next < blk1) fetch(next, next_page, vcache, v_sm, &bar[1]);
   }
+  if (*static_cast<volatile int*>(&abort_word)) {       // a copy that never arrived (there is no status word here): the row becomes NaN
+    __nanosleep(200000);
+    m = 0.f;
+    l = 1.f / 32.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) acc[k] = NAN;
+  }
+  l = warp_sum(l);
   // add the two key groups, then merge the 4 warps
 #pragma unroll
   for (int k = 0; k < 8; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 16);
@@ -857,7 +904,7 @@ extern "C" int rpeg_paged_decode_attn(const void* q, int ldq, int q_col0, const 
   if (B <= 0) return 0;
   const float scale_log2 = scale * 1.4426950408889634f;
   int* arrive = nsplit > 1 ? fused_combine_counters(B, H) : nullptr;
-  launch_pdl(paged_decode_attn_kernel, dim3(dim3(H, B, nsplit)), dim3(128), 0, STREAM(stream), 
+  launch_pdl(paged_decode_attn_kernel, dim3(H, B, nsplit), dim3(128), DA_SMEM, STREAM(stream), 
       static_cast<const __nv_bfloat16*>(q), ldq, q_col0, static_cast<const __nv_bfloat16*>(kcache),
       static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages, seq_lens,
       static_cast<__nv_bfloat16*>(out), scratch, H, Hkv, nsplit, scale_log2, static_cast<const int*>(nullptr), 0, nsplit, arrive);
@@ -886,7 +933,7 @@ extern "C" int rpeg_paged_decode_attn_grouped(const void* q, int ldq, int q_col0
   launch_pdl(paged_decode_attn_shared_kernel, dim3(H, B), dim3(128), 0, STREAM(stream), static_cast<const __nv_bfloat16*>(q), ldq,
              q_col0, static_cast<const __nv_bfloat16*>(kcache), static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages,
              group_rows, group_shared, scratch, H, Hkv, nslots, scale_log2);
-  launch_pdl(paged_decode_attn_kernel, dim3(H, B, nsplit), dim3(128), 0, STREAM(stream), static_cast<const __nv_bfloat16*>(q), ldq,
+  launch_pdl(paged_decode_attn_kernel, dim3(H, B, nsplit), dim3(128), DA_SMEM, STREAM(stream), static_cast<const __nv_bfloat16*>(q), ldq,
              q_col0, static_cast<const __nv_bfloat16*>(kcache), static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages,
              seq_lens, static_cast<__nv_bfloat16*>(out), scratch, H, Hkv, nsplit, scale_log2, row_key0, 1, nslots, arrive);
   if (arrive == nullptr)
@@ -936,7 +983,7 @@ extern "C" int rpeg_paged_decode_attn_grouped_tc(const void* q, int ldq, int q_c
   launch_pdl(paged_decode_attn_shared_tc_kernel, dim3(grid), dim3(GT_THREADS), GT_SMEM, STREAM(stream), tk, tv,
              static_cast<const __nv_bfloat16*>(q), ldq, q_col0, page_table, max_pages, group_rows, group_shared, scratch, B, H, Hkv,
              nslots, scale_log2, status);
-  launch_pdl(paged_decode_attn_kernel, dim3(H, B, nsplit), dim3(128), 0, STREAM(stream), static_cast<const __nv_bfloat16*>(q), ldq,
+  launch_pdl(paged_decode_attn_kernel, dim3(H, B, nsplit), dim3(128), DA_SMEM, STREAM(stream), static_cast<const __nv_bfloat16*>(q), ldq,
              q_col0, static_cast<const __nv_bfloat16*>(kcache), static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages,
              seq_lens, static_cast<__nv_bfloat16*>(out), scratch, H, Hkv, nsplit, scale_log2, row_key0, 1, nslots, arrive);
   if (arrive == nullptr)
@@ -987,7 +1034,7 @@ extern "C" int rpeg_paged_decode_attn_static(const void* q, int ldq, int q_col0,
   }
   float* scratch = g_static_scratch_ptr[dev];
   const float scale_log2 = scale * 1.4426950408889634f;
-  launch_pdl(paged_decode_attn_kernel, dim3(dim3(H, B, nsplit)), dim3(128), 0, STREAM(stream), 
+  launch_pdl(paged_decode_attn_kernel, dim3(H, B, nsplit), dim3(128), DA_SMEM, STREAM(stream), 
       static_cast<const __nv_bfloat16*>(q), ldq, q_col0, static_cast<const __nv_bfloat16*>(kcache),
       static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages, seq_lens, static_cast<__nv_bfloat16*>(out),
       scratch, H, Hkv, nsplit, scale_log2, static_cast<const int*>(nullptr), 0, nsplit, static_cast<int*>(nullptr));

@@ -129,11 +129,6 @@ __device__ __forceinline__ void load8(const float* p, uint64_t (&o)[4]) {
   const float4 a = load4(p), b = load4(p + 4);
   o[0] = pack2(a.x, a.y); o[1] = pack2(a.z, a.w); o[2] = pack2(b.x, b.y); o[3] = pack2(b.z, b.w);
 }
-__device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem_dst)),
-               "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
 
 // LPK lanes hold one key (8 dimensions each), a warp scores 32 / LPK keys side by side and RA_KEYS of them per lane
 // group in a row, for RA_HEADS query heads of the KV head (4 or 8, whichever leaves fewer idle). The RA_KEYS x RA_HEADS

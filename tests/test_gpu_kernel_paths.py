@@ -159,3 +159,25 @@ def test_flash_attn_fwd_units(cuda_device, h, hkv):
         assert _rel(out[at:at + n], want) < 2 ** -8                  # weights and output rounded to bf16
         assert float((lse[:, at:at + n] - s.logsumexp(-1)).abs().max()) < 1e-4
         at += n
+
+
+@pytest.mark.parametrize("h,hkv,nsplit", [(2, 2, 1), (4, 1, 1), (2, 2, 3)])
+def test_paged_decode_attn_blocks(cuda_device, h, hkv, nsplit):
+    hd, lens = 128, [0, 1, 7, 8, 9, 15, 16, 17, 63, 64, 65, 127, 200, 1025]      # edges of a lane group's 8 keys, a block's 16, a page's 64
+    g = torch.Generator(device=cuda_device).manual_seed(nsplit)
+    pages = max(lens) // 64 + 1
+    k, v = (torch.randn(len(lens) * pages, hkv, 64, hd, generator=g, device=cuda_device).bfloat16() for _ in range(2))
+    table = torch.randperm(len(lens) * pages, generator=g, device=cuda_device).int().view(len(lens), pages)
+    q = torch.randn(len(lens), h * hd, generator=g, device=cuda_device).bfloat16()
+    for i, n in enumerate(lens):                                                 # what lies behind a row's last key is never read
+        if n % 64:
+            k[table[i, n // 64].long(), :, n % 64:] = float("nan")
+            v[table[i, n // 64].long(), :, n % 64:] = float("nan")
+    out = K.paged_decode_attn(q, 0, k, v, table, torch.tensor(lens, dtype=torch.int32, device=cuda_device), h, hkv, hd, hd ** -0.5, nsplit=nsplit)
+    for i, n in enumerate(lens):
+        if n == 0:
+            assert bool((out[i] == 0).all())
+            continue
+        kk, vv = (t[table[i].long()].transpose(0, 1).reshape(hkv, -1, hd)[:, :n].double().repeat_interleave(h // hkv, 0) for t in (k, v))
+        w = (torch.einsum("hd,hkd->hk", q[i].double().view(h, hd), kk) * hd ** -0.5).softmax(-1)
+        assert _rel(out[i], torch.einsum("hk,hkd->hd", w, vv).reshape(-1)) < 2 ** -8
