@@ -406,68 +406,75 @@ __device__ __forceinline__ void load_partials8(const float* __restrict__ parts, 
 }
 
 // y = rmsnorm(sum_s parts[s] [+ res]) * w; h_out (optional) = the bf16 sum, i.e. the new residual stream.
+// One CTA per row, four columns a thread and turn: a decode step waits for this kernel, and what it waits for is one round trip to L2, so all
+// slabs of a row are requested at once (256 threads with 16 columns each took the slabs one after the other: 1 row 4.3 us, now 3.0; 16 rows 4.6 and 3.2; nine slabs, chained).
 template <int NV>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
 rmsnorm_fwd_partials_kernel(const float* __restrict__ parts, int splits, long long stride,
                             const __nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ w,
                             __nv_bfloat16* __restrict__ h_out, __nv_bfloat16* __restrict__ y, int d, float eps) {
   griddep_launch();
-  griddep_wait();   // may have been scheduled under the previous kernel's tail: nothing is read or written before this
-  __shared__ float warp_ss[8];
+  __shared__ float warp_ss[32];
   const int row = blockIdx.x;
-  const int nvec = d >> 3;
-  float v[NV][8];
+  const size_t row0 = static_cast<size_t>(row) * d;
+  uint2 wv[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {                   // no kernel of the step writes the weights
+    const int c = (threadIdx.x + k * blockDim.x) * 4;
+    wv[k] = c < d ? *reinterpret_cast<const uint2*>(w + c) : make_uint2(0u, 0u);
+  }
+  if (threadIdx.x < 32) warp_ss[threadIdx.x] = 0.f;
+  griddep_wait();   // may have been scheduled under the previous kernel's tail: nothing it writes is read before this
+  float4 v[NV];
+  uint2 r[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int c = (threadIdx.x + k * blockDim.x) * 4;
+    v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    r[k] = make_uint2(0u, 0u);
+    if (c < d) {
+      if (res) r[k] = *reinterpret_cast<const uint2*>(res + row0 + c);
+      for (int s0 = 0; s0 < splits; s0 += 8) {
+        float4 a[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (s0 + i < splits) a[i] = *reinterpret_cast<const float4*>(parts + (s0 + i) * stride + row0 + c);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (s0 + i < splits) { v[k].x += a[i].x; v[k].y += a[i].y; v[k].z += a[i].z; v[k].w += a[i].w; }
+      }
+    }
+  }
+  __syncthreads();                                 // warp_ss is cleared
   float ss = 0.f;
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    const int i = threadIdx.x + k * 256;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) v[k][e] = 0.f;
-    if (i < nvec) {
-      load_partials8(parts, splits, stride, static_cast<size_t>(row) * d + i * 8, v[k]);
-      if (res) {
-        const uint4 r = reinterpret_cast<const uint4*>(res + static_cast<size_t>(row) * d)[i];
-        const uint32_t* pr = reinterpret_cast<const uint32_t*>(&r);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = unpack_bf16x2(pr[e]);
-          v[k][2 * e] += f.x; v[k][2 * e + 1] += f.y;
-        }
-      }
-      // the residual stream is kept in bf16: round here so the norm sees exactly what is stored
-      uint4 hv;
-      uint32_t* ph = reinterpret_cast<uint32_t*>(&hv);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        ph[e] = pack_bf16x2(v[k][2 * e], v[k][2 * e + 1]);
-        const float2 f = unpack_bf16x2(ph[e]);
-        v[k][2 * e] = f.x; v[k][2 * e + 1] = f.y;
-        ss += f.x * f.x + f.y * f.y;
-      }
-      if (h_out) reinterpret_cast<uint4*>(h_out + static_cast<size_t>(row) * d)[i] = hv;
+    const int c = (threadIdx.x + k * blockDim.x) * 4;
+    if (res) {
+      const float2 r0 = unpack_bf16x2(r[k].x), r1 = unpack_bf16x2(r[k].y);
+      v[k].x += r0.x; v[k].y += r0.y; v[k].z += r1.x; v[k].w += r1.y;
+    }
+    // the residual stream is kept in bf16: round here so the norm sees exactly what is stored
+    const uint2 hv = make_uint2(pack_bf16x2(v[k].x, v[k].y), pack_bf16x2(v[k].z, v[k].w));
+    const float2 h0 = unpack_bf16x2(hv.x), h1 = unpack_bf16x2(hv.y);
+    v[k] = make_float4(h0.x, h0.y, h1.x, h1.y);
+    if (c < d) {
+      ss += h0.x * h0.x + h0.y * h0.y + h1.x * h1.x + h1.y * h1.y;
+      if (h_out) *reinterpret_cast<uint2*>(h_out + row0 + c) = hv;
     }
   }
   ss = warp_sum(ss);
   if ((threadIdx.x & 31) == 0) warp_ss[threadIdx.x >> 5] = ss;
   __syncthreads();
-  float tot = 0.f;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) tot += warp_ss[k];
+  const float tot = warp_sum(warp_ss[threadIdx.x & 31]);
   const float rstd = rsqrtf(tot / static_cast<float>(d) + eps);
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    const int i = threadIdx.x + k * 256;
-    if (i < nvec) {
-      const uint4 wv = reinterpret_cast<const uint4*>(w)[i];
-      const uint32_t* pw = reinterpret_cast<const uint32_t*>(&wv);
-      uint4 o;
-      uint32_t* po = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 b = unpack_bf16x2(pw[e]);
-        po[e] = pack_bf16x2(v[k][2 * e] * rstd * b.x, v[k][2 * e + 1] * rstd * b.y);
-      }
-      reinterpret_cast<uint4*>(y + static_cast<size_t>(row) * d)[i] = o;
+    const int c = (threadIdx.x + k * blockDim.x) * 4;
+    if (c < d) {
+      const float2 b0 = unpack_bf16x2(wv[k].x), b1 = unpack_bf16x2(wv[k].y);
+      *reinterpret_cast<uint2*>(y + row0 + c) =
+          make_uint2(pack_bf16x2(v[k].x * rstd * b0.x, v[k].y * rstd * b0.y), pack_bf16x2(v[k].z * rstd * b1.x, v[k].w * rstd * b1.y));
     }
   }
 }
@@ -703,10 +710,10 @@ extern "C" int rpeg_rmsnorm_fwd_partials(const float* parts, int splits, long lo
   if (T <= 0) return 0;
   const __nv_bfloat16 *rp = static_cast<const __nv_bfloat16*>(res), *wp = static_cast<const __nv_bfloat16*>(w);
   __nv_bfloat16 *hp = static_cast<__nv_bfloat16*>(h_out), *yp = static_cast<__nv_bfloat16*>(y);
-  const int nv = ((d >> 3) + 255) / 256;
-  if (nv == 1) launch_pdl(rmsnorm_fwd_partials_kernel<1>, dim3(T), dim3(256), 0, STREAM(stream), parts, splits, stride, rp, wp, hp, yp, d, eps);
-  else if (nv == 2) launch_pdl(rmsnorm_fwd_partials_kernel<2>, dim3(T), dim3(256), 0, STREAM(stream), parts, splits, stride, rp, wp, hp, yp, d, eps);
-  else if (nv <= 4) launch_pdl(rmsnorm_fwd_partials_kernel<4>, dim3(T), dim3(256), 0, STREAM(stream), parts, splits, stride, rp, wp, hp, yp, d, eps);
+  const int nv = (d / 4 + 1023) / 1024;
+  const dim3 block(((d / 4 + nv - 1) / nv + 31) & ~31);
+  if (nv == 1) launch_pdl(rmsnorm_fwd_partials_kernel<1>, dim3(T), block, 0, STREAM(stream), parts, splits, stride, rp, wp, hp, yp, d, eps);
+  else if (nv == 2) launch_pdl(rmsnorm_fwd_partials_kernel<2>, dim3(T), block, 0, STREAM(stream), parts, splits, stride, rp, wp, hp, yp, d, eps);
   else return -3;
   return LAUNCH_OK();
 }

@@ -181,3 +181,17 @@ def test_paged_decode_attn_blocks(cuda_device, h, hkv, nsplit):
         kk, vv = (t[table[i].long()].transpose(0, 1).reshape(hkv, -1, hd)[:, :n].double().repeat_interleave(h // hkv, 0) for t in (k, v))
         w = (torch.einsum("hd,hkd->hk", q[i].double().view(h, hd), kk) * hd ** -0.5).softmax(-1)
         assert _rel(out[i], torch.einsum("hk,hkd->hd", w, vv).reshape(-1)) < 2 ** -8
+
+
+@pytest.mark.parametrize("rows,d,splits", [(1, 8, 1), (3, 136, 9), (2, 4096, 9), (5, 4104, 17), (200, 2048, 2), (2, 8192, 8)])
+@pytest.mark.parametrize("residual", [True, False])
+def test_rmsnorm_partials_rows(cuda_device, rows, d, splits, residual):
+    g = torch.Generator(device=cuda_device).manual_seed(d)
+    parts = torch.randn(splits, rows, d, generator=g, device=cuda_device)
+    res = torch.randn(rows, d, generator=g, device=cuda_device).bfloat16() if residual else None
+    w = torch.randn(d, generator=g, device=cuda_device).bfloat16()
+    y, h = K.rmsnorm_fwd_partials(K.Partials(parts.view(-1), splits, rows, d), w, 1e-5, residual=res, want_sum=True)
+    total = parts.double().sum(0) + (res.double() if residual else 0)
+    assert _rel(h, total) < 2 ** -9
+    x = h.double()
+    assert _rel(y, x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-5) * w.double()) < 2 ** -9
