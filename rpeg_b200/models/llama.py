@@ -280,8 +280,7 @@ class LlamaModel:
             x, rstd1, h = K.rmsnorm_fwd(delta, p[f"l{i}.attn_norm"], cfg.rms_eps, residual=res, want_sum=True)
         qkv = K.gemm(x, p[f"l{i}.wqkv"], gate=gate)
         qkn = self._qk_norm(i, qkv, keep_acts) if cfg.qk_norm else None
-        K.rope_(qkv, ctx.pos, self.cos_t, self.sin_t, 0, cfg.n_heads, cfg.head_dim)
-        K.rope_(qkv, ctx.pos, self.cos_t, self.sin_t, cfg.q_width, cfg.n_kv_heads, cfg.head_dim)
+        K.rope_(qkv, ctx.pos, self.cos_t, self.sin_t, 0, cfg.n_heads + cfg.n_kv_heads, cfg.head_dim)      # q, then k
         attn, lse = K.flash_attn_fwd(qkv, 0, cfg.q_width, cfg.q_width + cfg.kv_width, ctx.cu_seqlens, ctx.max_seqlen,
                                      cfg.n_heads, cfg.n_kv_heads, cfg.head_dim)
         o = K.gemm(attn, p[f"l{i}.wo"])
@@ -336,8 +335,7 @@ class LlamaModel:
             x, rstd1, _ = K.rmsnorm_fwd(h, p[f"l{i}.attn_norm"], cfg.rms_eps)
             qkv = K.gemm(x, p[f"l{i}.wqkv"])
             qkn = self._qk_norm(i, qkv, True) if cfg.qk_norm else None
-            K.rope_(qkv, ctx.pos, self.cos_t, self.sin_t, 0, cfg.n_heads, cfg.head_dim)
-            K.rope_(qkv, ctx.pos, self.cos_t, self.sin_t, cfg.q_width, cfg.n_kv_heads, cfg.head_dim)
+            K.rope_(qkv, ctx.pos, self.cos_t, self.sin_t, 0, cfg.n_heads + cfg.n_kv_heads, cfg.head_dim)      # q, then k
             attn, lse = K.flash_attn_fwd(qkv, 0, cfg.q_width, cfg.q_width + cfg.kv_width, ctx.cu_seqlens,
                                          ctx.max_seqlen, cfg.n_heads, cfg.n_kv_heads, cfg.head_dim)
             o = K.gemm(attn, p[f"l{i}.wo"])
@@ -366,8 +364,7 @@ class LlamaModel:
         d_qkv = K.flash_attn_bwd(qkv, 0, cfg.q_width, cfg.q_width + cfg.kv_width, attn, d_attn, lse, ctx.cu_seqlens,
                                  ctx.max_seqlen, cfg.n_heads, cfg.n_kv_heads, cfg.head_dim)
         del d_attn, attn, qkv
-        K.rope_(d_qkv, ctx.pos, self.cos_t, self.sin_t, 0, cfg.n_heads, cfg.head_dim, backward=True)
-        K.rope_(d_qkv, ctx.pos, self.cos_t, self.sin_t, cfg.q_width, cfg.n_kv_heads, cfg.head_dim, backward=True)
+        K.rope_(d_qkv, ctx.pos, self.cos_t, self.sin_t, 0, cfg.n_heads + cfg.n_kv_heads, cfg.head_dim, backward=True)      # q, then k
         if cfg.qk_norm:
             pre, rq, rk = qkn
             for name, col0, nh, r in (("q_norm", 0, cfg.n_heads, rq), ("k_norm", cfg.q_width, cfg.n_kv_heads, rk)):

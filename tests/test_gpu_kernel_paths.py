@@ -183,6 +183,23 @@ def test_paged_decode_attn_blocks(cuda_device, h, hkv, nsplit):
         assert _rel(out[i], torch.einsum("hk,hkd->hd", w, vv).reshape(-1)) < 2 ** -8
 
 
+@pytest.mark.parametrize("t,heads,hd,col0,off", [(1, 1, 16, 0, 0), (5, 3, 128, 8, 0), (67, 9, 128, 0, 0), (33, 4, 48, 16, 0), (9, 5, 64, 4, 0), (9, 5, 64, 0, 4), (7, 2, 20, 0, 0)])
+@pytest.mark.parametrize("backward", [False, True])
+def test_rope_widths(cuda_device, t, heads, hd, col0, off, backward):
+    g = torch.Generator(device=cuda_device).manual_seed(t)
+    buf = torch.randn(t, (col0 + heads * hd + off + 15) // 8 * 8, generator=g, device=cuda_device).bfloat16()
+    view, want = buf[:, off:], buf.double().clone()
+    cos, sin = K.rope_tables(200, hd, 10000.0, cuda_device, 1.0)
+    pos = torch.randint(0, 200, (t,), generator=g, device=cuda_device, dtype=torch.int32)
+    c, s = (x[pos.long()].double()[:, None] for x in (cos, sin))
+    part = want[:, off + col0:off + col0 + heads * hd].reshape(t, heads, hd)
+    a, b = part[..., : hd // 2], part[..., hd // 2:]
+    s = -s if backward else s
+    want[:, off + col0:off + col0 + heads * hd] = torch.cat([a * c - b * s, b * c + a * s], -1).reshape(t, -1)
+    K.rope_(view, pos, cos, sin, col0, heads, hd, backward=backward)
+    assert _rel(buf, want) < 2 ** -9
+
+
 @pytest.mark.parametrize("rows,d,splits", [(1, 8, 1), (3, 136, 9), (2, 4096, 9), (5, 4104, 17), (200, 2048, 2), (2, 8192, 8)])
 @pytest.mark.parametrize("residual", [True, False])
 def test_rmsnorm_partials_rows(cuda_device, rows, d, splits, residual):
