@@ -52,8 +52,14 @@ moe_route_kernel(const float* __restrict__ logits, int splits, long long stride,
   float mx = -INFINITY;
   for (int e = lane; e < E; e += 32) {
     float z = lr[e];
-#pragma unroll 8
-    for (int s = 1; s < splits; ++s) z += lr[s * stride + e];
+    for (int s0 = 1; s0 < splits; s0 += 16) {              // 16 slabs in flight
+      float a[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) a[i] = s0 + i < splits ? lr[(s0 + i) * stride + e] : 0.f;
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (s0 + i < splits) z += a[i];
+    }
     sc[e] = z;
     mx = fmaxf(mx, z);
   }
