@@ -379,6 +379,23 @@ int make_tmap_bf16_2d(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_
   return r == CUDA_SUCCESS ? 0 : -11;
 }
 
+// 5-D bf16 tensor map; strides (of dimensions 1 to 4) in elements.
+int make_tmap_bf16_5d(CUtensorMap* out, const void* ptr, const uint64_t* dims, const uint64_t* strides, const uint32_t* box) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (fn == nullptr) return -10;
+  cuuint64_t d[5], st[4];
+  cuuint32_t b[5], estr[5];
+  for (int i = 0; i < 5; ++i) {
+    d[i] = dims[i];
+    b[i] = box[i];
+    estr[i] = 1;
+    if (i < 4) st[i] = strides[i] * 2;
+  }
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(ptr), d, st, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -11;
+}
+
 // fp32 tensor map of an output, 128-byte swizzle: d0 contiguous elements, d1 rows of `ld1` elements and, if rank is 3, d2 slabs of `ld2`; boxes
 // of b0 (32: one swizzle row) x b1 (x 1) elements.
 int make_tmap_f32_3d(CUtensorMap* out, void* ptr, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t ld1, uint64_t ld2, uint32_t b0, uint32_t b1,

@@ -384,6 +384,10 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 int make_tmap_bf16_2d(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner,
                       uint32_t box_outer);
 
+// moe_pair.cu
+int moe_pair(const void* A, long long a_rows_total, const void* X, const void* B, void* C, const int* seg_off, int n_routed, int n_shared,
+             int seg_rows, int N, int K, int lda, int ldx, int ldb, int ldc, int act, int num_sms, int* status, cudaStream_t stream);
+
 template <int BN, int ACT>
 static int launch_moe_gemm(const CUtensorMap& ta, const CUtensorMap& tx, const CUtensorMap& tb, void* C, const int* seg_off, int n_routed,
                            int n_shared, int seg_rows, int from_x, int N, int K, int ldc, int a_rows, long long max_tiles, int num_sms,
@@ -453,6 +457,15 @@ extern "C" int rpeg_moe_gemm(const void* A, long long a_rows_total, const void* 
   const long long active = choices < n_routed ? choices : n_routed;
   const long long m_tiles = choices / MG_BM + active + static_cast<long long>(n_shared) * ((seg_rows + MG_BM - 1) / MG_BM);
   int bn = bn_hint;
+  if (bn == 0) {
+    // Prompts: pairs of CTAs with tiles as high as a segment's rows ask for (moe_pair.cu), once experts have about 160 rows and there are six
+    // items a pair, with estimated halves for the last tiles (64 experts, 1024 x 4096 gated: 96 rows each 193 us either way, 192 rows 229 and 210
+    // us, 750 rows 683 and 607 us; few items, 8192 rows of 32 experts into 1024 columns: 71 us here, 79 us there).
+    const long long f_tiles = act == FF_SWIGLU ? (N + 127) / 128 : (N + 255) / 256;
+    const long long items = (choices / 256 + n_routed / 2 + static_cast<long long>(n_shared) * ((seg_rows + 255) / 256)) * f_tiles;
+    if (choices >= 160ll * n_routed && items >= 6ll * (num_sms / 2) && (act != FF_SWIGLU || (N & 15) == 0))
+      return moe_pair(A, a_rows_total, X, B, C, seg_off, n_routed, n_shared, seg_rows, N, K, lda, ldx, ldb, ldc, act, num_sms, status, STREAM(stream));
+  }
   if (bn == 0) {
     // widest tile that still gives every SM one, unless it wastes much more of the last column tile than a narrower one
     bn = 256;

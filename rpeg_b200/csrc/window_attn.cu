@@ -172,9 +172,11 @@ rows_attn_kernel(const RowsAttn a) {
   auto fetch = [&](int pg, int st) {
     const size_t off = (static_cast<size_t>(pt[pg]) * a.Hkv + hk) * WPAGE * dp;
     uint8_t* dst = ra_smem + static_cast<size_t>(st) * 2 * block_bytes;
-    mbar_expect_tx(&full_bar[st], 2 * block_bytes);
-    bulk_load(dst, kc + off, block_bytes, &full_bar[st]);
-    bulk_load(dst + block_bytes, vc + off, block_bytes, &full_bar[st]);
+    // nothing behind the row's last key: a row of 150 keys reads 2.3 pages, not three
+    const uint32_t bytes = static_cast<uint32_t>(min(WPAGE, L - pg * WPAGE) * dp * sizeof(T));
+    mbar_expect_tx(&full_bar[st], 2 * bytes);
+    bulk_load(dst, kc + off, bytes, &full_bar[st]);
+    bulk_load(dst + block_bytes, vc + off, bytes, &full_bar[st]);
   };
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) mbar_init(&full_bar[s], 1);

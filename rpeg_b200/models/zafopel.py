@@ -236,7 +236,7 @@ class ZafopelModel(ServedDecoder):
 
     prefill_spans = True
     KERNEL_SOURCES = ("gemm.cu", "gemm_pair.cu", "generate.cu", "loss.cu", "stream_update.cu", "latent.cu", "latent_decode.cu", "latent_prefill.cu", "head_gemm.cu",
-                      "moe.cu", "gemm_f32.cu")
+                      "moe.cu", "moe_pair.cu", "gemm_f32.cu")
 
     def __init__(self, cfg: ZafopelConfig, device, *, dtype: torch.dtype = torch.bfloat16, seed: Optional[int] = 0, trainable: bool = False):
         """``seed=None`` leaves the weights zero (a checkpoint is about to be loaded)."""

@@ -212,3 +212,28 @@ def test_rmsnorm_partials_rows(cuda_device, rows, d, splits, residual):
     assert _rel(h, total) < 2 ** -9
     x = h.double()
     assert _rel(y, x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-5) * w.double()) < 2 ** -9
+
+
+@pytest.mark.parametrize("e,top,shared,n,k,act", [(5, 2, 0, 4616, 72, "none"), (3, 1, 2, 4608, 136, "gelu"), (7, 3, 1, 3080, 64, "relu2"), (5, 2, 1, 2320, 200, "swiglu"),
+                                                  (0, 0, 1, 10240, 64, "gelu")])
+def test_moe_gemm_pair_tiles(cuda_device, e, top, shared, n, k, act):
+    t, dev = 3000, cuda_device
+    g = torch.Generator(device=dev).manual_seed(n)
+    x = torch.randn(t, k, generator=g, device=dev).bfloat16()
+    w = (torch.randn(e + shared, n * (2 if act == "swiglu" else 1), k, generator=g, device=dev) / k ** 0.5).bfloat16()
+    f = {"none": lambda z: z, "gelu": torch.nn.functional.gelu, "relu2": lambda z: torch.relu(z) ** 2,
+         "swiglu": lambda z: torch.nn.functional.silu(z[:, :n]) * z[:, n:]}[act]
+    if not e:
+        assert _rel(K.ff_first(x, w[0], act), f(x.double() @ w[0].double().T)) < 2 ** -8
+        return
+    logits = torch.randn(t, e, generator=g, device=dev)
+    logits[:, 0] -= 1.5                                              # experts of unlike size
+    counts = torch.zeros(e, dtype=torch.int32, device=dev)
+    ids, wts, ticket = K.moe_route(logits, e, top, counts)
+    r = K.moe_dispatch(x, ids, wts, ticket, counts, e)
+    got = K.moe_gemm(r.x_sorted, w, r, e, shared, shared_x=x if shared else None, act=act)
+    for i in range(e):
+        tok, col = (ids == i).nonzero(as_tuple=True)
+        assert _rel(got[r.row_of[tok, col].long()], f(x[tok].double() @ w[i].double().T)) < 2 ** -8
+    for s in range(shared):
+        assert _rel(got[t * top + s * t:t * top + (s + 1) * t], f(x.double() @ w[e + s].double().T)) < 2 ** -8
