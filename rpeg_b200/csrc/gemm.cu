@@ -704,7 +704,11 @@ extern "C" int rpeg_gemm_bf16_partials(const void* A, const void* B, int M, int 
     *k_splits_out = plan.splits;
     return gemm_pair(A, B, workspace, M, N, K, lda, ldb, N, 0, 0, 1, 0, plan, g_num_sms, pdl_enabled(), status, stream);
   }
-  const int bn = N >= 256 ? 256 : (N >= 128 ? 128 : (N >= 64 ? 64 : 32));
+  // Few rows: the wide tile, fewest reads of A. From 33 rows on the slabs weigh as much as that, and the narrow tile needs half as many to fill
+  // the SMs and stores one half while it multiplies the other (with the kernel that adds the slabs; 128 rows: 4096 x 4096 18.5 us at 256,
+  // 15.6 us at 128 columns, 12288 x 4096 34.7 and 30.9; 64 rows: 5120 x 4096 18.5 and 16.8, but 22016 x 4096 43.5 and 44.1; 16 rows: 12.2 and 12.7).
+  const bool narrow = M > 32 && (M > 64 || N <= 16384);
+  const int bn = N >= 256 && !narrow ? 256 : (N >= 128 ? 128 : (N >= 64 ? 64 : 32));
   const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);
   const int num_kb = (K + BK - 1) / BK;
   const double block_bytes = static_cast<double>(g_num_sms) * BK * (bn + BM) * 2.0;
@@ -717,7 +721,7 @@ extern "C" int rpeg_gemm_bf16_partials(const void* A, const void* B, int M, int 
     if (workspace_elems / per_split < sp) break;
     const int waves = (tiles * sp + g_num_sms - 1) / g_num_sms;
     // the consumer reads every partial once; no separate reduction pass writes and re-reads them
-    const double cost = waves * (kb_per + 2.0) + sp * per_split * 8.0 / block_bytes;
+    const double cost = waves * (kb_per + 2.0) + sp * per_split * (narrow ? 16.0 : 8.0) / block_bytes;
     if (cost < best - 1e-9) { best = cost; want = sp; }
   }
   const int kb_per = (num_kb + want - 1) / want;

@@ -130,9 +130,9 @@ def test_gemm_swiglu_pair_tiles(cuda_device, m, f, k):
     assert _rel(K.gemm_swiglu(x, w), torch.nn.functional.silu(gate) * up) < 2 ** -8
 
 
-@pytest.mark.parametrize("m", [129, 200, 256])
+@pytest.mark.parametrize("m", [32, 33, 64, 65, 128, 129, 200, 256])
 @pytest.mark.parametrize("n,k", [(136, 264), (1288, 4096), (12288, 1032)])
-def test_gemm_partials_of_two_row_tiles(cuda_device, m, n, k):
+def test_gemm_partials_rows(cuda_device, m, n, k):
     g = torch.Generator(device=cuda_device).manual_seed(m)
     a, b = (torch.randn(r, k, generator=g, device=cuda_device).bfloat16() for r in (m, n))
     want = a.double() @ b.double().T
