@@ -750,7 +750,7 @@ paged_decode_attn_shared_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, c
         asm volatile("bar.sync 1, 128;" ::: "memory");     // `red` may be rewritten by the next tile
         if (need) {                                        // the same decision in every thread: all hold the same m and tmax
           // PV of the previous tile must have landed before O is rescaled. Having seen s_full of this tile, the waiter
-          // is at most one completion behind on the barrier of that parity (see flash_attn_fwd_kernel).
+          // is at most one completion behind on the barrier of that parity: every MMA issued before this tile's Q K^T is complete.
           if (!__all_sync(0xffffffffu, mbar_wait(&pv_done[(t - 1) & 1], static_cast<uint32_t>((t - 1) >> 1) & 1u, abort_flag, status, 821))) { ok = false; break; }
           tc_fence_after_sync();
           float alpha[GROUP_MAX];

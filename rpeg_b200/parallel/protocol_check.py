@@ -291,8 +291,8 @@ def staleness_programs(tau: int, steps: int, *, slots: Optional[int] = None, n_g
 
 # ---------------------------------------------------------------------------------------------- the suite
 def flash_fwd_programs(n_tiles: int, rescale: Sequence[int] = (), *, pv_barriers: int = 2, in_order_consume: bool = False) -> List[Program]:
-    """The mbarrier pipeline of ``flash_attn_fwd_kernel`` (csrc/flash_attn.cu) for one CTA and ``n_tiles`` KV tiles, as
-    three agents: the MMA-issuing thread, the tensor pipe (completes the issued MMAs in issue order, each at an
+    """The mbarrier pipeline of an attention kernel with double-buffered scores (``paged_decode_attn_shared_tc_kernel`` in
+    csrc/decode_attn.cu; csrc/flash_attn.cu worked this way before it took two query tiles) for one CTA and ``n_tiles`` KV tiles, as three agents: the MMA-issuing thread, the tensor pipe (completes the issued MMAs in issue order, each at an
     arbitrary later time, and performs their commits) and one softmax warp. ``rescale``: the tiles at which the warp
     rescales O and therefore waits for the previous P*V product. Words count completed phases of a barrier.
 
