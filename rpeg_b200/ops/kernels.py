@@ -49,6 +49,12 @@ def check_status() -> None:
         raise KernelWaitTimeout(f"device wait timed out: code={vals[0]} where={vals[1]} block={vals[2]} extra={vals[3]}")
 
 
+def _overlap(a: torch.Tensor, b: torch.Tensor) -> bool:
+    """Whether the address ranges of two matrices of contiguous rows meet."""
+    (a0, a1), (b0, b1) = ((t.data_ptr(), t.data_ptr() + ((t.shape[0] - 1) * t.stride(0) + t.shape[1]) * t.element_size()) for t in (a, b))
+    return a0 < b1 and b0 < a1
+
+
 def _req(t: torch.Tensor, dtype: torch.dtype, name: str) -> None:
     if not t.is_cuda or t.dtype != dtype:
         raise TypeError(f"{name}: expected a CUDA {dtype} tensor, got {t.dtype} on {t.device}")
@@ -587,13 +593,18 @@ def flash_attn_fwd(qkv, q_col0, k_col0, v_col0, cu_seqlens, max_seqlen, n_heads,
 def flash_attn_bwd(qkv, q_col0, k_col0, v_col0, out, dout, lse, cu_seqlens, max_seqlen, n_heads, n_kv_heads, head_dim,
                    scale=None, dqkv: torch.Tensor | None = None) -> torch.Tensor:
     """Gradient of ``flash_attn_fwd`` w.r.t. the packed qkv buffer (same column blocks). ``dqkv``
-    may be passed in to reuse a buffer; columns outside the three blocks are left untouched."""
+    may be passed in to reuse a buffer, ``qkv`` itself too; columns outside the three blocks are left untouched."""
     T = qkv.shape[0]
     if _chk.active():
         _chk.packed_sequences("rpeg_flash_attn_bwd", cu_seqlens, T, max_seqlen)
     scale = 1.0 / math.sqrt(head_dim) if scale is None else scale
     if dqkv is None:
         dqkv = torch.empty_like(qkv)
+    elif _overlap(dqkv, qkv):
+        # dK and dV are written before the second pass reads K and V for dQ: the passes read a copy
+        copy = torch.empty((T, qkv.stride(0)), dtype=qkv.dtype, device=qkv.device)
+        copy[:, : qkv.shape[1]] = qkv
+        qkv = copy
     dvec = torch.empty((n_heads, T), dtype=torch.float32, device=qkv.device)
     check(lib().rpeg_flash_attn_bwd(qkv.data_ptr(), qkv.stride(0), q_col0, k_col0, v_col0, out.data_ptr(),
                                     dout.data_ptr(), lse.data_ptr(), cu_seqlens.data_ptr(), cu_seqlens.numel() - 1,

@@ -102,6 +102,27 @@ def test_flash_attn_bwd_tiles(cuda_device, lens, H, Hkv):
         assert float((got[:, lo:hi].double() - want).norm()) < 1e-2 * float(want.norm()) + 2e-3
 
 
+@pytest.mark.parametrize("lens", [[65, 300], [700]])
+@pytest.mark.parametrize("H,Hkv", [(2, 2), (4, 1)])
+def test_flash_attn_bwd_in_place(cuda_device, lens, H, Hkv):
+    """A gradient buffer that is ``qkv`` itself, or overlaps it, gets what a buffer of its own gets; other columns stay as they are."""
+    hd, T, dev = 128, sum(lens), cuda_device
+    g = torch.Generator(device=dev).manual_seed(T + H)
+    kc, vc, width = H * hd, (H + Hkv) * hd, (H + 2 * Hkv) * hd
+    store = torch.randn(T + 3, width + 8, generator=g, device=dev).bfloat16()
+    qkv = store[:T]
+    dout = torch.randn(T, H * hd, generator=g, device=dev).bfloat16()
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), device=dev, dtype=torch.int32)
+    out, lse = K.flash_attn_fwd(qkv, 0, kc, vc, cu, max(lens), H, Hkv, hd)
+    want = K.flash_attn_bwd(qkv, 0, kc, vc, out, dout, lse, cu, max(lens), H, Hkv, hd)
+    for first in (3, 0):
+        held = store.clone()
+        got = K.flash_attn_bwd(held[:T], 0, kc, vc, out, dout, lse, cu, max(lens), H, Hkv, hd, dqkv=held[first:first + T])
+        assert got.data_ptr() == held[first].data_ptr()
+        assert torch.equal(got[:, :width], want[:, :width])
+        assert torch.equal(held[:first], store[:first]) and torch.equal(got[:, width:], store[first:first + T, width:])
+
+
 # bf16 operands are exact in fp32, so an fp32 result is off by sums alone; a bf16 result by half a unit in its last place (2^-9) at most
 @pytest.mark.parametrize("m,n,k", [(1, 8, 1024), (129, 136, 1032), (257, 264, 1096), (300, 4096, 1024), (1000, 5000, 520), (2304, 8200, 72), (5000, 1288, 64)])
 @pytest.mark.parametrize("trans_a,trans_b", [(False, False), (True, False), (False, True), (True, True)])
