@@ -219,7 +219,7 @@ paged_decode_attn_kernel(const __nv_bfloat16* __restrict__ q, int ldq, int q_col
                          const int* __restrict__ page_table, int max_pages, const int* __restrict__ seq_lens,
                          __nv_bfloat16* __restrict__ out, float* __restrict__ partial, int H, int Hkv,
                          int nsplit, float scale_log2, const int* __restrict__ row_key0, int slot_base, int nslots,
-                         int* __restrict__ arrive) {
+                         int* __restrict__ arrive, int* status) {
   griddep_launch();
   griddep_wait();   // may have been scheduled under the previous kernel's tail: nothing is read or written before this
   extern __shared__ __align__(128) uint8_t kv_sm[];
@@ -283,7 +283,7 @@ paged_decode_attn_kernel(const __nv_bfloat16* __restrict__ q, int ldq, int q_col
     const int nk = min(DA_KEYS, L - blk * DA_KEYS) - grp * 8;   // valid keys of this group (may be <= 0)
     const uint4* kp = reinterpret_cast<const uint4*>(k_sm) + grp * 8 * (HD / 8) + c;      // this lane's chunk of the group's rows
     const uint4* vp = reinterpret_cast<const uint4*>(v_sm) + grp * 8 * (HD / 8) + c;
-    if (!__all_sync(0xffffffffu, mbar_wait(&bar[0], phase, &abort_word, nullptr, 0))) break;
+    if (!__all_sync(0xffffffffu, mbar_wait(&bar[0], phase, &abort_word, status, 830))) break;
     float part[8];
     if (nk >= 8) {
 #pragma unroll
@@ -307,7 +307,7 @@ paged_decode_attn_kernel(const __nv_bfloat16* __restrict__ q, int ldq, int q_col
 #pragma unroll
     for (int k = 0; k < 8; ++k) acc[k] *= alpha;
     m = nm;
-    if (!__all_sync(0xffffffffu, mbar_wait(&bar[1], phase, &abort_word, nullptr, 0))) break;
+    if (!__all_sync(0xffffffffu, mbar_wait(&bar[1], phase, &abort_word, status, 831))) break;
     if (nk >= 8) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) axpy8(acc, __shfl_sync(0xffffffffu, p, grp * 16 + j), vp[j * (HD / 8)]);
@@ -321,7 +321,7 @@ paged_decode_attn_kernel(const __nv_bfloat16* __restrict__ q, int ldq, int q_col
     __syncwarp();
     if (lane == 0 && next < blk1) fetch(next, next_page, vcache, v_sm, &bar[1]);
   }
-  if (*static_cast<volatile int*>(&abort_word)) {       // a copy that never arrived (there is no status word here): the row becomes NaN
+  if (*static_cast<volatile int*>(&abort_word)) {       // a copy that never arrived (in the status word): the row becomes NaN
     __nanosleep(200000);
     m = 0.f;
     l = 1.f / 32.f;
@@ -897,7 +897,7 @@ extern "C" long long rpeg_decode_attn_scratch_bytes(int B, int H, int nsplit) {
 extern "C" int rpeg_paged_decode_attn(const void* q, int ldq, int q_col0, const void* kcache, const void* vcache,
                                       const int* page_table, int max_pages, const int* seq_lens, void* out,
                                       float* scratch, int B, int H, int Hkv, int hd, int nsplit, float scale,
-                                      void* stream) {
+                                      int* status, void* stream) {
   if (hd != HD || H % Hkv != 0) return -2;
   if (nsplit < 1 || nsplit > 64) return -3;
   if (nsplit > 1 && scratch == nullptr) return -4;
@@ -907,7 +907,7 @@ extern "C" int rpeg_paged_decode_attn(const void* q, int ldq, int q_col0, const 
   launch_pdl(paged_decode_attn_kernel, dim3(H, B, nsplit), dim3(128), DA_SMEM, STREAM(stream), 
       static_cast<const __nv_bfloat16*>(q), ldq, q_col0, static_cast<const __nv_bfloat16*>(kcache),
       static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages, seq_lens,
-      static_cast<__nv_bfloat16*>(out), scratch, H, Hkv, nsplit, scale_log2, static_cast<const int*>(nullptr), 0, nsplit, arrive);
+      static_cast<__nv_bfloat16*>(out), scratch, H, Hkv, nsplit, scale_log2, static_cast<const int*>(nullptr), 0, nsplit, arrive, status);
   if (nsplit > 1 && arrive == nullptr)
     launch_pdl(decode_combine_kernel, dim3(dim3(H, B)), dim3(HD), 0, STREAM(stream), scratch, static_cast<__nv_bfloat16*>(out), H, nsplit);
   return LAUNCH_OK();
@@ -922,7 +922,7 @@ extern "C" int rpeg_paged_decode_attn_grouped(const void* q, int ldq, int q_col0
                                               const int* page_table, int max_pages, const int* seq_lens, void* out,
                                               float* scratch, int B, int H, int Hkv, int hd, int nsplit, float scale,
                                               const int* group_rows, const int* group_shared, const int* row_key0,
-                                              void* stream) {
+                                              int* status, void* stream) {
   if (hd != HD || H % Hkv != 0) return -2;
   if (nsplit < 1 || nsplit > 63) return -3;
   if (scratch == nullptr || group_rows == nullptr || group_shared == nullptr || row_key0 == nullptr) return -4;
@@ -935,7 +935,7 @@ extern "C" int rpeg_paged_decode_attn_grouped(const void* q, int ldq, int q_col0
              group_rows, group_shared, scratch, H, Hkv, nslots, scale_log2);
   launch_pdl(paged_decode_attn_kernel, dim3(H, B, nsplit), dim3(128), DA_SMEM, STREAM(stream), static_cast<const __nv_bfloat16*>(q), ldq,
              q_col0, static_cast<const __nv_bfloat16*>(kcache), static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages,
-             seq_lens, static_cast<__nv_bfloat16*>(out), scratch, H, Hkv, nsplit, scale_log2, row_key0, 1, nslots, arrive);
+             seq_lens, static_cast<__nv_bfloat16*>(out), scratch, H, Hkv, nsplit, scale_log2, row_key0, 1, nslots, arrive, status);
   if (arrive == nullptr)
     launch_pdl(decode_combine_kernel, dim3(H, B), dim3(HD), 0, STREAM(stream), scratch, static_cast<__nv_bfloat16*>(out), H, nslots);
   return LAUNCH_OK();
@@ -985,7 +985,7 @@ extern "C" int rpeg_paged_decode_attn_grouped_tc(const void* q, int ldq, int q_c
              nslots, scale_log2, status);
   launch_pdl(paged_decode_attn_kernel, dim3(H, B, nsplit), dim3(128), DA_SMEM, STREAM(stream), static_cast<const __nv_bfloat16*>(q), ldq,
              q_col0, static_cast<const __nv_bfloat16*>(kcache), static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages,
-             seq_lens, static_cast<__nv_bfloat16*>(out), scratch, H, Hkv, nsplit, scale_log2, row_key0, 1, nslots, arrive);
+             seq_lens, static_cast<__nv_bfloat16*>(out), scratch, H, Hkv, nsplit, scale_log2, row_key0, 1, nslots, arrive, status);
   if (arrive == nullptr)
     launch_pdl(decode_combine_kernel, dim3(H, B), dim3(HD), 0, STREAM(stream), scratch, static_cast<__nv_bfloat16*>(out), H, nslots);
   return LAUNCH_OK();
@@ -999,8 +999,10 @@ extern "C" int rpeg_paged_decode_attn_grouped_tc(const void* q, int ldq, int q_c
 namespace {
 constexpr long long STATIC_PARTIAL_FLOATS = static_cast<long long>(RPEG_DECODE_STATIC_MAX_PARTIALS) * (HD + 2);
 static __device__ __align__(256) float g_decode_static_scratch[STATIC_PARTIAL_FLOATS];
+static __device__ int g_decode_static_status[4];
 constexpr int STATIC_MAX_DEVICES = 64;
 float* g_static_scratch_ptr[STATIC_MAX_DEVICES] = {nullptr};
+int* g_static_status_ptr[STATIC_MAX_DEVICES] = {nullptr};
 }  // namespace
 
 extern "C" const char* rpeg_static_entry_strerror(int code) {
@@ -1026,19 +1028,29 @@ extern "C" int rpeg_paged_decode_attn_static(const void* q, int ldq, int q_col0,
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= STATIC_MAX_DEVICES) return RPEG_STATIC_ERR_SETUP;
   if (g_static_scratch_ptr[dev] == nullptr) {
-    // set-up, once per device: the array's address in this device's copy of the module
+    // set-up, once per device: the arrays' addresses in this device's copy of the module
     float* p = nullptr;
-    if (cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_decode_static_scratch) != cudaSuccess || p == nullptr)
+    int* st = nullptr;
+    if (cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_decode_static_scratch) != cudaSuccess || p == nullptr ||
+        cudaGetSymbolAddress(reinterpret_cast<void**>(&st), g_decode_static_status) != cudaSuccess || st == nullptr)
       return RPEG_STATIC_ERR_SETUP;
+    g_static_status_ptr[dev] = st;
     g_static_scratch_ptr[dev] = p;
   }
   float* scratch = g_static_scratch_ptr[dev];
+  int* status = g_static_status_ptr[dev];
   const float scale_log2 = scale * 1.4426950408889634f;
   launch_pdl(paged_decode_attn_kernel, dim3(H, B, nsplit), dim3(128), DA_SMEM, STREAM(stream), 
       static_cast<const __nv_bfloat16*>(q), ldq, q_col0, static_cast<const __nv_bfloat16*>(kcache),
       static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages, seq_lens, static_cast<__nv_bfloat16*>(out),
-      scratch, H, Hkv, nsplit, scale_log2, static_cast<const int*>(nullptr), 0, nsplit, static_cast<int*>(nullptr));
+      scratch, H, Hkv, nsplit, scale_log2, static_cast<const int*>(nullptr), 0, nsplit, static_cast<int*>(nullptr), status);
   if (nsplit > 1)
     launch_pdl(decode_combine_kernel, dim3(dim3(H, B)), dim3(HD), 0, STREAM(stream), scratch, static_cast<__nv_bfloat16*>(out), H, nsplit);
   return cudaGetLastError() == cudaSuccess ? 0 : RPEG_STATIC_ERR_LAUNCH;
+}
+
+extern "C" int rpeg_decode_static_status(int* out) {
+  static const int clear[4] = {0, 0, 0, 0};
+  if (cudaMemcpyFromSymbol(out, g_decode_static_status, sizeof(clear)) != cudaSuccess) return RPEG_STATIC_ERR_SETUP;
+  return out[0] == 0 || cudaMemcpyToSymbol(g_decode_static_status, clear, sizeof(clear)) == cudaSuccess ? 0 : RPEG_STATIC_ERR_SETUP;
 }
