@@ -417,22 +417,17 @@ rmsnorm_fwd_partials_kernel(const float* __restrict__ parts, int splits, long lo
   __shared__ float warp_ss[32];
   const int row = blockIdx.x;
   const size_t row0 = static_cast<size_t>(row) * d;
-  uint2 wv[NV];
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {                   // no kernel of the step writes the weights
-    const int c = (threadIdx.x + k * blockDim.x) * 4;
-    wv[k] = c < d ? *reinterpret_cast<const uint2*>(w + c) : make_uint2(0u, 0u);
-  }
   if (threadIdx.x < 32) warp_ss[threadIdx.x] = 0.f;
-  griddep_wait();   // may have been scheduled under the previous kernel's tail: nothing it writes is read before this
+  griddep_wait();   // may have been scheduled under the previous kernel's tail: nothing is read or written before this
   float4 v[NV];
-  uint2 r[NV];
+  uint2 r[NV], wv[NV];
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
     const int c = (threadIdx.x + k * blockDim.x) * 4;
     v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    r[k] = make_uint2(0u, 0u);
+    r[k] = wv[k] = make_uint2(0u, 0u);
     if (c < d) {
+      wv[k] = *reinterpret_cast<const uint2*>(w + c);
       if (res) r[k] = *reinterpret_cast<const uint2*>(res + row0 + c);
       for (int s0 = 0; s0 < splits; s0 += 8) {
         float4 a[8];
