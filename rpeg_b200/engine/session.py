@@ -97,12 +97,11 @@ class Session:
             try:
                 ids = np.frombuffer(array("i", list(tokens)), dtype=np.int32)
                 low, high = int(ids.min()), int(ids.max())
-            except (TypeError, OverflowError):              # not plain 32-bit integers
-                low, high = min(tokens), max(tokens)
-                ids = np.asarray(list(tokens)).astype(np.int32) if 0 <= low and high < g.cfg.vocab else np.zeros(0, np.int32)
-            arrays.append(ids)
+            except (TypeError, OverflowError):              # not plain 32-bit integers: converted below, once they are in range
+                ids, low, high = None, min(tokens), max(tokens)
             if low < 0 or high >= g.cfg.vocab:
                 raise ValueError(f"request {rid!r} brings a token outside the vocabulary")
+            arrays.append(ids if ids is not None else torch.tensor(list(tokens), dtype=torch.int32).numpy())      # refuses what is no number
             if len(want) and (min(want) < 0 or max(want) >= len(tokens)):
                 raise ValueError(f"request {rid!r} wants a place outside its tokens")
             have = self.requests[rid].length if rid in self.requests else 0
