@@ -238,6 +238,30 @@ class Generator:
         dev = torch.from_numpy(buf).to(self.dev)
         return [dev[o:o + a.size] for o, a in zip(at, arrays)]
 
+    #: bytes of pages that one copy may hold in its buffer
+    COPY_BYTES = 64 << 20
+
+    def _copy_pages(self, src: Sequence[int], dst: Sequence[int]) -> None:
+        """Copy KV pages (all layers, K and V): page ``src[i]`` onto ``dst[i]``. Pages pass through a buffer of at most ``COPY_BYTES``, as many at a time
+        as it holds (32 prompts of eight rows, four Llama-7B layers: 16 pages, 64 MiB); a larger page is copied in place."""
+        uniform = len(set(self.geometry)) == 1 and self.geometry[0][1] == self.geometry[0][2]
+        if uniform:                                      # layers of one shape: a single strided copy
+            pages = self.kcache[0].shape[0]
+            caches = [self.kv_storage.view(2 * self.cfg.n_layers, pages, -1).transpose(0, 1)]
+        else:
+            caches = [c for c in (*self.kcache, *self.vcache) if c.numel()]      # a layer may keep no values, or nothing of its own
+        page_bytes = max((c[0].numel() * c.element_size() for c in caches), default=1)
+        at_once = min(16, self.COPY_BYTES // page_bytes)
+        if at_once < 2:
+            for s, d in zip(src, dst):
+                for c in caches:
+                    c[d].copy_(c[s])
+            return
+        for i in range(0, len(src), at_once):
+            s_idx, d_idx = (x.long() for x in self._upload([np.asarray(v[i:i + at_once], dtype=np.int32) for v in (src, dst)]))
+            for c in caches:
+                c[d_idx] = c[s_idx]
+
     def prefill_hidden(self, pieces: List[torch.Tensor], slots: List[int], starts: Optional[List[int]] = None):
         """Run one piece of tokens per slot through the model, each continuing at position ``starts[i]`` (0 without it),
         and store the K/V through the slots' page-table rows. Returns the hidden rows of all pieces and their offsets."""
@@ -467,20 +491,6 @@ class Generator:
             if idx:
                 self.page_table.view(-1)[torch.tensor(idx, dtype=torch.long, device=dev)] = 0
 
-        def copy_pages(src: List[int], dst: List[int]) -> None:
-            """Copy KV pages (all layers, K and V): page ``src[i]`` onto ``dst[i]``, a few at a time (the copy passes through a buffer)."""
-            for i in range(0, len(src), 16):
-                s_idx, d_idx = self._upload([np.asarray(v[i:i + 16], dtype=np.int32) for v in (src, dst)])
-                s_idx, d_idx = s_idx.long(), d_idx.long()
-                if len(set(self.geometry)) > 1 or self.geometry[0][1] != self.geometry[0][2]:
-                    for c in (*self.kcache, *self.vcache):
-                        if c.numel():                    # a layer may keep no values, or nothing of its own
-                            c[d_idx] = c[s_idx]
-                else:
-                    pages = self.kcache[0].shape[0]      # layers of one shape: a single strided copy
-                    flat = self.kv_storage.view(2 * self.cfg.n_layers, pages, -1)
-                    flat[:, d_idx] = flat[:, s_idx]
-
         while retired < N:
             free = [s for s in range(n) if slot_row[s] < 0]
             # admit in batches: a prefill call stalls decoding, so wait until several slots are free
@@ -548,14 +558,14 @@ class Generator:
                                 if g["tail"]:               # keep the prompt's ragged tail for the rows that come later
                                     src.append(slot_pages[s][0])
                                     dst.append(g["tail"])
-                        copy_pages(src, dst)
+                        self._copy_pages(src, dst)
                         src, dst = [], []
                         for r, s in zip(new_rows, new_slots):   # rows that alias an already prefilled prompt need its tail
                             g = groups.get(r // G)
                             if g is not None and g["tail"] and r not in at:
                                 src.append(g["tail"])
                                 dst.append(slot_pages[s][0])
-                        copy_pages(src, dst)
+                        self._copy_pages(src, dst)
                         place = [fresh.get(r // G, -1) if (r // G) in groups else at[r] for r in new_rows]
                         if min(place) >= 0:
                             row_logits = logits[self._upload([np.asarray(place, dtype=np.int32)])[0].long()]
