@@ -37,9 +37,9 @@ Program = List[Instr]
 #   ("add", loc, n)                atomic add (arrival counter)
 #   ("wait", loc, minimum)         blocks while the word is below `minimum` (an acquire spin; bounded on the device)
 #   ("expect", loc, value, what)   a read that must see exactly `value`; anything else is reported as a race
-#   ("pwait", loc, parity)         mbarrier.try_wait.parity: the word counts the barrier's completed phases; the wait
-#                                  passes while the CURRENT phase's parity differs from `parity`, i.e. it cannot tell a
-#                                  phase that completed from one that completed two phases ago
+#   ("pwait", loc, parity[, n])    mbarrier.try_wait.parity: the word counts the barrier's arrivals, n of which (1 without it)
+#                                  complete a phase; the wait passes while the CURRENT phase's parity differs from `parity`,
+#                                  i.e. it cannot tell a phase that completed from one that completed two phases ago
 #   ("check", loc, minimum, what)  an assertion: the word must have reached `minimum` (reported as a race otherwise)
 TORN = "torn"
 
@@ -99,7 +99,7 @@ def explore(name: str, programs: Sequence[Program], initial: Optional[Dict[Hasha
                 if cur == TORN or not isinstance(cur, int) or cur < ins[2]:
                     continue
             elif op == "pwait":
-                if (int(cur) & 1) == (int(ins[2]) & 1):
+                if (int(cur) // (ins[3] if len(ins) > 3 else 1)) & 1 == int(ins[2]) & 1:
                     continue
             elif op == "check":
                 if not isinstance(cur, int) or cur < ins[2]:
@@ -290,10 +290,10 @@ def staleness_programs(tau: int, steps: int, *, slots: Optional[int] = None, n_g
 
 
 # ---------------------------------------------------------------------------------------------- the suite
-def flash_fwd_programs(n_tiles: int, rescale: Sequence[int] = (), *, pv_barriers: int = 2, in_order_consume: bool = False) -> List[Program]:
-    """The mbarrier pipeline of an attention kernel with double-buffered scores (``paged_decode_attn_shared_tc_kernel`` in
-    csrc/decode_attn.cu; csrc/flash_attn.cu worked this way before it took two query tiles) for one CTA and ``n_tiles`` KV tiles, as three agents: the MMA-issuing thread, the tensor pipe (completes the issued MMAs in issue order, each at an
-    arbitrary later time, and performs their commits) and one softmax warp. ``rescale``: the tiles at which the warp
+def group_decode_programs(n_tiles: int, rescale: Sequence[int] = (), *, pv_barriers: int = 2, in_order_consume: bool = False) -> List[Program]:
+    """The mbarrier pipeline of ``paged_decode_attn_shared_tc_kernel`` (csrc/decode_attn.cu), one query tile with double-buffered scores, for one
+    work item of ``n_tiles`` key tiles, as three agents: the MMA-issuing thread, the tensor pipe (completes the issued MMAs in issue order, each
+    at an arbitrary later time, and performs their commits) and one softmax warp. ``rescale``: the tiles at which the warp
     rescales O and therefore waits for the previous P*V product. Words count completed phases of a barrier.
 
     ``pv_barriers = 2``: P*V of tile j commits to ``pv_done[j & 1]`` and the warp waits on the wanted tile's barrier
@@ -341,6 +341,183 @@ def flash_fwd_programs(n_tiles: int, rescale: Sequence[int] = (), *, pv_barriers
     return [mma, pipe, warp]
 
 
+class _Pipe:
+    """The tensor pipe as an agent: ``issue`` appends an operation's effects (its reads, writes and commits) and returns the issuer's step. Operations
+    are performed in issue order, each at an arbitrary time after it was issued."""
+
+    def __init__(self) -> None:
+        self.program: Program = []
+        self.issued = 0
+
+    def issue(self, effects: Sequence[Instr]) -> Instr:
+        self.issued += 1
+        self.program += [("wait", "issued", self.issued), *effects]
+        return ("add", "issued", 1)
+
+
+def flash_fwd_programs(je: Tuple[int, int], rescale: Sequence[int] = (), *, keep_k_for_both: bool = True, wait_first_half: bool = True) -> List[Program]:
+    """The mbarrier pipeline of ``flash_attn_fwd_kernel`` (csrc/flash_attn.cu) for one CTA: two query tiles ("units") over the same key tiles, unit u
+    sees the first ``je[u]`` of them (0: absent). Agents: the TMA thread, the MMA-issuing thread, the tensor pipe and a softmax group per unit. The
+    weights P lie over the scores S in TMEM. ``rescale``: tiles at which both groups rescale O in place; no barrier guards that, since the
+    commit behind a unit's next Q K^T also covers its P V before it.
+
+    Ingredients that tests take out: K stays until BOTH units have used it, and P V of a tile's first keys waits for their weights."""
+    n = max(je)
+    tma: Program = [("add", "q_full", 1)]
+    for j in range(n):
+        for what in ("k", "v"):
+            tma += [("pwait", (what + "_empty", j & 1), (j >> 1 & 1) ^ 1), ("store", (what, j & 1), j + 1), ("add", (what + "_full", j & 1), 1)]
+    pipe = _Pipe()
+    mma: Program = [("pwait", "q_full", 0), ("pwait", ("k_full", 0), 0)]
+
+    def scores(u: int, j: int) -> None:
+        if j < je[u]:
+            mma.append(pipe.issue([("expect", ("k", j & 1), j + 1, f"Q K^T of unit {u} over tile {j}"), ("store", ("s", u, 0), ("scores", j)),
+                                   ("store", ("s", u, 1), ("scores", j)), ("add", ("s_full", u), 1)]))
+        if u == (1 if keep_k_for_both else 0):
+            mma.append(pipe.issue([("add", ("k_empty", j & 1), 1)]))
+
+    scores(0, 0)
+    scores(1, 0)
+    for j in range(n):
+        mma.append(("pwait", ("v_full", j & 1), j >> 1 & 1))
+        if j + 1 < n:
+            mma.append(("pwait", ("k_full", (j + 1) & 1), (j + 1) >> 1 & 1))
+        for u in range(2):
+            if j < je[u]:
+                for half in range(2):
+                    if half or wait_first_half:
+                        mma.append(("pwait", ("p_full" if half else "p_half", u), j & 1))
+                    mma.append(pipe.issue([("expect", ("v", j & 1), j + 1, f"P V of unit {u} over tile {j}"),
+                                           ("expect", ("s", u, half), ("weights", j), f"P V of unit {u} over tile {j}"), ("add", ("pv", u), 1)]))
+                if j + 1 == je[u]:
+                    mma.append(pipe.issue([("add", ("o_full", u), 1)]))
+            if u == 1:
+                mma.append(pipe.issue([("add", ("v_empty", j & 1), 1)]))
+            if j + 1 < n:
+                scores(u, j + 1)
+    groups: List[Program] = []
+    for u in range(2):
+        g: Program = []
+        for j in range(je[u]):
+            g += [("pwait", ("s_full", u), j & 1), ("expect", ("s", u, 0), ("scores", j), f"unit {u} reads its scores of tile {j}"),
+                  ("expect", ("s", u, 1), ("scores", j), f"unit {u} reads its scores of tile {j}")]
+            if j in rescale and j > 0:
+                g.append(("check", ("pv", u), 2 * j, f"unit {u} rescales O at tile {j} before P V of tile {j - 1} has landed"))
+            g += [("store", ("s", u, 0), ("weights", j)), ("add", ("p_half", u), 1), ("store", ("s", u, 1), ("weights", j)), ("add", ("p_full", u), 1)]
+        if je[u]:
+            g += [("pwait", ("o_full", u), 0), ("check", ("pv", u), 2 * je[u], f"unit {u} reads O before its last P V has landed")]
+        groups.append(g)
+    return [tma, mma, pipe.program, *groups]
+
+
+def flash_bwd_programs(n_sub: int, heads: int = 1, *, release_last: bool = True, lookahead: int = 2) -> List[Program]:
+    """The mbarrier pipeline of ``flash_attn_bwd_kernel`` (csrc/flash_attn_bwd.cu) for one CTA: ``n_sub`` streamed sub-tiles per head, two of them a TMA
+    stage, scores in two buffers that each belong to a group of warps. Agents: the TMA thread, the MMA-issuing thread, the tensor pipe, two groups.
+
+    Ingredients that tests take out: a stage is released behind its LAST sub-tile, and the scores of sub-tile u + 2 are issued behind the products
+    of u, which read their buffer (``lookahead`` 3: one sub-tile too early)."""
+    tiles, total = (n_sub + 1) // 2, n_sub * heads
+    tma: Program = [("add", "a_full", 1)]
+    for n in range(tiles * heads):
+        tma += [("pwait", ("b_empty", n & 1), (n >> 1 & 1) ^ 1), ("store", ("b", n & 1), n + 1), ("add", ("b_full", n & 1), 1)]
+    pipe = _Pipe()
+    mma: Program = [("pwait", "a_full", 0)]
+
+    def place(u: int) -> Tuple[int, int]:                # streamed tile, sub-tile inside its head
+        return u // n_sub * tiles + u % n_sub // 2, u % n_sub
+
+    def scores(u: int) -> None:
+        tile, sub = place(u)
+        if sub & 1 == 0:
+            mma.append(("pwait", ("b_full", tile & 1), tile >> 1 & 1))
+        mma.append(pipe.issue([("expect", ("b", tile & 1), tile + 1, f"scores of sub-tile {u}"), ("store", ("s", u & 1), ("scores", u)),
+                               ("add", ("s_full", u & 1), 1)]))
+
+    for u in range(min(lookahead, total)):
+        scores(u)
+    for u in range(total):
+        tile, sub = place(u)
+        mma.append(("pwait", ("p_full", u & 1), u >> 1 & 1))
+        mma.append(pipe.issue([("expect", ("s", u & 1), ("weights", u), f"products of sub-tile {u}"),
+                               ("expect", ("b", tile & 1), tile + 1, f"products of sub-tile {u}"), ("add", "products", 1)]))
+        if (sub & 1 == 1 or sub + 1 == n_sub) if release_last else sub & 1 == 0:
+            mma.append(pipe.issue([("add", ("b_empty", tile & 1), 1)]))
+        if u + lookahead < total:
+            scores(u + lookahead)
+    mma.append(pipe.issue([("add", "done", 1)]))
+    groups: List[Program] = []
+    for g in range(2):
+        prog: Program = []
+        for turn, u in enumerate(range(g, total, 2)):
+            prog += [("pwait", ("s_full", g), turn & 1), ("expect", ("s", g), ("scores", u), f"group {g} reads the scores of sub-tile {u}"),
+                     ("store", ("s", g), ("weights", u)), ("add", ("p_full", g), 1)]
+        prog += [("pwait", "done", 0), ("check", "products", total, f"group {g} stores before the last products have landed")]
+        groups.append(prog)
+    return [tma, mma, pipe.program, *groups]
+
+
+def pair_gemm_programs(items: int, blocks: int, *, stages: int = 2, both_epilogues: bool = True, both_producers: bool = True) -> List[Program]:
+    """The ring of a pair of CTAs (``gemm_pair_kernel`` in csrc/gemm_pair.cu, ``moe_pair_kernel`` in csrc/moe_pair.cu) over ``items`` tiles of ``blocks``
+    K blocks: each CTA loads its halves and counts its bytes on the EVEN CTA's full barrier, the even CTA issues the MMAs of both, the commits
+    arrive at both CTAs' barriers one after the other, and the epilogues of both release the accumulator at the even CTA. Agents: two TMA threads,
+    the MMA-issuing thread, the tensor pipe, an epilogue per CTA (its four warps arrive as one).
+
+    Ingredients that tests take out: the accumulator waits for the odd CTA's epilogue too, and the MMAs for the odd CTA's bytes."""
+    n_epi, n_tma = (2 if both_epilogues else 1), (2 if both_producers else 1)
+    order = [(i, kb) for i in range(items) for kb in range(blocks)]
+    producers: List[Program] = []
+    for c in range(2):
+        p: Program = []
+        for n in range(len(order)):
+            st, ph = n % stages, n // stages & 1
+            p += [("pwait", ("empty", c, st), ph ^ 1), ("store", ("stage", c, st), n + 1)]
+            if c == 0 or both_producers:
+                p.append(("add", ("full", st), 1))
+        producers.append(p)
+    pipe = _Pipe()
+    mma: Program = []
+    for n, (i, kb) in enumerate(order):
+        st, ph, buf = n % stages, n // stages & 1, i & 1
+        if kb == 0:
+            mma.append(("pwait", ("tempty", buf), (i >> 1 & 1) ^ 1, n_epi))
+        mma.append(("pwait", ("full", st), ph, n_tma))
+        effects: Program = [("expect", ("stage", c, st), n + 1, f"MMA of block {kb} of item {i}") for c in range(2)]
+        if kb == 0:
+            effects += [("check", ("read", c), i - 1, f"item {i} overwrites an accumulator that CTA {c} still reads") for c in range(2)]
+        if kb == blocks - 1:
+            effects.append(("store", ("acc", buf), i + 1))
+        effects += [("add", ("empty", c, st), 1) for c in range(2)]
+        if kb == blocks - 1:
+            effects += [("add", ("tfull", c, buf), 1) for c in range(2)]
+        mma.append(pipe.issue(effects))
+    epilogues: List[Program] = []
+    for c in range(2):
+        e: Program = []
+        for i in range(items):
+            e += [("pwait", ("tfull", c, i & 1), i >> 1 & 1), ("expect", ("acc", i & 1), i + 1, f"epilogue of item {i}"), ("add", ("read", c), 1)]
+            if c == 0 or both_epilogues:
+                e.append(("add", ("tempty", i & 1), 1))
+        epilogues.append(e)
+    return [*producers, mma, pipe.program, *epilogues]
+
+
+def decode_rows_programs(blocks: int, *, fetch_behind_use: bool = True) -> List[Program]:
+    """One warp of ``paged_decode_attn_kernel`` (csrc/decode_attn.cu) over ``blocks`` blocks of keys: one shared-memory buffer for K and one for V, each
+    refilled by a bulk copy as soon as its block has been used. Agents: the warp, the copies of K, the copies of V.
+
+    Ingredient that tests take out: the next copy is issued behind the last use of its buffer."""
+    warp: Program = [("add", ("asked", w), 1) for w in "kv"] if blocks else []
+    for i in range(blocks):
+        for w in "kv":
+            use: Program = [("pwait", (w, "bar"), i & 1), ("expect", (w, "buf"), i + 1, f"block {i} of {w}")]
+            ask: Program = [("add", ("asked", w), 1)] if i + 1 < blocks else []
+            warp += use + ask if fetch_behind_use else use[:1] + ask + use[1:]
+    copies: List[Program] = [[step for i in range(blocks) for step in [("wait", ("asked", w), i + 1), *bulk((w, "buf"), i + 1), ("add", (w, "bar"), 1)]]
+                             for w in "kv"]
+    return [warp, *copies]
+
+
 def one_shot_allreduce_programs(world: int, calls: int, *, slot_sets: int = 2) -> List[Program]:
     """The one-exchange all-reduce of the tensor-parallel decode step (``csrc/tp_decode.cu``,
     ``tp_allreduce_rmsnorm_ll_kernel``): in call k every rank stores its units {data, k} into its own slot of set
@@ -386,7 +563,16 @@ def check_all(verbose: bool = False) -> List[Result]:
     for n in (1, 2, 3, 5, 6):
         for k in range(0, min(n, 3)):
             for resc in itertools.combinations(range(1, n), k):
-                out.append(explore(f"flash forward pipeline, {n} tiles, rescale at {list(resc)}", flash_fwd_programs(n, resc)))
+                out.append(explore(f"group decode pipeline, {n} tiles, rescale at {list(resc)}", group_decode_programs(n, resc)))
+    for je in ((1, 0), (3, 0), (1, 2), (2, 3), (3, 4)):
+        for resc in ((), (1, 2)):
+            out.append(explore(f"flash forward, units of {je[0]} and {je[1]} key tiles, rescale at {list(resc)}", flash_fwd_programs(je, resc)))
+    for n, heads in ((1, 1), (2, 1), (3, 1), (4, 1), (7, 1), (1, 4), (3, 3), (4, 2)):
+        out.append(explore(f"flash backward, {n} sub-tiles, {heads} heads", flash_bwd_programs(n, heads)))
+    for items, blocks in ((1, 1), (1, 5), (3, 2), (4, 1)):
+        out.append(explore(f"pair of CTAs, {items} items of {blocks} blocks", pair_gemm_programs(items, blocks)))
+    for blocks in (1, 2, 5):
+        out.append(explore(f"decode attention, {blocks} blocks a warp", decode_rows_programs(blocks)))
     if verbose:
         for r in out:
             print(f"{'ok  ' if r.ok else 'FAIL'} {r.name}: {r.states} states" + ("" if r.ok else f" -- {r.finding}"))

@@ -167,19 +167,52 @@ def test_checked_mode_validators_name_the_offending_index():
     assert C.active() == prev
 
 
-def test_flash_forward_pipeline_needs_one_completion_barrier_per_buffer():
-    """The mbarrier pipeline of the flash attention forward kernel. With the P*V completion on ONE barrier that
+def test_group_decode_pipeline_needs_one_completion_barrier_per_buffer():
+    """The mbarrier pipeline of the tensor-core group decode kernel. With the P*V completion on ONE barrier that
     completes every tile and is consumed in order, a softmax warp can be two phases behind: the parity it waits for
     then names the running phase, which needs the warp's own next arrival (deadlock; on the GPU it ran into the
     bounded wait). Waiting directly on the wanted tile's parity of that single barrier passes too early instead. With
     one barrier per S/P buffer, as the kernel has it, every interleaving is clean for all rescale patterns."""
-    from rpeg_b200.parallel.protocol_check import explore, flash_fwd_programs
-    old = explore("in-order consumption of one barrier", flash_fwd_programs(5, (), pv_barriers=1, in_order_consume=True))
+    from rpeg_b200.parallel.protocol_check import explore, group_decode_programs
+    old = explore("in-order consumption of one barrier", group_decode_programs(5, (), pv_barriers=1, in_order_consume=True))
     assert old.finding is not None and old.finding.kind == "deadlock"
-    early = explore("direct wait on one barrier", flash_fwd_programs(5, (3,), pv_barriers=1, in_order_consume=False))
+    early = explore("direct wait on one barrier", group_decode_programs(5, (3,), pv_barriers=1, in_order_consume=False))
     assert early.finding is not None and early.finding.kind == "race" and "P*V" in early.finding.message
     for n, resc in ((1, ()), (2, (1,)), (4, ()), (5, (1, 3)), (6, (2, 3, 5)), (7, (6,))):
-        assert explore(f"{n} tiles", flash_fwd_programs(n, resc)).ok, (n, resc)
+        assert explore(f"{n} tiles", group_decode_programs(n, resc)).ok, (n, resc)
+
+
+def test_flash_forward_keeps_keys_for_both_units_and_waits_for_weights():
+    for je in ((1, 0), (1, 2), (2, 0), (3, 4)):
+        assert pc.explore("kernel", pc.flash_fwd_programs(je, range(1, 4))).ok, je
+    bad = pc.explore("K freed by the first unit", pc.flash_fwd_programs((3, 4), keep_k_for_both=False))
+    assert not bad.ok and bad.finding.kind == "race" and "Q K^T of unit 1" in bad.finding.message
+    bad = pc.explore("P V without its first weights", pc.flash_fwd_programs((1, 2), wait_first_half=False))
+    assert not bad.ok and bad.finding.kind == "race" and "P V of unit" in bad.finding.message
+
+
+def test_flash_backward_releases_stages_late_and_scores_behind_products():
+    for n, heads in ((1, 1), (1, 3), (2, 2), (3, 2), (5, 1)):
+        assert pc.explore("kernel", pc.flash_bwd_programs(n, heads)).ok, (n, heads)
+    bad = pc.explore("stage freed by its first half", pc.flash_bwd_programs(6, release_last=False))
+    assert not bad.ok and bad.finding.kind == "race" and "sub-tile" in bad.finding.message
+    bad = pc.explore("scores over weights that are still read", pc.flash_bwd_programs(6, lookahead=3))
+    assert not bad.ok
+
+
+def test_pair_of_ctas_waits_for_both():
+    for items, blocks, stages in ((1, 1, 2), (3, 1, 2), (2, 3, 2), (1, 7, 3)):
+        assert pc.explore("kernel", pc.pair_gemm_programs(items, blocks, stages=stages)).ok, (items, blocks)
+    bad = pc.explore("accumulator freed by the even epilogue", pc.pair_gemm_programs(4, 1, both_epilogues=False))
+    assert not bad.ok and bad.finding.kind == "race" and "CTA 1 still reads" in bad.finding.message
+    bad = pc.explore("MMA behind the even bytes", pc.pair_gemm_programs(1, 3, both_producers=False))
+    assert not bad.ok and bad.finding.kind == "race" and "MMA of block" in bad.finding.message
+
+
+def test_decode_attention_refills_behind_the_last_use():
+    assert pc.explore("kernel", pc.decode_rows_programs(4)).ok
+    bad = pc.explore("refilled before", pc.decode_rows_programs(4, fetch_behind_use=False))
+    assert not bad.ok and bad.finding.kind == "race" and "block" in bad.finding.message
 
 
 def test_one_exchange_allreduce_needs_two_slot_sets():
