@@ -20,6 +20,7 @@
 // linear_qkv / linear_proj / linear_fc1 / linear_fc2 / output_layer run them).
 #include <cstdlib>
 #include "common.cuh"
+#include "pair.cuh"
 #include "rpeg_kernels.h"
 
 namespace rpeg {
@@ -474,16 +475,6 @@ static int dispatch_major(int transA, int transB, const CUtensorMap& ta, const C
 }
 
 static int g_num_sms = 0;
-
-// gemm_pair.cu
-struct PairPlan {
-  int bn, splits, kb_per;
-};
-int gemm_pair(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int transA, int transB, int out_fp32,
-              int accumulate, PairPlan plan, int num_sms, int pdl, int* status, cudaStream_t stream);
-PairPlan pair_plan(int M, int N, int K, int transB, bool f32, long long slab_elems, int num_sms);
-int gemm_pair_swiglu(const void* A, const void* W, void* C, int M, int f, int K, int lda, int ldw, int ldc, int num_sms, int* status,
-                     cudaStream_t stream);
 
 }  // namespace rpeg
 

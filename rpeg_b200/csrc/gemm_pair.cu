@@ -31,9 +31,6 @@ constexpr int PG_STAGES = 6;
 constexpr int PG_SMEM = 1024 + PG_STAGES * PG_STAGE_BYTES + PG_STAGING + 512;
 static_assert(PG_SMEM <= 227 * 1024, "shared memory");
 
-struct PairPlan {                       // of pair_plan() below
-  int bn, splits, kb_per;
-};
 // Work of a launch: tiles of 256 rows x `bn` accumulator columns, each cut into `splits` pieces of `kb_per` K blocks (splits > 1: every piece
 // stores its own sums, `PG_F32` only).
 struct PairWork {

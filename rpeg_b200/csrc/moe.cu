@@ -15,6 +15,7 @@
 // Equal scores: the expert (or group) with the smaller number wins.
 #include "act_io.cuh"
 #include "moe_segments.cuh"
+#include "pair.cuh"
 #include "rpeg_kernels.h"
 
 namespace rpeg {
@@ -383,10 +384,6 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 
 int make_tmap_bf16_2d(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner,
                       uint32_t box_outer);
-
-// moe_pair.cu
-int moe_pair(const void* A, long long a_rows_total, const void* X, const void* B, void* C, const int* seg_off, int n_routed, int n_shared,
-             int seg_rows, int N, int K, int lda, int ldx, int ldb, int ldc, int act, int num_sms, int* status, cudaStream_t stream);
 
 template <int BN, int ACT>
 static int launch_moe_gemm(const CUtensorMap& ta, const CUtensorMap& tx, const CUtensorMap& tb, void* C, const int* seg_off, int n_routed,

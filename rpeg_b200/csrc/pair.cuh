@@ -60,4 +60,18 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
                : "memory");
 }
 
+// ---------------------------------------------------------------- host entries
+// gemm_pair.cu
+struct PairPlan {                       // of pair_plan()
+  int bn, splits, kb_per;
+};
+PairPlan pair_plan(int M, int N, int K, int transB, bool f32, long long slab_elems, int num_sms);
+int gemm_pair(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int transA, int transB, int out_fp32,
+              int accumulate, PairPlan plan, int num_sms, int pdl, int* status, cudaStream_t stream);
+int gemm_pair_swiglu(const void* A, const void* W, void* C, int M, int f, int K, int lda, int ldw, int ldc, int num_sms, int* status,
+                     cudaStream_t stream);
+// moe_pair.cu
+int moe_pair(const void* A, long long a_rows_total, const void* X, const void* B, void* C, const int* seg_off, int n_routed, int n_shared,
+             int seg_rows, int N, int K, int lda, int ldx, int ldb, int ldc, int act, int num_sms, int* status, cudaStream_t stream);
+
 }  // namespace rpeg
