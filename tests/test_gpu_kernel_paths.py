@@ -22,7 +22,7 @@ def _rel(a, b):
 F32 = 2e-6
 
 
-@pytest.mark.parametrize("m", [1, 2, 3, 4, 7, 8, 9, 16, 17, 65])
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 7, 8, 9, 16, 17, 31, 32, 33, 64, 65])      # passes of 16 rows, at most two of them; tiles of 64
 @pytest.mark.parametrize("n,k", [(1, 4), (5, 132), (130, 512), (700, 2052), (64, 65)])
 def test_gemm_f32_rows(cuda_device, m, n, k):
     g = torch.Generator(device=cuda_device).manual_seed(m * 1000 + n)
@@ -258,3 +258,49 @@ def test_moe_gemm_pair_tiles(cuda_device, e, top, shared, n, k, act):
         assert _rel(got[r.row_of[tok, col].long()], f(x[tok].double() @ w[i].double().T)) < 2 ** -8
     for s in range(shared):
         assert _rel(got[t * top + s * t:t * top + (s + 1) * t], f(x.double() @ w[e + s].double().T)) < 2 ** -8
+
+
+@pytest.mark.parametrize("act", ["none", "swiglu"])
+def test_moe_gemm_pair_ragged_experts(cuda_device, act):
+    """Experts without rows, with one, at the edges of the narrowest tile of 32 rows and of the widest of 256, among large ones."""
+    sizes, k, dev = [0, 1, 31, 32, 33, 0, 256, 257, 700, 1500, 0], 72, cuda_device
+    e, t, n = len(sizes), sum(sizes), 8200 if act == "none" else 4112
+    g = torch.Generator(device=dev).manual_seed(t)
+    x = torch.randn(t, k, generator=g, device=dev).bfloat16()
+    w = (torch.randn(e, n * (2 if act == "swiglu" else 1), k, generator=g, device=dev) / k ** 0.5).bfloat16()
+    expert = torch.repeat_interleave(torch.arange(e, device=dev), torch.tensor(sizes, device=dev))[torch.randperm(t, generator=g, device=dev)]
+    counts = torch.zeros(e, dtype=torch.int32, device=dev)
+    ids, wts, ticket = K.moe_route(torch.nn.functional.one_hot(expert, e).float() * 20, e, 1, counts)
+    assert torch.equal(ids[:, 0].long(), expert)
+    # the pair kernel's rule: 160 rows an expert on average, six items for each of 74 pairs
+    assert t >= 160 * e and (t // 256 + e // 2) * ((n + 255) // 256 if act == "none" else (n + 127) // 128) >= 6 * 74
+    r = K.moe_dispatch(x, ids, wts, ticket, counts, e)
+    got = K.moe_gemm(r.x_sorted, w, r, e, 0, act=act)
+    f = {"none": lambda z: z, "swiglu": lambda z: torch.nn.functional.silu(z[:, :n]) * z[:, n:]}[act]
+    for i in range(e):
+        tok = (expert == i).nonzero()[:, 0]
+        if len(tok):
+            assert _rel(got[r.row_of[tok, 0].long()], f(x[tok].double() @ w[i].double().T)) < 2 ** -8
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,vocab,shift", [(1, 1, 0), (3, 7, 0), (2, 8, 0), (5, 1003, 0), (4, 1003, 1), (3, 8192, 0), (2, 32003, 3)])
+def test_sample_rows(cuda_device, dtype, rows, vocab, shift):
+    """Rows of 16-byte loads with and without a tail of less than eight logits, and rows that are not aligned: the same tokens, argmax of the logits
+    (the first of equal ones) or of the logits plus noise that depends on the place alone, and log-probs under the full softmax."""
+    g = torch.Generator(device=cuda_device).manual_seed(vocab + shift)
+    aligned = torch.zeros(rows, (vocab + 15) // 8 * 8, device=cuda_device, dtype=dtype)[:, :vocab]
+    aligned.copy_(torch.randn(rows, vocab, generator=g, device=cuda_device) * 3)
+    aligned[:, vocab // 2:] = torch.minimum(aligned[:, vocab // 2:], aligned[:, : (vocab + 1) // 2].amax(1, keepdim=True))      # ties with earlier ones
+    odd = torch.empty(rows, vocab + 4, device=cuda_device, dtype=dtype)[:, shift:shift + vocab].copy_(aligned)
+    want = torch.log_softmax(aligned.double() / 0.7, -1)
+    first = (aligned == aligned.amax(1, keepdim=True)).int().argmax(1)
+    for x in (aligned, odd):
+        tok, lp = K.sample(x, 0.7, True, 9)
+        assert torch.equal(tok.long(), first)
+        # fp32 sums of `vocab` exponentials and a logarithm of about 10: 1e-5 of the result
+        assert float((lp - want.gather(1, tok.long()[:, None])[:, 0]).abs().max()) < 1e-4
+    drawn, lp = K.sample(aligned, 0.7, False, 77)
+    assert torch.equal(drawn, K.sample(odd, 0.7, False, 77)[0])
+    assert torch.equal(drawn, K.sample(aligned.float(), 0.7, False, 77)[0])
+    assert float((lp - want.gather(1, drawn.long()[:, None])[:, 0]).abs().max()) < 1e-4

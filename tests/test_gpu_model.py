@@ -201,6 +201,24 @@ def test_generation_with_page_preemption_matches_roomy_pool(cuda_device):
     assert tight.pool.available() == tight.pool.num_pages - 1
 
 
+@pytest.mark.parametrize("limit", [None, 3, 1])
+def test_shared_prompts_with_many_ragged_tails(cuda_device, limit):
+    """More ragged tails in one admission than a page copy takes at once (16 pages, or fewer by the buffer's size; None: the default)."""
+    cfg = LlamaConfig.tiny(n_layers=2)
+    model = LlamaModel(cfg, cuda_device, seed=9)
+    P, Kq, S = 20, 3, 75
+    prompts = torch.randint(2, cfg.vocab, (P, S), device=cuda_device, dtype=torch.int32).repeat_interleave(Kq, dim=0).contiguous()
+    gen = Generator(model, max_slots=64, max_seq_len=S + 24, kv_budget_bytes=1e9, eos_id=1)
+    plain = gen.generate(prompts, 24, greedy=True)
+    if limit is not None:
+        gen.COPY_BYTES = limit * 2 * cfg.n_layers * cfg.n_kv_heads * K.KV_PAGE * cfg.head_dim * 2
+    shared = gen.generate(prompts, 24, greedy=True, group_size=Kq)
+    assert shared.counters["prompts_prefilled"] == P and shared.counters["shared_prompt_pages"] == P * (S // K.KV_PAGE)
+    # the same keys in other pages, prefilled once instead of three times: the prefill's packing may flip a near tie
+    same = sum(int(torch.equal(plain.tokens[i], shared.tokens[i])) for i in range(P * Kq))
+    assert same >= P * Kq - 3, f"only {same} of {P * Kq} rows identical"
+
+
 @pytest.mark.parametrize("S", [128, 150])
 def test_generation_with_shared_prompt_pages(cuda_device, S):
     """K samples per prompt with the prompt's KV pages shared by the group: one prefill per prompt, fewer pages, and
