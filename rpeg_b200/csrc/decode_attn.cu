@@ -201,39 +201,37 @@ __device__ __forceinline__ void axpy8(float (&acc)[8], float p, const uint4& vv)
 // q: [B, ldq] with head h at column q_col0 + h*HD. out: [B, H*HD] bf16.
 // partial (when nsplit > 1): [B, H, nsplit, HD + 2] fp32 = {o[HD], m, l}.
 //
-// Bound by streaming the cache: a block of 16 keys (4 KB of K and of V) comes into a warp's own shared memory as one bulk copy each, the
-// next K as soon as this one's scores are taken, so 24 warps an SM keep up to 192 KB in flight whatever their registers allow (loads to
-// registers waited four times per 32 keys: 16 rows of 280 keys, 32 heads 31 -> 23 us, 256 rows of 540 410 -> 323 us, 7.0 TB/s;
-// 256 rows in groups of eight over 512 shared keys 256 -> 199 us).
-// Work split inside a warp: the 32 lanes form two groups of 16; a group reads one 256-byte K (or V) row per load instruction, lane c of the
-// group owning the 16-byte chunk c (head dims 8c..8c+7). Group g takes keys g*8..g*8+7 of a block; the 8 partial dot products of a lane are
-// summed across the group by a transposing butterfly that leaves the score of key `lane & 7` in two lanes. For PV each lane
-// accumulates its 8 head dims over the group's keys; the two groups are added at the end.
+// Bound by streaming the cache. A warp takes blocks of 16 keys; its 32 lanes form two groups of 16, a group reads one 256-byte K (or V) row per
+// load instruction, lane c of the group owning the 16-byte chunk c (head dims 8c..8c+7), so every load is coalesced. Group g takes keys
+// g*8..g*8+7 of a block; the 8 partial dot products of a lane are summed across the group by a transposing butterfly that leaves the score of
+// key `lane & 7` in two lanes. For PV each lane accumulates its 8 head dims over the group's keys; the two groups are added at the end.
+// A row's last block is loaded without a branch per key (K rows past the end repeat the last one, V rows are zero): a branch per key serialised its
+// loads (256 rows of 540 keys, blocks of 32: 411 us with the branches, 344 without).
+//
+// MIN_CTAS: how many CTAs an SM is to hold, against how early V is requested. What a short wave needs is bytes in flight per warp, what a
+// long one needs is warps (32 heads; keys copied to shared memory by bulk copies, 6 CTAs an SM, in brackets):
+//   4: V together with K, one round trip a block.  16 rows of 1900 keys 73 us (93), with 8 KV heads 46 (72); 1 row of 48 keys 2.4 (2.6)
+//   6: V behind the scores, under the softmax.     24 rows of 1900 keys 107 us (119), with 8 KV heads 63 (74); 48 rows of 1000 113 (114)
+//   7: V behind the softmax.                       32 rows of 1900 keys 142 us (172), with 8 KV heads 77 (88); 64 rows of 540 84 (90); 256 rows
+//      of 540 317 (315), in groups of eight over 512 shared keys 168 (188); of 150 keys 98 (93)
 constexpr int DA_KEYS = 16;                          // keys of a block, a divisor of the page
-constexpr int DA_BLOCK_BYTES = DA_KEYS * HD * 2;
-constexpr int DA_SMEM = 4 * 2 * DA_BLOCK_BYTES;      // per warp: a block of K and of V
 
-__global__ void __launch_bounds__(128)
+template <int MIN_CTAS>
+__global__ void __launch_bounds__(128, MIN_CTAS)
 paged_decode_attn_kernel(const __nv_bfloat16* __restrict__ q, int ldq, int q_col0,
                          const __nv_bfloat16* __restrict__ kcache, const __nv_bfloat16* __restrict__ vcache,
                          const int* __restrict__ page_table, int max_pages, const int* __restrict__ seq_lens,
                          __nv_bfloat16* __restrict__ out, float* __restrict__ partial, int H, int Hkv,
                          int nsplit, float scale_log2, const int* __restrict__ row_key0, int slot_base, int nslots,
-                         int* __restrict__ arrive, int* status) {
+                         int* __restrict__ arrive) {
   griddep_launch();
   griddep_wait();   // may have been scheduled under the previous kernel's tail: nothing is read or written before this
-  extern __shared__ __align__(128) uint8_t kv_sm[];
-  __shared__ uint64_t kv_bar[4][2];
-  __shared__ int abort_word;
   __shared__ float red_m[4], red_l[4];
   __shared__ int is_last;
   __shared__ __align__(16) float red_o[4][HD];
   const int h = blockIdx.x, b = blockIdx.y, split = blockIdx.z;
   const int hk = h / (H / Hkv);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint8_t* const k_sm = kv_sm + warp * 2 * DA_BLOCK_BYTES;
-  uint8_t* const v_sm = k_sm + DA_BLOCK_BYTES;
-  uint64_t* const bar = kv_bar[warp];
   const int grp = lane >> 4, c = lane & 15;
   const int L = seq_lens[b];
   const int nblk = (L + DA_KEYS - 1) / DA_KEYS;
@@ -260,43 +258,41 @@ paged_decode_attn_kernel(const __nv_bfloat16* __restrict__ q, int ldq, int q_col
   const int* pt = page_table + static_cast<size_t>(b) * max_pages;
   const int first = blk0 + warp;
   int page = first < blk1 ? pt[(first * DA_KEYS) / PAGE] : 0;
-  auto fetch = [&](int blk, int pg, const __nv_bfloat16* cache, uint8_t* dst, uint64_t* done) {     // one lane
-    const uint32_t bytes = min(DA_KEYS, L - blk * DA_KEYS) * (HD * 2);
-    mbar_expect_tx(done, bytes);
-    bulk_load(dst, cache + ((static_cast<size_t>(pg) * Hkv + hk) * PAGE + (blk * DA_KEYS) % PAGE) * HD, bytes, done);
-  };
-  if (lane == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    if (warp == 0) abort_word = 0;
-    fence_mbar_init();
-    if (first < blk1) {
-      fetch(first, page, kcache, k_sm, &bar[0]);
-      fetch(first, page, vcache, v_sm, &bar[1]);
-    }
-  }
-  __syncthreads();
-  uint32_t phase = 0;
-  for (int blk = first; blk < blk1; blk += 4, phase ^= 1u) {
+  uint4 kv[8], vv[8];
+  for (int blk = first; blk < blk1; blk += 4) {
     const int next = blk + 4;
     const int next_page = next < blk1 ? pt[(next * DA_KEYS) / PAGE] : 0;
-    const int nk = min(DA_KEYS, L - blk * DA_KEYS) - grp * 8;   // valid keys of this group (may be <= 0)
-    const uint4* kp = reinterpret_cast<const uint4*>(k_sm) + grp * 8 * (HD / 8) + c;      // this lane's chunk of the group's rows
-    const uint4* vp = reinterpret_cast<const uint4*>(v_sm) + grp * 8 * (HD / 8) + c;
-    if (!__all_sync(0xffffffffu, mbar_wait(&bar[0], phase, &abort_word, status, 830))) break;
-    float part[8];
+    const int nk = min(DA_KEYS, L - blk * DA_KEYS) - grp * 8;   // valid keys of this group (group 1: may be <= 0)
+    // this lane's chunk of the group's rows
+    const size_t base = ((static_cast<size_t>(page) * Hkv + hk) * PAGE + (blk * DA_KEYS) % PAGE + grp * 8) * HD + c * 8;
+    const uint4* kp = reinterpret_cast<const uint4*>(kcache + base);
+    const uint4* vp = reinterpret_cast<const uint4*>(vcache + base);
+    page = next_page;
     if (nk >= 8) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) part[j] = dot8(kp[j * (HD / 8)], qr);
+      for (int j = 0; j < 8; ++j) kv[j] = kp[j * (HD / 8)];
     } else {
+      const int last = nk > 0 ? nk - 1 : -grp * 8;              // a group without keys reads the block's first
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        part[j] = 0.f;
-        if (j < nk) part[j] = dot8(kp[j * (HD / 8)], qr);
-      }
+      for (int j = 0; j < 8; ++j) kv[j] = kp[min(j, last) * (HD / 8)];
     }
-    __syncwarp();
-    if (lane == 0 && next < blk1) fetch(next, next_page, kcache, k_sm, &bar[0]);
+    auto load_v = [&]() {
+      if (nk >= 8) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) vv[j] = vp[j * (HD / 8)];
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          vv[j] = make_uint4(0u, 0u, 0u, 0u);
+          if (j < nk) vv[j] = vp[j * (HD / 8)];
+        }
+      }
+    };
+    if constexpr (MIN_CTAS == 4) load_v();
+    float part[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) part[j] = dot8(kv[j], qr);
+    if constexpr (MIN_CTAS == 6) load_v();
     const int key = lane & 7;
     float s = transpose_reduce8(part, lane);        // score of key `key` of the group, in two lanes
     if (key >= nk) s = -INFINITY;
@@ -307,26 +303,9 @@ paged_decode_attn_kernel(const __nv_bfloat16* __restrict__ q, int ldq, int q_col
 #pragma unroll
     for (int k = 0; k < 8; ++k) acc[k] *= alpha;
     m = nm;
-    if (!__all_sync(0xffffffffu, mbar_wait(&bar[1], phase, &abort_word, status, 831))) break;
-    if (nk >= 8) {
+    if constexpr (MIN_CTAS == 7) load_v();
 #pragma unroll
-      for (int j = 0; j < 8; ++j) axpy8(acc, __shfl_sync(0xffffffffu, p, grp * 16 + j), vp[j * (HD / 8)]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float pj = __shfl_sync(0xffffffffu, p, grp * 16 + j);
-        if (j < nk) axpy8(acc, pj, vp[j * (HD / 8)]);
-      }
-    }
-    __syncwarp();
-    if (lane == 0 && next < blk1) fetch(next, next_page, vcache, v_sm, &bar[1]);
-  }
-  if (*static_cast<volatile int*>(&abort_word)) {       // a copy that never arrived (in the status word): the row becomes NaN
-    __nanosleep(200000);
-    m = 0.f;
-    l = 1.f / 32.f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) acc[k] = NAN;
+    for (int j = 0; j < 8; ++j) axpy8(acc, __shfl_sync(0xffffffffu, p, grp * 16 + j), vv[j]);
   }
   l = warp_sum(l);
   // add the two key groups, then merge the 4 warps
@@ -383,6 +362,23 @@ paged_decode_attn_kernel(const __nv_bfloat16* __restrict__ q, int ldq, int q_col
       out[(static_cast<size_t>(b) * H + h) * HD + threadIdx.x] = __float2bfloat16(gl > 0.f ? o / gl : 0.f);
     }
   }
+}
+
+// Which of the three forms. Up to four CTAs an SM, the first. Then whichever of six and seven CTAs an SM leaves less of its last wave empty; a
+// last wave costs at least 0.6 of a full one (48 rows of 32 heads, 1000 keys: 113 us at six, 119 at seven; 32 rows: 93 and 76); in one wave, six.
+static cudaError_t launch_decode_attn(int H, int B, int nsplit, cudaStream_t stream, const void* q, int ldq, int q_col0, const void* kcache,
+                                      const void* vcache, const int* page_table, int max_pages, const int* seq_lens, void* out, float* partial,
+                                      int Hkv, float scale_log2, const int* row_key0, int slot_base, int nslots, int* arrive) {
+  const long long ctas = static_cast<long long>(H) * B * nsplit, sms = 148;
+  auto cost = [&](long long slots) {
+    const long long rest = ctas % slots;
+    return (ctas - rest) * 10 + (rest == 0 ? 0 : rest * 10 > slots * 6 ? rest * 10 : slots * 6);
+  };
+  auto kern = ctas <= 4 * sms ? paged_decode_attn_kernel<4>
+              : ctas <= 6 * sms || cost(6 * sms) < cost(7 * sms) ? paged_decode_attn_kernel<6> : paged_decode_attn_kernel<7>;
+  return launch_pdl(kern, dim3(H, B, nsplit), dim3(128), 0, stream, static_cast<const __nv_bfloat16*>(q), ldq, q_col0,
+                    static_cast<const __nv_bfloat16*>(kcache), static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages, seq_lens,
+                    static_cast<__nv_bfloat16*>(out), partial, H, Hkv, nsplit, scale_log2, row_key0, slot_base, nslots, arrive);
 }
 
 // Arrival counters of the fused combine, one per (row, head); zero between launches. One split-KV decode attention
@@ -897,17 +893,15 @@ extern "C" long long rpeg_decode_attn_scratch_bytes(int B, int H, int nsplit) {
 extern "C" int rpeg_paged_decode_attn(const void* q, int ldq, int q_col0, const void* kcache, const void* vcache,
                                       const int* page_table, int max_pages, const int* seq_lens, void* out,
                                       float* scratch, int B, int H, int Hkv, int hd, int nsplit, float scale,
-                                      int* status, void* stream) {
+                                      void* stream) {
   if (hd != HD || H % Hkv != 0) return -2;
   if (nsplit < 1 || nsplit > 64) return -3;
   if (nsplit > 1 && scratch == nullptr) return -4;
   if (B <= 0) return 0;
   const float scale_log2 = scale * 1.4426950408889634f;
   int* arrive = nsplit > 1 ? fused_combine_counters(B, H) : nullptr;
-  launch_pdl(paged_decode_attn_kernel, dim3(H, B, nsplit), dim3(128), DA_SMEM, STREAM(stream), 
-      static_cast<const __nv_bfloat16*>(q), ldq, q_col0, static_cast<const __nv_bfloat16*>(kcache),
-      static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages, seq_lens,
-      static_cast<__nv_bfloat16*>(out), scratch, H, Hkv, nsplit, scale_log2, static_cast<const int*>(nullptr), 0, nsplit, arrive, status);
+  launch_decode_attn(H, B, nsplit, STREAM(stream), q, ldq, q_col0, kcache, vcache, page_table, max_pages, seq_lens, out, scratch, Hkv, scale_log2,
+                     nullptr, 0, nsplit, arrive);
   if (nsplit > 1 && arrive == nullptr)
     launch_pdl(decode_combine_kernel, dim3(dim3(H, B)), dim3(HD), 0, STREAM(stream), scratch, static_cast<__nv_bfloat16*>(out), H, nsplit);
   return LAUNCH_OK();
@@ -922,7 +916,7 @@ extern "C" int rpeg_paged_decode_attn_grouped(const void* q, int ldq, int q_col0
                                               const int* page_table, int max_pages, const int* seq_lens, void* out,
                                               float* scratch, int B, int H, int Hkv, int hd, int nsplit, float scale,
                                               const int* group_rows, const int* group_shared, const int* row_key0,
-                                              int* status, void* stream) {
+                                              void* stream) {
   if (hd != HD || H % Hkv != 0) return -2;
   if (nsplit < 1 || nsplit > 63) return -3;
   if (scratch == nullptr || group_rows == nullptr || group_shared == nullptr || row_key0 == nullptr) return -4;
@@ -933,9 +927,8 @@ extern "C" int rpeg_paged_decode_attn_grouped(const void* q, int ldq, int q_col0
   launch_pdl(paged_decode_attn_shared_kernel, dim3(H, B), dim3(128), 0, STREAM(stream), static_cast<const __nv_bfloat16*>(q), ldq,
              q_col0, static_cast<const __nv_bfloat16*>(kcache), static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages,
              group_rows, group_shared, scratch, H, Hkv, nslots, scale_log2);
-  launch_pdl(paged_decode_attn_kernel, dim3(H, B, nsplit), dim3(128), DA_SMEM, STREAM(stream), static_cast<const __nv_bfloat16*>(q), ldq,
-             q_col0, static_cast<const __nv_bfloat16*>(kcache), static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages,
-             seq_lens, static_cast<__nv_bfloat16*>(out), scratch, H, Hkv, nsplit, scale_log2, row_key0, 1, nslots, arrive, status);
+  launch_decode_attn(H, B, nsplit, STREAM(stream), q, ldq, q_col0, kcache, vcache, page_table, max_pages, seq_lens, out, scratch, Hkv, scale_log2,
+                     row_key0, 1, nslots, arrive);
   if (arrive == nullptr)
     launch_pdl(decode_combine_kernel, dim3(H, B), dim3(HD), 0, STREAM(stream), scratch, static_cast<__nv_bfloat16*>(out), H, nslots);
   return LAUNCH_OK();
@@ -983,9 +976,8 @@ extern "C" int rpeg_paged_decode_attn_grouped_tc(const void* q, int ldq, int q_c
   launch_pdl(paged_decode_attn_shared_tc_kernel, dim3(grid), dim3(GT_THREADS), GT_SMEM, STREAM(stream), tk, tv,
              static_cast<const __nv_bfloat16*>(q), ldq, q_col0, page_table, max_pages, group_rows, group_shared, scratch, B, H, Hkv,
              nslots, scale_log2, status);
-  launch_pdl(paged_decode_attn_kernel, dim3(H, B, nsplit), dim3(128), DA_SMEM, STREAM(stream), static_cast<const __nv_bfloat16*>(q), ldq,
-             q_col0, static_cast<const __nv_bfloat16*>(kcache), static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages,
-             seq_lens, static_cast<__nv_bfloat16*>(out), scratch, H, Hkv, nsplit, scale_log2, row_key0, 1, nslots, arrive, status);
+  launch_decode_attn(H, B, nsplit, STREAM(stream), q, ldq, q_col0, kcache, vcache, page_table, max_pages, seq_lens, out, scratch, Hkv, scale_log2,
+                     row_key0, 1, nslots, arrive);
   if (arrive == nullptr)
     launch_pdl(decode_combine_kernel, dim3(H, B), dim3(HD), 0, STREAM(stream), scratch, static_cast<__nv_bfloat16*>(out), H, nslots);
   return LAUNCH_OK();
@@ -999,10 +991,8 @@ extern "C" int rpeg_paged_decode_attn_grouped_tc(const void* q, int ldq, int q_c
 namespace {
 constexpr long long STATIC_PARTIAL_FLOATS = static_cast<long long>(RPEG_DECODE_STATIC_MAX_PARTIALS) * (HD + 2);
 static __device__ __align__(256) float g_decode_static_scratch[STATIC_PARTIAL_FLOATS];
-static __device__ int g_decode_static_status[4];
 constexpr int STATIC_MAX_DEVICES = 64;
 float* g_static_scratch_ptr[STATIC_MAX_DEVICES] = {nullptr};
-int* g_static_status_ptr[STATIC_MAX_DEVICES] = {nullptr};
 }  // namespace
 
 extern "C" const char* rpeg_static_entry_strerror(int code) {
@@ -1028,29 +1018,17 @@ extern "C" int rpeg_paged_decode_attn_static(const void* q, int ldq, int q_col0,
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= STATIC_MAX_DEVICES) return RPEG_STATIC_ERR_SETUP;
   if (g_static_scratch_ptr[dev] == nullptr) {
-    // set-up, once per device: the arrays' addresses in this device's copy of the module
+    // set-up, once per device: the array's address in this device's copy of the module
     float* p = nullptr;
-    int* st = nullptr;
-    if (cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_decode_static_scratch) != cudaSuccess || p == nullptr ||
-        cudaGetSymbolAddress(reinterpret_cast<void**>(&st), g_decode_static_status) != cudaSuccess || st == nullptr)
+    if (cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_decode_static_scratch) != cudaSuccess || p == nullptr)
       return RPEG_STATIC_ERR_SETUP;
-    g_static_status_ptr[dev] = st;
     g_static_scratch_ptr[dev] = p;
   }
   float* scratch = g_static_scratch_ptr[dev];
-  int* status = g_static_status_ptr[dev];
   const float scale_log2 = scale * 1.4426950408889634f;
-  launch_pdl(paged_decode_attn_kernel, dim3(H, B, nsplit), dim3(128), DA_SMEM, STREAM(stream), 
-      static_cast<const __nv_bfloat16*>(q), ldq, q_col0, static_cast<const __nv_bfloat16*>(kcache),
-      static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages, seq_lens, static_cast<__nv_bfloat16*>(out),
-      scratch, H, Hkv, nsplit, scale_log2, static_cast<const int*>(nullptr), 0, nsplit, static_cast<int*>(nullptr), status);
+  launch_decode_attn(H, B, nsplit, STREAM(stream), q, ldq, q_col0, kcache, vcache, page_table, max_pages, seq_lens, out, scratch, Hkv, scale_log2,
+                     nullptr, 0, nsplit, nullptr);
   if (nsplit > 1)
     launch_pdl(decode_combine_kernel, dim3(dim3(H, B)), dim3(HD), 0, STREAM(stream), scratch, static_cast<__nv_bfloat16*>(out), H, nsplit);
   return cudaGetLastError() == cudaSuccess ? 0 : RPEG_STATIC_ERR_LAUNCH;
-}
-
-extern "C" int rpeg_decode_static_status(int* out) {
-  static const int clear[4] = {0, 0, 0, 0};
-  if (cudaMemcpyFromSymbol(out, g_decode_static_status, sizeof(clear)) != cudaSuccess) return RPEG_STATIC_ERR_SETUP;
-  return out[0] == 0 || cudaMemcpyToSymbol(g_decode_static_status, clear, sizeof(clear)) == cudaSuccess ? 0 : RPEG_STATIC_ERR_SETUP;
 }

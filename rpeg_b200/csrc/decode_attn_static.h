@@ -17,8 +17,6 @@
 //     split pass of the same call.
 //   * There is ONE array per device. Two calls whose kernels may overlap in time (different streams,
 //     or different host threads) race on it; keep all calls on a device in one stream, or order them.
-//   * The kernel's waits for its own copies are bounded. One that runs out turns the row into NaN and is recorded
-//     in a device word of the library, which rpeg_decode_static_status() reads.
 //   * No cudaMalloc / cudaFree and no allocating library routine is called, on the first call or later.
 #pragma once
 
@@ -37,10 +35,6 @@ extern "C" {
 int rpeg_paged_decode_attn_static(const void* q, int ldq, int q_col0, const void* kcache, const void* vcache,
                                   const int* page_table, int max_pages, const int* seq_lens, void* out, int B, int H,
                                   int Hkv, int hd, int nsplit, float scale, void* stream);
-
-// Copies the current device's record of the first wait that ran out to out[4] (code, place, block, detail; code 0: none) and clears
-// it. Waits for the device; not for use under stream capture. Returns 0 or RPEG_STATIC_ERR_SETUP.
-int rpeg_decode_static_status(int* out);
 
 // Human-readable text for the codes above (a static string; never NULL).
 const char* rpeg_static_entry_strerror(int code);

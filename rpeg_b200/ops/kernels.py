@@ -562,8 +562,7 @@ def paged_decode_attn(q, q_col0, kcache, vcache, page_table, seq_lens, n_heads, 
         check(lib().rpeg_paged_decode_attn_grouped(q.data_ptr(), q.stride(0), q_col0, kcache.data_ptr(), vcache.data_ptr(),
                                                    page_table.data_ptr(), page_table.stride(0), seq_lens.data_ptr(), out.data_ptr(),
                                                    scratch.data_ptr(), B, n_heads, n_kv_heads, head_dim, nsplit, scale,
-                                                   group_rows.data_ptr(), group_shared.data_ptr(), row_key0.data_ptr(),
-                                                   status_word(q.device).data_ptr(), _stream()),
+                                                   group_rows.data_ptr(), group_shared.data_ptr(), row_key0.data_ptr(), _stream()),
               "rpeg_paged_decode_attn_grouped")
         return out
     if nsplit > 1 and scratch is None:
@@ -571,7 +570,7 @@ def paged_decode_attn(q, q_col0, kcache, vcache, page_table, seq_lens, n_heads, 
     check(lib().rpeg_paged_decode_attn(q.data_ptr(), q.stride(0), q_col0, kcache.data_ptr(), vcache.data_ptr(),
                                        page_table.data_ptr(), page_table.stride(0), seq_lens.data_ptr(),
                                        out.data_ptr(), _ptr(scratch), B, n_heads, n_kv_heads, head_dim, nsplit,
-                                       scale, status_word(q.device).data_ptr(), _stream()), "rpeg_paged_decode_attn")
+                                       scale, _stream()), "rpeg_paged_decode_attn")
     return out
 
 

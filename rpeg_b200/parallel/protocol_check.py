@@ -502,22 +502,6 @@ def pair_gemm_programs(items: int, blocks: int, *, stages: int = 2, both_epilogu
     return [*producers, mma, pipe.program, *epilogues]
 
 
-def decode_rows_programs(blocks: int, *, fetch_behind_use: bool = True) -> List[Program]:
-    """One warp of ``paged_decode_attn_kernel`` (csrc/decode_attn.cu) over ``blocks`` blocks of keys: one shared-memory buffer for K and one for V, each
-    refilled by a bulk copy as soon as its block has been used. Agents: the warp, the copies of K, the copies of V.
-
-    Ingredient that tests take out: the next copy is issued behind the last use of its buffer."""
-    warp: Program = [("add", ("asked", w), 1) for w in "kv"] if blocks else []
-    for i in range(blocks):
-        for w in "kv":
-            use: Program = [("pwait", (w, "bar"), i & 1), ("expect", (w, "buf"), i + 1, f"block {i} of {w}")]
-            ask: Program = [("add", ("asked", w), 1)] if i + 1 < blocks else []
-            warp += use + ask if fetch_behind_use else use[:1] + ask + use[1:]
-    copies: List[Program] = [[step for i in range(blocks) for step in [("wait", ("asked", w), i + 1), *bulk((w, "buf"), i + 1), ("add", (w, "bar"), 1)]]
-                             for w in "kv"]
-    return [warp, *copies]
-
-
 def one_shot_allreduce_programs(world: int, calls: int, *, slot_sets: int = 2) -> List[Program]:
     """The one-exchange all-reduce of the tensor-parallel decode step (``csrc/tp_decode.cu``,
     ``tp_allreduce_rmsnorm_ll_kernel``): in call k every rank stores its units {data, k} into its own slot of set
@@ -571,8 +555,6 @@ def check_all(verbose: bool = False) -> List[Result]:
         out.append(explore(f"flash backward, {n} sub-tiles, {heads} heads", flash_bwd_programs(n, heads)))
     for items, blocks in ((1, 1), (1, 5), (3, 2), (4, 1)):
         out.append(explore(f"pair of CTAs, {items} items of {blocks} blocks", pair_gemm_programs(items, blocks)))
-    for blocks in (1, 2, 5):
-        out.append(explore(f"decode attention, {blocks} blocks a warp", decode_rows_programs(blocks)))
     if verbose:
         for r in out:
             print(f"{'ok  ' if r.ok else 'FAIL'} {r.name}: {r.states} states" + ("" if r.ok else f" -- {r.finding}"))

@@ -182,7 +182,8 @@ def test_flash_attn_fwd_units(cuda_device, h, hkv):
         at += n
 
 
-@pytest.mark.parametrize("h,hkv,nsplit", [(2, 2, 1), (4, 1, 1), (2, 2, 3)])
+# 14 rows of so many heads and splits: up to four CTAs an SM, up to six, more (672 and 896 CTAs), and a second wave that six an SM fill better (1344)
+@pytest.mark.parametrize("h,hkv,nsplit", [(2, 2, 1), (4, 1, 1), (2, 2, 3), (48, 6, 1), (64, 8, 1), (16, 2, 4), (48, 6, 2)])
 def test_paged_decode_attn_blocks(cuda_device, h, hkv, nsplit):
     hd, lens = 128, [0, 1, 7, 8, 9, 15, 16, 17, 63, 64, 65, 127, 200, 1025]      # edges of a lane group's 8 keys, a block's 16, a page's 64
     g = torch.Generator(device=cuda_device).manual_seed(nsplit)

@@ -209,12 +209,6 @@ def test_pair_of_ctas_waits_for_both():
     assert not bad.ok and bad.finding.kind == "race" and "MMA of block" in bad.finding.message
 
 
-def test_decode_attention_refills_behind_the_last_use():
-    assert pc.explore("kernel", pc.decode_rows_programs(4)).ok
-    bad = pc.explore("refilled before", pc.decode_rows_programs(4, fetch_behind_use=False))
-    assert not bad.ok and bad.finding.kind == "race" and "block" in bad.finding.message
-
-
 def test_one_exchange_allreduce_needs_two_slot_sets():
     """The all-reduce that pushes self-validating units and never acknowledges them: clean with the two slot sets the
     kernel alternates between, and the checker finds the overwritten units when there is only one."""

@@ -91,16 +91,3 @@ def test_static_scratch_entry_refuses_what_does_not_fit(cuda_device):
     assert err(0) == b"ok"
     torch.cuda.synchronize()
     K.check_status()
-
-
-def test_static_scratch_entry_reports_its_waits(cuda_device):
-    """Nothing ran out, so the record reads clear, also after calls of the entry (a wait that runs out needs a broken copy)."""
-    lib = ctypes.CDLL(LIB)
-    lib.rpeg_decode_static_status.restype, lib.rpeg_decode_static_status.argtypes = I, [P]
-    fn, err = _entry()
-    q, kc, vc, table, seq = _case(cuda_device, [300, 20], 8, 8, seed=4)
-    out = torch.empty_like(q)
-    assert fn(q.data_ptr(), q.stride(0), 0, kc.data_ptr(), vc.data_ptr(), table.data_ptr(), table.stride(0), seq.data_ptr(), out.data_ptr(), 2, 8, 8, 128,
-              2, 0.1, torch.cuda.current_stream().cuda_stream) == 0
-    record = (I * 4)(7, 7, 7, 7)
-    assert lib.rpeg_decode_static_status(record) == 0 and list(record) == [0, 0, 0, 0]
