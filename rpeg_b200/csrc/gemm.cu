@@ -538,15 +538,25 @@ static int gemm_impl(const void* A, const void* B, void* C, int M, int N, int K,
   // bit 0x1000 of the tile-width hint: the caller chains this GEMM into a decode step (see `pdl` below)
   const bool chain = (bn_hint & 0x1000) != 0;
   bn_hint &= 0xfff;
-  // Two CTAs per tile (gemm_pair.cu), unless the product is small: short K loops over few tiles do not repay the pair's set-up
-  // (256 x 256 x 256: 8 us here, 10 us there; 1024 x 512 columns, 700 rows: 10 and 12 us), long ones do at any M (16 x 12288 x 4096: 47
-  // and 33 us; 637 x 4096 x 11008: 115 and 66 us; 8192 x 22016 x 4096: 1233 and 1003 us). Added gradients always go there: this kernel
-  // reads and writes them a row per thread (4096 x 4096, 637 tokens: 132 and 48 us). With a workspace (decode) up to 128 rows stay
-  // here, where split K keeps every SM on the weights; beyond, a second row tile would stream them twice (256 x 22016 x 4096: 77 and 50 us).
+  // Two CTAs per tile (gemm_pair.cu) or one (this kernel)? Times are us here and there.
+  //  * Pairs: long K loops over few tiles (16 x 12288 x 4096: 42 and 22; 637 x 4096 x 11008: 115 and 66), and many tiles (8192 x 22016 x 4096:
+  //    1233 and 1003; 512 x 12288 x 128: 13 and 8). Short loops over few tiles do not repay the set-up (256 x 256 x 256: 8 and 10); with B stored
+  //    [K, N], whose tiles are 128 columns at least, that goes up to K = 2048 (1500 x 256 x 1024: 8.6 and 9.4).
+  //  * Here: rows that leave the pair's last row tile half empty and cost it a wave more than a single CTA's tiles of 128 x 256
+  //    (300 x 22016 x 11008: 153 and 176; 640 rows: 231 and 254; but 400 rows: 211 and 180).
+  //  * Here: up to 128 rows where tiles of 128 columns fill the SMs anyway (16 x 32000 x 2048: 27 and 33) or K is short (16 x 22016 x 512: 9 and 10),
+  //    and a few rows or a short K in between (1 x 4096 x 4096: 21 and 26; 32 x 4096 x 1024: 7.5 and 8.2; but 16 x 4096 x 11008: 51 and 40).
+  //  * Added gradients always go to the pairs: this kernel reads and writes them a row per thread (4096 x 4096, 637 tokens: 132 and 48).
+  //  * With a workspace (decode) up to 128 rows stay here, where split K keeps every SM on the weights; beyond, a second row tile would stream
+  //    them twice (256 x 22016 x 4096: 77 and 50).
   const bool split_k = workspace != nullptr && !out_fp32 && !accumulate && M <= 2 * BM;
   if (bn_hint == 0 && gate.flags == nullptr && (!split_k || M > BM)) {
-    const int wide = ((M + 255) / 256) * ((N + 255) / 256);
-    if ((out_fp32 && accumulate) || K >= 1024 || wide >= g_num_sms / 4) {
+    const int cols = (N + 255) / 256, wide = ((M + 255) / 256) * cols;
+    const int waves = ((M + BM - 1) / BM * cols + g_num_sms - 1) / g_num_sms, pair_waves = (wide + g_num_sms / 2 - 1) / (g_num_sms / 2);
+    const bool deep = K >= (transB ? 2048 : 1024);
+    const bool few = N >= g_num_sms * 128 || (N >= 2048 && N < 8192 && (M < 8 || K < 2048));       // of up to 128 rows
+    const bool half_empty = K >= 2048 && waves >= 2 && 3 * pair_waves >= 4 * waves;
+    if ((out_fp32 && accumulate) || (M <= BM ? deep && !few : (deep || wide >= g_num_sms / 4) && (split_k || !half_empty))) {
       const PairPlan plan = pair_plan(M, N, K, transB, out_fp32 != 0, split_k ? workspace_elems : 0, g_num_sms);
       const int pdl = (split_k || chain) ? pdl_enabled() : 0;
       if (plan.splits == 1)
@@ -648,8 +658,11 @@ extern "C" int rpeg_gemm_swiglu(const void* A, const void* W, void* C, int M, in
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
-  // up to 128 rows a pair's tile would be half empty
-  if (M > BM) return gemm_pair_swiglu(A, W, C, M, f, K, lda, ldw, ldc, g_num_sms, status, stream);
+  // Pairs, unless this kernel's tiles are one wave (512 rows, f = 4096, K = 2048: 15 us here, 16 there; 640: 26 and 25), K is short (2000 rows, f =
+  // 11008, K = 256: 32 and 35) or a half-empty last row tile costs the pairs a wave more (300 rows, f = 11008, K = 4096: 60 and 67; 400: 82 and 69).
+  const int tiles = ((M + BM - 1) / BM) * (f / 128), pair_tiles = ((M + 2 * BM - 1) / (2 * BM)) * (f / 128), half = g_num_sms / 2;
+  if (K >= 1024 && tiles > g_num_sms && (pair_tiles + half - 1) / half <= (tiles + g_num_sms - 1) / g_num_sms)
+    return gemm_pair_swiglu(A, W, C, M, f, K, lda, ldw, ldc, g_num_sms, status, stream);
   CUtensorMap ta, tb;
   int rc = make_tmap_bf16_2d(&ta, A, K, M, lda, BK, BM);
   if (rc) return rc;
@@ -662,15 +675,14 @@ extern "C" int rpeg_gemm_swiglu(const void* A, const void* W, void* C, int M, in
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) != cudaSuccess) return -20;
     configured = true;
   }
-  const int tiles = ((M + BM - 1) / BM) * (f / 128);
   const int grid = tiles < g_num_sms ? tiles : g_num_sms;
   kern<<<grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream>>>(ta, tb, C, M, f, K, ldc, 0, 1, 0, status, WeightGate{nullptr, 0, 0u, 0ull}, 0, BM);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
 // Skinny GEMM that leaves its split-K partials for the consumer: C_s[M,N] (fp32, s = 0..splits-1, `M*N`
-// apart in `workspace`) with sum_s C_s = A[M,K] * B[N,K]^T. The split count is chosen by the same cost
-// model as rpeg_gemm_bf16 and returned in *k_splits_out; kernels that read the result (RMSNorm, SwiGLU,
+// apart in `workspace`) with sum_s C_s = A[M,K] * B[N,K]^T. The split count is chosen by a cost model like that of
+// rpeg_gemm_bf16, with a tile width and a weight of the slabs of its own, and returned in *k_splits_out; kernels that read the result (RMSNorm, SwiGLU,
 // RoPE + KV append for decode) add the partials while they load them, so the separate reduction pass
 // and its round trip through memory disappear.
 extern "C" int rpeg_gemm_bf16_partials(const void* A, const void* B, int M, int N, int K, int lda, int ldb,
@@ -696,8 +708,9 @@ extern "C" int rpeg_gemm_bf16_partials(const void* A, const void* B, int M, int 
     return gemm_pair(A, B, workspace, M, N, K, lda, ldb, N, 0, 0, 1, 0, plan, g_num_sms, pdl_enabled(), status, stream);
   }
   // Few rows: the wide tile, fewest reads of A. From 33 rows on the slabs weigh as much as that, and the narrow tile needs half as many to fill
-  // the SMs and stores one half while it multiplies the other (with the kernel that adds the slabs; 128 rows: 4096 x 4096 18.5 us at 256,
-  // 15.6 us at 128 columns, 12288 x 4096 34.7 and 30.9; 64 rows: 5120 x 4096 18.5 and 16.8, but 22016 x 4096 43.5 and 44.1; 16 rows: 12.2 and 12.7).
+  // the SMs and stores one half while it multiplies the other. With the kernel that adds the slabs, K = 4096, us at 256 and at 128 columns: 33 / 64 /
+  // 128 rows of 4096 14.3 and 13.2 / 15.7 and 14.2 / 19.1 and 16.1; of 12288 25.7 and 24.4 / 28.3 and 26.9 / 34.5 and 31.1; of 16384 29.3 and 30.2 /
+  // 31.3 and 31.2 / 36.5 and 33.7; of 20480 38.4 and 41.3 / 43.1 and 44.7 / 53.2 and 49.0: up to 64 rows they change over about 16384.
   const bool narrow = M > 32 && (M > 64 || N <= 16384);
   const int bn = N >= 256 && !narrow ? 256 : (N >= 128 ? 128 : (N >= 64 ? 64 : 32));
   const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);
@@ -711,7 +724,8 @@ extern "C" int rpeg_gemm_bf16_partials(const void* A, const void* B, int M, int 
     if ((num_kb + kb_per - 1) / kb_per != sp) continue;
     if (workspace_elems / per_split < sp) break;
     const int waves = (tiles * sp + g_num_sms - 1) / g_num_sms;
-    // the consumer reads every partial once; no separate reduction pass writes and re-reads them
+    // The consumer reads every partial once; no separate reduction pass writes and re-reads them. A narrow tile's slabs weigh twice as much
+    // (128 rows of 22016: two of them 50.2 us, the four that the lower weight chooses 56.8; up to 64 rows both choose the same).
     const double cost = waves * (kb_per + 2.0) + sp * per_split * (narrow ? 16.0 : 8.0) / block_bytes;
     if (cost < best - 1e-9) { best = cost; want = sp; }
   }
