@@ -385,9 +385,9 @@ __device__ __forceinline__ float logit_at(const float* p) { return *p; }
 
 // One CTA per row; a decode step waits for it. Eight logits a turn: their maximum first, so that their exponentials do not wait for one
 // another (one at a time in 256 threads: 32000 bf16 logits 8.2 us greedy and 18.6 us with noise, now 4.9 and 9.8; 256 rows 54 us with noise, now 20).
-constexpr int SAMPLE_THREADS = 1024;
-template <typename T>
-__global__ void __launch_bounds__(SAMPLE_THREADS)
+// THREADS: 1024, or 256 below 8192 logits, which are at most four turns of them (256 rows of 1000: 4.9 us with 1024, 3.1 with 256).
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 sample_kernel(const T* __restrict__ logits, int V, int ld, float inv_temp, int greedy,
               unsigned long long seed, const unsigned long long* __restrict__ seed_offset,
               const int* __restrict__ forced, int* __restrict__ token_out, float* __restrict__ logp_out) {
@@ -434,7 +434,7 @@ sample_kernel(const T* __restrict__ logits, int V, int ld, float inv_temp, int g
     const uint4* lv = reinterpret_cast<const uint4*>(lr);
     const int nvec = V >> 3;
 #pragma unroll 2
-    for (int j = threadIdx.x; j < nvec; j += SAMPLE_THREADS) {
+    for (int j = threadIdx.x; j < nvec; j += THREADS) {
       float x[8];
       if constexpr (PER == 8) {
         const uint4 a = lv[j];
@@ -453,9 +453,9 @@ sample_kernel(const T* __restrict__ logits, int V, int ld, float inv_temp, int g
       }
       take8(j * 8, x);
     }
-    for (int i = (nvec << 3) + threadIdx.x; i < V; i += SAMPLE_THREADS) take(i, logit_at(lr + i));
+    for (int i = (nvec << 3) + threadIdx.x; i < V; i += THREADS) take(i, logit_at(lr + i));
   } else {
-    for (int i = threadIdx.x; i < V; i += SAMPLE_THREADS) take(i, logit_at(lr + i));
+    for (int i = threadIdx.x; i < V; i += THREADS) take(i, logit_at(lr + i));
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   auto best_of_warp = [&]() {
@@ -470,8 +470,8 @@ sample_kernel(const T* __restrict__ logits, int V, int ld, float inv_temp, int g
   if (lane == 0) { sm_best[warp] = best; sm_idx[warp] = best_i; }
   block_lse(m, s, sm_m, sm_s);  // contains __syncthreads
   if (warp == 0) {
-    best = sm_best[lane];
-    best_i = sm_idx[lane];
+    best = lane < THREADS / 32 ? sm_best[lane] : -INFINITY;
+    best_i = lane < THREADS / 32 ? sm_idx[lane] : 0x7fffffff;
     best_of_warp();
     if (lane == 0) {
       if (forced != nullptr && forced[row] >= 0) best_i = forced[row];
@@ -700,7 +700,8 @@ template <typename T>
 static int launch_sample(const void* logits, int B, int V, int ld, float temperature, int greedy, unsigned long long seed,
                          const unsigned long long* seed_offset, const int* forced, int* token_out, float* logp_out, void* stream) {
   if (B <= 0) return 0;
-  launch_pdl(sample_kernel<T>, dim3(B), dim3(SAMPLE_THREADS), 0, STREAM(stream), static_cast<const T*>(logits), V, ld, 1.f / temperature,
+  const bool few = V < 8192;
+  launch_pdl(few ? sample_kernel<T, 256> : sample_kernel<T, 1024>, dim3(B), dim3(few ? 256 : 1024), 0, STREAM(stream), static_cast<const T*>(logits), V, ld, 1.f / temperature,
              greedy, seed, seed_offset, forced, token_out, logp_out);
   return LAUNCH_OK();
 }
