@@ -529,7 +529,8 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ buf, const int* __restri
 
 // The same for heads of 16 columns or a multiple, everything on 16-byte boundaries: a thread turns 8 pairs of up to ROPE_HEADS heads, whose
 // angles it reads once. Bound by reading and writing the heads (one pair of words a thread: 6900 tokens x 64 heads 77 us, now 36, 6.3 TB/s; 10356 tokens 113 and 52 us).
-constexpr int ROPE_HEADS = 4;
+// From ROPE_WIDE_MIN threads on: fewer leave SMs idle, and then a thread's longer chain shows (100 tokens x 8 heads 1.8 and 2.4 us, 1000 x 2 1.8 and 2.3).
+constexpr int ROPE_HEADS = 4, ROPE_WIDE_MIN = 20000;
 __global__ void __launch_bounds__(256)
 rope_wide_kernel(__nv_bfloat16* __restrict__ buf, const int* __restrict__ pos, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                  int T, int ld, int col0, int nheads, int hd, float sign) {
@@ -775,8 +776,8 @@ extern "C" int rpeg_rope(void* buf, const int* pos, const float* cos_t, const fl
   const float sign = backward ? -1.f : 1.f;
   __nv_bfloat16* b = static_cast<__nv_bfloat16*>(buf);
   const bool aligned = !((reinterpret_cast<uintptr_t>(buf) | reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t)) & 15);
-  if (aligned && (hd & 15) == 0 && ((ld | col0) & 7) == 0) {
-    const long long m = static_cast<long long>(T) * ((nheads + ROPE_HEADS - 1) / ROPE_HEADS) * (hd >> 4);
+  const long long m = static_cast<long long>(T) * ((nheads + ROPE_HEADS - 1) / ROPE_HEADS) * (hd >> 4);
+  if (aligned && (hd & 15) == 0 && ((ld | col0) & 7) == 0 && m >= ROPE_WIDE_MIN) {
     rope_wide_kernel<<<static_cast<unsigned>((m + 255) / 256), 256, 0, STREAM(stream)>>>(b, pos, cos_t, sin_t, T, ld, col0, nheads, hd, sign);
     return LAUNCH_OK();
   }
