@@ -153,7 +153,7 @@ def bench_non_gemm(dev, batch: int = 64, seq: int = 640) -> Dict[str, float]:
     cu = torch.arange(0, T + 1, seq, device=dev, dtype=torch.int32)
     cos_t, sin_t = K.rope_tables(seq, hd, 10000.0, dev)
     t_norm = timed(lambda: K.rmsnorm_fwd(x, w, 1e-5, residual=x, want_sum=True))
-    t_rope = timed(lambda: (K.rope_(qkv, pos, cos_t, sin_t, 0, H, hd), K.rope_(qkv, pos, cos_t, sin_t, d, H, hd)))
+    t_rope = timed(lambda: K.rope_(qkv, pos, cos_t, sin_t, 0, 2 * H, hd))      # queries and keys side by side, as the model turns them
     t_act = timed(lambda: K.swiglu_fwd(gu))
     t_attn = timed(lambda: K.flash_attn_fwd(qkv, 0, d, 2 * d, cu, seq, H, H, hd))
     return {"non_gemm_constant": 2 * t_norm, "non_gemm_scaling": t_rope + t_act + t_attn, "non_gemm_batch_cal": float(batch),
