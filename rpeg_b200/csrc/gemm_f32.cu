@@ -4,8 +4,8 @@
 // mixture, see moe.cu for the segment layout and the activations); or batched: the same product for every head, at fixed
 // strides, with B either [N, K] or [K, N].
 //
-// Two kernels. gemm_f32_kernel: 64 x 64 tiles, bound by the FMA rate once M fills them. gemm_f32_rows_kernel: up to SR_MAX rows
-// (decode), bound by streaming B once from memory.
+// Two kernels. gemm_f32_kernel: 64 x 64 tiles, bound by the FMA rate once M fills them. gemm_f32_rows_kernel: up to SR_ROWS rows
+// (decode), bound by streaming B from memory, once for every SR_MAX rows.
 #include "act_io.cuh"
 #include "moe_segments.cuh"
 #include "rpeg_kernels.h"
@@ -53,31 +53,35 @@ gemm_f32_kernel(const GemmF32 p) {
   const int m0 = blockIdx.y * SG_T, n0 = blockIdx.x * SG_T;
   if (m0 >= M) return;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  // what this thread carries of a slice: of row lr, columns lk + 16 v .. + 3 of A and B; of B stored [K, N], columns 4 (tid % 16) .. of the
-  // rows tid / 16 + 16 v
-  const int lr = tid >> 2, lk = (tid & 3) * 4;
+  // What this thread carries of a slice. VEC: of row tid / 4, four columns in a row. Otherwise one float of each of four rows, side by side over
+  // the threads (four in a row per thread took 1000 rows, N = 2048, K = 2050 from 308 to 362 us); of B stored [K, N] as well.
+  const int vr = tid >> 2, vk = (tid & 3) * 4;
   float ra[NV][4], rb[NB][NV][4];
   auto row4 = [&](const float* base, bool live, int k, float (&v)[4]) {
-    if constexpr (VEC) {
-      const float4 t = live && k < p.K ? load4(base + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = live && k + i < p.K ? base[k + i] : 0.f;
-    }
+    const float4 t = live && k < p.K ? load4(base + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
   };
   auto fetch = [&](int k0) {
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-      row4(a + static_cast<size_t>(m0 + lr) * p.lda, m0 + lr < M, k0 + lk + 16 * v, ra[v]);
-      if constexpr (MODE == SG_BATCHED_KN) {
-        const int n = n0 + tx * 4, k = k0 + ty + 16 * v;
-        const float* src = B + static_cast<size_t>(k) * p.ldb;
+      if constexpr (VEC) {
+        row4(a + static_cast<size_t>(m0 + vr) * p.lda, m0 + vr < M, k0 + vk + 16 * v, ra[v]);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) rb[0][v][i] = n + i < p.N && k < p.K ? src[n + i] : 0.f;
+        for (int g = 0; g < NB; ++g) row4(B + (static_cast<size_t>(g) * p.N + n0 + vr) * p.ldb, n0 + vr < p.N, k0 + vk + 16 * v, rb[g][v]);
       } else {
+        const int k = k0 + 16 * v + tx;
 #pragma unroll
-        for (int g = 0; g < NB; ++g) row4(B + (static_cast<size_t>(g) * p.N + n0 + lr) * p.ldb, n0 + lr < p.N, k0 + lk + 16 * v, rb[g][v]);
+        for (int i = 0; i < 4; ++i) {
+          const int r = ty + 16 * i;
+          ra[v][i] = m0 + r < M && k < p.K ? a[static_cast<size_t>(m0 + r) * p.lda + k] : 0.f;
+          if constexpr (MODE == SG_BATCHED_KN) {
+            const int n = n0 + (tid & 63), kk = k0 + 16 * v + (tid >> 6) + 4 * i;
+            rb[0][v][i] = n < p.N && kk < p.K ? B[static_cast<size_t>(kk) * p.ldb + n] : 0.f;
+          } else {
+#pragma unroll
+            for (int g = 0; g < NB; ++g) rb[g][v][i] = n0 + r < p.N && k < p.K ? B[(static_cast<size_t>(g) * p.N + n0 + r) * p.ldb + k] : 0.f;
+          }
+        }
       }
     }
   };
@@ -86,11 +90,12 @@ gemm_f32_kernel(const GemmF32 p) {
     for (int v = 0; v < NV; ++v)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        as[buf][lk + 16 * v + i][lr] = ra[v][i];
+        const int k = 16 * v + (VEC ? vk + i : tx), r = VEC ? vr : ty + 16 * i;
+        as[buf][k][r] = ra[v][i];
 #pragma unroll
         for (int g = 0; g < NB; ++g) {
-          if constexpr (MODE == SG_BATCHED_KN) bs[buf][g][ty + 16 * v][tx * 4 + i] = rb[g][v][i];
-          else bs[buf][g][lk + 16 * v + i][lr] = rb[g][v][i];
+          if constexpr (MODE == SG_BATCHED_KN) bs[buf][g][16 * v + (tid >> 6) + 4 * i][tid & 63] = rb[g][v][i];
+          else bs[buf][g][k][r] = rb[g][v][i];
         }
       }
   };
