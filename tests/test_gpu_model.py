@@ -207,7 +207,8 @@ def test_shared_prompts_with_many_ragged_tails(cuda_device, limit):
     cfg = LlamaConfig.tiny(n_layers=2)
     model = LlamaModel(cfg, cuda_device, seed=9)
     P, Kq, S = 20, 3, 75
-    prompts = torch.randint(2, cfg.vocab, (P, S), device=cuda_device, dtype=torch.int32).repeat_interleave(Kq, dim=0).contiguous()
+    g = torch.Generator(device=cuda_device).manual_seed(P)
+    prompts = torch.randint(2, cfg.vocab, (P, S), generator=g, device=cuda_device, dtype=torch.int32).repeat_interleave(Kq, dim=0).contiguous()
     gen = Generator(model, max_slots=64, max_seq_len=S + 24, kv_budget_bytes=1e9, eos_id=1)
     plain = gen.generate(prompts, 24, greedy=True)
     if limit is not None:
