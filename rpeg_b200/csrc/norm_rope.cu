@@ -407,9 +407,10 @@ __device__ __forceinline__ void load_partials8(const float* __restrict__ parts, 
 
 // y = rmsnorm(sum_s parts[s] [+ res]) * w; h_out (optional) = the bf16 sum, i.e. the new residual stream.
 // One CTA per row, four columns a thread and turn: a decode step waits for this kernel, and what it waits for is one round trip to L2, so all
-// slabs of a row are requested at once (256 threads with 16 columns each took the slabs one after the other: 1 row 4.3 us, now 3.0; 16 rows 4.6 and 3.2; nine slabs, chained).
+// slabs of a row are requested at once (256 threads with 16 columns each took the slabs one after the other: 1 row 4.1 us, now 2.6; 16 rows 4.3 and 2.6; nine slabs
+// of 4096 columns, chained; one slab 2.5 and 1.7).
 template <int NV>
-__global__ void __launch_bounds__(1024)
+__global__ void __launch_bounds__(NV <= 2 ? 1024 : 256)
 rmsnorm_fwd_partials_kernel(const float* __restrict__ parts, int splits, long long stride,
                             const __nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ w,
                             __nv_bfloat16* __restrict__ h_out, __nv_bfloat16* __restrict__ y, int d, float eps) {
@@ -421,23 +422,42 @@ rmsnorm_fwd_partials_kernel(const float* __restrict__ parts, int splits, long lo
   griddep_wait();   // may have been scheduled under the previous kernel's tail: nothing is read or written before this
   float4 v[NV];
   uint2 r[NV], wv[NV];
+  auto slab = [&](int s, int c) { return *reinterpret_cast<const float4*>(parts + s * stride + row0 + c); };
+  auto add = [](float4& x, const float4& y) { x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w; };
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
     const int c = (threadIdx.x + k * blockDim.x) * 4;
-    v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     r[k] = wv[k] = make_uint2(0u, 0u);
+    v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (c < d) {
       wv[k] = *reinterpret_cast<const uint2*>(w + c);
       if (res) r[k] = *reinterpret_cast<const uint2*>(res + row0 + c);
-      for (int s0 = 0; s0 < splits; s0 += 8) {
-        float4 a[8];
+      v[k] = slab(0, c);
+    }
+  }
+  if (splits == 2) {
+    float4 a[NV];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-          if (s0 + i < splits) a[i] = *reinterpret_cast<const float4*>(parts + (s0 + i) * stride + row0 + c);
+    for (int k = 0; k < NV; ++k) {
+      const int c = (threadIdx.x + k * blockDim.x) * 4;
+      a[k] = c < d ? slab(1, c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-          if (s0 + i < splits) { v[k].x += a[i].x; v[k].y += a[i].y; v[k].z += a[i].z; v[k].w += a[i].w; }
-      }
+    for (int k = 0; k < NV; ++k) add(v[k], a[k]);
+  } else if (splits > 2) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const int c = (threadIdx.x + k * blockDim.x) * 4;
+      if (c < d)
+        for (int s0 = 1; s0 < splits; s0 += 8) {
+          float4 a[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if (s0 + i < splits) a[i] = slab(s0 + i, c);
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if (s0 + i < splits) add(v[k], a[i]);
+        }
     }
   }
   __syncthreads();                                 // warp_ss is cleared
@@ -750,11 +770,13 @@ extern "C" int rpeg_rmsnorm_fwd_partials(const float* parts, int splits, long lo
   if (T <= 0) return 0;
   const __nv_bfloat16 *rp = static_cast<const __nv_bfloat16*>(res), *wp = static_cast<const __nv_bfloat16*>(w);
   __nv_bfloat16 *hp = static_cast<__nv_bfloat16*>(h_out), *yp = static_cast<__nv_bfloat16*>(y);
-  const int nv = (d / 4 + 1023) / 1024;
+  if (d > 8192) return -3;
+  // More rows than SMs, of one or two slabs: 256 threads, so that an SM holds more rows (256 rows of 4096, one slab: 4.3 us in 1024 threads, 2.3 in 256;
+  // 128 rows, two slabs: 2.3 and 2.7).
+  const int most = T > 148 && splits <= 2 ? 256 : 1024, per = (d / 4 + most - 1) / most, nv = per <= 2 ? per : per <= 4 ? 4 : 8;
   const dim3 block(((d / 4 + nv - 1) / nv + 31) & ~31);
-  if (nv == 1) launch_pdl(rmsnorm_fwd_partials_kernel<1>, dim3(T), block, 0, STREAM(stream), parts, splits, stride, rp, wp, hp, yp, d, eps);
-  else if (nv == 2) launch_pdl(rmsnorm_fwd_partials_kernel<2>, dim3(T), block, 0, STREAM(stream), parts, splits, stride, rp, wp, hp, yp, d, eps);
-  else return -3;
+  auto kern = nv == 1 ? rmsnorm_fwd_partials_kernel<1> : nv == 2 ? rmsnorm_fwd_partials_kernel<2> : nv == 4 ? rmsnorm_fwd_partials_kernel<4> : rmsnorm_fwd_partials_kernel<8>;
+  launch_pdl(kern, dim3(T), block, 0, STREAM(stream), parts, splits, stride, rp, wp, hp, yp, d, eps);
   return LAUNCH_OK();
 }
 

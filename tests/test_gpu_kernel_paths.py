@@ -230,8 +230,8 @@ def test_rope_widths(cuda_device, t, heads, hd, col0, off, backward):
 
 
 @pytest.mark.parametrize("rows,d,splits", [(1, 8, 1), (3, 136, 9), (2, 4096, 9), (5, 4104, 17), (200, 2048, 2), (2, 8192, 8),
-                                           # 64 rows of up to two slabs: 256 threads with one, two, four or eight groups of columns
-                                           (63, 4096, 2), (64, 136, 1), (64, 1032, 2), (65, 4096, 1), (64, 5120, 2), (64, 8192, 1), (64, 4096, 3)])
+                                           # more rows than SMs of up to two slabs: 256 threads with one, two, four or eight groups of columns
+                                           (148, 4096, 2), (149, 136, 1), (149, 1032, 2), (150, 4096, 1), (149, 5120, 2), (149, 8192, 1), (149, 4096, 3)])
 @pytest.mark.parametrize("residual", [True, False])
 def test_rmsnorm_partials_rows(cuda_device, rows, d, splits, residual):
     g = torch.Generator(device=cuda_device).manual_seed(d)
