@@ -1,0 +1,346 @@
+// Paged decode attention for rows that alias pages (the samples of one prompt share its pages): a key is read once for up to eight queries.
+//
+// A CTA owns eight query columns: the G query heads of one KV head times 8 / G neighbouring rows. It lists the 16-key blocks that any of its rows
+// sees, a physical page that several rows share once, with the columns it is for; its warps take turns at the list. A block is scored against all
+// eight columns by mma.m16n8k16 with the KEYS on the M axis,
+//     S^T [16 keys x 8] = K [16 x 128] Q^T,      O^T [128 x 8] += V^T [128 x 16] P^T,
+// on fragments that are loaded straight from the pages: a lane's 16-byte chunks of K are two k steps each (the order of the head dimensions inside
+// a step is free, Q has the same), V's keys 2t, 2t + 1, 2t + 8, 2t + 9 are paired by byte permutes, P^T turns by movmatrix. Every warp keeps its own
+// softmax state for the eight columns; the four are merged at the end, splits by the last one to arrive.
+//
+// P stays fp32: it enters the product as three bf16 parts (8 + 8 + 8 bits, exact). Columns a block is not for are neither scored nor added to, so
+// what one row holds (infinities, NaN) never reaches another.
+//
+// Bound by the bytes of the pages; the row kernel (decode_attn.cu) reads the shared ones once per row, from L2.
+#include <cmath>
+#include "common.cuh"
+#include "rpeg_kernels.h"
+
+namespace rpeg {
+
+constexpr int DP_PAGE = RPEG_KV_PAGE, DP_HD = 128, DP_COLS = 8, DP_WARPS = 4, DP_THREADS = DP_WARPS * 32;
+constexpr int DP_WINDOW = 32;                                // logical pages listed at a time
+constexpr int DP_LIST = DP_WINDOW * DP_COLS * (DP_PAGE / 16);
+constexpr int DP_ITEMS = 1 << 16;
+static_assert(DP_PAGE == 64, "a page is four blocks");
+
+// Arrival counters of the splits of an item, zero between launches; launches of one GPU that split run in stream order.
+__device__ int g_packed_arrive[DP_ITEMS];
+
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t v) {
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
+}
+// The leading bf16 parts of two numbers; `a` and `b` keep the (exact) remainders.
+__device__ __forceinline__ uint32_t take_bf16x2(float& a, float& b) {
+  const uint32_t x = __float_as_uint(a), y = __float_as_uint(b);
+  a -= __uint_as_float(x & 0xffff0000u);
+  b -= __uint_as_float(y & 0xffff0000u);
+  return __byte_perm(x, y, 0x7632);
+}
+
+template <int G>
+__global__ void __launch_bounds__(DP_THREADS, 3)
+paged_decode_attn_packed_kernel(const __nv_bfloat16* __restrict__ q, int ldq, int q_col0, const __nv_bfloat16* __restrict__ kcache,
+                                const __nv_bfloat16* __restrict__ vcache, const int* __restrict__ page_table, int max_pages,
+                                const int* __restrict__ seq_lens, __nv_bfloat16* __restrict__ out, float* __restrict__ partial, int B, int H,
+                                int Hkv, int nsplit, float scale_log2) {
+  griddep_launch();
+  griddep_wait();   // may have been scheduled under the previous kernel's tail: nothing is read or written before this
+  __shared__ int2 list[DP_LIST];                             // first cache row of a block; its first key | columns << 24 | keys - 1
+  __shared__ int lens_s[DP_COLS], warp_total[DP_WARPS], is_last;
+  __shared__ float red_m[DP_WARPS][DP_COLS], red_l[DP_WARPS][DP_COLS];
+  __shared__ __align__(16) float red_o[DP_WARPS][DP_COLS][DP_HD];
+  constexpr int rows = DP_COLS / G;
+  const int hk = blockIdx.x, row0 = blockIdx.y * rows, split = blockIdx.z;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  if (tid < DP_COLS) lens_s[tid] = tid < rows && row0 + tid < B ? seq_lens[row0 + tid] : 0;
+  const int pr = tid & 7, pi = tid >> 3;                     // this thread's row and page in a listing
+  const int* table = page_table + static_cast<size_t>(min(row0 + pr, B - 1)) * max_pages;
+  int pages[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) pages[i] = pr < rows && pi + 16 * i < max_pages ? table[pi + 16 * i] : 0;
+  // query column g: head hk G + g % G of row g / G
+  uint32_t qf[16];
+  {
+    const int r = min(row0 + g / G, B - 1);
+    const uint4* src = reinterpret_cast<const uint4*>(q + static_cast<size_t>(r) * ldq + q_col0 + (hk * G + g % G) * DP_HD + t * 8);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const uint4 v = src[c * 4];
+      qf[c * 4] = v.x; qf[c * 4 + 1] = v.y; qf[c * 4 + 2] = v.z; qf[c * 4 + 3] = v.w;
+    }
+  }
+  __syncthreads();
+  const int len0 = lens_s[2 * t / G], len1 = lens_s[(2 * t + 1) / G];     // of this lane's columns 2t, 2t + 1
+  int longest = 0, live = 0;
+#pragma unroll
+  for (int c = 0; c < DP_COLS; ++c) {
+    const int n = lens_s[c / G];
+    longest = max(longest, n);
+    live |= (n > 0 ? 1 : 0) << c;
+  }
+  const int n_pages = min(max_pages, (longest + DP_PAGE - 1) / DP_PAGE);
+
+  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+  float acc[8][4] = {};                                      // [i]: dimensions 8g + i (columns 2t, 2t + 1) and 64 + 8g + i
+  for (int w0 = 0; w0 < n_pages; w0 += DP_WINDOW) {
+    // ---- list the window's blocks
+    int count[2], mask[2], keys[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int page = w0 + pi + 16 * i, left = lens_s[pr] - page * DP_PAGE;
+      if (w0 > 0) pages[i] = pr < rows && page < n_pages ? table[page] : 0;
+      const int own = pr < rows && page < n_pages ? max(0, min(left, DP_PAGE)) : 0;      // keys of this page that the row sees
+      int most = own, cols = 0;
+      bool first = own > 0;
+#pragma unroll
+      for (int r = 0; r < rows; ++r) {                       // rows with the same page
+        const int o = __shfl_sync(0xffffffffu, own, (lane & 24) | r), other = __shfl_sync(0xffffffffu, pages[i], (lane & 24) | r);
+        if (o > 0 && other == pages[i]) {
+          most = max(most, o);
+          cols |= ((1 << G) - 1) << (r * G);
+          first = first && r >= pr;
+        }
+      }
+      keys[i] = most;
+      mask[i] = cols;
+      count[i] = first ? (most + 15) / 16 : 0;
+    }
+    int at = count[0] + count[1];
+    const int mine = at;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, at, o);
+      if (lane >= o) at += u;
+    }
+    if (lane == 31) warp_total[warp] = at;
+    __syncthreads();
+    at -= mine;
+    int total = 0;
+#pragma unroll
+    for (int w = 0; w < DP_WARPS; ++w) {
+      if (w < warp) at += warp_total[w];
+      total += warp_total[w];
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int key0 = (w0 + pi + 16 * i) * DP_PAGE, first = (pages[i] * Hkv + hk) * DP_PAGE;
+      for (int k = 0; k < count[i]; ++k)
+        list[at++] = make_int2(first + 16 * k, static_cast<int>(static_cast<uint32_t>(mask[i]) << 24) | (key0 + 16 * k) | (min(16, keys[i] - 16 * k) - 1));
+    }
+    __syncthreads();
+    const int lo = static_cast<int>(static_cast<long long>(total) * split / nsplit), hi = static_cast<int>(static_cast<long long>(total) * (split + 1) / nsplit);
+
+    // ---- this warp's blocks: K of the next one is requested behind the scores, V behind the averages
+    uint4 kv[8], vv[4][2];
+    auto load_k = [&](int row) {
+      const uint4* p = reinterpret_cast<const uint4*>(kcache + (static_cast<size_t>(row) + g) * DP_HD + t * 8);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        kv[c] = p[c * 4];
+        kv[4 + c] = p[8 * (DP_HD / 8) + c * 4];
+      }
+    };
+    auto load_v = [&](int row) {
+      const uint4* p = reinterpret_cast<const uint4*>(vcache + (static_cast<size_t>(row) + 2 * t) * DP_HD + g * 8);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) vv[j][c] = p[((j & 1) + (j >> 1) * 8) * (DP_HD / 8) + c * 8];
+    };
+    int b = lo + warp;
+    int2 e = make_int2(0, 0);
+    if (b < hi) {
+      e = list[b];
+      load_k(e.x);
+      load_v(e.x);
+    }
+    while (b < hi) {
+      const int next = b + DP_WARPS;
+      const int2 en = next < hi ? list[next] : make_int2(0, 0);
+      const int key0 = e.y & 0xfffff0, valid = (e.y & 15) + 1, cols = static_cast<int>(static_cast<uint32_t>(e.y) >> 24);
+      float s[4] = {}, s2[4] = {};
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        mma_16816(s, kv[c].x, kv[4 + c].x, kv[c].y, kv[4 + c].y, qf[c * 4], qf[c * 4 + 1]);
+        mma_16816(s2, kv[c].z, kv[4 + c].z, kv[c].w, kv[4 + c].w, qf[c * 4 + 2], qf[c * 4 + 3]);
+      }
+      if (next < hi) load_k(en.x);
+      // keys key0 + g (+ 8), columns 2t and 2t + 1
+      const bool c0 = (cols >> (2 * t)) & 1, c1 = (cols >> (2 * t + 1)) & 1;
+      const int ka = key0 + g, kb = ka + 8;
+      const float a0 = c0 && ka < len0 ? (s[0] + s2[0]) * scale_log2 : -INFINITY, a1 = c1 && ka < len1 ? (s[1] + s2[1]) * scale_log2 : -INFINITY;
+      const float b0 = c0 && kb < len0 ? (s[2] + s2[2]) * scale_log2 : -INFINITY, b1 = c1 && kb < len1 ? (s[3] + s2[3]) * scale_log2 : -INFINITY;
+      float x0 = fmaxf(a0, b0), x1 = fmaxf(a1, b1);
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) {
+        x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, o));
+        x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
+      }
+      if (__any_sync(0xffffffffu, x0 > m0 || x1 > m1)) {
+        const float n0 = fmaxf(m0, x0), n1 = fmaxf(m1, x1);
+        const float f0 = n0 == m0 ? 1.f : exp2f(m0 - n0), f1 = n1 == m1 ? 1.f : exp2f(m1 - n1);
+        l0 *= f0; l1 *= f1;
+        m0 = n0; m1 = n1;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { acc[i][0] *= f0; acc[i][1] *= f1; acc[i][2] *= f0; acc[i][3] *= f1; }
+      }
+      float pa0 = c0 && ka < len0 ? exp2f(a0 - m0) : 0.f, pa1 = c1 && ka < len1 ? exp2f(a1 - m1) : 0.f;
+      float pb0 = c0 && kb < len0 ? exp2f(b0 - m0) : 0.f, pb1 = c1 && kb < len1 ? exp2f(b1 - m1) : 0.f;
+      l0 += pa0 + pb0;
+      l1 += pa1 + pb1;
+      uint32_t pf[3][2];
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        pf[p][0] = transpose_8x8(take_bf16x2(pa0, pa1));
+        pf[p][1] = transpose_8x8(take_bf16x2(pb0, pb1));
+      }
+      pf[2][0] = transpose_8x8(pack_bf16x2(pa0, pa1));
+      pf[2][1] = transpose_8x8(pack_bf16x2(pb0, pb1));
+      if (valid < 16) {                                      // a row's last block: what lies behind its last key has no weight, whatever it holds
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (2 * t + (j & 1) + (j >> 1) * 8 >= valid) vv[j][0] = vv[j][1] = make_uint4(0u, 0u, 0u, 0u);
+      }
+      const uint32_t* v0 = reinterpret_cast<const uint32_t*>(&vv[0][0]);     // [j][c]: four words each
+      auto fragment = [&](int i, uint32_t (&a)[4]) {
+        const uint32_t pick = i & 1 ? 0x7632 : 0x5410;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) a[k] = __byte_perm(v0[((k >> 1) * 4 + (k & 1)) * 4 + (i >> 1)], v0[((k >> 1) * 4 + 2 + (k & 1)) * 4 + (i >> 1)], pick);
+      };
+      if ((cols & live) == live) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          uint32_t a[4];
+          fragment(i, a);
+#pragma unroll
+          for (int p = 0; p < 3; ++p) mma_16816(acc[i], a[0], a[1], a[2], a[3], pf[p][0], pf[p][1]);
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          uint32_t a[4];
+          fragment(i, a);
+          float d[4] = {};
+#pragma unroll
+          for (int p = 0; p < 3; ++p) mma_16816(d, a[0], a[1], a[2], a[3], pf[p][0], pf[p][1]);
+          acc[i][0] += c0 ? d[0] : 0.f; acc[i][1] += c1 ? d[1] : 0.f; acc[i][2] += c0 ? d[2] : 0.f; acc[i][3] += c1 ? d[3] : 0.f;
+        }
+      }
+      if (next < hi) load_v(en.x);
+      b = next;
+      e = en;
+    }
+    if (w0 + DP_WINDOW < n_pages) __syncthreads();           // the list is rewritten
+  }
+
+  // ---- merge the warps
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) {
+    l0 += __shfl_xor_sync(0xffffffffu, l0, o);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, o);
+  }
+  if (g == 0) {
+    red_m[warp][2 * t] = m0; red_m[warp][2 * t + 1] = m1;
+    red_l[warp][2 * t] = l0; red_l[warp][2 * t + 1] = l1;
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float* dst = &red_o[warp][2 * t + (e & 1)][(e >> 1) * 64 + g * 8];
+    *reinterpret_cast<float4*>(dst) = make_float4(acc[0][e], acc[1][e], acc[2][e], acc[3][e]);
+    *reinterpret_cast<float4*>(dst + 4) = make_float4(acc[4][e], acc[5][e], acc[6][e], acc[7][e]);
+  }
+  __syncthreads();
+  const int col = tid >> 4, d0 = (tid & 15) * 8, row = row0 + col / G;       // eight dimensions of a column per thread
+  float gm = -INFINITY, gl = 0.f, o[8] = {};
+#pragma unroll
+  for (int w = 0; w < DP_WARPS; ++w) gm = fmaxf(gm, red_m[w][col]);
+#pragma unroll
+  for (int w = 0; w < DP_WARPS; ++w) {
+    const float mw = red_m[w][col];
+    if (mw == -INFINITY) continue;                           // a warp that saw no key of this column holds nothing for it
+    const float f = exp2f(mw - gm);
+    gl += red_l[w][col] * f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o[i] += red_o[w][col][d0 + i] * f;
+  }
+  auto store = [&](const float (&v)[8], float l) {
+    uint32_t u[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) u[i] = l > 0.f ? pack_bf16x2(v[2 * i] / l, v[2 * i + 1] / l) : 0u;
+    *reinterpret_cast<uint4*>(out + (static_cast<size_t>(row) * H + hk * G + col % G) * DP_HD + d0) = make_uint4(u[0], u[1], u[2], u[3]);
+  };
+  if (nsplit == 1) {
+    if (row < B) store(o, gl);
+    return;
+  }
+  // partial sums [B H nsplit][128], then (maximum, sum) [B H nsplit][2]
+  const size_t slot0 = (static_cast<size_t>(row) * H + hk * G + col % G) * nsplit;
+  float* ml = partial + static_cast<size_t>(B) * H * nsplit * DP_HD;
+  if (row < B) {
+    float* pp = partial + (slot0 + split) * DP_HD + d0;
+    *reinterpret_cast<float4*>(pp) = make_float4(o[0], o[1], o[2], o[3]);
+    *reinterpret_cast<float4*>(pp + 4) = make_float4(o[4], o[5], o[6], o[7]);
+    if (d0 == 0) *reinterpret_cast<float2*>(ml + (slot0 + split) * 2) = make_float2(gm, gl);
+  }
+  int* arrive = &g_packed_arrive[blockIdx.y * Hkv + hk];
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) is_last = atomicAdd(arrive, 1) == nsplit - 1 ? 1 : 0;
+  __syncthreads();
+  if (!is_last) return;
+  if (tid == 0) *arrive = 0;
+  __threadfence();
+  if (row >= B) return;
+  gm = -INFINITY;
+  gl = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) o[i] = 0.f;
+#pragma unroll 4
+  for (int s = 0; s < nsplit; ++s) {
+    const float2 x = __ldcg(reinterpret_cast<const float2*>(ml + (slot0 + s) * 2));
+    const float4 u = __ldcg(reinterpret_cast<const float4*>(partial + (slot0 + s) * DP_HD + d0));
+    const float4 v = __ldcg(reinterpret_cast<const float4*>(partial + (slot0 + s) * DP_HD + d0 + 4));
+    if (x.x == -INFINITY) continue;
+    const float nm = fmaxf(gm, x.x), f0 = exp2f(gm - nm), f = exp2f(x.x - nm);
+    const float e[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+    gm = nm;
+    gl = gl * f0 + x.y * f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o[i] = o[i] * f0 + e[i] * f;
+  }
+  store(o, gl);
+}
+
+}  // namespace rpeg
+
+using namespace rpeg;
+
+// rpeg_paged_decode_attn for rows that may alias pages; scratch as there. H / Hkv must divide 8.
+extern "C" int rpeg_paged_decode_attn_packed(const void* q, int ldq, int q_col0, const void* kcache, const void* vcache, const int* page_table,
+                                             int max_pages, const int* seq_lens, void* out, float* scratch, int B, int H, int Hkv, int hd, int nsplit,
+                                             float scale, void* stream) {
+  if (hd != DP_HD || Hkv <= 0 || H % Hkv != 0 || H / Hkv > DP_COLS || DP_COLS % (H / Hkv) != 0) return -2;
+  if (nsplit < 1 || nsplit > 64) return -3;
+  if (nsplit > 1 && scratch == nullptr) return -4;
+  if ((ldq | q_col0) & 7) return -5;
+  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache) | reinterpret_cast<uintptr_t>(out) |
+       reinterpret_cast<uintptr_t>(scratch)) & 15) return -1;
+  if (max_pages < 1 || max_pages > (1 << 24) / DP_PAGE) return -6;         // a block's first key has 24 bits
+  if (B <= 0) return 0;
+  const int rows = DP_COLS / (H / Hkv), items = (B + rows - 1) / rows;
+  if (items > 65535 || (nsplit > 1 && static_cast<long long>(items) * Hkv > DP_ITEMS)) return -7;
+  auto kern = H == Hkv ? paged_decode_attn_packed_kernel<1>
+              : H == 2 * Hkv ? paged_decode_attn_packed_kernel<2> : H == 4 * Hkv ? paged_decode_attn_packed_kernel<4> : paged_decode_attn_packed_kernel<8>;
+  return launch_pdl(kern, dim3(Hkv, items, nsplit), dim3(DP_THREADS), 0, reinterpret_cast<cudaStream_t>(stream),
+                    static_cast<const __nv_bfloat16*>(q), ldq, q_col0, static_cast<const __nv_bfloat16*>(kcache),
+                    static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages, seq_lens, static_cast<__nv_bfloat16*>(out), scratch, B, H, Hkv,
+                    nsplit, scale * 1.4426950408889634f) == cudaSuccess ? 0 : -21;
+}

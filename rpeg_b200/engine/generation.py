@@ -82,6 +82,11 @@ class Generator:
     GROUP_MAX = 8              # queries the group attention kernel scores per K/V tile
     GROUP_MIN_BATCH = 128      # the group kernel is one more launch per layer: it pays only while many rows are live
     GROUP_MIN = 3              # smaller groups are cheaper row by row
+    # From this many (row, head) pairs on, and while the keys that rows share weigh this much in what they see, aliased rows are attended to eight at a
+    # time (``K.ALIASED``). us per layer, 32 heads, eight rows a prompt, row by row and so: 512 shared keys and 1 to 48 own ones, 256 rows
+    # 163 and 79, 32 rows 24 and 15, 8 rows 12 and 11; 100 to 500 own ones (0.55 of the keys) 276 and 253; 300 to 1500 (0.32) 583 and 606.
+    ALIASED_MIN_HEADS = 1024
+    ALIASED_MIN_SAVED = 0.4
 
     @staticmethod
     def kv_bytes_for(cfg, slots: int, max_seq_len: int, tp: int = 1) -> int:
@@ -150,6 +155,7 @@ class Generator:
         self.group_shared = torch.zeros(n, **i32)
         self.row_key0 = torch.zeros(n, **i32)
         self._group_state = None
+        self._aliased = False      # whether the next steps read what rows share once for eight of them
         self.token = torch.zeros(n, **i32)
         self.pos = torch.zeros(n, **i32)
         self.seq_len = torch.zeros(n, **i32)
@@ -183,7 +189,9 @@ class Generator:
         # (a tensor-parallel step is made of short kernels at every batch size: always chained)
         # (so is the decode step of a model that asks for it)
         K.set_pdl(b <= getattr(m, "pdl_max_batch", self.PDL_MAX_BATCH) or getattr(m, "tp", 1) > 1)
-        groups = (self.group_rows[:b], self.group_shared[:b], self.row_key0[:b]) if (self.group_attention and b >= self.group_min_batch) else None
+        groups = K.ALIASED if self._aliased else None
+        if self.group_attention and b >= self.group_min_batch:
+            groups = (self.group_rows[:b], self.group_shared[:b], self.row_key0[:b])
         K.set_group_tc(self.group_tc)
         xf = m.decode_step(self.token[:b], self.pos[:b], self.slot_ids[:b], self.seq_len[:b], self.page_table[:b],
                            self.kcache, self.vcache, nsplit=self._nsplit(b), groups=groups)
@@ -201,7 +209,7 @@ class Generator:
             self._decode_body(b, temperature, greedy, seed, top_k, top_p)
             return
         key = (b, self.out_tok.shape[1], float(temperature), bool(greedy), int(seed), self.out_tok.data_ptr(), int(top_k), float(top_p),
-               self.group_attention)
+               self.group_attention, self._aliased)
         g = self._graphs.get(key)
         if g is None:
             # warm up and capture with every slot parked, so neither pass advances real rows
@@ -379,6 +387,7 @@ class Generator:
         if self.zero_cache:
             self.kv_storage.zero_()
         self._group_state = None
+        self._aliased = False
         self.group_shared.zero_()
         self.row_key0.zero_()
         slot_row = [-1] * n
@@ -595,6 +604,11 @@ class Generator:
             b = self._bucket(used)
             if self.group_attention:
                 self._sync_groups(live, slot_row, slot_shared, G)
+            if G > 1 and not self.cached_prefill and not self.group_attention:
+                first = {slot_row[s] // G: slot_shared[s] for s in live}
+                saved = (sum(slot_shared[s] for s in live) - sum(first.values())) * PAGE       # shared keys beyond one reading of each
+                heads = b * getattr(self.model, "n_heads_local", getattr(self.cfg, "n_heads", 1))
+                self._aliased = heads >= self.ALIASED_MIN_HEADS and saved >= self.ALIASED_MIN_SAVED * sum(slot_bound[s] for s in live)
             for _ in range(horizon):
                 self._step(b, temperature, greedy, seed, top_k, top_p)
             counters["decode_steps"] += horizon

@@ -456,12 +456,12 @@ class LlamaModel:
         """One autoregressive step for ``B`` slots: appends this token's K/V to the paged cache at
         ``pos`` and attends over ``seq_len`` cached keys. Returns the final normalised hidden ``[B, d]``.
         All GEMMs have ``M = B <= 256`` and run split-K so every SM streams a slice of the weights.
-        ``groups`` (see ``ops.kernels.paged_decode_attn``) names the rows that share their first KV pages."""
+        ``groups`` (see ``ops.kernels.paged_decode_attn``) says which rows share their first KV pages."""
         cfg, p = self.cfg, self.p
         ws = self._workspace()
         scale = 1.0 / math.sqrt(cfg.head_dim)
         if cfg.qk_norm:
-            return self._decode_step_unfused(token, pos, slot_ids, seq_len, page_table, kcache, vcache, nsplit)
+            return self._decode_step_unfused(token, pos, slot_ids, seq_len, page_table, kcache, vcache, nsplit, groups)
         # Every GEMM leaves its split-K partials in the workspace and the next kernel adds them up while it
         # loads them (one stream, so a consumer always runs before the next GEMM reuses the workspace).
         B = token.shape[0]
@@ -484,7 +484,7 @@ class LlamaModel:
                                           want_sum=not last)
         return x
 
-    def _decode_step_unfused(self, token, pos, slot_ids, seq_len, page_table, kcache, vcache, nsplit: int = 1) -> torch.Tensor:
+    def _decode_step_unfused(self, token, pos, slot_ids, seq_len, page_table, kcache, vcache, nsplit: int = 1, groups=None) -> torch.Tensor:
         """The same step with reduced GEMM outputs (needed when q and k are normalised per head before RoPE)."""
         cfg, p = self.cfg, self.p
         ws = self._workspace()
@@ -502,7 +502,7 @@ class LlamaModel:
             K.rope_kv_append_(qkv, 0, cfg.q_width, cfg.q_width + cfg.kv_width, slot_ids, pos, self.cos_t, self.sin_t,
                               page_table, kcache[i], vcache[i], cfg.n_heads, cfg.n_kv_heads, cfg.head_dim)
             attn = K.paged_decode_attn(qkv, 0, kcache[i], vcache[i], page_table, seq_len, cfg.n_heads, cfg.n_kv_heads,
-                                       cfg.head_dim, scale, nsplit=nsplit)
+                                       cfg.head_dim, scale, nsplit=nsplit, groups=groups)
             o = K.gemm(attn, p[f"l{i}.wo"], workspace=ws)
             x2, _, h1 = K.rmsnorm_fwd(o, p[f"l{i}.mlp_norm"], cfg.rms_eps, residual=h, want_sum=True)
             gu = K.gemm(x2, p[f"l{i}.w_gate_up"], workspace=ws)

@@ -525,6 +525,17 @@ def decode_scratch_numel(B: int, H: int, nsplit: int) -> int:
     return int(lib().rpeg_decode_attn_scratch_bytes(B, H, nsplit)) // 4
 
 
+#: ``paged_decode_attn(groups=ALIASED)``: neighbouring rows of the batch may share pages (the page table tells which)
+ALIASED = "aliased"
+
+
+def packed_decode_splits(B: int, n_heads: int, n_kv_heads: int, pages: int) -> int:
+    """Splits of the kernel for aliased rows: three CTAs an SM, twice as many where rows may be long (their last wave weighs more: 64 rows of
+    1000 to 2000 keys 311 us whole, 245 in three; 256 rows of 512 + 30 keys 79 whole, 92 in two)."""
+    ctas = -(-B // (8 * n_kv_heads // n_heads)) * n_kv_heads
+    return max(1, min(8, 444 // ctas, pages // 2)) if pages < 24 else max(2, min(8, 888 // ctas))
+
+
 _GROUP_TC = False
 
 
@@ -541,11 +552,26 @@ def paged_decode_attn(q, q_col0, kcache, vcache, page_table, seq_lens, n_heads, 
     """``groups = (group_rows [B, 8] int32, group_shared [B] int32, row_key0 [B] int32)``: rows that alias their first
     KV pages in groups (K samples of one prompt); the shared keys are then read once per group (``scratch`` must
     hold ``nsplit + 1`` partials per row and head). ``group_tc``: score the groups on the tensor cores (tcgen05, keys on
-    the M axis) instead of the CUDA-core kernel."""
+    the M axis) instead of the CUDA-core kernel. ``groups = ALIASED``: any rows may share pages, what eight neighbours share is
+    read once (the splits are then chosen here)."""
     B = q.shape[0]
     if _chk.active():
         _chk.paged_attention("rpeg_paged_decode_attn", B, seq_lens, page_table, kcache, n_kv_heads, head_dim)
     out = torch.empty((B, n_heads * head_dim), dtype=torch.bfloat16, device=q.device) if out is None else out
+    if groups is ALIASED:
+        groups = None
+        if 8 % (n_heads // n_kv_heads) == 0 and (q.stride(0) | q_col0) % 8 == 0 and B <= 8192:
+            nsplit = packed_decode_splits(B, n_heads, n_kv_heads, page_table.shape[1])
+            if scratch is not None:
+                while nsplit > 1 and decode_scratch_numel(B, n_heads, nsplit) > scratch.numel():
+                    nsplit -= 1
+            elif nsplit > 1:
+                scratch = torch.empty(decode_scratch_numel(B, n_heads, nsplit), dtype=torch.float32, device=q.device)
+            check(lib().rpeg_paged_decode_attn_packed(q.data_ptr(), q.stride(0), q_col0, kcache.data_ptr(), vcache.data_ptr(),
+                                                      page_table.data_ptr(), page_table.stride(0), seq_lens.data_ptr(), out.data_ptr(),
+                                                      _ptr(scratch) if nsplit > 1 else None, B, n_heads, n_kv_heads, head_dim, nsplit, scale,
+                                                      _stream()), "rpeg_paged_decode_attn_packed")
+            return out
     if groups is not None:
         group_rows, group_shared, row_key0 = groups
         if scratch is None:

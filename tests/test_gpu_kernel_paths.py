@@ -314,3 +314,47 @@ def test_sample_rows(cuda_device, dtype, rows, vocab, shift):
     assert torch.equal(drawn, K.sample(odd, 0.7, False, 77)[0])
     assert torch.equal(drawn, K.sample(aligned.float(), 0.7, False, 77)[0])
     assert float((lp - want.gather(1, drawn.long()[:, None])[:, 0]).abs().max()) < 1e-4
+
+
+# 11 rows: groups that share one, two or 33 pages (a second listing of 32), a row of its own, an empty one; eight columns of 8, 4, 2 and 1 rows
+@pytest.mark.parametrize("h,hkv", [(3, 3), (4, 2), (8, 2), (8, 1)])
+@pytest.mark.parametrize("split", [True, False])
+def test_paged_decode_attn_aliased_rows(cuda_device, h, hkv, split):
+    hd, dev = 128, cuda_device
+    groups = [(33, [0, 1, 15, 16]), (1, [17, 63, 64]), (2, [65]), (0, [1, 130, 0])]      # shared pages, own keys of every row
+    g = torch.Generator(device=dev).manual_seed(h)
+    lens = [64 * s + n for s, own in groups for n in own]
+    table = torch.zeros(len(lens), 36, dtype=torch.int32)
+    at, row = 1, 0
+    for s, own in groups:
+        for n in own:
+            table[row, :s] = torch.arange(at, at + s)
+            row += 1
+        at += s
+    for i, n in enumerate(lens):
+        s = int((table[i] > 0).sum())
+        need = -(-n // 64) - s
+        table[i, s:s + need] = torch.arange(at, at + need)
+        at += need
+    k, v = (torch.randn(at, hkv, 64, hd, generator=g, device=dev).bfloat16() for _ in range(2))
+    q = torch.randn(len(lens), h * hd, generator=g, device=dev).bfloat16()
+    for i, n in enumerate(lens):                                  # what lies behind a row's last key is never used
+        if n % 64:
+            k[table[i, n // 64].long(), :, n % 64:] = float("nan")
+            v[table[i, n // 64].long(), :, n % 64:] = float("nan")
+    v[table[6, 1].long(), :, 3] = float("inf")                    # and what one row holds never reaches another
+    table = table.to(dev)
+    seq = torch.tensor(lens, dtype=torch.int32, device=dev)
+    scratch = None if split else torch.empty(0, device=dev)       # no room for splits
+    out = K.paged_decode_attn(q, 0, k, v, table, seq, h, hkv, hd, hd ** -0.5, groups=K.ALIASED, scratch=scratch)
+    for i, n in enumerate(lens):
+        if n == 0:
+            assert bool((out[i] == 0).all())
+            continue
+        kk, vv = (t[table[i].long()].transpose(0, 1).reshape(hkv, -1, hd)[:, :n].double().repeat_interleave(h // hkv, 0) for t in (k, v))
+        w = (torch.einsum("hd,hkd->hk", q[i].double().view(h, hd), kk) * hd ** -0.5).softmax(-1)
+        want = torch.einsum("hk,hkd->hd", w, vv).reshape(-1)
+        if i == 6:
+            assert not bool(out[i].isfinite().any()) and not bool(want.isfinite().any())
+        else:
+            assert _rel(out[i], want) < 2 ** -8
