@@ -179,7 +179,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const int* _
       if (!__all_sync(0xffffffffu, mbar_wait(&s_full[ui], static_cast<uint32_t>(j) & 1u, abort_flag, status, 520))) { ok = false; break; }
       tc_fence_after_sync();
       const int k0 = j * FA_BN;
-      WpRow row;
+      WpRow<4> row;
       wp_load_row(ts, row);
       if (k0 + FA_BN - 1 > q0 || L - q0 < FA_BM) wp_mask_row(row, k0, lo, hi);
       const float tmax = wp_max_row(row) * scale_log2;        // scale > 0, so max commutes with the scaling

@@ -9,7 +9,7 @@
 //
 // Like the chunked kernel (window_prefill.cu) one CTA works on two 128-row query tiles ("units") of one head over the same key tiles, and while
 // the softmax warps of one unit turn its scores into weights the tensor cores multiply for the other. Roles: a TMA warp, an MMA
-// warp, four softmax warps per unit (thread = query row); weights replace the scores in place as two bf16 parts. What differs:
+// warp, eight softmax warps per unit (two threads a query row, prefill_softmax.cuh); weights replace the scores in place as two bf16 parts. What differs:
 //   * A query / key row is KA atoms of 64 columns (unrotated ones, then rotated ones), a value row VA atoms. The TMA unit pads narrower ones.
 //   * Key and value atoms (128 rows x 128 bytes) share one ring, freed atom by atom: with 192-wide keys and 128-wide values two key
 //     tiles and a value tile are in flight.
@@ -19,14 +19,14 @@
 
 namespace rpeg {
 
-constexpr int LP_BM = 128, LP_BN = 128, LP_THREADS = 320, LP_ATOM = 128 * 128;
+constexpr int LP_BM = 128, LP_BN = 128, LP_THREADS = WP_BLOCK, LP_ATOM = 128 * 128;
 
 template <int KA, int VA>
 struct LatentPrefillCfg {
   static constexpr int Q_BYTES = 2 * KA * LP_ATOM;
-  static constexpr int RAW = (227 * 1024 - 1536 - Q_BYTES) / LP_ATOM;
+  static constexpr int RAW = (227 * 1024 - 1280 - WP_EXCHANGE - Q_BYTES) / LP_ATOM;
   static constexpr int SLOTS = RAW > 10 ? 10 : RAW;
-  static constexpr int SMEM = Q_BYTES + SLOTS * LP_ATOM + 1536;
+  static constexpr int SMEM = Q_BYTES + SLOTS * LP_ATOM + 1280 + WP_EXCHANGE;
   static_assert(SLOTS >= KA + VA, "a key tile and a value tile must fit");
 };
 
@@ -81,17 +81,17 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_
   uint64_t* full = bars + 1;                // [SLOTS]
   uint64_t* empty = full + SLOTS;           // [SLOTS]
   uint64_t* s_full = empty + SLOTS;         // [2], per unit: S of its next tile is complete (and its P V before that)
-  uint64_t* p_half = s_full + 2;            // [2], per unit: its weights for the first 64 keys are in place
-  uint64_t* p_full = p_half + 2;            // [2], per unit: and for the others
+  uint64_t* p_full = s_full + 2;            // [2], per unit: its weights are in place
   uint64_t* o_full = p_full + 2;            // [2], per unit: O is final
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint16_t* exchange = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(bars) + 256);    // [2 units][2 halves][128 rows]
 
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int s = 0; s < SLOTS; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int u = 0; u < 2; ++u) { mbar_init(&s_full[u], 1); mbar_init(&p_half[u], 4); mbar_init(&p_full[u], 4); mbar_init(&o_full[u], 1); }
+    for (int u = 0; u < 2; ++u) { mbar_init(&s_full[u], 1); mbar_init(&p_full[u], WP_WARPS); mbar_init(&o_full[u], 1); }
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -107,6 +107,9 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_
   auto slot_of = [](int i) { return i % SLOTS; };
   auto parity_of = [](int i) { return static_cast<uint32_t>(i / SLOTS) & 1u; };
 
+  if (warp < WP_FIRST) {
+    wp_few_registers();
+  }
   if (warp == 0) {
     if (lane == 0) {
       const int row0 = a.off[b] + kb - a.lo[b];
@@ -173,7 +176,6 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_
       issue_qk(1, 0);
       for (int j = 0; j < n_tiles && ok; ++j) {
         if (!wait_atoms(j * TA + KA, VA)) break;
-        if (j + 1 < n_tiles && !wait_atoms((j + 1) * TA, KA)) break;
         const int v0 = slot_of(j * TA + KA), v1 = slot_of(j * TA + KA + VA - 1);
         const uint64_t vd0 = smem_desc_at(vd, v0 * LP_ATOM);
         const bool joined = VA == 2 && v1 == v0 + 1;         // neighbouring atoms are one product of 128 columns
@@ -182,35 +184,30 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_
           if (active(u, j)) {
             const int n = j - (u ? u1.jb : u0.jb);           // tiles of this unit before this one
             const uint32_t tp = tmem_base + u * 128, to = tmem_base + 256 + u * 128;
+            ok = wait(&p_full[u], static_cast<uint32_t>(n) & 1u, 1213);
+            if (!ok) break;
+            tc_fence_after_sync();
+            // 16 keys a step: 8 packed columns of P, 16 rows (2 KiB) of the value atoms
+            if (joined) {
 #pragma unroll
-            for (int half = 0; half < 2 && ok; ++half) {     // the first keys are multiplied while the last ones are exponentiated
-              ok = wait(half ? &p_full[u] : &p_half[u], static_cast<uint32_t>(n) & 1u, 1213 + half);
-              if (!ok) break;
-              tc_fence_after_sync();
-              // 16 keys a step: 8 packed columns of P, 16 rows (2 KiB) of the value atoms
-              if (joined) {
+              for (int part = 0; part < 2; ++part)
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                  if (leader)
+                    umma_bf16_ts(to, tp + (k >> 1) * 32 + part * 16 + (k & 1) * 8, smem_desc_at(vd0, k * 2048), idesc_pv2, (n | part | k) != 0 ? 1u : 0u);
+            } else {
+#pragma unroll
+              for (int va = 0; va < VA; ++va) {
+                const uint64_t vda = smem_desc_at(vd, (va ? v1 : v0) * LP_ATOM);
 #pragma unroll
                 for (int part = 0; part < 2; ++part)
 #pragma unroll
-                  for (int k = half * 4; k < half * 4 + 4; ++k)
+                  for (int k = 0; k < 8; ++k)
                     if (leader)
-                      umma_bf16_ts(to, tp + (k >> 1) * 32 + part * 16 + (k & 1) * 8, smem_desc_at(vd0, k * 2048), idesc_pv2,
-                                   (n | half | part | (k & 3)) != 0 ? 1u : 0u);
-              } else {
-#pragma unroll
-                for (int va = 0; va < VA; ++va) {
-                  const uint64_t vda = smem_desc_at(vd, (va ? v1 : v0) * LP_ATOM);
-#pragma unroll
-                  for (int part = 0; part < 2; ++part)
-#pragma unroll
-                    for (int k = half * 4; k < half * 4 + 4; ++k)
-                      if (leader)
-                        umma_bf16_ts(to + va * 64, tp + (k >> 1) * 32 + part * 16 + (k & 1) * 8, smem_desc_at(vda, k * 2048), idesc_pv,
-                                     (n | half | part | (k & 3)) != 0 ? 1u : 0u);
-                }
+                      umma_bf16_ts(to + va * 64, tp + (k >> 1) * 32 + part * 16 + (k & 1) * 8, smem_desc_at(vda, k * 2048), idesc_pv,
+                                   (n | part | k) != 0 ? 1u : 0u);
               }
             }
-            if (!ok) break;
             if (leader && j + 1 == (u ? u1.je : u0.je)) umma_commit(&o_full[u]);
           }
           if (u == 1)
@@ -218,74 +215,80 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_
             for (int va = 0; va < VA; ++va)
               if (leader) umma_commit(&empty[va ? v1 : v0]);
           tc_fence_after_sync();
-          if (j + 1 < n_tiles) issue_qk(u, j + 1);
+          if (j + 1 < n_tiles) {
+            // the next keys arrive in slots that values of the tile before have left: they are not waited for any earlier
+            if (u == 0) ok = wait_atoms((j + 1) * TA, KA);
+            if (!ok) break;
+            issue_qk(u, j + 1);
+          }
         }
       }
     }
-  } else {
-    const int ui = (warp - 2) >> 2;
+  } else if (warp >= WP_FIRST) {
+    wp_many_registers();
+    const int ui = (warp - WP_FIRST) / WP_WARPS, half = ((warp - WP_FIRST) >> 2) & 1;
     const LatentUnit w = ui ? u1 : u0;
-    const int quad = warp & 3;
+    const int quad = warp & 3, pair = ui * 4 + quad;
     const int r = quad * 32 + lane;
     const bool row_valid = w.q0 + r < L;
     const int qi = w.p0 + r;
     const int lo = row_valid ? first_key(qi) : 1, hi = row_valid ? qi : 0;     // an absent row sees nothing
     const uint32_t ts = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + ui * 128;
-    const uint32_t to = ts + 256;
+    const uint32_t to = ts + 256 + half * (VA * 32);         // this thread's half of O
     const float sink_l2 = a.sink != nullptr ? a.sink[h] * 1.4426950408889634f : -INFINITY;
     float m_ref = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = w.jb; j < w.je; ++j) {
       const int n = j - w.jb;
-      if (!__all_sync(0xffffffffu, mbar_wait(&s_full[ui], static_cast<uint32_t>(n) & 1u, abort_flag, a.status, 1220))) { ok = false; break; }
+      ok = __all_sync(0xffffffffu, mbar_wait(&s_full[ui], static_cast<uint32_t>(n) & 1u, abort_flag, a.status, 1220));
       tc_fence_after_sync();
-      const int k0 = kb + j * LP_BN;
-      const bool need_mask = k0 + LP_BN - 1 > w.p0 || k0 < w.last_lo || w.p_last - w.p0 < LP_BM - 1;
+      const int k0 = kb + j * LP_BN + half * 64;
+      const bool need_mask = k0 + 63 > w.p0 || k0 < w.last_lo || w.p_last - w.p0 < LP_BM - 1;
       // scale > 0, so the largest score is the scaled largest product
-      WpRow row;
-      wp_load_row(ts, row);
+      WpRow<2> row;
+      wp_load_row(ts + half * 64, row);
       if (need_mask) wp_mask_row(row, k0, lo, hi);
-      const float tmax = wp_max_row(row) * a.scale_log2;
+      float tmax = wp_max_row(row);
+      ok = wp_agree(ok, tmax, exchange + ui * 256, half, r, pair);
+      if (!ok) break;
+      tmax *= a.scale_log2;
       if (n == 0) {
         m_ref = fmaxf(tmax, sink_l2);
-        if (sink_l2 != -INFINITY) l = exp2f(sink_l2 - m_ref);
+        if (sink_l2 != -INFINITY && half == 0) l = exp2f(sink_l2 - m_ref);
       } else {
         const bool need = tmax > m_ref + WP_RESCALE;
         if (__any_sync(0xffffffffu, need)) {
           // a row that has seen no key yet (its window starts in a later tile) has nothing to rescale
           const float alpha = need ? (m_ref == -INFINITY ? 0.f : exp2f(m_ref - tmax)) : 1.f;
           if (need) { m_ref = tmax; l *= alpha; }
-#pragma unroll 1
-          for (int c = 0; c < VA * 2; ++c) {
-            uint32_t v[32];
-            tmem_ld_32x32(to + c * 32, v);
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-            tmem_st_32x32(to + c * 32, v);
-          }
+          wp_rescale(to, VA, alpha);
         }
       }
       const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
-      l += wp_exp_row(row, ts, a.scale_log2, m_use, &p_half[ui]);
+      l += wp_exp_row(row, ts + half * 64, a.scale_log2, m_use);
       tmem_wait_st();
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[ui]);
     }
-    if (ok && w.je > w.jb && __all_sync(0xffffffffu, mbar_wait(&o_full[ui], 0, abort_flag, a.status, 1222))) {
+    if (ok && w.je > w.jb) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&o_full[ui], 0, abort_flag, a.status, 1222));
+      // the unit's products are done: its queries' shared memory is free
+      ok = wp_add(ok, l, reinterpret_cast<float*>(q_sm + ui * KA * LP_ATOM), half, r, pair);
+    }
+    if (ok && w.je > w.jb) {
       tc_fence_after_sync();
       const float inv_l = l > 0.f ? 1.f / l : 0.f;
-      __nv_bfloat16* orow = a.out + static_cast<size_t>(tok0 + w.q0 + r) * a.ldo + h * a.vdim_p;
+      __nv_bfloat16* orow = a.out + static_cast<size_t>(tok0 + w.q0 + r) * a.ldo + h * a.vdim_p + half * (VA * 32);
 #pragma unroll 1
-      for (int c = 0; c < VA * 2; ++c) {
+      for (int c = 0; c < VA; ++c) {
         uint32_t v[32];
         tmem_ld_32x32(to + c * 32, v);
         tmem_wait_ld();
         if (row_valid) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            if (c * 32 + i * 8 < a.vdim_p) {
+            if (half * (VA * 32) + c * 32 + i * 8 < a.vdim_p) {
               uint32_t o[4];
 #pragma unroll
               for (int e = 0; e < 4; ++e)

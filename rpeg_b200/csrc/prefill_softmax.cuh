@@ -1,26 +1,44 @@
-// The softmax side of the tensor-core prompt attention kernels: a thread owns one query row, whose 128 scores of a key tile lie in TMEM.
+// The softmax side of the tensor-core prompt attention kernels. The 128 scores of a query row over a key tile lie in TMEM and belong to one thread
+// (flash_attn.cu) or two, 64 each (window_prefill.cu, latent_prefill.cu).
+//
+// A unit (128 query rows) is a chain: scores, weights, product, scores of the next tile. Weights of two bf16 parts took one thread a row 2800 of the
+// 7100 clocks that two units needed per tile, in which the tensor cores were busy for 3600; two threads a row halve that link. Plain bf16 weights
+// (1500 of 3700) are bound by the exponential unit, which both units share: more threads lost a tenth there. (Half as many keys a step, scores in
+// two buffers, gained nothing either: a product of 64 columns costs the tensor cores 57 clocks, one of 128 columns 61.)
+// The two threads agree on the reference of a row's exponentials: their maxima, rounded to bf16, meet in shared memory.
 #pragma once
 #include "act_io.cuh"
 
 namespace rpeg {
 
 constexpr float WP_RESCALE = 8.0f;       // log2: how far a row's maximum may grow before its accumulator is rescaled
+constexpr int WP_WARPS = 8;              // softmax warps of a unit: two for every 32 rows
+// A CTA's 20 warps: a TMA warp, an MMA warp, two that idle, and the softmax warps. It is launched with 96 registers a thread, of which the first
+// four warps leave some to the others: 4 x 32 x 64 + 16 x 32 x 104 = 640 x 96 (with 32 and 112 the MMA warp's descriptors did not fit).
+constexpr int WP_FIRST = 4, WP_BLOCK = 32 * (WP_FIRST + 2 * WP_WARPS);
+constexpr int WP_EXCHANGE = 2 * 2 * 128 * 2;        // bytes of shared memory: [unit][half][row]
 
-// A row's 128 scores of one tile, in registers from the maximum to the weights: S is read from TMEM once.
+__device__ __forceinline__ void wp_few_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 64;"); }
+__device__ __forceinline__ void wp_many_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 104;"); }
+
+// A thread's 32 C scores, in registers from the maximum to the weights: S is read from TMEM once.
+template <int C>
 struct WpRow {
-  uint32_t s[4][32];
+  uint32_t s[C][32];
 };
 
-__device__ __forceinline__ void wp_load_row(uint32_t ts, WpRow& row) {
+template <int C>
+__device__ __forceinline__ void wp_load_row(uint32_t ts, WpRow<C>& row) {
 #pragma unroll
-  for (int c = 0; c < 4; ++c) tmem_ld_32x32(ts + c * 32, row.s[c]);
+  for (int c = 0; c < C; ++c) tmem_ld_32x32(ts + c * 32, row.s[c]);
   tmem_wait_ld();
 }
 
-// Keys outside [lo, hi] of the tile that starts at k0 get no weight, whatever their (finite or not) score is.
-__device__ __forceinline__ void wp_mask_row(WpRow& row, int k0, int lo, int hi) {
+// Keys outside [lo, hi] of those that start at k0 get no weight, whatever their (finite or not) score is.
+template <int C>
+__device__ __forceinline__ void wp_mask_row(WpRow<C>& row, int k0, int lo, int hi) {
 #pragma unroll
-  for (int c = 0; c < 4; ++c)
+  for (int c = 0; c < C; ++c)
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
       const int kj = k0 + c * 32 + i;
@@ -28,28 +46,30 @@ __device__ __forceinline__ void wp_mask_row(WpRow& row, int k0, int lo, int hi) 
     }
 }
 
-__device__ __forceinline__ float wp_max_row(const WpRow& row) {
+template <int C>
+__device__ __forceinline__ float wp_max_row(const WpRow<C>& row) {
   float m[4];
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    m[c] = __uint_as_float(row.s[c][0]);
+    m[c] = __uint_as_float(row.s[c * C / 4][c * C % 4 * 8]);
 #pragma unroll
-    for (int i = 1; i < 32; ++i) m[c] = fmaxf(m[c], __uint_as_float(row.s[c][i]));
+    for (int i = 1; i < 8 * C; ++i) m[c] = fmaxf(m[c], __uint_as_float(row.s[(c * 8 * C + i) / 32][(c * 8 * C + i) % 32]));
   }
   return fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
 }
 
-// P = exp2(s * scale - m_ref) over S in place (columns 32 c .. + 15: leading parts of chunk c, + 16 .. + 31: remainders);
-// returns its row sum. `half_bar` gets this warp's arrival once the first 64 keys are in place.
-__device__ __forceinline__ float wp_exp_row(const WpRow& row, uint32_t ts, float scale_log2, float m_ref, uint64_t* half_bar) {
+// P = exp2(s * scale - m_ref) over S in place (columns 32 c .. + 15: leading parts of chunk c, + 16 .. + 31: remainders); returns its sum. 16 keys at a
+// time: the words of more would not fit beside the scores.
+__device__ __forceinline__ float wp_exp_row(const WpRow<2>& row, uint32_t ts, float scale_log2, float m_ref) {
   const uint64_t scale2 = pack2(scale_log2, scale_log2), shift2 = pack2(-m_ref, -m_ref), minus2 = pack2(-1.f, -1.f);
   uint64_t sum2[2] = {0ull, 0ull};
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    uint32_t head[16], rest[16];
+    uint32_t head[8], rest[8];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const float2 t = unpack2(fma2(pack2(__uint_as_float(row.s[c][2 * i]), __uint_as_float(row.s[c][2 * i + 1])), scale2, shift2));
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t* s = &row.s[c >> 1][(c & 1) * 16 + 2 * i];
+      const float2 t = unpack2(fma2(pack2(__uint_as_float(s[0]), __uint_as_float(s[1])), scale2, shift2));
       const float p0 = exp2f(t.x), p1 = exp2f(t.y);
       const uint64_t p = pack2(p0, p1);
       sum2[i & 1] = add2(sum2[i & 1], p);
@@ -59,21 +79,16 @@ __device__ __forceinline__ float wp_exp_row(const WpRow& row, uint32_t ts, float
       const float2 r = unpack2(fma2(pack2(__uint_as_float(w0 & 0xffff0000u), __uint_as_float(w1 & 0xffff0000u)), minus2, p));
       rest[i] = pack_bf16x2(r.x, r.y);
     }
-    tmem_st_32x16(ts + c * 32, head);
-    tmem_st_32x16(ts + c * 32 + 16, rest);
-    if (c == 1) {
-      tmem_wait_st();
-      tc_fence_before_sync();
-      __syncwarp();
-      if ((threadIdx.x & 31) == 0) mbar_arrive(half_bar);
-    }
+    tmem_st_32x8(ts + (c >> 1) * 32 + (c & 1) * 8, head);
+    tmem_st_32x8(ts + (c >> 1) * 32 + 16 + (c & 1) * 8, rest);
   }
   const float2 s0 = unpack2(sum2[0]), s1 = unpack2(sum2[1]);
   return (s0.x + s0.y) + (s1.x + s1.y);
 }
 
-// The same with plain bf16 weights: P over the first 64 columns of S, 16 columns a chunk.
-__device__ __forceinline__ float wp_exp_row_bf16(const WpRow& row, uint32_t ts, float scale_log2, float m_ref, uint64_t* half_bar) {
+// One thread a row, plain bf16 weights over the first 64 columns of S, 16 columns a chunk. `half_bar` gets this warp's arrival once the first 64 keys are
+// in place.
+__device__ __forceinline__ float wp_exp_row_bf16(const WpRow<4>& row, uint32_t ts, float scale_log2, float m_ref, uint64_t* half_bar) {
   const uint64_t scale2 = pack2(scale_log2, scale_log2), shift2 = pack2(-m_ref, -m_ref);
   uint64_t sum2[2] = {0ull, 0ull};
 #pragma unroll
@@ -96,6 +111,48 @@ __device__ __forceinline__ float wp_exp_row_bf16(const WpRow& row, uint32_t ts, 
   }
   const float2 s0 = unpack2(sum2[0]), s1 = unpack2(sum2[1]);
   return (s0.x + s0.y) + (s1.x + s1.y);
+}
+
+// Whether both of a row's threads are well (their waits have not run out): a barrier of the two warps.
+__device__ __forceinline__ bool wp_meet(bool ok, int pair) {
+  uint32_t both;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 q, %1, 0;\n\t"
+      "barrier.cta.red.and.pred p, %2, 64, q;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(both)
+      : "r"(ok ? 1u : 0u), "r"(pair + 1)
+      : "memory");
+  return both != 0;
+}
+// `m`: the larger of the two threads' maxima, as both see it. `words`: [half][row] of the unit. Behind it both have read their scores.
+__device__ __forceinline__ bool wp_agree(bool ok, float& m, uint16_t* words, int half, int r, int pair) {
+  const __nv_bfloat16 own = __float2bfloat16(m);
+  words[half * 128 + r] = __bfloat16_as_ushort(own);
+  ok = wp_meet(ok, pair);
+  m = fmaxf(__bfloat162float(own), __bfloat162float(__ushort_as_bfloat16(words[(half ^ 1) * 128 + r])));
+  return ok;
+}
+// `l`: the sum of the two threads' sums.
+__device__ __forceinline__ bool wp_add(bool ok, float& l, float* words, int half, int r, int pair) {
+  words[half * 128 + r] = l;
+  ok = wp_meet(ok, pair);
+  l += words[(half ^ 1) * 128 + r];
+  return ok;
+}
+
+// O of a row times alpha (columns to .. to + 32 chunks).
+__device__ __forceinline__ void wp_rescale(uint32_t to, int chunks, float alpha) {
+#pragma unroll 1
+  for (int c = 0; c < chunks; ++c) {
+    uint32_t v[32];
+    tmem_ld_32x32(to + c * 32, v);
+    tmem_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
+    tmem_st_32x32(to + c * 32, v);
+  }
 }
 
 }  // namespace rpeg

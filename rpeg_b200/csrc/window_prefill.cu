@@ -8,8 +8,8 @@
 //
 // One CTA works on two 128-row query tiles ("units") over the same key tiles: the same rows of two heads of one KV head,
 // or, when the KV head has an odd number of query heads, two neighbouring row tiles of one head. While the softmax warps of one
-// unit turn its scores into weights, the tensor cores multiply for the other one. Roles: a TMA warp, an MMA warp, four softmax
-// warps per unit (thread = query row).
+// unit turn its scores into weights, the tensor cores multiply for the other one. Roles: a TMA warp, an MMA warp, eight softmax
+// warps per unit (two threads a query row, prefill_softmax.cuh).
 //   * TMEM: S (128 columns) and O (up to 128) of each unit. A unit's weights replace its scores in place, 32-key chunk by
 //     chunk: a weight is handed to the tensor cores as the sum of two bf16 numbers (16 bits), so that rounding the operands
 //     of P V does not show; its two parts take 16 of the chunk's 32 columns each.
@@ -26,12 +26,12 @@
 
 namespace rpeg {
 
-constexpr int WP_BM = 128, WP_BN = 128, WP_THREADS = 320, WP_STAGES = 2;
+constexpr int WP_BM = 128, WP_BN = 128, WP_THREADS = WP_BLOCK, WP_STAGES = 2;
 
 template <int HDT>
 struct PrefillCfg {
   static constexpr int TILE = 128 * HDT * 2;               // HDT / 64 atoms of 128 rows x 128 bytes
-  static constexpr int SMEM = TILE * (2 + 2 * WP_STAGES) + 1024 + 256;
+  static constexpr int SMEM = TILE * (2 + 2 * WP_STAGES) + 1024 + 256 + WP_EXCHANGE;
 };
 
 struct Prefill {
@@ -92,11 +92,11 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   uint64_t* v_full = k_empty + WP_STAGES;
   uint64_t* v_empty = v_full + WP_STAGES;
   uint64_t* s_full = v_empty + WP_STAGES;   // [2], per unit: S of its next tile is complete (and its P V before that)
-  uint64_t* p_half = s_full + 2;            // [2], per unit: its weights for the first 64 keys are in place
-  uint64_t* p_full = p_half + 2;            // [2], per unit: and for the others
+  uint64_t* p_full = s_full + 2;            // [2], per unit: its weights are in place
   uint64_t* o_full = p_full + 2;            // [2], per unit: O is final
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint16_t* exchange = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(bars) + 256);    // [2 units][2 halves][128 rows]
 
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -105,7 +105,7 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1);
       mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1);
     }
-    for (int u = 0; u < 2; ++u) { mbar_init(&s_full[u], 1); mbar_init(&p_half[u], 4); mbar_init(&p_full[u], 4); mbar_init(&o_full[u], 1); }
+    for (int u = 0; u < 2; ++u) { mbar_init(&s_full[u], 1); mbar_init(&p_full[u], WP_WARPS); mbar_init(&o_full[u], 1); }
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -118,6 +118,9 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
+  if (warp < WP_FIRST) {
+    wp_few_registers();
+  }
   if (warp == 0) {
     if (lane == 0) {
       const int* pt = a.page_table + static_cast<size_t>(a.slot[tok0]) * a.max_pages;
@@ -191,20 +194,15 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
           if (active(u, j)) {
             const int n = j - (u ? u1.jb : u0.jb);           // tiles of this unit before this one
             const uint32_t tp = tmem_base + u * 128, to = tmem_base + 256 + u * 128;
-#pragma unroll
-            for (int half = 0; half < 2 && ok; ++half) {     // the first keys are multiplied while the last ones are exponentiated
-              ok = wait(half ? &p_full[u] : &p_half[u], static_cast<uint32_t>(n) & 1u, 913 + half);
-              if (!ok) break;
-              tc_fence_after_sync();
-#pragma unroll
-              for (int part = 0; part < 2; ++part)
-#pragma unroll
-                for (int k = half * 4; k < half * 4 + 4; ++k)     // 16 keys: 8 packed columns of P, 16 rows (2 KiB) of the V tile
-                  if (leader)
-                    umma_bf16_ts(to, tp + (k >> 1) * 32 + part * 16 + (k & 1) * 8, smem_desc_at(va, k * 2048), idesc_pv,
-                                 (n | half | part | (k & 3)) != 0 ? 1u : 0u);
-            }
+            ok = wait(&p_full[u], static_cast<uint32_t>(n) & 1u, 913);
             if (!ok) break;
+            tc_fence_after_sync();
+#pragma unroll
+            for (int part = 0; part < 2; ++part)
+#pragma unroll
+              for (int k = 0; k < 8; ++k)     // 16 keys: 8 packed columns of P, 16 rows (2 KiB) of the V tile
+                if (leader)
+                  umma_bf16_ts(to, tp + (k >> 1) * 32 + part * 16 + (k & 1) * 8, smem_desc_at(va, k * 2048), idesc_pv, (n | part | k) != 0 ? 1u : 0u);
             if (leader && j + 1 == (u ? u1.je : u0.je)) umma_commit(&o_full[u]);
           }
           if (leader && u == 1) umma_commit(&v_empty[st]);
@@ -213,10 +211,11 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         }
       }
     }
-  } else {
-    const int ui = (warp - 2) >> 2;
+  } else if (warp >= WP_FIRST) {
+    wp_many_registers();
+    const int ui = (warp - WP_FIRST) / WP_WARPS, half = ((warp - WP_FIRST) >> 2) & 1;
     const PrefillUnit w = ui ? u1 : u0;
-    const int quad = warp & 3;
+    const int quad = warp & 3, pair = ui * 4 + quad;
     const int r = quad * 32 + lane;
     const bool row_valid = w.q0 + r < L;
     const int qi = w.p0 + r;
@@ -224,61 +223,61 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     const int lo = row_valid ? (a.window > 0 ? qi / a.window * a.window : 0) : 1;
     const int hi = row_valid ? qi : 0;
     const uint32_t ts = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + ui * 128;
-    const uint32_t to = ts + 256;
+    const uint32_t to = ts + 256 + half * (HDT / 64 * 32);         // this thread's half of O
     const float sink_l2 = a.sink != nullptr ? a.sink[w.h] * 1.4426950408889634f : -INFINITY;
     float m_ref = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = w.jb; j < w.je; ++j) {
       const int n = j - w.jb;
-      if (!__all_sync(0xffffffffu, mbar_wait(&s_full[ui], static_cast<uint32_t>(n) & 1u, abort_flag, a.status, 920))) { ok = false; break; }
+      ok = __all_sync(0xffffffffu, mbar_wait(&s_full[ui], static_cast<uint32_t>(n) & 1u, abort_flag, a.status, 920));
       tc_fence_after_sync();
-      const int k0 = kb + j * WP_BN;
-      const bool need_mask = k0 + WP_BN - 1 > w.p0 || k0 < w.last_lo || w.p_last - w.p0 < WP_BM - 1;
+      const int k0 = kb + j * WP_BN + half * 64;
+      const bool need_mask = k0 + 63 > w.p0 || k0 < w.last_lo || w.p_last - w.p0 < WP_BM - 1;
       // scale > 0, so the largest score is the scaled largest product
-      WpRow row;
-      wp_load_row(ts, row);
+      WpRow<2> row;
+      wp_load_row(ts + half * 64, row);
       if (need_mask) wp_mask_row(row, k0, lo, hi);
-      const float tmax = wp_max_row(row) * a.scale_log2;
+      float tmax = wp_max_row(row);
+      ok = wp_agree(ok, tmax, exchange + ui * 256, half, r, pair);
+      if (!ok) break;
+      tmax *= a.scale_log2;
       if (n == 0) {
         m_ref = fmaxf(tmax, sink_l2);
-        if (sink_l2 != -INFINITY) l = exp2f(sink_l2 - m_ref);
+        if (sink_l2 != -INFINITY && half == 0) l = exp2f(sink_l2 - m_ref);
       } else {
         const bool need = tmax > m_ref + WP_RESCALE;
         if (__any_sync(0xffffffffu, need)) {
           const float alpha = need ? exp2f(m_ref - tmax) : 1.f;
           if (need) { m_ref = tmax; l *= alpha; }
-#pragma unroll 1
-          for (int c = 0; c < HDT / 32; ++c) {
-            uint32_t v[32];
-            tmem_ld_32x32(to + c * 32, v);
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-            tmem_st_32x32(to + c * 32, v);
-          }
+          wp_rescale(to, HDT / 64, alpha);
         }
       }
       // a row that has seen no key yet and has no sink: every weight of this tile is masked to zero
       const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
-      l += wp_exp_row(row, ts, a.scale_log2, m_use, &p_half[ui]);
+      l += wp_exp_row(row, ts + half * 64, a.scale_log2, m_use);
       tmem_wait_st();
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[ui]);
     }
-    if (ok && w.je > w.jb && __all_sync(0xffffffffu, mbar_wait(&o_full[ui], 0, abort_flag, a.status, 922))) {
+    if (ok && w.je > w.jb) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&o_full[ui], 0, abort_flag, a.status, 922));
+      // the unit's products are done: its queries' shared memory is free
+      ok = wp_add(ok, l, reinterpret_cast<float*>(q_sm + ui * TILE), half, r, pair);
+    }
+    if (ok && w.je > w.jb) {
       tc_fence_after_sync();
       const float inv_l = l > 0.f ? 1.f / l : 0.f;
-      __nv_bfloat16* orow = a.out + static_cast<size_t>(tok0 + w.q0 + r) * a.ldo + w.h * a.dp;
+      __nv_bfloat16* orow = a.out + static_cast<size_t>(tok0 + w.q0 + r) * a.ldo + w.h * a.dp + half * (HDT / 2);
 #pragma unroll 1
-      for (int c = 0; c < HDT / 32; ++c) {
+      for (int c = 0; c < HDT / 64; ++c) {
         uint32_t v[32];
         tmem_ld_32x32(to + c * 32, v);
         tmem_wait_ld();
         if (row_valid) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            if (c * 32 + i * 8 < a.dp) {
+            if (half * (HDT / 2) + c * 32 + i * 8 < a.dp) {
               uint4 o;
               o.x = pack_bf16x2(__uint_as_float(v[i * 8 + 0]) * inv_l, __uint_as_float(v[i * 8 + 1]) * inv_l);
               o.y = pack_bf16x2(__uint_as_float(v[i * 8 + 2]) * inv_l, __uint_as_float(v[i * 8 + 3]) * inv_l);
