@@ -659,9 +659,11 @@ extern "C" int rpeg_gemm_swiglu(const void* A, const void* W, void* C, int M, in
     cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
   // Pairs, unless this kernel's tiles are one wave (512 rows, f = 4096, K = 2048: 15 us here, 16 there; 640: 26 and 25), K is short (2000 rows, f =
-  // 11008, K = 256: 32 and 35) or a half-empty last row tile costs the pairs a wave more (300 rows, f = 11008, K = 4096: 60 and 67; 400: 82 and 69).
+  // 11008, K = 256: 32 and 35) or a half-empty last row tile costs the pairs more than a fifth of the waves, which take them 26 us for 32 here (300 rows,
+  // f = 11008, K = 4096, two waves and three: 60 and 67; 1600 rows, eight and nine: 230 and 209; 3700: 487 and 437).
   const int tiles = ((M + BM - 1) / BM) * (f / 128), pair_tiles = ((M + 2 * BM - 1) / (2 * BM)) * (f / 128), half = g_num_sms / 2;
-  if (K >= 1024 && tiles > g_num_sms && (pair_tiles + half - 1) / half <= (tiles + g_num_sms - 1) / g_num_sms)
+  const int waves = (tiles + g_num_sms - 1) / g_num_sms, pair_waves = (pair_tiles + half - 1) / half;
+  if (K >= 1024 && tiles > g_num_sms && 5 * pair_waves <= 6 * waves)
     return gemm_pair_swiglu(A, W, C, M, f, K, lda, ldw, ldc, g_num_sms, status, stream);
   CUtensorMap ta, tb;
   int rc = make_tmap_bf16_2d(&ta, A, K, M, lda, BK, BM);
