@@ -140,6 +140,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
+      const uint64_t policy = l2_policy(pdl && m_tiles == 1);      // weights that one row tile reads
       int skip = 0;                      // k-blocks of the first item that the early weight prefetch already issued
       if (gate.flags != nullptr) {
         const uint64_t t0 = global_timer_ns();
@@ -168,7 +169,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
             const int pre = min(STAGES, kb1 - kb0);
             for (int i = 0; i < pre; ++i) {            // weights first: they do not depend on the previous kernel
               mbar_expect_tx(&full_bar[i], stage_tx);
-              tma_load_2d(smem + i * Cfg::STAGE_BYTES + Cfg::A_BYTES, &tmap_b, &full_bar[i], (kb0 + i) * BK, tn * BN);  // never EPI_SWIGLU
+              tma_load_2d_hint(smem + i * Cfg::STAGE_BYTES + Cfg::A_BYTES, &tmap_b, &full_bar[i], (kb0 + i) * BK, tn * BN, policy);  // never EPI_SWIGLU
             }
             griddep_wait();
             for (int i = 0; i < pre; ++i)
@@ -206,7 +207,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
             tma_load_2d(sb, &tmap_b, &full_bar[stage], kb * BK, n0);
             tma_load_2d(sb + (BN / 2) * BK * 2, &tmap_b, &full_bar[stage], kb * BK, N + n0);
           } else if constexpr (!B_MN) {
-            tma_load_2d(sb, &tmap_b, &full_bar[stage], kb * BK, n0);
+            tma_load_2d_hint(sb, &tmap_b, &full_bar[stage], kb * BK, n0, policy);
           } else {
 #pragma unroll
             for (int c = 0; c < BN / 64; ++c)

@@ -4,8 +4,8 @@
 // mixture, see moe.cu for the segment layout and the activations); or batched: the same product for every head, at fixed
 // strides, with B either [N, K] or [K, N].
 //
-// Two kernels. gemm_f32_kernel: 64 x 64 tiles, bound by the FMA rate once M fills them. gemm_f32_rows_kernel: up to SR_ROWS rows
-// (decode), bound by streaming B from memory, once for every SR_MAX rows.
+// gemm_f32_tile_kernel: tiles, bound by the FMA rate once there are enough of them; gemm_f32_kernel: the same for rows that are not aligned.
+// gemm_f32_rows_kernel: up to SR_ROWS rows (decode), bound by streaming B from memory, once for every SR_MAX rows.
 #include "act_io.cuh"
 #include "moe_segments.cuh"
 #include "rpeg_kernels.h"
@@ -145,9 +145,9 @@ constexpr int SR_MAX = 16;      // rows of A per pass over B
 constexpr int SR_ROWS = 32;     // most rows of A
 constexpr int SR_WARPS = 4, SR_N = 4;   // a warp's rows of B
 
-__device__ __forceinline__ float4 stream4(const float* p) {   // read once: leaves the L1 to A
+__device__ __forceinline__ float4 stream4(const float* p, uint64_t once) {   // read once: leaves the L1 to A, and L2 before anything else
   float4 v;
-  asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(once));
   return v;
 }
 
@@ -182,6 +182,7 @@ __device__ __forceinline__ void rows_dot(const float* a, int lda, int M, const f
   constexpr int U = MR <= 4 ? 4 : 2;      // float4 of each B row in flight
   float acc[SR_N * MR] = {};
   const int k4 = K >> 2, step = 32 * ks;
+  const uint64_t once = l2_policy(true);
   auto fold = [&](int f, const float4 (&w)[SR_N]) {
 #pragma unroll
     for (int m = 0; m < MR; ++m) {
@@ -199,14 +200,14 @@ __device__ __forceinline__ void rows_dot(const float* a, int lda, int M, const f
 #pragma unroll
     for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int r = 0; r < SR_N; ++r) w[u][r] = stream4(b[r] + static_cast<size_t>(f + u * step) * 4);
+      for (int r = 0; r < SR_N; ++r) w[u][r] = stream4(b[r] + static_cast<size_t>(f + u * step) * 4, once);
 #pragma unroll
     for (int u = 0; u < U; ++u) fold(f + u * step, w[u]);
   }
   for (; f < k4; f += step) {
     float4 w[SR_N];
 #pragma unroll
-    for (int r = 0; r < SR_N; ++r) w[r] = stream4(b[r] + static_cast<size_t>(f) * 4);
+    for (int r = 0; r < SR_N; ++r) w[r] = stream4(b[r] + static_cast<size_t>(f) * 4, once);
     fold(f, w);
   }
   int first;

@@ -108,6 +108,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
   if (warp == 0) {
     if (lane == 0) {
+      const uint64_t policy = l2_policy(EPI == PG_F32 && m_tiles == 1);      // decode: weights that one row tile reads
       int stage = 0;
       uint32_t phase = 0;
       for (int w = first; w < num_items; w += step) {
@@ -128,7 +129,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             for (int c = 0; c < PG_BM / 64; ++c) tma_load_2d_pair(sa + c * (64 * PG_BK * 2), &tmap_a, bar, m0 + c * 64, kb * PG_BK);
           }
           if constexpr (!B_MN) {
-            tma_load_2d_pair(sb, &tmap_b, bar, kb * PG_BK, n0);
+            tma_load_2d_pair_hint(sb, &tmap_b, bar, kb * PG_BK, n0, policy);
           } else {
             for (int c = 0; c * 64 < BN / 2; ++c) tma_load_2d_pair(sb + c * (64 * PG_BK * 2), &tmap_b, bar, n0 + c * 64, kb * PG_BK);
           }
