@@ -25,11 +25,10 @@ struct GemmF32 {
 
 enum { SG_PLAIN = 0, SG_GROUPED = 1, SG_GATED = 2, SG_BATCHED = 3, SG_BATCHED_KN = 4 };   // KN: B is stored [K, N]
 
-// 64 x 64 outputs per CTA, 4 x 4 per thread, K slices in two shared-memory buffers: the next slice is in registers while this one is
-// multiplied, one barrier a slice. A slice is 32 deep, long enough to cover a memory access (16 where two tiles of B leave no room).
-// VEC: rows of A and B are read as float4 (16-byte aligned operands, K and pitches multiples of 4). Every output is one fp32 sum in the
-// order of k. 282 rows, N = K = 2048: 221 -> 151 us; N = 32000: 1542 -> 1230 us (one scalar slice at a time before).
-template <int MODE, bool VEC>
+// Rows that are not aligned, and B stored [K, N]: 64 x 64 outputs per CTA, 4 x 4 per thread, K slices in two shared-memory buffers: the next
+// slice is in registers while this one is multiplied, one barrier a slice. A slice is 32 deep, long enough to cover a memory access (16 where
+// two tiles of B leave no room). Every output is one fp32 sum in the order of k.
+template <int MODE>
 __global__ void __launch_bounds__(256)
 gemm_f32_kernel(const GemmF32 p) {
   constexpr bool GATED = MODE == SG_GATED;
@@ -53,34 +52,23 @@ gemm_f32_kernel(const GemmF32 p) {
   const int m0 = blockIdx.y * SG_T, n0 = blockIdx.x * SG_T;
   if (m0 >= M) return;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  // What this thread carries of a slice. VEC: of row tid / 4, four columns in a row. Otherwise one float of each of four rows, side by side over
-  // the threads (four in a row per thread took 1000 rows, N = 2048, K = 2050 from 308 to 362 us); of B stored [K, N] as well.
-  const int vr = tid >> 2, vk = (tid & 3) * 4;
+  // What this thread carries of a slice: one float of each of four rows, side by side over the threads (four in a row per thread took 1000
+  // rows, N = 2048, K = 2050 from 308 to 362 us); of B stored [K, N] as well.
   float ra[NV][4], rb[NB][NV][4];
-  auto row4 = [&](const float* base, bool live, int k, float (&v)[4]) {
-    const float4 t = live && k < p.K ? load4(base + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-  };
   auto fetch = [&](int k0) {
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-      if constexpr (VEC) {
-        row4(a + static_cast<size_t>(m0 + vr) * p.lda, m0 + vr < M, k0 + vk + 16 * v, ra[v]);
+      const int k = k0 + 16 * v + tx;
 #pragma unroll
-        for (int g = 0; g < NB; ++g) row4(B + (static_cast<size_t>(g) * p.N + n0 + vr) * p.ldb, n0 + vr < p.N, k0 + vk + 16 * v, rb[g][v]);
-      } else {
-        const int k = k0 + 16 * v + tx;
+      for (int i = 0; i < 4; ++i) {
+        const int r = ty + 16 * i;
+        ra[v][i] = m0 + r < M && k < p.K ? a[static_cast<size_t>(m0 + r) * p.lda + k] : 0.f;
+        if constexpr (MODE == SG_BATCHED_KN) {
+          const int n = n0 + (tid & 63), kk = k0 + 16 * v + (tid >> 6) + 4 * i;
+          rb[0][v][i] = n < p.N && kk < p.K ? B[static_cast<size_t>(kk) * p.ldb + n] : 0.f;
+        } else {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int r = ty + 16 * i;
-          ra[v][i] = m0 + r < M && k < p.K ? a[static_cast<size_t>(m0 + r) * p.lda + k] : 0.f;
-          if constexpr (MODE == SG_BATCHED_KN) {
-            const int n = n0 + (tid & 63), kk = k0 + 16 * v + (tid >> 6) + 4 * i;
-            rb[0][v][i] = n < p.N && kk < p.K ? B[static_cast<size_t>(kk) * p.ldb + n] : 0.f;
-          } else {
-#pragma unroll
-            for (int g = 0; g < NB; ++g) rb[g][v][i] = n0 + r < p.N && k < p.K ? B[(static_cast<size_t>(g) * p.N + n0 + r) * p.ldb + k] : 0.f;
-          }
+          for (int g = 0; g < NB; ++g) rb[g][v][i] = n0 + r < p.N && k < p.K ? B[(static_cast<size_t>(g) * p.N + n0 + r) * p.ldb + k] : 0.f;
         }
       }
     }
@@ -90,7 +78,7 @@ gemm_f32_kernel(const GemmF32 p) {
     for (int v = 0; v < NV; ++v)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int k = 16 * v + (VEC ? vk + i : tx), r = VEC ? vr : ty + 16 * i;
+        const int k = 16 * v + tx, r = ty + 16 * i;
         as[buf][k][r] = ra[v][i];
 #pragma unroll
         for (int g = 0; g < NB; ++g) {
@@ -137,6 +125,131 @@ gemm_f32_kernel(const GemmF32 p) {
       if constexpr (MODE == SG_GROUPED) v = p.act == FF_GELU ? ff_act<FF_GELU>(v) : (p.act == FF_RELU2 ? ff_act<FF_RELU2>(v) : v);
       C[static_cast<size_t>(m) * p.ldc + n] = v;
     }
+  }
+}
+
+// ---------------------------------------------------------------------------------- tiles
+// TM x 64 products per CTA (gated: 32 outputs, gate and up), 256 threads in four groups that take every fourth 16-deep slice of K each: a grid of
+// few tiles still has eight warps an SM with independent loads. A thread has TM / 8 x 8 sums. What bounds it is shared memory, whose loads fill
+// registers at 128 bytes a clock: 4 x 8 sums take 12 clocks of it a warp and k for 8 of products, 8 x 8 take 16 and 16 (packed products with
+// doubled columns: 20 and 8, 71 us where these take 46). 33 rows, N = 2560, K = 2048: 84 us with 4 x 4 sums a thread and one group, now 46; 240
+// rows 147 and 118; 512 rows, N = 32000 2000 and 1690 (40 TFLOP/s).
+// A group's slices pass through two buffers of its own, and its 64 threads wait for each other only. The four sums of an output are added
+// at the end. Rows of A and B are read as float4 (16-byte aligned operands, K and pitches multiples of 4).
+constexpr int ST_N = 64, ST_K = 16, ST_GROUPS = 4, ST_THREADS = 64 * ST_GROUPS;
+
+template <int TM>
+struct SgemmTile {
+  static constexpr int LA = TM + 4, LB = ST_N + 4, BUF = ST_K * (LA + LB);           // one slice, rows of k
+  static constexpr int WORDS = ST_GROUPS * 2 * BUF > ST_GROUPS * TM * ST_N ? ST_GROUPS * 2 * BUF : ST_GROUPS * TM * ST_N;
+  static constexpr int SMEM = WORDS * 4;
+};
+
+__device__ __forceinline__ void group_barrier(int group) { asm volatile("bar.sync %0, 64;" ::"r"(group + 1) : "memory"); }
+
+template <int MODE, int TM>
+__global__ void __launch_bounds__(ST_THREADS)
+gemm_f32_tile_kernel(const GemmF32 p) {
+  using Cfg = SgemmTile<TM>;
+  constexpr bool GATED = MODE == SG_GATED;
+  constexpr int TN = ST_N, TO = GATED ? TN / 2 : TN, MR = TM / 8, NR = TN / 8, NA = TM / 16, NB = TN / 16;
+  extern __shared__ __align__(16) float st_sm[];
+  int M = p.M;
+  const float *a = p.A, *B = p.B;
+  float* C = p.C;
+  if constexpr (MODE == SG_GROUPED || GATED) {
+    const MoeSegment sg = moe_segment(p.seg_off, p.n_routed, p.seg_rows, blockIdx.z);
+    M = sg.rows;
+    B += static_cast<size_t>(blockIdx.z) * p.N * (GATED ? 2 : 1) * p.ldb;
+    a = p.X != nullptr && static_cast<int>(blockIdx.z) >= p.n_routed ? p.X : p.A + static_cast<size_t>(sg.row0) * p.lda;
+    C += static_cast<size_t>(sg.row0) * p.ldc;
+  }
+  if constexpr (MODE == SG_BATCHED) {
+    a += blockIdx.z * p.a_stride;
+    B += blockIdx.z * p.b_stride;
+    C += blockIdx.z * p.c_stride;
+  }
+  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TO;
+  if (m0 >= M) return;
+  const int group = threadIdx.x >> 6, tid = threadIdx.x & 63, tx = tid & 7, ty = tid >> 3;
+  float* mine = st_sm + group * 2 * Cfg::BUF;
+  // what this thread carries of a slice: four columns in a row of NA rows of A and NB of B
+  const int vr = tid >> 2, vk = (tid & 3) * 4;
+  const float *arow[NA], *brow[NB];
+#pragma unroll
+  for (int i = 0; i < NA; ++i) arow[i] = m0 + vr + 16 * i < M ? a + static_cast<size_t>(m0 + vr + 16 * i) * p.lda : nullptr;
+#pragma unroll
+  for (int i = 0; i < NB; ++i) {
+    const int r = vr + 16 * i, n = n0 + (GATED ? r % TO : r);          // gated: the gate rows, then the up rows of the same outputs
+    brow[i] = n < p.N ? B + static_cast<size_t>(GATED && r >= TO ? p.N + n : n) * p.ldb : nullptr;
+  }
+  float4 ra[NA], rb[NB];
+  auto fetch = [&](int k0) {
+    const bool in = k0 + vk < p.K;
+#pragma unroll
+    for (int i = 0; i < NA; ++i) ra[i] = in && arow[i] != nullptr ? load4(arow[i] + k0 + vk) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < NB; ++i) rb[i] = in && brow[i] != nullptr ? load4(brow[i] + k0 + vk) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  auto put = [](float* at, int ld, float4 v) { at[0] = v.x; at[ld] = v.y; at[2 * ld] = v.z; at[3 * ld] = v.w; };
+  auto stash = [&](int buf) {
+    float *as = mine + buf * Cfg::BUF + vk * Cfg::LA + vr, *bs = mine + buf * Cfg::BUF + ST_K * Cfg::LA + vk * Cfg::LB + vr;
+#pragma unroll
+    for (int i = 0; i < NA; ++i) put(as + 16 * i, Cfg::LA, ra[i]);
+#pragma unroll
+    for (int i = 0; i < NB; ++i) put(bs + 16 * i, Cfg::LB, rb[i]);
+  };
+  // rows 4 ty .. + 3 and every 32nd from there, columns 4 tx .. + 3 and every 32nd from there
+  float acc[MR][NR] = {};
+  int k0 = group * ST_K, buf = 0;
+  if (k0 < p.K) {
+    fetch(k0);
+    stash(0);
+    group_barrier(group);
+  }
+  for (; k0 < p.K; k0 += ST_GROUPS * ST_K, buf ^= 1) {
+    const bool more = k0 + ST_GROUPS * ST_K < p.K;
+    if (more) fetch(k0 + ST_GROUPS * ST_K);
+    const float *as = mine + buf * Cfg::BUF + ty * 4, *bs = mine + buf * Cfg::BUF + ST_K * Cfg::LA + tx * 4;
+#pragma unroll
+    for (int k = 0; k < ST_K; ++k) {
+      float x[MR], y[NR];
+#pragma unroll
+      for (int h = 0; h < MR / 4; ++h) *reinterpret_cast<float4*>(&x[4 * h]) = load4(as + k * Cfg::LA + 32 * h);
+#pragma unroll
+      for (int h = 0; h < NR / 4; ++h) *reinterpret_cast<float4*>(&y[4 * h]) = load4(bs + k * Cfg::LB + 32 * h);
+#pragma unroll
+      for (int i = 0; i < MR; ++i)
+#pragma unroll
+        for (int j = 0; j < NR; ++j) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
+    }
+    if (more) {
+      stash(buf ^ 1);            // last read before the previous barrier
+      group_barrier(group);
+    }
+  }
+  __syncthreads();               // the buffers turn into the groups' sums [group][TM][TN]
+  float* sums = st_sm + group * TM * TN;
+#pragma unroll
+  for (int i = 0; i < MR; ++i)
+#pragma unroll
+    for (int h = 0; h < NR / 4; ++h)
+      store4(sums + ((i >> 2) * 32 + ty * 4 + (i & 3)) * TN + 32 * h + tx * 4, make_float4(acc[i][4 * h], acc[i][4 * h + 1], acc[i][4 * h + 2], acc[i][4 * h + 3]));
+  __syncthreads();
+  auto total = [&](int at) {
+    float v = st_sm[at];
+#pragma unroll
+    for (int g = 1; g < ST_GROUPS; ++g) v += st_sm[g * TM * TN + at];
+    return v;
+  };
+#pragma unroll 4
+  for (int e = threadIdx.x; e < TM * TO; e += ST_THREADS) {
+    const int r = e / TO, c = e % TO;
+    if (m0 + r >= M || n0 + c >= p.N) continue;
+    float v = total(r * TN + c);
+    if constexpr (GATED) v = silu_mul(v, total(r * TN + TO + c));
+    if constexpr (MODE == SG_GROUPED) v = p.act == FF_GELU ? ff_act<FF_GELU>(v) : (p.act == FF_RELU2 ? ff_act<FF_RELU2>(v) : v);
+    C[static_cast<size_t>(m0 + r) * p.ldc + n0 + c] = v;
   }
 }
 
@@ -288,6 +401,21 @@ static bool vector_rows(const GemmF32& p) {
   return MODE != SG_BATCHED || ((p.a_stride | p.b_stride) & 3) == 0;
 }
 
+template <int MODE, int TM>
+static int launch_tiles(const GemmF32& p, int rows, int batch, cudaStream_t stream) {
+  auto kern = gemm_f32_tile_kernel<MODE, TM>;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SgemmTile<TM>::SMEM) != cudaSuccess) return -20;
+    configured = true;
+  }
+  constexpr int width = MODE == SG_GATED ? ST_N / 2 : ST_N;
+  const dim3 grid((p.N + width - 1) / width, (rows + TM - 1) / TM, batch);
+  if (grid.y > 65535u) return -2;
+  kern<<<grid, ST_THREADS, SgemmTile<TM>::SMEM, stream>>>(p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+}
+
 template <int MODE>
 static int launch_gemm_f32(const GemmF32& p, int rows, int batch, void* stream_v) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
@@ -305,11 +433,17 @@ static int launch_gemm_f32(const GemmF32& p, int rows, int batch, void* stream_v
         return launch_pdl(gemm_f32_rows_kernel<MODE>, dim3((p.N + per - 1) / per, 1, batch), dim3(SR_WARPS * 32), 0, stream, p, ks) == cudaSuccess
                    ? 0 : -21;
       }
-      gemm_f32_kernel<MODE, true><<<grid, 256, 0, stream>>>(p);
-      return cudaGetLastError() == cudaSuccess ? 0 : -21;
+      // Which tile: one wave of 32-row tiles takes 45 us (K = 2048), every wave of two an SM 73, a wave of 64-row tiles, one an SM, 60. Of segments only
+      // the bound of their rows is known: 32 experts of which every row takes four change over at 500 rows (40 rows, 1024 x 2048: 145 and 239 us, 240
+      // rows 223 and 250, 500 rows 376 and 375, 960 rows 692 and 630). Tiles of 64 x 128 gained nothing (240 rows, N = K = 4096: 247 us, 236 with 64).
+      constexpr int width = MODE == SG_GATED ? ST_N / 2 : ST_N;
+      const long long cols = static_cast<long long>((p.N + width - 1) / width) * batch, low = (rows + 31) / 32 * cols, high = (rows + 63) / 64 * cols;
+      const long long cost_low = low <= 148 ? 45 : (low + 295) / 296 * 73, cost_high = (high + 147) / 148 * 60;
+      const bool segments = MODE == SG_GROUPED || MODE == SG_GATED;
+      return (segments ? rows < 500 : cost_low <= cost_high) ? launch_tiles<MODE, 32>(p, rows, batch, stream) : launch_tiles<MODE, 64>(p, rows, batch, stream);
     }
   }
-  gemm_f32_kernel<MODE, false><<<grid, 256, 0, stream>>>(p);
+  gemm_f32_kernel<MODE><<<grid, 256, 0, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
