@@ -22,6 +22,7 @@
 #include "common.cuh"
 #include "pair.cuh"
 #include "rpeg_kernels.h"
+#include "skinny.cuh"
 
 namespace rpeg {
 
@@ -710,11 +711,17 @@ extern "C" int rpeg_gemm_bf16_partials(const void* A, const void* B, int M, int 
     *k_splits_out = plan.splits;
     return gemm_pair(A, B, workspace, M, N, K, lda, ldb, N, 0, 0, 1, 0, plan, g_num_sms, pdl_enabled(), status, stream);
   }
+  // From 33 rows on, of matrices that several SMs share, gemm_skinny.cu: K = 4096, us here (tiles of 128 rows x 128 or 256 columns) and there: 33 / 64 / 128 rows
+  // of 2048 6.4 and 5.7 / 7.0 and 6.1 / 8.4 and 6.5; of 12288 20.2 and 18.5 / 22.5 and 19.7 / 26.9 and 23.4; of 22016 35.1 and 32.8 / 38.4 and 32.8 / 44.7 and
+  // 36.9; but of 1024 4.8 and 5.5 / 5.3 and 6.6 / 7.1 and 5.8, and at K = 128 of 4096 3.6 and 4.3.
+  if (M > 32 && N >= 2048 && static_cast<long long>(N) * K >= 2048ll * 1024) {
+    const SkinnyPlan plan = skinny_plan(M, N, K, workspace_elems, g_num_sms);
+    *k_splits_out = plan.splits;
+    return skinny_partials(A, B, workspace, M, N, K, lda, ldb, plan, status, stream);
+  }
   // Few rows: the wide tile, fewest reads of A. From 33 rows on the slabs weigh as much as that, and the narrow tile needs half as many to fill
-  // the SMs and stores one half while it multiplies the other. With the kernel that adds the slabs, K = 4096, us at 256 and at 128 columns: 33 / 64 /
-  // 128 rows of 4096 14.3 and 13.2 / 15.7 and 14.2 / 19.1 and 16.1; of 12288 25.7 and 24.4 / 28.3 and 26.9 / 34.5 and 31.1; of 16384 29.3 and 30.2 /
-  // 31.3 and 31.2 / 36.5 and 33.7; of 20480 38.4 and 41.3 / 43.1 and 44.7 / 53.2 and 49.0: up to 64 rows they change over about 16384.
-  const bool narrow = M > 32 && (M > 64 || N <= 16384);
+  // the SMs and stores one half while it multiplies the other.
+  const bool narrow = M > 32;
   const int bn = N >= 256 && !narrow ? 256 : (N >= 128 ? 128 : (N >= 64 ? 64 : 32));
   const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);
   const int num_kb = (K + BK - 1) / BK;
@@ -727,8 +734,7 @@ extern "C" int rpeg_gemm_bf16_partials(const void* A, const void* B, int M, int 
     if ((num_kb + kb_per - 1) / kb_per != sp) continue;
     if (workspace_elems / per_split < sp) break;
     const int waves = (tiles * sp + g_num_sms - 1) / g_num_sms;
-    // The consumer reads every partial once; no separate reduction pass writes and re-reads them. A narrow tile's slabs weigh twice as much
-    // (128 rows of 22016: two of them 50.2 us, the four that the lower weight chooses 56.8; up to 64 rows both choose the same).
+    // The consumer reads every partial once; no separate reduction pass writes and re-reads them. A narrow tile's slabs weigh twice as much.
     const double cost = waves * (kb_per + 2.0) + sp * per_split * (narrow ? 16.0 : 8.0) / block_bytes;
     if (cost < best - 1e-9) { best = cost; want = sp; }
   }

@@ -1,0 +1,376 @@
+// Products of few activation rows (decode): the weights go on the M axis of tcgen05.mma, the rows on N.
+//
+//   partial sums    C_s[m, f], s = 0 .. splits - 1 (fp32 slabs), sum_s C_s = X[m, 0..K) * W[f, 0..K)^T, up to 128 rows
+//   experts         C[r, f] = act( X[r, 0..K) * W_e[f, 0..K)^T ) for every row r of segment e (segments as in moe.cu), up to 128 rows a segment
+//
+// Bound by streaming the weights. With rows on the M axis a tile was 128 rows high, whatever their number: the accumulator of 6 rows was read by one
+// warp, 256 columns of it one after the other. Here a tile is 128 weight rows x 16 .. 128 columns, all four epilogue warps hold a feature per
+// lane, and what a K block brings in beside 16 KB of weights is 2 KB for every 16 rows.
+//
+// Dense products are cut evenly: the K blocks of all tiles form one list, of which every CTA takes an equal run (whole tiles cut in equal pieces left
+// up to a fifth of the last wave empty and needed more slabs). A tile's pieces are numbered by CTA; where a tile has fewer pieces than another,
+// its last one stores zeros for the rest.
+//
+// Roles (192 threads, persistent): warp 0 TMA producer, warp 1 issues the MMAs, warps 2..5 epilogue (32 features each). A grid that was launched as a
+// programmatic dependent requests its first weights before it waits for the kernel before (dense: weights are known; experts: they depend on it).
+#include "act_io.cuh"
+#include "moe_segments.cuh"
+#include "rpeg_kernels.h"
+#include "skinny.cuh"
+
+namespace rpeg {
+
+int make_tmap_bf16_2d(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner, uint32_t box_outer);
+int make_tmap_bf16_5d(CUtensorMap* out, const void* ptr, const uint64_t* dims, const uint64_t* strides, const uint32_t* box);
+
+constexpr int SK_BK = 64, SK_THREADS = 192, SK_F = 128;              // features per tile (gated: 64 gate and 64 up rows)
+constexpr int SK_W_BYTES = SK_F * SK_BK * 2;
+constexpr int SK_MAX_SEGMENTS = 1024;
+
+enum { SK_PARTS = 0, SK_EXPERTS = 1 };
+
+template <int NT, int MODE>
+struct SkinnyCfg {
+  static constexpr int STAGE_BYTES = SK_W_BYTES + NT * SK_BK * 2;
+  static constexpr int LIST_BYTES = MODE == SK_EXPERTS ? (SK_MAX_SEGMENTS * 3 + 4) * 4 : 0;
+  static constexpr int RAW = (227 * 1024 - 1024 - 512 - LIST_BYTES) / STAGE_BYTES;
+  static constexpr int STAGES = RAW > 12 ? 12 : RAW;
+  static constexpr int BUFS = NT <= 64 ? 4 : 2;                      // accumulators of NT columns
+  static constexpr int TMEM_COLS = BUFS * NT;
+  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 512 + LIST_BYTES;
+};
+
+struct Skinny {
+  int M, N, K, splits;
+  float* parts;                                                      // SK_PARTS
+  const int* seg_off;                                                // SK_EXPERTS
+  int n_routed, n_shared, seg_rows, shared_from_x, ldc;
+  __nv_bfloat16* C;
+  int* status;
+};
+
+struct SkinnyItem {
+  int w0, f0, row0, rows, kb0, kb1, slot, seg;                       // w0: first weight row; rows [row0, row0 + rows) of X and C
+};
+
+template <int NT, int MODE, int ACT>
+__global__ void __launch_bounds__(SK_THREADS, 1)
+gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_s,
+                   const Skinny p) {
+  using Cfg = SkinnyCfg<NT, MODE>;
+  constexpr int STAGES = Cfg::STAGES, BUFS = Cfg::BUFS;
+  constexpr bool GATED = ACT == FF_SWIGLU;
+  constexpr int TF = GATED ? SK_F / 2 : SK_F;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES);
+  uint64_t* empty_bar = full_bar + STAGES;
+  uint64_t* tfull_bar = empty_bar + STAGES;
+  uint64_t* tempty_bar = tfull_bar + BUFS;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + BUFS);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  int* list = reinterpret_cast<int*>(smem + STAGES * Cfg::STAGE_BYTES + 512);     // SK_EXPERTS: how many segments have rows, then {segment, row0, rows}
+
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int b = 0; b < BUFS; ++b) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 4); }
+    *abort_flag = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tmap_w);
+    tma_prefetch_desc(&tmap_x);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
+    tmem_relinquish();
+  }
+  griddep_launch();
+  if constexpr (MODE == SK_EXPERTS) {
+    griddep_wait();
+    if (warp == 2) {
+      const int S = p.n_routed + p.n_shared;
+      int n = 0;
+      for (int s0 = 0; s0 < S; s0 += 32) {
+        const int s = s0 + lane;
+        MoeSegment sg{0, 0};
+        if (s < S) sg = moe_segment(p.seg_off, p.n_routed, p.seg_rows, s);
+        const uint32_t has = __ballot_sync(0xffffffffu, sg.rows > 0);
+        if (sg.rows > 0) {
+          int* e = list + 1 + 3 * (n + __popc(has & ((1u << lane) - 1)));
+          e[0] = s; e[1] = static_cast<int>(sg.row0); e[2] = sg.rows;
+        }
+        n += __popc(has);
+      }
+      if (lane == 0) list[0] = n;
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  if constexpr (MODE == SK_PARTS) {
+    if (threadIdx.x != 0) griddep_wait();     // the producer waits behind its first weights
+  }
+
+  const int num_kb = (p.K + SK_BK - 1) / SK_BK, tiles = (p.N + TF - 1) / TF;
+  // SK_PARTS: this CTA's run of the list of K blocks; the CTA of block x is the largest c with c * total / grid <= x
+  const long long total = static_cast<long long>(tiles) * num_kb;
+  const int grid = gridDim.x, cta = blockIdx.x;
+  const int run0 = static_cast<int>(total * cta / grid), run1 = static_cast<int>(total * (cta + 1) / grid);
+  const int begin = MODE == SK_PARTS ? run0 : cta;
+  auto next = [&](int& at, SkinnyItem& it) -> bool {
+    if constexpr (MODE == SK_PARTS) {
+      if (at >= run1) return false;
+      const int tile = at / num_kb, kb = at - tile * num_kb, n = min(num_kb - kb, run1 - at);
+      const int first = static_cast<int>(((static_cast<long long>(tile) * num_kb + 1) * grid - 1) / total);
+      it = {tile * TF, tile * TF, 0, p.M, kb, kb + n, cta - first, 0};
+      at += n;
+    } else {
+      if (at >= list[0] * tiles) return false;
+      const int k = at / tiles, f0 = (at - k * tiles) * TF;
+      const int* e = list + 1 + 3 * k;
+      it = {e[0] * p.N + f0, f0, e[1], e[2], 0, num_kb, 0, e[0]};
+      at += grid;
+    }
+    return true;
+  };
+  // K blocks bring 16 rows a box for experts (as many as the segment has), one box of NT rows for dense products
+  auto boxes = [&](const SkinnyItem& it) -> int { return MODE == SK_PARTS ? 1 : (it.rows + 15) / 16; };
+  constexpr int BOX = MODE == SK_PARTS ? NT : 16;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      SkinnyItem it;
+      const uint64_t once = l2_policy(true);
+      auto load_w = [&](int stage, int kb) {
+        uint8_t* sw = smem + stage * Cfg::STAGE_BYTES;
+        mbar_expect_tx(&full_bar[stage], SK_W_BYTES + boxes(it) * BOX * SK_BK * 2);
+        if constexpr (GATED) {
+          asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5, %6, %7}], [%2], %8;" ::"r"(
+                           smem_u32(sw)),
+                       "l"(reinterpret_cast<uint64_t>(&tmap_w)), "r"(smem_u32(&full_bar[stage])), "r"(kb * SK_BK), "r"(0), "r"(0), "r"(it.f0 / 16),
+                       "r"(it.seg), "l"(once)
+                       : "memory");
+        } else {
+          tma_load_2d_hint(sw, &tmap_w, &full_bar[stage], kb * SK_BK, it.w0, once);
+        }
+      };
+      int ahead = 0;
+      if constexpr (MODE == SK_PARTS) {
+        for (int at = begin; ahead < STAGES && next(at, it);)
+          for (int kb = it.kb0; kb < it.kb1 && ahead < STAGES; ++kb) load_w(ahead++, kb);
+        griddep_wait();
+      }
+      int stage = 0, i = 0;
+      uint32_t phase = 0;
+      for (int at = begin; next(at, it);) {
+        const bool shared = MODE == SK_EXPERTS && p.shared_from_x && it.seg >= p.n_routed;
+        const CUtensorMap* tx = shared ? &tmap_s : &tmap_x;
+        const int row0 = shared ? 0 : it.row0, nb = boxes(it);
+        for (int kb = it.kb0; kb < it.kb1; ++kb, ++i) {
+          if (i >= ahead) {
+            if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, 1300)) goto producer_done;
+            load_w(stage, kb);
+          }
+          uint8_t* sx = smem + stage * Cfg::STAGE_BYTES + SK_W_BYTES;
+          for (int b = 0; b < nb; ++b) tma_load_2d(sx + b * BOX * SK_BK * 2, tx, &full_bar[stage], kb * SK_BK, row0 + b * BOX);
+          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+        }
+      }
+    producer_done:;
+    }
+  } else if (warp == 1) {
+    const uint32_t s0 = smem_u32(smem);
+    const uint64_t dw0 = make_smem_desc_sw128(s0, 16, 1024), dx0 = make_smem_desc_sw128(s0 + SK_W_BYTES, 16, 1024);
+    int stage = 0, buf = 0;
+    uint32_t phase = 0, acc_phase = 0;
+    bool ok = true;
+    SkinnyItem it;
+    for (int at = begin; ok && next(at, it);) {
+      const uint32_t idesc = make_idesc_bf16(SK_F, boxes(it) * BOX, 0, 0);
+      ok = __all_sync(0xffffffffu, mbar_wait(&tempty_bar[buf], acc_phase ^ 1u, abort_flag, p.status, 1301));
+      if (!ok) break;
+      tc_fence_after_sync();
+      const uint32_t tacc = tmem_base + static_cast<uint32_t>(buf * NT);
+      for (int kb = it.kb0; kb < it.kb1; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, abort_flag, p.status, 1302));
+        if (!ok) break;
+        tc_fence_after_sync();
+        const uint64_t dw = smem_desc_at(dw0, stage * Cfg::STAGE_BYTES), dx = smem_desc_at(dx0, stage * Cfg::STAGE_BYTES);
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < SK_BK / 16; ++k)
+            umma_bf16_ss(tacc, smem_desc_at(dw, k * 32), smem_desc_at(dx, k * 32), idesc, (kb != it.kb0 || k != 0) ? 1u : 0u);
+          umma_commit(&empty_bar[stage]);
+          if (kb == it.kb1 - 1) umma_commit(&tfull_bar[buf]);
+        }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+      }
+      if (++buf == BUFS) { buf = 0; acc_phase ^= 1u; }
+    }
+  } else {
+    const int quad = warp & 3;          // TMEM lane quadrant this warp may read: 32 weight rows of the tile
+    int buf = 0;
+    uint32_t acc_phase = 0;
+    SkinnyItem it;
+    for (int at = begin; next(at, it);) {
+      if (!__all_sync(0xffffffffu, mbar_wait(&tfull_bar[buf], acc_phase, abort_flag, p.status, 1303))) break;
+      tc_fence_after_sync();
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(buf * NT);
+#pragma unroll 1
+      for (int c = 0; c * 16 < it.rows; ++c) {
+        uint32_t v[16];
+        tmem_ld_32x16(taddr + c * 16, v);
+        tmem_wait_ld();
+        if constexpr (MODE == SK_PARTS) {
+          const int f = it.f0 + quad * 32 + lane;
+          if (f < p.N) {
+            const size_t slab = static_cast<size_t>(p.M) * p.N;
+            float* out = p.parts + it.slot * slab + static_cast<size_t>(c * 16) * p.N + f;
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (c * 16 + j < it.rows) out[static_cast<size_t>(j) * p.N] = __uint_as_float(v[j]);
+            if (it.kb1 == num_kb)
+              for (int s = it.slot + 1; s < p.splits; ++s) {
+                out += slab;
+                for (int j = 0; j < 16 && c * 16 + j < it.rows; ++j) out[static_cast<size_t>(j) * p.N] = 0.f;
+              }
+          }
+        } else if constexpr (GATED) {   // rows of the tile: 16 gate rows, 16 up rows of the same features, and so on
+          const bool up = lane >= 16;
+          const int f = it.f0 + quad * 16 + (lane & 15);
+          __nv_bfloat16* out = p.C + static_cast<size_t>(it.row0 + c * 16) * p.ldc + f;
+#pragma unroll
+          for (int j = 0; j < 16; j += 2) {                // lanes 0..15 finish row j, the others row j + 1
+            const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(up ? v[j] : v[j + 1]), 16);
+            const float own = __uint_as_float(up ? v[j + 1] : v[j]);
+            const int r = j + (up ? 1 : 0);
+            if (f < p.N && c * 16 + r < it.rows) out[static_cast<size_t>(r) * p.ldc] = __float2bfloat16(up ? silu_mul(other, own) : silu_mul(own, other));
+          }
+        } else {
+          const int f = it.f0 + quad * 32 + lane;
+          if (f < p.N) {
+            __nv_bfloat16* out = p.C + static_cast<size_t>(it.row0 + c * 16) * p.ldc + f;
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (c * 16 + j < it.rows) out[static_cast<size_t>(j) * p.ldc] = __float2bfloat16(ff_act<ACT>(__uint_as_float(v[j])));
+          }
+        }
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty_bar[buf]);
+      if (++buf == BUFS) { buf = 0; acc_phase ^= 1u; }
+    }
+  }
+
+  // Teardown. After an aborted wait there may be bulk copies in flight; give them time to land before the block exits.
+  __syncwarp();
+  if (*abort_flag) __nanosleep(200000);
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+  }
+}
+
+template <int NT, int MODE, int ACT>
+static int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& ts, const Skinny& p, int grid, cudaStream_t stream) {
+  using Cfg = SkinnyCfg<NT, MODE>;
+  auto kern = gemm_skinny_kernel<NT, MODE, ACT>;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess) return -20;
+    configured = true;
+  }
+  return launch_pdl(kern, dim3(grid), dim3(SK_THREADS), static_cast<size_t>(Cfg::SMEM), stream, tw, tx, ts, p) == cudaSuccess ? 0 : -21;
+}
+
+// CTAs and slabs: every SM, or as many CTAs as cut every tile in equal pieces, whichever costs less in K blocks of a CTA (16 KB of weights) and slabs
+// that are written and read again (N = K = 4096, 128 rows: 148 CTAs and six slabs 13.9 us, 128 and four 12.6; N = 22016: 148 and two 39 us). A CTA takes
+// four K blocks at least, and a tile is cut into at most 16 pieces.
+SkinnyPlan skinny_plan(int M, int N, int K, long long slab_elems, int num_sms) {
+  const int num_kb = (K + SK_BK - 1) / SK_BK, tiles = (N + SK_F - 1) / SK_F;
+  const long long total = static_cast<long long>(tiles) * num_kb, slab = static_cast<long long>(M) * N;
+  const int least = num_kb / 15 > 3 ? num_kb / 15 + 1 : 4;
+  long long most = (total + least - 1) / least;
+  if (most > num_sms) most = num_sms;
+  auto pieces = [&](long long grid) {
+    int splits = 1;
+    for (int t = 0; t < tiles; ++t) {
+      const long long a = ((static_cast<long long>(t) * num_kb + 1) * grid - 1) / total, b = ((t + 1ll) * num_kb * grid - 1) / total;
+      if (b - a + 1 > splits) splits = static_cast<int>(b - a + 1);
+    }
+    return splits;
+  };
+  SkinnyPlan best{0, 0};
+  double least_cost = 1e300;
+  auto consider = [&](long long grid) {
+    if (grid < 1 || grid > most) return;
+    const int splits = pieces(grid);
+    if (splits * slab > slab_elems) return;
+    const double cost = static_cast<double>((total + grid - 1) / grid) + static_cast<double>(splits * slab) * 8.0 / (num_sms * SK_W_BYTES);
+    if (cost < least_cost) { least_cost = cost; best = {static_cast<int>(grid), splits}; }
+  };
+  consider(most);
+  for (long long s = 1; tiles * s <= most; ++s) consider(tiles * s);
+  for (long long grid = most * 3 / 4; best.grid == 0; grid = grid * 3 / 4) {       // little scratch, more tiles than CTAs
+    if (grid < 1) grid = 1;
+    consider(grid);
+    if (grid == 1) break;
+  }
+  return best;
+}
+
+int skinny_partials(const void* X, const void* W, float* parts, int M, int N, int K, int ldx, int ldw, SkinnyPlan plan, int* status, cudaStream_t stream) {
+  const int nt = M <= 64 ? 64 : 128;
+  CUtensorMap tw, tx;
+  int rc = make_tmap_bf16_2d(&tx, X, K, M, ldx, SK_BK, nt);
+  if (rc) return rc;
+  rc = make_tmap_bf16_2d(&tw, W, K, N, ldw, SK_BK, SK_F);
+  if (rc) return rc - 100;
+  Skinny p{};
+  p.M = M; p.N = N; p.K = K; p.splits = plan.splits; p.parts = parts; p.status = status;
+  return nt == 64 ? launch_skinny<64, SK_PARTS, FF_NONE>(tw, tx, tx, p, plan.grid, stream) : launch_skinny<128, SK_PARTS, FF_NONE>(tw, tx, tx, p, plan.grid, stream);
+}
+
+template <int NT>
+static int skinny_act(int act, const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& ts, const Skinny& p, int grid, cudaStream_t stream) {
+  switch (act) {
+    case FF_NONE: return launch_skinny<NT, SK_EXPERTS, FF_NONE>(tw, tx, ts, p, grid, stream);
+    case FF_GELU: return launch_skinny<NT, SK_EXPERTS, FF_GELU>(tw, tx, ts, p, grid, stream);
+    case FF_SWIGLU: return launch_skinny<NT, SK_EXPERTS, FF_SWIGLU>(tw, tx, ts, p, grid, stream);
+    case FF_RELU2: return launch_skinny<NT, SK_EXPERTS, FF_RELU2>(tw, tx, ts, p, grid, stream);
+    default: return -4;
+  }
+}
+
+// Arguments are those of rpeg_moe_gemm, checked there; seg_rows <= 128; gated: N a multiple of 16.
+int skinny_experts(const void* A, long long a_rows_total, const void* X, const void* B, void* C, const int* seg_off, int n_routed, int n_shared,
+                   int seg_rows, int N, int K, int lda, int ldx, int ldb, int ldc, int act, int grid, int* status, cudaStream_t stream) {
+  const int S = n_routed + n_shared;
+  CUtensorMap tw, tx, ts;
+  int rc = make_tmap_bf16_2d(&tx, A, K, a_rows_total, lda, SK_BK, 16);
+  if (rc) return rc;
+  rc = X != nullptr ? make_tmap_bf16_2d(&ts, X, K, seg_rows, ldx, SK_BK, 16) : make_tmap_bf16_2d(&ts, A, K, a_rows_total, lda, SK_BK, 16);
+  if (rc) return rc - 100;
+  if (act == FF_SWIGLU) {
+    const uint64_t row = ldb, dims[5] = {static_cast<uint64_t>(K), 16, 2, static_cast<uint64_t>(N / 16), static_cast<uint64_t>(S)};
+    const uint64_t strides[4] = {row, N * row, 16 * row, 2 * N * row};
+    const uint32_t box[5] = {SK_BK, 16, 2, 4, 1};
+    rc = make_tmap_bf16_5d(&tw, B, dims, strides, box);
+  } else {
+    rc = make_tmap_bf16_2d(&tw, B, K, static_cast<uint64_t>(S) * N, ldb, SK_BK, SK_F);
+  }
+  if (rc) return rc - 200;
+  Skinny p{};
+  p.N = N; p.K = K; p.seg_off = seg_off; p.n_routed = n_routed; p.n_shared = n_shared; p.seg_rows = seg_rows;
+  p.shared_from_x = X != nullptr; p.ldc = ldc; p.C = static_cast<__nv_bfloat16*>(C); p.status = status;
+  if (seg_rows <= 16) return skinny_act<16>(act, tw, tx, ts, p, grid, stream);
+  if (seg_rows <= 64) return skinny_act<64>(act, tw, tx, ts, p, grid, stream);
+  return skinny_act<128>(act, tw, tx, ts, p, grid, stream);
+}
+
+}  // namespace rpeg

@@ -17,6 +17,7 @@
 #include "moe_segments.cuh"
 #include "pair.cuh"
 #include "rpeg_kernels.h"
+#include "skinny.cuh"
 
 namespace rpeg {
 
@@ -454,6 +455,11 @@ extern "C" int rpeg_moe_gemm(const void* A, long long a_rows_total, const void* 
   const long long active = choices < n_routed ? choices : n_routed;
   const long long m_tiles = choices / MG_BM + active + static_cast<long long>(n_shared) * ((seg_rows + MG_BM - 1) / MG_BM);
   int bn = bn_hint;
+  if (bn == 0 && seg_rows <= (act == FF_SWIGLU ? 128 : 64) && (act != FF_SWIGLU || (N & 15) == 0)) {
+    const long long items = (active + n_shared) * (act == FF_SWIGLU ? (N + 63) / 64 : (N + 127) / 128);
+    return skinny_experts(A, a_rows_total, X, B, C, seg_off, n_routed, n_shared, seg_rows, N, K, lda, ldx, ldb, ldc, act,
+                          static_cast<int>(items < num_sms ? items : num_sms), status, STREAM(stream));
+  }
   if (bn == 0) {
     // Prompts: pairs of CTAs with tiles as high as a segment's rows ask for (moe_pair.cu), once experts have about 160 rows and there are six
     // items a pair, with estimated halves for the last tiles (64 experts, 1024 x 4096 gated: 96 rows each 193 us either way, 192 rows 229 and 210

@@ -1,0 +1,15 @@
+// Host entries of gemm_skinny.cu: products of up to 128 activation rows.
+#pragma once
+#include "common.cuh"
+
+namespace rpeg {
+
+struct SkinnyPlan {                     // of skinny_plan(): CTAs, slabs of partial sums
+  int grid, splits;
+};
+SkinnyPlan skinny_plan(int M, int N, int K, long long slab_elems, int num_sms);
+int skinny_partials(const void* X, const void* W, float* parts, int M, int N, int K, int ldx, int ldw, SkinnyPlan plan, int* status, cudaStream_t stream);
+int skinny_experts(const void* A, long long a_rows_total, const void* X, const void* B, void* C, const int* seg_off, int n_routed, int n_shared,
+                   int seg_rows, int N, int K, int lda, int ldx, int ldb, int ldc, int act, int grid, int* status, cudaStream_t stream);
+
+}  // namespace rpeg

@@ -235,7 +235,7 @@ class ZafopelModel(ServedDecoder):
     """Weights and kernels of one model on one GPU."""
 
     prefill_spans = True
-    KERNEL_SOURCES = ("gemm.cu", "gemm_pair.cu", "generate.cu", "loss.cu", "stream_update.cu", "latent.cu", "latent_decode.cu", "latent_prefill.cu", "head_gemm.cu",
+    KERNEL_SOURCES = ("gemm.cu", "gemm_pair.cu", "gemm_skinny.cu", "generate.cu", "loss.cu", "stream_update.cu", "latent.cu", "latent_decode.cu", "latent_prefill.cu", "head_gemm.cu",
                       "moe.cu", "moe_pair.cu", "gemm_f32.cu")
 
     def __init__(self, cfg: ZafopelConfig, device, *, dtype: torch.dtype = torch.bfloat16, seed: Optional[int] = 0, trainable: bool = False):

@@ -358,3 +358,38 @@ def test_paged_decode_attn_aliased_rows(cuda_device, h, hkv, split):
             assert not bool(out[i].isfinite().any()) and not bool(want.isfinite().any())
         else:
             assert _rel(out[i], want) < 2 ** -8
+
+
+# tiles of 128 features, columns for 16, 32, 64 and 128 rows; runs of K blocks that cross tiles, fewer blocks than CTAs, scratch for one slab only
+@pytest.mark.parametrize("m", [1, 15, 16, 17, 32, 33, 64, 65, 127, 128])
+@pytest.mark.parametrize("n,k,slabs", [(8, 8, 1), (136, 72, 4), (128, 4096, 20), (1288, 1032, 20), (12288, 520, 2), (2056, 4096, 1)])
+def test_gemm_partials_few_rows(cuda_device, m, n, k, slabs):
+    g = torch.Generator(device=cuda_device).manual_seed(m)
+    a, b = (torch.randn(r, k, generator=g, device=cuda_device).bfloat16() for r in (m, n))
+    ws = torch.full((slabs * m * n + 3,), float("nan"), device=cuda_device)
+    p = K.gemm_partials(a, b, ws)
+    assert p.splits <= slabs
+    # the tensor cores cut a sum off where they add 16 products to it: up to 2^-23 of it at each of the k / 16 additions of a slab, half of it on average
+    assert _rel(p.buf[: p.splits * m * n].view(p.splits, m, n).sum(0), a.double() @ b.double().T) < F32 + k / 16 * 2 ** -24
+
+
+@pytest.mark.parametrize("t", [1, 7, 16, 17, 33, 64, 65, 128])
+@pytest.mark.parametrize("e,top,shared,n,k,act", [(5, 2, 0, 136, 72, "none"), (40, 3, 2, 264, 136, "gelu"), (3, 3, 1, 128, 64, "relu2"), (6, 2, 0, 144, 200, "swiglu"), (2, 1, 1, 16, 4096, "swiglu")])
+def test_moe_gemm_few_rows(cuda_device, t, e, top, shared, n, k, act):
+    dev, g = cuda_device, torch.Generator(device=cuda_device).manual_seed(t)
+    x = torch.randn(t, k, generator=g, device=dev).bfloat16()
+    w = (torch.randn(e + shared, n * (2 if act == "swiglu" else 1), k, generator=g, device=dev) / k ** 0.5).bfloat16()
+    counts = torch.zeros(e, dtype=torch.int32, device=dev)
+    scores = torch.randn(t, e, generator=g, device=dev)
+    scores[:, 0] += 2.0                                           # one expert has most of the rows, others none
+    ids, wts, ticket = K.moe_route(scores, e, top, counts)
+    r = K.moe_dispatch(x, ids, wts, ticket, counts, e)
+    got = K.moe_gemm(r.x_sorted, w, r, e, shared, shared_x=x if shared else None, act=act)
+    f = {"none": lambda z: z, "gelu": torch.nn.functional.gelu, "relu2": lambda z: torch.relu(z) ** 2,
+         "swiglu": lambda z: torch.nn.functional.silu(z[:, :n]) * z[:, n:]}[act]
+    off = r.seg_off.tolist()
+    spans = [(off[i], off[i + 1]) for i in range(e)] + [(off[e] + s * t, off[e] + (s + 1) * t) for s in range(shared)]
+    for i, (lo, hi) in enumerate(spans):
+        rows = r.x_sorted[lo:hi] if i < e else x
+        if hi > lo:
+            assert _rel(got[lo:hi, :n], f(rows.double() @ w[i].double().T)) < 2 ** -8
