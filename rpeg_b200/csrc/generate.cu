@@ -10,6 +10,7 @@
 // The reference keeps this state in Python per generation call and compacts KV rows on the host
 // side after every EOS (RPEG/runtime/workers/megatron_worker.py:2463-2598).
 #include "common.cuh"
+#include "decode_state.cuh"
 #include "rpeg_kernels.h"
 
 namespace rpeg {
@@ -40,20 +41,8 @@ __global__ void decode_advance_kernel(const int* __restrict__ sampled, const flo
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s == 0 && step_counter != nullptr) step_counter[0] += 1;
   if (s >= n_slots || !active[s]) return;
-  const int t = sampled[s];
-  const int g = gen_count[s];
-  out_tok[static_cast<size_t>(s) * max_new + g] = t;
-  out_lp[static_cast<size_t>(s) * max_new + g] = sampled_lp[s];
-  gen_count[s] = g + 1;
-  if (t == eos || g + 1 >= max_new) {
-    active[s] = 0;
-    seq_len[s] = 0;  // attention of a retired slot reads nothing
-    atomicAdd(n_finished, 1);
-  } else {
-    token[s] = t;
-    pos[s] += 1;
-    seq_len[s] += 1;
-  }
+  advance_row(DecodeState{nullptr, token, pos, seq_len, active, gen_count, out_tok, out_lp, max_new, eos, n_finished, nullptr, nullptr}, s, sampled[s],
+              sampled_lp[s]);
 }
 
 // out[i, :] = x[rows[i], :]   (bf16 rows, 16-byte vectors)

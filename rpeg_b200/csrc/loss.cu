@@ -10,6 +10,7 @@
 // :4361-4387 (GRPO), :4388-4417 (PPO actor), :4650 (critic), group advantages :4418, and the
 // sampler is megatron_worker.py:83-123.
 #include "common.cuh"
+#include "decode_state.cuh"
 #include "rpeg_kernels.h"
 
 namespace rpeg {
@@ -386,11 +387,13 @@ __device__ __forceinline__ float logit_at(const float* p) { return *p; }
 // One CTA per row; a decode step waits for it. Eight logits a turn: their maximum first, so that their exponentials do not wait for one
 // another (one at a time in 256 threads: 32000 bf16 logits 8.2 us greedy and 18.6 us with noise, now 4.9 and 9.8; 256 rows 54 us with noise, now 20).
 // THREADS: 1024, or 256 below 8192 logits, which are at most four turns of them (256 rows of 1000: 4.9 us with 1024, 3.1 with 256).
-template <typename T, int THREADS>
+// STEP: the bookkeeping of a decode step around the choice (generate.cu: the forced token before it, the row's state behind it), which were launches of
+// their own; the last CTA advances the step counter, which is the others' noise.
+template <typename T, int THREADS, bool STEP>
 __global__ void __launch_bounds__(THREADS)
 sample_kernel(const T* __restrict__ logits, int V, int ld, float inv_temp, int greedy,
-              unsigned long long seed, const unsigned long long* __restrict__ seed_offset,
-              const int* __restrict__ forced, int* __restrict__ token_out, float* __restrict__ logp_out) {
+              unsigned long long seed, const unsigned long long* seed_offset,
+              const int* __restrict__ forced, int* __restrict__ token_out, float* __restrict__ logp_out, const DecodeState st) {
   griddep_launch();
   griddep_wait();   // may have been scheduled under the previous kernel's tail: nothing is read or written before this
   __shared__ float sm_m[32], sm_s[32], sm_best[32];
@@ -474,9 +477,22 @@ sample_kernel(const T* __restrict__ logits, int V, int ld, float inv_temp, int g
     best_i = lane < THREADS / 32 ? sm_idx[lane] : 0x7fffffff;
     best_of_warp();
     if (lane == 0) {
-      if (forced != nullptr && forced[row] >= 0) best_i = forced[row];
+      if constexpr (STEP) {
+        best_i = forced_token(st, row, best_i);
+      } else {
+        if (forced != nullptr && forced[row] >= 0) best_i = forced[row];
+      }
+      const float lp = logit_at(lr + best_i) * inv_temp - (m + __logf(s));
       token_out[row] = best_i;
-      logp_out[row] = logit_at(lr + best_i) * inv_temp - (m + __logf(s));
+      logp_out[row] = lp;
+      if constexpr (STEP) {
+        advance_row(st, row, best_i, lp);
+        __threadfence();
+        if (atomicAdd(st.arrived, 1) == static_cast<int>(gridDim.x) - 1) {
+          *st.arrived = 0;
+          *st.step_counter += 1;
+        }
+      }
     }
   }
 }
@@ -701,8 +717,16 @@ static int launch_sample(const void* logits, int B, int V, int ld, float tempera
                          const unsigned long long* seed_offset, const int* forced, int* token_out, float* logp_out, void* stream) {
   if (B <= 0) return 0;
   const bool few = V < 8192;
-  launch_pdl(few ? sample_kernel<T, 256> : sample_kernel<T, 1024>, dim3(B), dim3(few ? 256 : 1024), 0, STREAM(stream), static_cast<const T*>(logits), V, ld, 1.f / temperature,
-             greedy, seed, seed_offset, forced, token_out, logp_out);
+  launch_pdl(few ? sample_kernel<T, 256, false> : sample_kernel<T, 1024, false>, dim3(B), dim3(few ? 256 : 1024), 0, STREAM(stream), static_cast<const T*>(logits), V, ld,
+             1.f / temperature, greedy, seed, seed_offset, forced, token_out, logp_out, DecodeState{});
+  return LAUNCH_OK();
+}
+template <typename T>
+static int launch_sample_step(const void* logits, int B, int V, int ld, float temperature, int greedy, unsigned long long seed, int* token_out,
+                              float* logp_out, const DecodeState& st, void* stream) {
+  const bool few = V < 8192;
+  launch_pdl(few ? sample_kernel<T, 256, true> : sample_kernel<T, 1024, true>, dim3(B), dim3(few ? 256 : 1024), 0, STREAM(stream), static_cast<const T*>(logits), V, ld,
+             1.f / temperature, greedy, seed, st.step_counter, nullptr, token_out, logp_out, st);
   return LAUNCH_OK();
 }
 template <typename T>
@@ -724,6 +748,17 @@ extern "C" int rpeg_sample_f32(const void* logits, int B, int V, int ld, float t
                                unsigned long long seed, const unsigned long long* seed_offset, const int* forced,
                                int* token_out, float* logp_out, void* stream) {
   return launch_sample<float>(logits, B, V, ld, temperature, greedy, seed, seed_offset, forced, token_out, logp_out, stream);
+}
+// rpeg_decode_prepare, rpeg_sample (noise by the step counter) and rpeg_decode_advance in one launch. `arrived`: one int, zero between launches.
+extern "C" int rpeg_sample_step(const void* logits, int B, int V, int ld, int f32, float temperature, int greedy, unsigned long long seed,
+                                const int* forced_len, int* sampled, float* sampled_lp, int* token, int* pos, int* seq_len, int* active,
+                                int* gen_count, int* out_tok, float* out_lp, int max_new, int eos, int* n_finished, unsigned long long* step_counter,
+                                int* arrived, void* stream) {
+  if (B <= 0) return 0;
+  if (step_counter == nullptr || arrived == nullptr) return -2;
+  const DecodeState st{forced_len, token, pos, seq_len, active, gen_count, out_tok, out_lp, max_new, eos, n_finished, step_counter, arrived};
+  return f32 ? launch_sample_step<float>(logits, B, V, ld, temperature, greedy, seed, sampled, sampled_lp, st, stream)
+             : launch_sample_step<__nv_bfloat16>(logits, B, V, ld, temperature, greedy, seed, sampled, sampled_lp, st, stream);
 }
 extern "C" int rpeg_sample_filtered(const void* logits, int B, int V, int ld, float temperature, int top_k, float top_p,
                                     unsigned long long seed, const unsigned long long* seed_offset, const int* forced,

@@ -128,6 +128,11 @@ int rpeg_kv_append(const void* qkv, int ld, int k_col0, int v_col0, const int* s
 int rpeg_rope_kv_append(void* qkv, int ld, int q_col0, int k_col0, int v_col0, const int* seq_id, const int* pos,
                         const float* cos_t, const float* sin_t, const int* page_table, int max_pages, void* kcache,
                         void* vcache, int T, int H, int Hkv, int hd, void* stream);
+int rpeg_embed_rmsnorm_fwd(const int* ids, const void* table, const void* w, void* h, void* y, int T, int d, float eps, void* stream);
+int rpeg_sample_step(const void* logits, int B, int V, int ld, int f32, float temperature, int greedy, unsigned long long seed,
+                     const int* forced_len, int* sampled, float* sampled_lp, int* token, int* pos, int* seq_len, int* active, int* gen_count,
+                     int* out_tok, float* out_lp, int max_new, int eos, int* n_finished, unsigned long long* step_counter, int* arrived,
+                     void* stream);
 long long rpeg_decode_attn_scratch_bytes(int B, int H, int nsplit);
 int rpeg_paged_decode_attn(const void* q, int ldq, int q_col0, const void* kcache, const void* vcache,
                            const int* page_table, int max_pages, const int* seq_lens, void* out, float* scratch,

@@ -169,6 +169,7 @@ class Generator:
         self.sampled_lp = torch.zeros(n, dtype=torch.float32, device=self.dev)
         self.n_finished = torch.zeros(1, **i32)
         self.step_counter = torch.zeros(1, dtype=torch.int64, device=self.dev)
+        self.arrived = torch.zeros(1, **i32)
         self.out_tok: Optional[torch.Tensor] = None
         self.out_lp: Optional[torch.Tensor] = None
         self._graphs: Dict[tuple, torch.cuda.CUDAGraph] = {}
@@ -196,6 +197,12 @@ class Generator:
         xf = m.decode_step(self.token[:b], self.pos[:b], self.slot_ids[:b], self.seq_len[:b], self.page_table[:b],
                            self.kcache, self.vcache, nsplit=self._nsplit(b), groups=groups)
         logits = m.lm_logits(xf, decode=True)
+        if greedy or not (0 < top_k < logits.shape[1] or top_p < 1.0):
+            K.sample_step(logits, temperature, greedy, seed, self.forced_len[:b], self.sampled[:b], self.sampled_lp[:b], self.token[:b], self.pos[:b],
+                          self.seq_len[:b], self.active[:b], self.gen_count[:b], self.out_tok[:b], self.out_lp[:b], self.eos_id, self.n_finished,
+                          self.step_counter, self.arrived)
+            K.set_pdl(True)
+            return
         K.decode_prepare(self.active[:b], self.gen_count[:b], self.forced_len[:b], self.forced[:b], self.eos_id)
         K.sample(logits, temperature, greedy, seed, forced=self.forced[:b], token_out=self.sampled[:b],
                  logp_out=self.sampled_lp[:b], seed_offset=self.step_counter, top_k=top_k, top_p=top_p)

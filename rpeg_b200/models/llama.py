@@ -465,8 +465,7 @@ class LlamaModel:
         # Every GEMM leaves its split-K partials in the workspace and the next kernel adds them up while it
         # loads them (one stream, so a consumer always runs before the next GEMM reuses the workspace).
         B = token.shape[0]
-        h = K.embed_fwd(token, p["embed"])
-        x, _, _ = K.rmsnorm_fwd(h, p["l0.attn_norm"], cfg.rms_eps)
+        x, h = K.embed_rmsnorm_fwd(token, p["embed"], p["l0.attn_norm"], cfg.rms_eps)
         qkv = torch.empty((B, cfg.qkv_width), dtype=torch.bfloat16, device=self.device)
         for i in range(cfg.n_layers):
             parts = K.gemm_partials(x, p[f"l{i}.wqkv"], ws)
@@ -489,11 +488,10 @@ class LlamaModel:
         cfg, p = self.cfg, self.p
         ws = self._workspace()
         scale = 1.0 / math.sqrt(cfg.head_dim)
-        res, delta = K.embed_fwd(token, p["embed"]), None
+        res = delta = None
         for i in range(cfg.n_layers):
             if delta is None:
-                h = res
-                x, _, _ = K.rmsnorm_fwd(h, p[f"l{i}.attn_norm"], cfg.rms_eps)
+                x, h = K.embed_rmsnorm_fwd(token, p["embed"], p[f"l{i}.attn_norm"], cfg.rms_eps)
             else:
                 x, _, h = K.rmsnorm_fwd(delta, p[f"l{i}.attn_norm"], cfg.rms_eps, residual=res, want_sum=True)
             qkv = K.gemm(x, p[f"l{i}.wqkv"], workspace=ws)

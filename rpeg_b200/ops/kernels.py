@@ -261,6 +261,22 @@ def embed_fwd(ids: torch.Tensor, table: torch.Tensor, out: torch.Tensor | None =
     return out
 
 
+def embed_rmsnorm_fwd(ids: torch.Tensor, table: torch.Tensor, w: torch.Tensor, eps: float):
+    """``(rmsnorm(h) * w, h)`` of the embedding rows ``h = table[ids]``, in one launch."""
+    if table.shape[1] > 8192:
+        h = embed_fwd(ids, table)
+        return rmsnorm_fwd(h, w, eps)[0], h
+    _req(ids, torch.int32, "ids")
+    _req(table, torch.bfloat16, "table")
+    if _chk.active():
+        _chk.embed("rpeg_embed_rmsnorm_fwd", ids, table.shape[0])
+    h = torch.empty((ids.numel(), table.shape[1]), dtype=table.dtype, device=table.device)
+    y = torch.empty_like(h)
+    check(lib().rpeg_embed_rmsnorm_fwd(ids.data_ptr(), table.data_ptr(), w.data_ptr(), h.data_ptr(), y.data_ptr(), ids.numel(), table.shape[1], eps,
+                                       _stream()), "rpeg_embed_rmsnorm_fwd")
+    return y, h
+
+
 def embed_bwd(ids: torch.Tensor, dout: torch.Tensor, dtable: torch.Tensor) -> None:
     if _chk.active():
         _chk.embed("rpeg_embed_bwd", ids, dtable.numel() // dout.shape[1])
@@ -652,6 +668,18 @@ def decode_advance(sampled, sampled_lp, token, pos, seq_len, active, gen_count, 
                                     seq_len.data_ptr(), active.data_ptr(), gen_count.data_ptr(), out_tok.data_ptr(),
                                     out_lp.data_ptr(), active.numel(), out_tok.shape[1], eos, n_finished.data_ptr(),
                                     _ptr(step_counter), _stream()), "rpeg_decode_advance")
+
+
+def sample_step(logits, temperature: float, greedy: bool, seed: int, forced_len, sampled, sampled_lp, token, pos, seq_len, active, gen_count,
+                out_tok, out_lp, eos: int, n_finished, step_counter, arrived) -> None:
+    """``decode_prepare``, ``sample`` (noise by ``step_counter``) and ``decode_advance`` in one launch; ``arrived``: one int32, zero."""
+    if logits.dtype not in (torch.bfloat16, torch.float32):
+        raise TypeError(f"sample_step: logits must be bf16 or fp32, got {logits.dtype}")
+    check(lib().rpeg_sample_step(logits.data_ptr(), logits.shape[0], logits.shape[1], logits.stride(0), int(logits.dtype == torch.float32), temperature,
+                                 int(greedy), seed & 0xFFFFFFFFFFFFFFFF, _ptr(forced_len), sampled.data_ptr(), sampled_lp.data_ptr(),
+                                 token.data_ptr(), pos.data_ptr(), seq_len.data_ptr(), active.data_ptr(), gen_count.data_ptr(), out_tok.data_ptr(),
+                                 out_lp.data_ptr(), out_tok.shape[1], eos, n_finished.data_ptr(), step_counter.data_ptr(), arrived.data_ptr(),
+                                 _stream()), "rpeg_sample_step")
 
 
 def gather_rows(x: torch.Tensor, rows: torch.Tensor) -> torch.Tensor:

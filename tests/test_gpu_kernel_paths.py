@@ -393,3 +393,42 @@ def test_moe_gemm_few_rows(cuda_device, t, e, top, shared, n, k, act):
         rows = r.x_sorted[lo:hi] if i < e else x
         if hi > lo:
             assert _rel(got[lo:hi, :n], f(rows.double() @ w[i].double().T)) < 2 ** -8
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,vocab", [(1, 1003), (5, 8192), (37, 640)])
+@pytest.mark.parametrize("greedy", [True, False])
+def test_sample_step_is_prepare_sample_advance(cuda_device, dtype, rows, vocab, greedy):
+    dev, g = cuda_device, torch.Generator(device=cuda_device).manual_seed(rows)
+    logits = torch.randn(rows, vocab, generator=g, device=dev).to(dtype)
+    eos, max_new = 2, 9
+
+    def state():
+        h = torch.Generator(device=dev).manual_seed(rows)
+        ints = lambda lo, hi: torch.randint(lo, hi, (rows,), generator=h, device=dev, dtype=torch.int32)  # noqa: E731
+        zero = lambda n=rows, t=torch.int32: torch.zeros(n, dtype=t, device=dev)  # noqa: E731
+        return dict(forced_len=ints(0, 6), token=ints(3, 100), pos=ints(5, 50), seq_len=ints(5, 50), active=ints(0, 2), gen_count=ints(1, max_new),
+                    out_tok=zero(rows * max_new).view(rows, max_new), out_lp=zero(rows * max_new, torch.float32).view(rows, max_new), n_finished=zero(1),
+                    step_counter=torch.full((1,), 7, dtype=torch.int64, device=dev))
+
+    a, b = state(), state()
+    forced, sampled, lp = torch.zeros_like(a["token"]), torch.zeros_like(a["token"]), torch.zeros(rows, device=dev)
+    arrived = torch.zeros(1, dtype=torch.int32, device=dev)
+    for _ in range(3):
+        K.decode_prepare(a["active"], a["gen_count"], a["forced_len"], forced, eos)
+        K.sample(logits, 0.7, greedy, 11, forced=forced, token_out=sampled, logp_out=lp, seed_offset=a["step_counter"])
+        K.decode_advance(sampled, lp, a["token"], a["pos"], a["seq_len"], a["active"], a["gen_count"], a["out_tok"], a["out_lp"], eos, a["n_finished"], a["step_counter"])
+        K.sample_step(logits, 0.7, greedy, 11, b["forced_len"], torch.zeros_like(sampled), torch.zeros_like(lp), b["token"], b["pos"], b["seq_len"], b["active"],
+                      b["gen_count"], b["out_tok"], b["out_lp"], eos, b["n_finished"], b["step_counter"], arrived)
+    assert int(arrived) == 0
+    for name in a:
+        assert torch.equal(a[name], b[name]), name
+
+
+@pytest.mark.parametrize("rows,d", [(1, 8), (3, 2056), (5, 8192), (2, 8200)])
+def test_embed_rmsnorm_rows(cuda_device, rows, d):
+    g = torch.Generator(device=cuda_device).manual_seed(d)
+    table, w = (torch.randn(n, d, generator=g, device=cuda_device).bfloat16() for n in (7, 1))
+    ids = torch.randint(0, 7, (rows,), generator=g, device=cuda_device, dtype=torch.int32)
+    y, h = K.embed_rmsnorm_fwd(ids, table, w[0], 1e-5)
+    assert torch.equal(h, table[ids.long()]) and torch.equal(y, K.rmsnorm_fwd(h, w[0], 1e-5)[0])
