@@ -616,10 +616,15 @@ class Generator:
                 saved = (sum(slot_shared[s] for s in live) - sum(first.values())) * PAGE       # shared keys beyond one reading of each
                 heads = b * getattr(self.model, "n_heads_local", getattr(self.cfg, "n_heads", 1))
                 self._aliased = heads >= self.ALIASED_MIN_HEADS and saved >= self.ALIASED_MIN_SAVED * sum(slot_bound[s] for s in live)
-            for _ in range(horizon):
+            # no row is longer than its cap: the last steps of a horizon may have none left to advance (10 new tokens are nine steps, not 16). The noise of
+            # whatever is sampled next is that of the whole horizon all the same.
+            steps = min(horizon, max(slot_prompt[s] + max_new - slot_bound[s] for s in live))
+            for _ in range(steps):
                 self._step(b, temperature, greedy, seed, top_k, top_p)
-            counters["decode_steps"] += horizon
-            counters["graph_replays"] += horizon if self.use_graphs else 0
+            if steps < horizon:
+                self.step_counter += horizon - steps
+            counters["decode_steps"] += steps
+            counters["graph_replays"] += steps if self.use_graphs else 0
             for s in live:
                 slot_bound[s] = min(slot_bound[s] + horizon, slot_prompt[s] + max_new)
             nf = int(self.n_finished.item())
