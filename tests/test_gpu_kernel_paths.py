@@ -432,3 +432,12 @@ def test_embed_rmsnorm_rows(cuda_device, rows, d):
     ids = torch.randint(0, 7, (rows,), generator=g, device=cuda_device, dtype=torch.int32)
     y, h = K.embed_rmsnorm_fwd(ids, table, w[0], 1e-5)
     assert torch.equal(h, table[ids.long()]) and torch.equal(y, K.rmsnorm_fwd(h, w[0], 1e-5)[0])
+
+
+# output heads whose tiles are narrower than 256: one wave of 224, two of 160 where 256 takes three
+@pytest.mark.parametrize("m,n,k", [(1, 32000, 264), (17, 32008, 520), (128, 37000, 136), (3, 70000, 72)])
+def test_gemm_narrow_wave(cuda_device, m, n, k):
+    g = torch.Generator(device=cuda_device).manual_seed(m)
+    a, b = (torch.randn(r, k, generator=g, device=cuda_device).bfloat16() for r in (m, n))
+    ws = torch.empty(1 << 20, device=cuda_device)
+    assert _rel(K.gemm(a, b, workspace=ws), a.double() @ b.double().T) < 2 ** -8
