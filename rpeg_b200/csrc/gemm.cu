@@ -29,7 +29,7 @@ namespace rpeg {
 constexpr int BM = 128;
 constexpr int BK = 64;  // 64 bf16 = one 128-byte swizzle row
 constexpr int GEMM_THREADS = 192;
-constexpr int SMEM_BUDGET = 227 * 1024 - 2048;
+constexpr int SMEM_BUDGET = 196 * 1024 - 2048;         // not all of it: see gemm_skinny.cu on kernels that are chained
 
 // AR: rows of the A tile that exist in shared memory (128 in every instantiation in use). A variant with AR = 32 for
 // decode GEMMs of up to 32 rows (6 stages of 256-wide weight tiles instead of 4) measured 5 % SLOWER per decode step:
@@ -121,10 +121,11 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   const uint32_t tmem_base = *tmem_slot;
   // Launched as a programmatic dependent (decode: B is a weight matrix that no kernel of the step writes): the
   // set-up above already ran under the previous kernel's tail, and the producer streams the first weight tiles
-  // before it waits for that kernel; every other thread waits here, before it can touch A, C or the workspace.
+  // before it waits for that kernel; every other warp waits here, before it can touch A, C or the workspace. (Not the producer's other
+  // lanes: a wait of theirs holds up the whole warp.)
   if (pdl) {
     griddep_launch();
-    if (threadIdx.x != 0) griddep_wait();
+    if (warp != 0) griddep_wait();
   }
 
   // Tile order: groups of 8 M-tiles sweep N together so the A rows stay in L2.
@@ -697,7 +698,7 @@ extern "C" int rpeg_gemm_swiglu(const void* A, const void* W, void* C, int M, in
     configured = true;
   }
   const int grid = tiles < g_num_sms ? tiles : g_num_sms;
-  kern<<<grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream>>>(ta, tb, C, M, f, K, ldc, 0, 1, 0, status, WeightGate{nullptr, 0, 0u, 0ull}, 0, BM);
+  kern<<<grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream>>>(ta, tb, C, M, f, K, ldc, 0, 1, 0, status, WeightGate{nullptr, 0, 0u, 0ull}, 0, BM, 256);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
@@ -728,16 +729,17 @@ extern "C" int rpeg_gemm_bf16_partials(const void* A, const void* B, int M, int 
     *k_splits_out = plan.splits;
     return gemm_pair(A, B, workspace, M, N, K, lda, ldb, N, 0, 0, 1, 0, plan, g_num_sms, pdl_enabled(), status, stream);
   }
-  // From 33 rows on, of matrices that several SMs share, gemm_skinny.cu: K = 4096, us here (tiles of 128 rows x 128 or 256 columns) and there: 33 / 64 / 128 rows
-  // of 2048 6.4 and 5.7 / 7.0 and 6.1 / 8.4 and 6.5; of 12288 20.2 and 18.5 / 22.5 and 19.7 / 26.9 and 23.4; of 22016 35.1 and 32.8 / 38.4 and 32.8 / 44.7 and
-  // 36.9; but of 1024 4.8 and 5.5 / 5.3 and 6.6 / 7.1 and 5.8, and at K = 128 of 4096 3.6 and 4.3.
-  if (M > 32 && N >= 2048 && static_cast<long long>(N) * K >= 2048ll * 1024) {
+  // Of matrices that many SMs share, gemm_skinny.cu: K = 4096, us here (tiles of 128 rows x 128 or 256 columns) and there: 33 / 64 / 128 rows of 2048
+  // 6.4 and 5.7 / 7.0 and 6.1 / 8.4 and 6.5; of 12288 20.2 and 18.5 / 22.5 and 19.7 / 26.9 and 23.4; of 22016 35.1 and 32.8 / 38.4 and 32.8 / 44.7 and 36.9; but
+  // of 1024 4.8 and 5.5 / 5.3 and 6.6 / 7.1 and 5.8, and at K = 128 of 4096 3.6 and 4.3. Fewer rows are level alone, but not in a step, where
+  // there are fewer slabs to add: 4 Llama-7B layers, 1 / 16 / 32 rows 0.408 and 0.405 / 0.462 and 0.453 / 0.532 and 0.503 ms.
+  if (N >= 2048 && static_cast<long long>(N) * K >= 2048ll * 1024) {
     const SkinnyPlan plan = skinny_plan(M, N, K, workspace_elems, g_num_sms);
     *k_splits_out = plan.splits;
     return skinny_partials(A, B, workspace, M, N, K, lda, ldb, plan, status, stream);
   }
-  // Few rows: the wide tile, fewest reads of A. From 33 rows on the slabs weigh as much as that, and the narrow tile needs half as many to fill
-  // the SMs and stores one half while it multiplies the other.
+  // The wide tile, fewest reads of A. From 33 rows on the slabs weigh as much as that, and the narrow tile needs half as many to fill the SMs and
+  // stores one half while it multiplies the other.
   const bool narrow = M > 32;
   const int bn = N >= 256 && !narrow ? 256 : (N >= 128 ? 128 : (N >= 64 ? 64 : 32));
   const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);

@@ -27,9 +27,10 @@ constexpr int PG_STAGING = 4 * 2 * 4096;
 
 constexpr int PG_A_BYTES = PG_BM * PG_BK * 2;
 constexpr int PG_STAGE_BYTES = PG_A_BYTES + 128 * PG_BK * 2;     // up to 128 columns of B per CTA
-constexpr int PG_STAGES = 6;
-constexpr int PG_SMEM = 1024 + PG_STAGES * PG_STAGE_BYTES + PG_STAGING + 512;
-static_assert(PG_SMEM <= 227 * 1024, "shared memory");
+// Stages: six, or five for the partial sums of a decode step (see gemm_skinny.cu on the shared memory of chained kernels).
+constexpr int pair_stages(int epi) { return epi == 1 ? 5 : 6; }
+constexpr int pair_smem(int epi) { return 1024 + pair_stages(epi) * PG_STAGE_BYTES + PG_STAGING + 512; }
+static_assert(pair_smem(0) <= 227 * 1024 && pair_smem(1) <= 196 * 1024, "shared memory");
 
 // Work of a launch: tiles of 256 rows x `bn` accumulator columns, each cut into `splits` pieces of `kb_per` K blocks (splits > 1: every piece
 // stores its own sums, `PG_F32` only).
@@ -43,7 +44,7 @@ template <int EPI, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(PG_THREADS, 1) __cluster_dims__(2, 1, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                  const __grid_constant__ CUtensorMap tmap_c, const PairWork pw, int* status) {
-  constexpr int STAGES = PG_STAGES;
+  constexpr int STAGES = pair_stages(EPI);
   const int M = pw.M, N = pw.N, BN = pw.bn;
   const int TN = EPI == PG_SWIGLU ? BN / 2 : BN;           // output columns per tile
   extern __shared__ uint8_t smem_raw[];
@@ -276,7 +277,7 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
   auto kern = gemm_pair_kernel<EPI, A_MN, B_MN>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PG_SMEM) != cudaSuccess) return -20;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_smem(EPI)) != cudaSuccess) return -20;
     configured = true;
   }
   const int tn = EPI == PG_SWIGLU ? pw.bn / 2 : pw.bn;
@@ -285,7 +286,7 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs);
   cfg.blockDim = dim3(PG_THREADS);
-  cfg.dynamicSmemBytes = PG_SMEM;
+  cfg.dynamicSmemBytes = pair_smem(EPI);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -33,7 +33,11 @@ template <int NT, int MODE>
 struct SkinnyCfg {
   static constexpr int STAGE_BYTES = SK_W_BYTES + NT * SK_BK * 2;
   static constexpr int LIST_BYTES = MODE == SK_EXPERTS ? (SK_MAX_SEGMENTS * 3 + 4) * 4 : 0;
-  static constexpr int RAW = (227 * 1024 - 1024 - 512 - LIST_BYTES) / STAGE_BYTES;
+  // Dense products run in chains of programmatic dependents, whose small kernels share an SM with the next product's waiting CTA: what it leaves of
+  // shared memory counts for more than its deepest stages. The line is 196 KB, the last way but one to part an SM's memory between the two kinds of
+  // kernels (Llama-7B shapes, 4 layers, a step of 64 rows with 222 KB 0.670 ms, 194 KB 0.622, 130 KB 0.634; of 16 rows with 200 KB 0.479, 182 KB 0.453).
+  static constexpr int BUDGET = (MODE == SK_PARTS || NT == 16 ? 196 : 227) * 1024;
+  static constexpr int RAW = (BUDGET - 1024 - 512 - LIST_BYTES) / STAGE_BYTES;
   static constexpr int STAGES = RAW > 12 ? 12 : RAW;
   static constexpr int BUFS = NT <= 64 ? 4 : 2;                      // accumulators of NT columns
   static constexpr int TMEM_COLS = BUFS * NT;
@@ -109,7 +113,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   if constexpr (MODE == SK_PARTS) {
-    if (threadIdx.x != 0) griddep_wait();     // the producer waits behind its first weights
+    if (warp != 0) griddep_wait();            // the producer waits behind its first weights; a wait of its other lanes would hold it up
   }
 
   const int num_kb = (p.K + SK_BK - 1) / SK_BK, tiles = (p.N + TF - 1) / TF;
@@ -325,7 +329,7 @@ SkinnyPlan skinny_plan(int M, int N, int K, long long slab_elems, int num_sms) {
 }
 
 int skinny_partials(const void* X, const void* W, float* parts, int M, int N, int K, int ldx, int ldw, SkinnyPlan plan, int* status, cudaStream_t stream) {
-  const int nt = M <= 64 ? 64 : 128;
+  const int nt = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
   CUtensorMap tw, tx;
   int rc = make_tmap_bf16_2d(&tx, X, K, M, ldx, SK_BK, nt);
   if (rc) return rc;
@@ -333,7 +337,12 @@ int skinny_partials(const void* X, const void* W, float* parts, int M, int N, in
   if (rc) return rc - 100;
   Skinny p{};
   p.M = M; p.N = N; p.K = K; p.splits = plan.splits; p.parts = parts; p.status = status;
-  return nt == 64 ? launch_skinny<64, SK_PARTS, FF_NONE>(tw, tx, tx, p, plan.grid, stream) : launch_skinny<128, SK_PARTS, FF_NONE>(tw, tx, tx, p, plan.grid, stream);
+  switch (nt) {
+    case 16: return launch_skinny<16, SK_PARTS, FF_NONE>(tw, tx, tx, p, plan.grid, stream);
+    case 32: return launch_skinny<32, SK_PARTS, FF_NONE>(tw, tx, tx, p, plan.grid, stream);
+    case 64: return launch_skinny<64, SK_PARTS, FF_NONE>(tw, tx, tx, p, plan.grid, stream);
+    default: return launch_skinny<128, SK_PARTS, FF_NONE>(tw, tx, tx, p, plan.grid, stream);
+  }
 }
 
 template <int NT>
