@@ -90,14 +90,19 @@ rope_kv_append_kernel(__nv_bfloat16* __restrict__ qkv, int ld, int q_col0, int k
 }
 
 // The same job list as rope_kv_append_kernel, but the qkv row is the sum of split-K partials
-// (fp32 [splits][T][ld]): the head slice is summed, rounded to bf16, rotated (q, k) and stored: q into
-// the bf16 qkv buffer the attention kernel reads, k and v into the paged cache.
+// (fp32 [splits][T][ld]): the head slice is summed, rounded to bf16, normalised (NORM: RMSNorm over the head with one
+// weight vector for all query heads and one for all key heads), rotated (q, k) and stored: q into the bf16 qkv buffer the
+// attention kernel reads, k and v into the paged cache. NORM replaces a reduction, two norms and a rotation of their own
+// (Qwen3-8B, 4
+// layers, a step of 128 rows, with the other products' partial sums added up by their readers too: 0.98 -> 0.80 ms).
+template <bool NORM>
 __global__ void __launch_bounds__(256)
 rope_kv_append_partials_kernel(const float* __restrict__ parts, int splits, long long stride, __nv_bfloat16* __restrict__ qkv,
                                int ld, int q_col0, int k_col0, int v_col0, const int* __restrict__ seq_id,
                                const int* __restrict__ pos, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                const int* __restrict__ page_table, int max_pages, __nv_bfloat16* __restrict__ kcache,
-                               __nv_bfloat16* __restrict__ vcache, int T, int H, int Hkv) {
+                               __nv_bfloat16* __restrict__ vcache, int T, int H, int Hkv, const __nv_bfloat16* __restrict__ q_norm,
+                               const __nv_bfloat16* __restrict__ k_norm, float eps) {
   griddep_launch();
   griddep_wait();   // may have been scheduled under the previous kernel's tail: nothing is read or written before this
   const int jobs = H + 2 * Hkv;
@@ -125,7 +130,14 @@ rope_kv_append_partials_kernel(const float* __restrict__ parts, int splits, long
   }
   uint32_t lo = pack_bf16x2(lo0, lo1), hi = pack_bf16x2(hi0, hi1);
   if (job < H + Hkv) {
-    const float2 a = unpack_bf16x2(lo), b = unpack_bf16x2(hi);
+    float2 a = unpack_bf16x2(lo), b = unpack_bf16x2(hi);
+    if constexpr (NORM) {                    // rounded where headnorm_fwd_kernel rounds
+      const __nv_bfloat16* w = job < H ? q_norm : k_norm;
+      const float rstd = rsqrtf(warp_sum(a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y) * (1.f / HD) + eps);
+      const float2 wa = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(w + i)), wb = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(w + i + half));
+      a = unpack_bf16x2(pack_bf16x2(a.x * rstd * wa.x, a.y * rstd * wa.y));
+      b = unpack_bf16x2(pack_bf16x2(b.x * rstd * wb.x, b.y * rstd * wb.y));
+    }
     const float2 c = *reinterpret_cast<const float2*>(cos_t + static_cast<size_t>(p) * half + i);
     const float2 sn = *reinterpret_cast<const float2*>(sin_t + static_cast<size_t>(p) * half + i);
     lo = pack_bf16x2(a.x * c.x - b.x * sn.x, a.y * c.y - b.y * sn.y);
@@ -875,14 +887,18 @@ extern "C" int rpeg_rope_kv_append(void* qkv, int ld, int q_col0, int k_col0, in
 extern "C" int rpeg_rope_kv_append_partials(const float* parts, int splits, long long stride, void* qkv, int ld, int q_col0,
                                             int k_col0, int v_col0, const int* seq_id, const int* pos, const float* cos_t,
                                             const float* sin_t, const int* page_table, int max_pages, void* kcache,
-                                            void* vcache, int T, int H, int Hkv, int hd, void* stream) {
+                                            void* vcache, int T, int H, int Hkv, int hd, const void* q_norm, const void* k_norm,
+                                            float eps, void* stream) {
   if (hd != HD || splits < 1) return -2;
   if ((ld | q_col0 | k_col0 | v_col0) & 7) return -3;
+  if ((q_norm == nullptr) != (k_norm == nullptr)) return -4;
   const long long threads = static_cast<long long>(T) * (H + 2 * Hkv) * 32;
   if (threads <= 0) return 0;
-  launch_pdl(rope_kv_append_partials_kernel, dim3(static_cast<unsigned>((threads + 255) / 256)), dim3(256), 0, STREAM(stream), 
+  auto kern = q_norm != nullptr ? rope_kv_append_partials_kernel<true> : rope_kv_append_partials_kernel<false>;
+  launch_pdl(kern, dim3(static_cast<unsigned>((threads + 255) / 256)), dim3(256), 0, STREAM(stream),
       parts, splits, stride, static_cast<__nv_bfloat16*>(qkv), ld, q_col0, k_col0, v_col0, seq_id, pos, cos_t, sin_t, page_table,
-      max_pages, static_cast<__nv_bfloat16*>(kcache), static_cast<__nv_bfloat16*>(vcache), T, H, Hkv);
+      max_pages, static_cast<__nv_bfloat16*>(kcache), static_cast<__nv_bfloat16*>(vcache), T, H, Hkv,
+      static_cast<const __nv_bfloat16*>(q_norm), static_cast<const __nv_bfloat16*>(k_norm), eps);
   return LAUNCH_OK();
 }
 

@@ -40,7 +40,7 @@ int rpeg_swiglu_fwd_partials(const float* parts, int splits, long long stride, v
 int rpeg_rope_kv_append_partials(const float* parts, int splits, long long stride, void* qkv, int ld, int q_col0, int k_col0,
                                  int v_col0, const int* seq_id, const int* pos, const float* cos_t, const float* sin_t,
                                  const int* page_table, int max_pages, void* kcache, void* vcache, int T, int H, int Hkv,
-                                 int hd, void* stream);
+                                 int hd, const void* q_norm, const void* k_norm, float eps, void* stream);
 int rpeg_rope(void* buf, const int* pos, const float* cos_t, const float* sin_t, int T, int ld, int col0,
               int nheads, int hd, int backward, void* stream);
 int rpeg_swiglu_fwd(const void* gu, void* out, long long T, int f, void* stream);

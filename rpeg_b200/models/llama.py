@@ -460,8 +460,6 @@ class LlamaModel:
         cfg, p = self.cfg, self.p
         ws = self._workspace()
         scale = 1.0 / math.sqrt(cfg.head_dim)
-        if cfg.qk_norm:
-            return self._decode_step_unfused(token, pos, slot_ids, seq_len, page_table, kcache, vcache, nsplit, groups)
         # Every GEMM leaves its split-K partials in the workspace and the next kernel adds them up while it
         # loads them (one stream, so a consumer always runs before the next GEMM reuses the workspace).
         B = token.shape[0]
@@ -470,7 +468,8 @@ class LlamaModel:
         for i in range(cfg.n_layers):
             parts = K.gemm_partials(x, p[f"l{i}.wqkv"], ws)
             K.rope_kv_append_partials_(parts, qkv, 0, cfg.q_width, cfg.q_width + cfg.kv_width, slot_ids, pos, self.cos_t,
-                                       self.sin_t, page_table, kcache[i], vcache[i], cfg.n_heads, cfg.n_kv_heads, cfg.head_dim)
+                                       self.sin_t, page_table, kcache[i], vcache[i], cfg.n_heads, cfg.n_kv_heads, cfg.head_dim,
+                                       p.get(f"l{i}.q_norm"), p.get(f"l{i}.k_norm"), cfg.rms_eps)
             attn = K.paged_decode_attn(qkv, 0, kcache[i], vcache[i], page_table, seq_len, cfg.n_heads, cfg.n_kv_heads,
                                        cfg.head_dim, scale, nsplit=nsplit, groups=groups)
             parts = K.gemm_partials(attn, p[f"l{i}.wo"], ws)
@@ -482,33 +481,6 @@ class LlamaModel:
             x, h = K.rmsnorm_fwd_partials(parts, p["final_norm"] if last else p[f"l{i + 1}.attn_norm"], cfg.rms_eps, residual=h1,
                                           want_sum=not last)
         return x
-
-    def _decode_step_unfused(self, token, pos, slot_ids, seq_len, page_table, kcache, vcache, nsplit: int = 1, groups=None) -> torch.Tensor:
-        """The same step with reduced GEMM outputs (needed when q and k are normalised per head before RoPE)."""
-        cfg, p = self.cfg, self.p
-        ws = self._workspace()
-        scale = 1.0 / math.sqrt(cfg.head_dim)
-        res = delta = None
-        for i in range(cfg.n_layers):
-            if delta is None:
-                x, h = K.embed_rmsnorm_fwd(token, p["embed"], p[f"l{i}.attn_norm"], cfg.rms_eps)
-            else:
-                x, _, h = K.rmsnorm_fwd(delta, p[f"l{i}.attn_norm"], cfg.rms_eps, residual=res, want_sum=True)
-            qkv = K.gemm(x, p[f"l{i}.wqkv"], workspace=ws)
-            if cfg.qk_norm:
-                self._qk_norm(i, qkv, False)
-            K.rope_kv_append_(qkv, 0, cfg.q_width, cfg.q_width + cfg.kv_width, slot_ids, pos, self.cos_t, self.sin_t,
-                              page_table, kcache[i], vcache[i], cfg.n_heads, cfg.n_kv_heads, cfg.head_dim)
-            attn = K.paged_decode_attn(qkv, 0, kcache[i], vcache[i], page_table, seq_len, cfg.n_heads, cfg.n_kv_heads,
-                                       cfg.head_dim, scale, nsplit=nsplit, groups=groups)
-            o = K.gemm(attn, p[f"l{i}.wo"], workspace=ws)
-            x2, _, h1 = K.rmsnorm_fwd(o, p[f"l{i}.mlp_norm"], cfg.rms_eps, residual=h, want_sum=True)
-            gu = K.gemm(x2, p[f"l{i}.w_gate_up"], workspace=ws)
-            act = K.swiglu_fwd(gu)
-            delta = K.gemm(act, p[f"l{i}.w_down"], workspace=ws)
-            res = h1
-        xf, _, _ = K.rmsnorm_fwd(delta, p["final_norm"], cfg.rms_eps, residual=res)
-        return xf
 
     def lm_logits(self, xf: torch.Tensor, decode: bool = False) -> torch.Tensor:
         return K.gemm(xf, self.p["lm_head"], workspace=self._workspace() if decode else None)

@@ -53,7 +53,7 @@ _SIGNATURES = {
     "rpeg_gemm_bf16_partials": [P, P, I, I, I, I, I, P, c_longlong, P, P, P],
     "rpeg_rmsnorm_fwd_partials": [P, I, c_longlong, P, P, P, P, I, I, F, P],
     "rpeg_swiglu_fwd_partials": [P, I, c_longlong, P, c_longlong, I, P],
-    "rpeg_rope_kv_append_partials": [P, I, c_longlong, P, I, I, I, I, P, P, P, P, P, I, P, P, I, I, I, I, P],
+    "rpeg_rope_kv_append_partials": [P, I, c_longlong, P, I, I, I, I, P, P, P, P, P, I, P, P, I, I, I, I, P, P, F, P],
     "rpeg_headnorm_fwd": [P, I, I, I, I, P, P, I, F, P],
     "rpeg_headnorm_bwd": [P, I, P, I, I, I, I, P, P, P, I, P],
     "rpeg_ag_gemm": [P, P, P, P, I, I, I, I, I, I, I, I, c_uint, P, P],

@@ -493,15 +493,17 @@ def swiglu_fwd_partials(parts: Partials) -> torch.Tensor:
 
 
 def rope_kv_append_partials_(parts: Partials, qkv: torch.Tensor, q_col0, k_col0, v_col0, seq_id, pos, cos_t, sin_t, page_table,
-                             kcache, vcache, n_heads, n_kv_heads, head_dim) -> None:
-    """Sum the partials of a QKV projection, rotate q and k, store q into ``qkv`` (bf16, the attention
-    kernel's query input) and k, v into the paged cache."""
+                             kcache, vcache, n_heads, n_kv_heads, head_dim, q_norm=None, k_norm=None, eps=0.0) -> None:
+    """Sum the partials of a QKV projection, normalise q and k per head where ``q_norm`` and ``k_norm`` (bf16
+    ``[head_dim]``) are given, rotate them, store q into ``qkv`` (bf16, the attention kernel's query input) and
+    k, v into the paged cache."""
     if _chk.active():
         _chk.kv_append("rpeg_rope_kv_append_partials", parts.M, seq_id, pos, page_table, kcache, n_kv_heads, head_dim, cos_t)
     check(lib().rpeg_rope_kv_append_partials(parts.buf.data_ptr(), parts.splits, parts.stride, qkv.data_ptr(), qkv.stride(0), q_col0,
                                              k_col0, v_col0, seq_id.data_ptr(), pos.data_ptr(), cos_t.data_ptr(), sin_t.data_ptr(),
                                              page_table.data_ptr(), page_table.stride(0), kcache.data_ptr(), vcache.data_ptr(),
-                                             parts.M, n_heads, n_kv_heads, head_dim, _stream()), "rpeg_rope_kv_append_partials")
+                                             parts.M, n_heads, n_kv_heads, head_dim, _ptr(q_norm), _ptr(k_norm), eps, _stream()),
+          "rpeg_rope_kv_append_partials")
 
 
 def scatter_rows_by_index(src: torch.Tensor, global_idx: torch.Tensor, rows_per_rank: int, dst_ptr_array, world: int) -> None:

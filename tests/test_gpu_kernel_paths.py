@@ -441,3 +441,33 @@ def test_gemm_narrow_wave(cuda_device, m, n, k):
     a, b = (torch.randn(r, k, generator=g, device=cuda_device).bfloat16() for r in (m, n))
     ws = torch.empty(1 << 20, device=cuda_device)
     assert _rel(K.gemm(a, b, workspace=ws), a.double() @ b.double().T) < 2 ** -8
+
+
+@pytest.mark.parametrize("rows,splits,h,hkv", [(1, 1, 4, 4), (3, 2, 8, 2), (17, 5, 5, 1)])
+def test_rope_append_partials_normalises_heads(cuda_device, rows, splits, h, hkv):
+    """Sum, per-head RMSNorm, rotation and append in one kernel against the kernels for each. The slabs are multiples of 1/64: their sums are exact."""
+    dev, hd, n = cuda_device, 128, (h + 2 * hkv) * 128
+    g = torch.Generator(device=dev).manual_seed(rows)
+    slabs = torch.randint(-64, 65, (splits, rows, n), generator=g, device=dev).float() / 64
+    parts = K.Partials(slabs.flatten(), splits, rows, n)
+    wq, wk = (torch.randn(hd, generator=g, device=dev).bfloat16() for _ in range(2))
+    pos = torch.randint(0, 190, (rows,), generator=g, device=dev, dtype=torch.int32)
+    seq = torch.arange(rows, device=dev, dtype=torch.int32)
+    table = torch.arange(rows * 3, device=dev, dtype=torch.int32).view(rows, 3)
+    cos_t, sin_t = K.rope_tables(256, hd, 10000.0, dev)
+    out = []
+    for fused in (False, True):
+        kc, vc = (torch.zeros(rows * 3, hkv, K.KV_PAGE, hd, device=dev, dtype=torch.bfloat16) for _ in range(2))
+        if fused:
+            q = torch.zeros(rows, n, device=dev, dtype=torch.bfloat16)
+            K.rope_kv_append_partials_(parts, q, 0, h * hd, (h + hkv) * hd, seq, pos, cos_t, sin_t, table, kc, vc, h, hkv, hd, wq, wk, 1e-6)
+        else:
+            q = slabs.sum(0).bfloat16()
+            K.headnorm_fwd_(q, 0, h, hd, wq, 1e-6, want_rstd=False)
+            K.headnorm_fwd_(q, h * hd, hkv, hd, wk, 1e-6, want_rstd=False)
+            K.rope_kv_append_(q, 0, h * hd, (h + hkv) * hd, seq, pos, cos_t, sin_t, table, kc, vc, h, hkv, hd)
+        out.append((q[:, :h * hd], kc, vc))
+    (q0, k0, v0), (q1, k1, v1) = out
+    # the two sum a head's squares in unlike orders: where that flips a rounding to bf16 (twice on the way), a value moves by 2^-8 of itself each time
+    assert _rel(q1, q0) < 2 ** -7 and _rel(k1, k0) < 2 ** -7
+    assert torch.equal(v0, v1)
