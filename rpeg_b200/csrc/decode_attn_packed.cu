@@ -6,14 +6,15 @@
 //     S^T [16 keys x 8] = K [16 x 128] Q^T,      O^T [128 x 8] += V^T [128 x 16] P^T,
 // on fragments that are loaded straight from the pages: a lane's 16-byte chunks of K are two k steps each (the order of the head dimensions inside
 // a step is free, Q has the same), V's keys 2t, 2t + 1, 2t + 8, 2t + 9 are paired by byte permutes, P^T turns by movmatrix. Every warp keeps its own
-// softmax state for the eight columns; the four are merged at the end, splits by the last one to arrive.
+// softmax state for the eight columns; the four are merged at the end. The splits of
+// an item are a cluster and are merged through each other's shared memory: no scratch, and no counters that launches on two streams would share.
 //
 // P stays fp32: it enters the product as three bf16 parts (8 + 8 + 8 bits, exact). Columns a block is not for are neither scored nor added to, so
 // what one row holds (infinities, NaN) never reaches another.
 //
 // Bound by the bytes of the pages; the row kernel (decode_attn.cu) reads the shared ones once per row, from L2.
 #include <cmath>
-#include "common.cuh"
+#include "pair.cuh"
 #include "rpeg_kernels.h"
 
 namespace rpeg {
@@ -21,12 +22,18 @@ namespace rpeg {
 constexpr int DP_PAGE = RPEG_KV_PAGE, DP_HD = 128, DP_COLS = 8, DP_WARPS = 4, DP_THREADS = DP_WARPS * 32;
 constexpr int DP_WINDOW = 32;                                // logical pages listed at a time
 constexpr int DP_LIST = DP_WINDOW * DP_COLS * (DP_PAGE / 16);
-constexpr int DP_ITEMS = 1 << 16;
 static_assert(DP_PAGE == 64, "a page is four blocks");
 
-// Arrival counters of the splits of an item, zero between launches; launches of one GPU that split run in stream order.
-__device__ int g_packed_arrive[DP_ITEMS];
-
+__device__ __forceinline__ float4 cluster_load4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 cluster_load2(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -49,12 +56,13 @@ template <int G>
 __global__ void __launch_bounds__(DP_THREADS, 3)
 paged_decode_attn_packed_kernel(const __nv_bfloat16* __restrict__ q, int ldq, int q_col0, const __nv_bfloat16* __restrict__ kcache,
                                 const __nv_bfloat16* __restrict__ vcache, const int* __restrict__ page_table, int max_pages,
-                                const int* __restrict__ seq_lens, __nv_bfloat16* __restrict__ out, float* __restrict__ partial, int B, int H,
-                                int Hkv, int nsplit, float scale_log2) {
+                                const int* __restrict__ seq_lens, __nv_bfloat16* __restrict__ out, int B, int H, int Hkv, int nsplit,
+                                float scale_log2) {
   griddep_launch();
   griddep_wait();   // may have been scheduled under the previous kernel's tail: nothing is read or written before this
   __shared__ int2 list[DP_LIST];                             // first cache row of a block; its first key | columns << 24 | keys - 1
-  __shared__ int lens_s[DP_COLS], warp_total[DP_WARPS], is_last;
+  __shared__ int lens_s[DP_COLS], warp_total[DP_WARPS];
+  __shared__ __align__(8) float2 sum_ml[DP_COLS];             // this split's maxima and sums
   __shared__ float red_m[DP_WARPS][DP_COLS], red_l[DP_WARPS][DP_COLS];
   __shared__ __align__(16) float red_o[DP_WARPS][DP_COLS][DP_HD];
   constexpr int rows = DP_COLS / G;
@@ -281,66 +289,67 @@ paged_decode_attn_packed_kernel(const __nv_bfloat16* __restrict__ q, int ldq, in
     if (row < B) store(o, gl);
     return;
   }
-  // partial sums [B H nsplit][128], then (maximum, sum) [B H nsplit][2]
-  const size_t slot0 = (static_cast<size_t>(row) * H + hk * G + col % G) * nsplit;
-  float* ml = partial + static_cast<size_t>(B) * H * nsplit * DP_HD;
-  if (row < B) {
-    float* pp = partial + (slot0 + split) * DP_HD + d0;
-    *reinterpret_cast<float4*>(pp) = make_float4(o[0], o[1], o[2], o[3]);
-    *reinterpret_cast<float4*>(pp + 4) = make_float4(o[4], o[5], o[6], o[7]);
-    if (d0 == 0) *reinterpret_cast<float2*>(ml + (slot0 + split) * 2) = make_float2(gm, gl);
-  }
-  int* arrive = &g_packed_arrive[blockIdx.y * Hkv + hk];
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) is_last = atomicAdd(arrive, 1) == nsplit - 1 ? 1 : 0;
-  __syncthreads();
-  if (!is_last) return;
-  if (tid == 0) *arrive = 0;
-  __threadfence();
-  if (row >= B) return;
-  gm = -INFINITY;
-  gl = 0.f;
+  // every (column, eight dimensions) was read by the thread that now rewrites it; the splits share the merge out among themselves
+  float* own = &red_o[0][col][d0];
+  *reinterpret_cast<float4*>(own) = make_float4(o[0], o[1], o[2], o[3]);
+  *reinterpret_cast<float4*>(own + 4) = make_float4(o[4], o[5], o[6], o[7]);
+  if (d0 == 0) sum_ml[col] = make_float2(gm, gl);
+  __syncwarp();
+  cluster_sync_all();
+  if (tid % nsplit == split && row < B) {
+    gm = -INFINITY;
+    gl = 0.f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) o[i] = 0.f;
+    for (int i = 0; i < 8; ++i) o[i] = 0.f;
 #pragma unroll 4
-  for (int s = 0; s < nsplit; ++s) {
-    const float2 x = __ldcg(reinterpret_cast<const float2*>(ml + (slot0 + s) * 2));
-    const float4 u = __ldcg(reinterpret_cast<const float4*>(partial + (slot0 + s) * DP_HD + d0));
-    const float4 v = __ldcg(reinterpret_cast<const float4*>(partial + (slot0 + s) * DP_HD + d0 + 4));
-    if (x.x == -INFINITY) continue;
-    const float nm = fmaxf(gm, x.x), f0 = exp2f(gm - nm), f = exp2f(x.x - nm);
-    const float e[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
-    gm = nm;
-    gl = gl * f0 + x.y * f;
+    for (int s = 0; s < nsplit; ++s) {
+      const float2 x = cluster_load2(cluster_addr(&sum_ml[col], s));
+      const float4 u = cluster_load4(cluster_addr(own, s)), v = cluster_load4(cluster_addr(own + 4, s));
+      if (x.x == -INFINITY) continue;
+      const float nm = fmaxf(gm, x.x), f0 = exp2f(gm - nm), f = exp2f(x.x - nm);
+      const float e[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+      gm = nm;
+      gl = gl * f0 + x.y * f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) o[i] = o[i] * f0 + e[i] * f;
+      for (int i = 0; i < 8; ++i) o[i] = o[i] * f0 + e[i] * f;
+    }
+    store(o, gl);
   }
-  store(o, gl);
+  __syncwarp();
+  cluster_sync_all();                                        // nobody's shared memory goes while another reads it
 }
 
 }  // namespace rpeg
 
 using namespace rpeg;
 
-// rpeg_paged_decode_attn for rows that may alias pages; scratch as there. H / Hkv must divide 8.
+// rpeg_paged_decode_attn for rows that may alias pages, without scratch. H / Hkv must divide 8; at most eight splits.
 extern "C" int rpeg_paged_decode_attn_packed(const void* q, int ldq, int q_col0, const void* kcache, const void* vcache, const int* page_table,
-                                             int max_pages, const int* seq_lens, void* out, float* scratch, int B, int H, int Hkv, int hd, int nsplit,
-                                             float scale, void* stream) {
+                                             int max_pages, const int* seq_lens, void* out, int B, int H, int Hkv, int hd, int nsplit, float scale,
+                                             void* stream) {
   if (hd != DP_HD || Hkv <= 0 || H % Hkv != 0 || H / Hkv > DP_COLS || DP_COLS % (H / Hkv) != 0) return -2;
-  if (nsplit < 1 || nsplit > 64) return -3;
-  if (nsplit > 1 && scratch == nullptr) return -4;
+  if (nsplit < 1 || nsplit > 8) return -3;
   if ((ldq | q_col0) & 7) return -5;
-  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache) | reinterpret_cast<uintptr_t>(out) |
-       reinterpret_cast<uintptr_t>(scratch)) & 15) return -1;
+  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache) | reinterpret_cast<uintptr_t>(out)) &
+      15) return -1;
   if (max_pages < 1 || max_pages > (1 << 24) / DP_PAGE) return -6;         // a block's first key has 24 bits
   if (B <= 0) return 0;
   const int rows = DP_COLS / (H / Hkv), items = (B + rows - 1) / rows;
-  if (items > 65535 || (nsplit > 1 && static_cast<long long>(items) * Hkv > DP_ITEMS)) return -7;
+  if (items > 65535) return -7;
   auto kern = H == Hkv ? paged_decode_attn_packed_kernel<1>
               : H == 2 * Hkv ? paged_decode_attn_packed_kernel<2> : H == 4 * Hkv ? paged_decode_attn_packed_kernel<4> : paged_decode_attn_packed_kernel<8>;
-  return launch_pdl(kern, dim3(Hkv, items, nsplit), dim3(DP_THREADS), 0, reinterpret_cast<cudaStream_t>(stream),
-                    static_cast<const __nv_bfloat16*>(q), ldq, q_col0, static_cast<const __nv_bfloat16*>(kcache),
-                    static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages, seq_lens, static_cast<__nv_bfloat16*>(out), scratch, B, H, Hkv,
-                    nsplit, scale * 1.4426950408889634f) == cudaSuccess ? 0 : -21;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim = {1, 1, static_cast<unsigned>(nsplit)};
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(Hkv, items, nsplit);
+  cfg.blockDim = dim3(DP_THREADS);
+  cfg.stream = reinterpret_cast<cudaStream_t>(stream);
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<const __nv_bfloat16*>(q), ldq, q_col0, static_cast<const __nv_bfloat16*>(kcache),
+                            static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages, seq_lens, static_cast<__nv_bfloat16*>(out), B, H, Hkv,
+                            nsplit, scale * 1.4426950408889634f) == cudaSuccess ? 0 : -21;
 }

@@ -548,10 +548,18 @@ ALIASED = "aliased"
 
 
 def packed_decode_splits(B: int, n_heads: int, n_kv_heads: int, pages: int) -> int:
-    """Splits of the kernel for aliased rows: three CTAs an SM, twice as many where rows may be long (their last wave weighs more: 64 rows of
-    1000 to 2000 keys 311 us whole, 245 in three; 256 rows of 512 + 30 keys 79 whole, 92 in two)."""
+    """Splits of the kernel for aliased rows: three CTAs an SM, twice as many where rows of one query head a KV head may be long (their last wave
+    weighs more: 64 rows of 1000 to 2000 keys 311 us whole, 245 in three; 256 rows of 512 + 30 keys 79 whole, 92 in two; 48 rows of 400 to 1000
+    keys, 32 heads, 8 KV heads 31.0 in two, 36.2 in four)."""
     ctas = -(-B // (8 * n_kv_heads // n_heads)) * n_kv_heads
-    return max(1, min(8, 444 // ctas, pages // 2)) if pages < 24 else max(2, min(8, 888 // ctas))
+    return max(1, min(8, 444 // ctas, pages // 2)) if pages < 24 or n_heads > n_kv_heads else max(2, min(8, 888 // ctas))
+
+
+#: From this many (row, head) pairs on, the kernel for aliased rows is the faster one for four or eight query heads a KV head, pages shared or not: it
+#: scores their eight columns on the tensor cores (us, 32 heads, 8 KV heads, keys up to 64 / 200 / 500, row by row and so: 32 rows 5.4 / 10.2 / 19.9 and
+#: 6.6 / 11.3 / 15.5; 48 rows 8.1 / 15.2 / 28.6 and 7.3 / 12.1 / 19.1; 128 rows 17.3 / 32.3 / 64.0 and 13.1 / 24.2 / 46.5; 16 heads, 8 KV heads, 192
+#: rows 14.1 / 27.5 and 11.8 / 25.0, 128 rows 10.3 / 19.5 / 39.9 and 11.2 / 22.2 / 44.9).
+PACKED_MIN_HEADS = 1536
 
 
 _GROUP_TC = False
@@ -571,24 +579,21 @@ def paged_decode_attn(q, q_col0, kcache, vcache, page_table, seq_lens, n_heads, 
     KV pages in groups (K samples of one prompt); the shared keys are then read once per group (``scratch`` must
     hold ``nsplit + 1`` partials per row and head). ``group_tc``: score the groups on the tensor cores (tcgen05, keys on
     the M axis) instead of the CUDA-core kernel. ``groups = ALIASED``: any rows may share pages, what eight neighbours share is
-    read once (the splits are then chosen here)."""
+    read once (the splits are then chosen here, without scratch)."""
     B = q.shape[0]
     if _chk.active():
         _chk.paged_attention("rpeg_paged_decode_attn", B, seq_lens, page_table, kcache, n_kv_heads, head_dim)
     out = torch.empty((B, n_heads * head_dim), dtype=torch.bfloat16, device=q.device) if out is None else out
+    if groups is None and nsplit == 1 and n_heads >= 4 * n_kv_heads and B * n_heads >= PACKED_MIN_HEADS:
+        groups = ALIASED
     if groups is ALIASED:
         groups = None
-        if 8 % (n_heads // n_kv_heads) == 0 and (q.stride(0) | q_col0) % 8 == 0 and B <= 8192:
+        aligned = (q.data_ptr() | kcache.data_ptr() | vcache.data_ptr() | out.data_ptr()) % 16 == 0 and (q.stride(0) | q_col0) % 8 == 0
+        if 8 % (n_heads // n_kv_heads) == 0 and aligned and B <= 8192 and page_table.shape[1] <= 1 << 18:
             nsplit = packed_decode_splits(B, n_heads, n_kv_heads, page_table.shape[1])
-            if scratch is not None:
-                while nsplit > 1 and decode_scratch_numel(B, n_heads, nsplit) > scratch.numel():
-                    nsplit -= 1
-            elif nsplit > 1:
-                scratch = torch.empty(decode_scratch_numel(B, n_heads, nsplit), dtype=torch.float32, device=q.device)
             check(lib().rpeg_paged_decode_attn_packed(q.data_ptr(), q.stride(0), q_col0, kcache.data_ptr(), vcache.data_ptr(),
-                                                      page_table.data_ptr(), page_table.stride(0), seq_lens.data_ptr(), out.data_ptr(),
-                                                      _ptr(scratch) if nsplit > 1 else None, B, n_heads, n_kv_heads, head_dim, nsplit, scale,
-                                                      _stream()), "rpeg_paged_decode_attn_packed")
+                                                      page_table.data_ptr(), page_table.stride(0), seq_lens.data_ptr(), out.data_ptr(), B, n_heads,
+                                                      n_kv_heads, head_dim, nsplit, scale, _stream()), "rpeg_paged_decode_attn_packed")
             return out
     if groups is not None:
         group_rows, group_shared, row_key0 = groups

@@ -318,9 +318,10 @@ def test_sample_rows(cuda_device, dtype, rows, vocab, shift):
 
 # 11 rows: groups that share one, two or 33 pages (a second listing of 32), a row of its own, an empty one; eight columns of 8, 4, 2 and 1 rows
 @pytest.mark.parametrize("h,hkv", [(3, 3), (4, 2), (8, 2), (8, 1)])
-@pytest.mark.parametrize("split", [True, False])
-def test_paged_decode_attn_aliased_rows(cuda_device, h, hkv, split):
+@pytest.mark.parametrize("split", [1, 3, 8])
+def test_paged_decode_attn_aliased_rows(cuda_device, monkeypatch, h, hkv, split):
     hd, dev = 128, cuda_device
+    monkeypatch.setattr(K, "packed_decode_splits", lambda *a: split)
     groups = [(33, [0, 1, 15, 16]), (1, [17, 63, 64]), (2, [65]), (0, [1, 130, 0])]      # shared pages, own keys of every row
     g = torch.Generator(device=dev).manual_seed(h)
     lens = [64 * s + n for s, own in groups for n in own]
@@ -345,8 +346,7 @@ def test_paged_decode_attn_aliased_rows(cuda_device, h, hkv, split):
     v[table[6, 1].long(), :, 3] = float("inf")                    # and what one row holds never reaches another
     table = table.to(dev)
     seq = torch.tensor(lens, dtype=torch.int32, device=dev)
-    scratch = None if split else torch.empty(0, device=dev)       # no room for splits
-    out = K.paged_decode_attn(q, 0, k, v, table, seq, h, hkv, hd, hd ** -0.5, groups=K.ALIASED, scratch=scratch)
+    out = K.paged_decode_attn(q, 0, k, v, table, seq, h, hkv, hd, hd ** -0.5, groups=K.ALIASED)
     for i, n in enumerate(lens):
         if n == 0:
             assert bool((out[i] == 0).all())
@@ -471,3 +471,25 @@ def test_rope_append_partials_normalises_heads(cuda_device, rows, splits, h, hkv
     # the two sum a head's squares in unlike orders: where that flips a rounding to bf16 (twice on the way), a value moves by 2^-8 of itself each time
     assert _rel(q1, q0) < 2 ** -7 and _rel(k1, k0) < 2 ** -7
     assert torch.equal(v0, v1)
+
+
+# eight columns of two rows and of one; the last group of rows is not full; whole and in splits; room for long rows
+@pytest.mark.parametrize("rows,h,hkv,pages", [(193, 8, 2, 3), (49, 32, 8, 6), (48, 32, 4, 30)])
+def test_paged_decode_attn_many_rows(cuda_device, rows, h, hkv, pages):
+    hd, dev = 128, cuda_device
+    assert rows * h >= K.PACKED_MIN_HEADS
+    g = torch.Generator(device=dev).manual_seed(rows)
+    table = torch.randperm(rows * pages, generator=g, device=dev).to(torch.int32).view(rows, pages)
+    lens = torch.randint(1, min(pages, 6) * 64 + 1, (rows,), generator=g, device=dev, dtype=torch.int32)
+    lens[0], lens[1], lens[-1] = pages * 64, 0, 1
+    k, v = (torch.randn(rows * pages, hkv, 64, hd, generator=g, device=dev).bfloat16() for _ in range(2))
+    q = torch.randn(rows, (h + 2 * hkv) * hd, generator=g, device=dev).bfloat16()
+    out = K.paged_decode_attn(q, 0, k, v, table, lens, h, hkv, hd, hd ** -0.5)
+    row = K.paged_decode_attn(q, 0, k, v, table, lens, h, hkv, hd, hd ** -0.5, nsplit=2)       # the kernel for single rows
+    assert bool((out[1] == 0).all())
+    for i in (0, 2, rows // 2, rows - 2, rows - 1):
+        n = int(lens[i])
+        kk, vv = (t[table[i].long()].transpose(0, 1).reshape(hkv, -1, hd)[:, :n].double().repeat_interleave(h // hkv, 0) for t in (k, v))
+        w = (torch.einsum("hd,hkd->hk", q[i, :h * hd].double().view(h, hd), kk) * hd ** -0.5).softmax(-1)
+        assert _rel(out[i], torch.einsum("hk,hkd->hd", w, vv).reshape(-1)) < 2 ** -8
+    assert _rel(out, row) < 2 ** -8                               # both round the same sums to bf16
