@@ -131,13 +131,20 @@ inline int& pdl_state() {
   static int v = -1;            // -1 = not read yet, 0 = off, 1 = on, 2 = off by the environment
   return v;
 }
+// Whether this thread's launches follow a kernel of the same chain that let its dependents start only when it had itself waited: what was written before
+// the chain is then visible to all of it, and a product may request its weights ahead of its own wait.
+inline int& pdl_chain() {
+  static thread_local int v = 0;
+  return v;
+}
+// 0: off; 1: on; 2: on, in a chain
 inline int pdl_enabled() {
   int& v = pdl_state();
   if (v < 0) {
     const char* e = getenv("RPEG_PDL");
     v = (e != nullptr && e[0] == '0') ? 2 : 1;
   }
-  return v == 1;
+  return v != 1 ? 0 : pdl_chain() ? 2 : 1;
 }
 
 // Launch `kernel` as a programmatic dependent of the previous kernel in `stream`: its blocks may become resident

@@ -121,7 +121,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   const uint32_t tmem_base = *tmem_slot;
   // Launched as a programmatic dependent (decode: B is a weight matrix that no kernel of the step writes): the
   // set-up above already ran under the previous kernel's tail, and the producer streams the first weight tiles
-  // before it waits for that kernel; every other warp waits here, before it can touch A, C or the workspace. (Not the producer's other
+  // before it waits for that kernel (pdl == 2: what wrote them is known to be done); every other warp waits here, before it can touch A, C or the workspace. (Not the producer's other
   // lanes: a wait of theirs holds up the whole warp.)
   if (pdl) {
     griddep_launch();
@@ -171,6 +171,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
             tile_coords(blockIdx.x / k_splits, tm, tn);
             const int kb0 = (blockIdx.x % k_splits) * kb_per, kb1 = min(num_kb, kb0 + kb_per);
             const int pre = min(STAGES, kb1 - kb0);
+            if (pdl != 2) griddep_wait();
             for (int i = 0; i < pre; ++i) {            // weights first: they do not depend on the previous kernel
               mbar_expect_tx(&full_bar[i], stage_tx);
               tma_load_2d_hint(smem + i * Cfg::STAGE_BYTES + Cfg::A_BYTES, &tmap_b, &full_bar[i], (kb0 + i) * BK, tn * bn, policy);  // never EPI_SWIGLU

@@ -11,8 +11,8 @@
 // up to a fifth of the last wave empty and needed more slabs). A tile's pieces are numbered by CTA; where a tile has fewer pieces than another,
 // its last one stores zeros for the rest.
 //
-// Roles (192 threads, persistent): warp 0 TMA producer, warp 1 issues the MMAs, warps 2..5 epilogue (32 features each). A grid that was launched as a
-// programmatic dependent requests its first weights before it waits for the kernel before (dense: weights are known; experts: they depend on it).
+// Roles (192 threads, persistent): warp 0 TMA producer, warp 1 issues the MMAs, warps 2..5 epilogue (32 features each). In a chain of
+// programmatic dependents a grid requests its first weights before it waits for the kernel before (dense: weights are known; experts: they depend on it).
 #include "act_io.cuh"
 #include "moe_segments.cuh"
 #include "rpeg_kernels.h"
@@ -45,7 +45,7 @@ struct SkinnyCfg {
 };
 
 struct Skinny {
-  int M, N, K, splits;
+  int M, N, K, splits, early;                                        // early: weights may be requested before the wait
   float* parts;                                                      // SK_PARTS
   const int* seg_off;                                                // SK_EXPERTS
   int n_routed, n_shared, seg_rows, shared_from_x, ldc;
@@ -161,6 +161,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       };
       int ahead = 0;
       if constexpr (MODE == SK_PARTS) {
+        if (!p.early) griddep_wait();
         for (int at = begin; ahead < STAGES && next(at, it);)
           for (int kb = it.kb0; kb < it.kb1 && ahead < STAGES; ++kb) load_w(ahead++, kb);
         griddep_wait();
@@ -337,6 +338,7 @@ int skinny_partials(const void* X, const void* W, float* parts, int M, int N, in
   if (rc) return rc - 100;
   Skinny p{};
   p.M = M; p.N = N; p.K = K; p.splits = plan.splits; p.parts = parts; p.status = status;
+  p.early = pdl_enabled() == 2;
   switch (nt) {
     case 16: return launch_skinny<16, SK_PARTS, FF_NONE>(tw, tx, tx, p, plan.grid, stream);
     case 32: return launch_skinny<32, SK_PARTS, FF_NONE>(tw, tx, tx, p, plan.grid, stream);

@@ -260,8 +260,9 @@ __global__ void __launch_bounds__(256)
 rmsnorm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ ids, const __nv_bfloat16* __restrict__ res,
                        const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ h_out,
                        __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out, int d, float eps) {
-  griddep_launch();
+  if (ids == nullptr) griddep_launch();
   griddep_wait();   // may have been scheduled under the previous kernel's tail: nothing is read or written before this
+  if (ids != nullptr) griddep_launch();       // a chain's first kernel (see pdl_chain())
   __shared__ float warp_ss[8];
   const int row = blockIdx.x;
   const int nvec = d >> 3;
@@ -669,8 +670,8 @@ __global__ void add_bf16_kernel(const __nv_bfloat16* __restrict__ a, const __nv_
 // Row gather of an embedding table and its backward scatter-add into an fp32 gradient.
 __global__ void embed_fwd_kernel(const int* __restrict__ ids, const __nv_bfloat16* __restrict__ table,
                                  __nv_bfloat16* __restrict__ out, int T, int d) {
-  griddep_launch();
-  griddep_wait();   // may have been scheduled under the previous kernel's tail: nothing is read or written before this
+  griddep_wait();
+  griddep_launch();                           // a chain's first kernel (see pdl_chain())
   const int dv = d >> 3;
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= static_cast<long long>(T) * dv) return;

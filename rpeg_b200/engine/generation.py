@@ -189,7 +189,14 @@ class Generator:
         # kernel before it (4 Llama-7B layers: 96 rows 0.802 -> 0.741, 128 rows 0.924 -> 0.870, 256 rows 1.411 -> 1.396 ms)
         # (a tensor-parallel step is made of short kernels at every batch size: always chained)
         # (so is the decode step of a model that asks for it)
-        K.set_pdl(b <= getattr(m, "pdl_max_batch", self.PDL_MAX_BATCH) or getattr(m, "tp", 1) > 1)
+        K.set_pdl(b <= getattr(m, "pdl_max_batch", self.PDL_MAX_BATCH) or getattr(m, "tp", 1) > 1, chain=True)
+        try:
+            self._decode_kernels(b, temperature, greedy, seed, top_k, top_p)
+        finally:
+            K.set_pdl(True)
+
+    def _decode_kernels(self, b: int, temperature: float, greedy: bool, seed: int, top_k: int, top_p: float) -> None:
+        m = self.model
         groups = K.ALIASED if self._aliased else None
         if self.group_attention and b >= self.group_min_batch:
             groups = (self.group_rows[:b], self.group_shared[:b], self.row_key0[:b])
@@ -201,7 +208,6 @@ class Generator:
             K.sample_step(logits, temperature, greedy, seed, self.forced_len[:b], self.sampled[:b], self.sampled_lp[:b], self.token[:b], self.pos[:b],
                           self.seq_len[:b], self.active[:b], self.gen_count[:b], self.out_tok[:b], self.out_lp[:b], self.eos_id, self.n_finished,
                           self.step_counter, self.arrived)
-            K.set_pdl(True)
             return
         K.decode_prepare(self.active[:b], self.gen_count[:b], self.forced_len[:b], self.forced[:b], self.eos_id)
         K.sample(logits, temperature, greedy, seed, forced=self.forced[:b], token_out=self.sampled[:b],
@@ -209,7 +215,6 @@ class Generator:
         K.decode_advance(self.sampled[:b], self.sampled_lp[:b], self.token[:b], self.pos[:b], self.seq_len[:b],
                          self.active[:b], self.gen_count[:b], self.out_tok[:b], self.out_lp[:b], self.eos_id,
                          self.n_finished, self.step_counter)
-        K.set_pdl(True)
 
     def _step(self, b: int, temperature: float, greedy: bool, seed: int, top_k: int = 0, top_p: float = 1.0) -> None:
         if not self.use_graphs:

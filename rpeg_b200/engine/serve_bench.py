@@ -243,7 +243,7 @@ def decode_kernels(tab: Table, d, ll, B: int, ctx: int) -> None:
     cos_t, sin_t = d._tables[(m.rot_base, m.rot_dims)]
     rep = 4
     nsp = 1 if B * H >= 296 else min(8, (296 + B * H - 1) // (B * H))
-    K.set_pdl(True)
+    K.set_pdl(True, chain=True)
     L = [i for _ in range(rep) for i in R]
 
     def wbytes(rows, cols):

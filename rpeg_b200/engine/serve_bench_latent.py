@@ -137,7 +137,7 @@ def decode_kernels(tab: S.Table, z, d, ll, B: int, ctx: int) -> None:
     C = [i for _ in range(4) for i in range(4)]
     ws, ws1 = z._workspace(), z._workspace(1)
     h, x32 = torch.randn(B, w, **bf), torch.randn(B, w, device=dev)
-    K.set_pdl(True)
+    K.set_pdl(True, chain=True)
 
     def gemm(name, a, key, like, space=ws):
         ws_ = [q[key] for q in p]

@@ -138,9 +138,10 @@ def gemm_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor | No
     return out
 
 
-def set_pdl(on: bool) -> None:
-    """Programmatic dependent launches for the kernels launched from now on (a captured graph keeps its setting)."""
-    lib().rpeg_set_pdl(int(bool(on)))
+def set_pdl(on: bool, chain: bool = False) -> None:
+    """Programmatic dependent launches for the kernels launched from now on (a captured graph keeps its setting). ``chain``: what this thread launches
+    next is a decode step, whose products may request weights before the kernel in front of them is through."""
+    lib().rpeg_set_pdl(2 if on and chain else int(bool(on)))
 
 
 def publish_version(flag_ptrs, word: int, version: int) -> None:
