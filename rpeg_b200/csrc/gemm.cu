@@ -563,7 +563,7 @@ static int gemm_impl(const void* A, const void* B, void* C, int M, int N, int K,
     const bool few = N >= g_num_sms * 128 || (N >= 2048 && N < 8192 && (M < 8 || K < 2048));       // of up to 128 rows
     const bool half_empty = K >= 2048 && waves >= 2 && 3 * pair_waves >= 4 * waves;
     if ((out_fp32 && accumulate) || (M <= BM ? deep && !few : (deep || wide >= g_num_sms / 4) && (split_k || !half_empty))) {
-      const PairPlan plan = pair_plan(M, N, K, transB, out_fp32 != 0, split_k ? workspace_elems : 0, g_num_sms);
+      const PairPlan plan = pair_plan(M, N, K, transB, out_fp32 != 0, split_k ? workspace_elems : 0, true, g_num_sms);
       const int pdl = (split_k || chain) ? pdl_enabled() : 0;
       if (plan.splits == 1)
         return gemm_pair(A, B, C, M, N, K, lda, ldb, ldc, transA, transB, out_fp32, accumulate, plan, g_num_sms, pdl, status, stream);
@@ -726,7 +726,7 @@ extern "C" int rpeg_gemm_bf16_partials(const void* A, const void* B, int M, int 
     cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
   if (M > BM) {                                            // two row tiles: pairs read the weights once (see gemm_impl)
-    const PairPlan plan = pair_plan(M, N, K, 0, true, workspace_elems, g_num_sms);
+    const PairPlan plan = pair_plan(M, N, K, 0, true, workspace_elems, false, g_num_sms);
     *k_splits_out = plan.splits;
     return gemm_pair(A, B, workspace, M, N, K, lda, ldb, N, 0, 0, 1, 0, plan, g_num_sms, pdl_enabled(), status, stream);
   }

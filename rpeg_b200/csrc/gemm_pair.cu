@@ -34,8 +34,9 @@ static_assert(pair_smem(0) <= 227 * 1024 && pair_smem(1) <= 196 * 1024, "shared 
 
 // Work of a launch: tiles of 256 rows x `bn` accumulator columns, each cut into `splits` pieces of `kb_per` K blocks (splits > 1: every piece
 // stores its own sums, `PG_F32` only).
+// pdl: of pdl_enabled(), 2 means that the first blocks of B may be requested before the wait for the kernel in front.
 struct PairWork {
-  int M, N, K, bn, splits, kb_per;
+  int M, N, K, bn, splits, kb_per, pdl;
 };
 
 enum { PG_BF16 = 0, PG_F32 = 1, PG_F32_ADD = 2, PG_SWIGLU = 3 };
@@ -92,7 +93,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   griddep_launch();
-  griddep_wait();                       // returns at once unless this grid was launched as a programmatic dependent
+  if (warp != 0) griddep_wait();        // returns at once unless this grid was launched as a programmatic dependent; the producer waits further down
 
   // Item order: groups of eight row tiles sweep N together, so that their rows of A stay in L2; the pieces of a tile follow each other.
   struct Item { int tm, tn, split, kb0, kb1; };
@@ -109,30 +110,42 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
   if (warp == 0) {
     if (lane == 0) {
-      const uint64_t policy = l2_policy(EPI == PG_F32 && m_tiles == 1);      // decode: weights that one row tile reads
-      int stage = 0;
+      const uint64_t policy = l2_policy(m_tiles == 1 && (EPI == PG_F32 || pw.pdl != 0));      // decode: weights that one row tile reads
+      auto load_b = [&](const Item& it, int stage, int kb) {
+        uint8_t* sb = smem + stage * PG_STAGE_BYTES + PG_A_BYTES;
+        // swiglu: the even CTA holds the gate rows of the tile's columns, the odd one the up rows (N = f rows further on)
+        const int n0 = EPI == PG_SWIGLU ? it.tn * TN + static_cast<int>(rank) * N : it.tn * TN + static_cast<int>(rank) * (BN / 2);
+        if (rank == 0) mbar_expect_tx(&full_bar[stage], stage_tx);
+        const uint32_t bar = cluster_addr(&full_bar[stage], 0);
+        if constexpr (!B_MN) {
+          tma_load_2d_pair_hint(sb, &tmap_b, bar, kb * PG_BK, n0, policy);
+        } else {
+          for (int c = 0; c * 64 < BN / 2; ++c) tma_load_2d_pair(sb + c * (64 * PG_BK * 2), &tmap_b, bar, n0 + c * 64, kb * PG_BK);
+        }
+      };
+      int ahead = 0;
+      if (pw.pdl == 2 && first < num_items) {
+        const Item it = item(first);
+        for (int kb = it.kb0; kb < it.kb1 && ahead < STAGES; ++kb) load_b(it, ahead++, kb);
+      }
+      griddep_wait();
+      int stage = 0, i = 0;
       uint32_t phase = 0;
       for (int w = first; w < num_items; w += step) {
         const Item it = item(w);
         const int m0 = it.tm * 2 * PG_BM + static_cast<int>(rank) * PG_BM;
-        // swiglu: the even CTA holds the gate rows of the tile's columns, the odd one the up rows (N = f rows further on)
-        const int n0 = EPI == PG_SWIGLU ? it.tn * TN + static_cast<int>(rank) * N : it.tn * TN + static_cast<int>(rank) * (BN / 2);
-        for (int kb = it.kb0; kb < it.kb1; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, status, 160)) goto producer_done;
+        for (int kb = it.kb0; kb < it.kb1; ++kb, ++i) {
+          if (i >= ahead) {
+            if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, status, 160)) goto producer_done;
+            load_b(it, stage, kb);
+          }
           uint8_t* sa = smem + stage * PG_STAGE_BYTES;
-          uint8_t* sb = sa + PG_A_BYTES;
-          if (rank == 0) mbar_expect_tx(&full_bar[stage], stage_tx);
           const uint32_t bar = cluster_addr(&full_bar[stage], 0);
           if constexpr (!A_MN) {
             tma_load_2d_pair(sa, &tmap_a, bar, kb * PG_BK, m0);
           } else {
 #pragma unroll
             for (int c = 0; c < PG_BM / 64; ++c) tma_load_2d_pair(sa + c * (64 * PG_BK * 2), &tmap_a, bar, m0 + c * 64, kb * PG_BK);
-          }
-          if constexpr (!B_MN) {
-            tma_load_2d_pair_hint(sb, &tmap_b, bar, kb * PG_BK, n0, policy);
-          } else {
-            for (int c = 0; c * 64 < BN / 2; ++c) tma_load_2d_pair(sb + c * (64 * PG_BK * 2), &tmap_b, bar, n0 + c * 64, kb * PG_BK);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
@@ -272,7 +285,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 }
 
 template <int EPI, bool A_MN, bool B_MN>
-static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const PairWork& pw, int num_sms, int pdl, int* status,
+static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const PairWork& pw, int num_sms, int* status,
                        cudaStream_t stream) {
   auto kern = gemm_pair_kernel<EPI, A_MN, B_MN>;
   static bool configured = false;
@@ -292,25 +305,26 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cfg.numAttrs = pw.pdl ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, pw, status) == cudaSuccess ? 0 : -21;
 }
 
 template <int EPI>
 static int pair_major(int transA, int transB, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const PairWork& pw, int num_sms,
-                      int pdl, int* status, cudaStream_t stream) {
-  if (!transA && !transB) return launch_pair<EPI, false, false>(ta, tb, tc, pw, num_sms, pdl, status, stream);
-  if (transA && !transB) return launch_pair<EPI, true, false>(ta, tb, tc, pw, num_sms, pdl, status, stream);
-  if (!transA) return launch_pair<EPI, false, true>(ta, tb, tc, pw, num_sms, pdl, status, stream);
-  return launch_pair<EPI, true, true>(ta, tb, tc, pw, num_sms, pdl, status, stream);
+                      int* status, cudaStream_t stream) {
+  if (!transA && !transB) return launch_pair<EPI, false, false>(ta, tb, tc, pw, num_sms, status, stream);
+  if (transA && !transB) return launch_pair<EPI, true, false>(ta, tb, tc, pw, num_sms, status, stream);
+  if (!transA) return launch_pair<EPI, false, true>(ta, tb, tc, pw, num_sms, status, stream);
+  return launch_pair<EPI, true, true>(ta, tb, tc, pw, num_sms, status, stream);
 }
 
 // Accumulator columns of a tile (`bn`) and K pieces (`splits` of `kb_per` 64-deep blocks; slab_elems: fp32 words for their sums, 0: one piece).
 // What a K block of a tile costs, in that of 256 columns, measured over whole waves of tiles (8192 x 4096 x 4096: 26.2 us a wave of 256,
 // 20.0 of 192, 18.9 of 128, 18.0 of 64): narrow tiles read A as often for less work, so they are for sizes whose wide tiles leave the
 // last wave nearly empty (700 x 4096 x 4096: 33 us at 256, 27 us at 192; 5900 rows: 135 and 139 us). An item starts and ends in about four
-// blocks' time, and every slab is written and read once more (256 x 12288 x 4096: 1 us each).
-PairPlan pair_plan(int M, int N, int K, int transB, bool f32, long long slab_elems, int num_sms) {
+// blocks' time, and every slab is written and read once more (256 x 12288 x 4096: 1 us each); where a reduction of its own reads them, `reduced`,
+// more than L2 holds takes longer (256 x 32000 x 4096: 61 + 14 us in two pieces, 53 whole; 160 x 4096 x 4096: 14.5 in four, 16.2 in fewer).
+PairPlan pair_plan(int M, int N, int K, int transB, bool f32, long long slab_elems, bool reduced, int num_sms) {
   static const struct { int bn; double cost; bool any_b, any_out; } widths[] = {      // B stored [K, N] comes in boxes of 64 columns a CTA;
       {256, 1.0, true, true}, {224, 0.88, false, false}, {192, 0.77, false, true},    // a bf16 line of the output has 64 columns
       {160, 0.75, false, false}, {128, 0.72, true, true}, {64, 0.69, false, true}};
@@ -326,7 +340,8 @@ PairPlan pair_plan(int M, int N, int K, int transB, bool f32, long long slab_ele
       const int kb_per = (num_kb + sp - 1) / sp;
       if ((num_kb + kb_per - 1) / kb_per != sp) continue;
       if (sp == 1 && !f32 && !w.any_out) continue;
-      const double cost = static_cast<double>((tiles * sp + pairs - 1) / pairs) * (kb_per * w.cost + 4.0) + (sp > 1 || slab_elems > 0 ? sp * slab_cost : 0.0);
+      const double cost = static_cast<double>((tiles * sp + pairs - 1) / pairs) * (kb_per * w.cost + 4.0) +
+                          (sp == 1 && (reduced || slab_elems == 0) ? 0.0 : sp * slab_cost * (reduced && sp * slab > (6 << 20) ? 2.5 : 1.0));
       if (cost < least * 0.999) { least = cost; best = PairPlan{w.bn, sp, kb_per}; }
     }
   }
@@ -346,10 +361,10 @@ int gemm_pair(const void* A, const void* B, void* C, int M, int N, int K, int ld
   rc = out_fp32 ? make_tmap_f32_3d(&tc, C, N, M, splits, ldc, static_cast<uint64_t>(M) * ldc, 32, 32, accumulate ? 2 : 3)
                 : make_tmap_bf16_2d(&tc, C, N, M, ldc, 64, 32);
   if (rc) return rc - 200;
-  const PairWork pw{M, N, K, bn, splits, plan.kb_per};
-  if (!out_fp32) return pair_major<PG_BF16>(transA, transB, ta, tb, tc, pw, num_sms, pdl, status, stream);
-  if (accumulate) return pair_major<PG_F32_ADD>(transA, transB, ta, tb, tc, pw, num_sms, pdl, status, stream);
-  return pair_major<PG_F32>(transA, transB, ta, tb, tc, pw, num_sms, pdl, status, stream);
+  const PairWork pw{M, N, K, bn, splits, plan.kb_per, pdl};
+  if (!out_fp32) return pair_major<PG_BF16>(transA, transB, ta, tb, tc, pw, num_sms, status, stream);
+  if (accumulate) return pair_major<PG_F32_ADD>(transA, transB, ta, tb, tc, pw, num_sms, status, stream);
+  return pair_major<PG_F32>(transA, transB, ta, tb, tc, pw, num_sms, status, stream);
 }
 
 int gemm_pair_swiglu(const void* A, const void* W, void* C, int M, int f, int K, int lda, int ldw, int ldc, int num_sms, int* status,
@@ -361,7 +376,7 @@ int gemm_pair_swiglu(const void* A, const void* W, void* C, int M, int f, int K,
   if (rc) return rc - 100;
   rc = make_tmap_bf16_2d(&tc, C, f, M, ldc, 64, 32);
   if (rc) return rc - 200;
-  return launch_pair<PG_SWIGLU, false, false>(ta, tb, tc, PairWork{M, f, K, 256, 1, (K + PG_BK - 1) / PG_BK}, num_sms, 0, status, stream);
+  return launch_pair<PG_SWIGLU, false, false>(ta, tb, tc, PairWork{M, f, K, 256, 1, (K + PG_BK - 1) / PG_BK, 0}, num_sms, status, stream);
 }
 
 }  // namespace rpeg

@@ -71,7 +71,7 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
 struct PairPlan {                       // of pair_plan()
   int bn, splits, kb_per;
 };
-PairPlan pair_plan(int M, int N, int K, int transB, bool f32, long long slab_elems, int num_sms);
+PairPlan pair_plan(int M, int N, int K, int transB, bool f32, long long slab_elems, bool reduced, int num_sms);
 int gemm_pair(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int transA, int transB, int out_fp32,
               int accumulate, PairPlan plan, int num_sms, int pdl, int* status, cudaStream_t stream);
 int gemm_pair_swiglu(const void* A, const void* W, void* C, int M, int f, int K, int lda, int ldw, int ldc, int num_sms, int* status,

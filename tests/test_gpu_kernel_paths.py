@@ -434,12 +434,12 @@ def test_embed_rmsnorm_rows(cuda_device, rows, d):
     assert torch.equal(h, table[ids.long()]) and torch.equal(y, K.rmsnorm_fwd(h, w[0], 1e-5)[0])
 
 
-# output heads whose tiles are narrower than 256: one wave of 224, two of 160 where 256 takes three
-@pytest.mark.parametrize("m,n,k", [(1, 32000, 264), (17, 32008, 520), (128, 37000, 136), (3, 70000, 72)])
+# output heads whose tiles are narrower than 256: one wave of 224, two of 160 where 256 takes three; of more rows: whole although there is room for pieces
+@pytest.mark.parametrize("m,n,k", [(1, 32000, 264), (17, 32008, 520), (128, 37000, 136), (3, 70000, 72), (129, 32000, 4096), (256, 32008, 1096)])
 def test_gemm_narrow_wave(cuda_device, m, n, k):
     g = torch.Generator(device=cuda_device).manual_seed(m)
     a, b = (torch.randn(r, k, generator=g, device=cuda_device).bfloat16() for r in (m, n))
-    ws = torch.empty(1 << 20, device=cuda_device)
+    ws = torch.empty(1 << 20 if m <= 128 else 24 << 20, device=cuda_device)
     assert _rel(K.gemm(a, b, workspace=ws), a.double() @ b.double().T) < 2 ** -8
 
 
