@@ -14,6 +14,29 @@ __device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<f
 __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
   *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
 }
+// Eight columns: one 16-byte access of bf16, two of fp32.
+struct float8 { float4 lo, hi; };
+__device__ __forceinline__ float8 load8(const float* p) { return {load4(p), load4(p + 4)}; }
+__device__ __forceinline__ float8 widen(float8 v) { return v; }
+__device__ __forceinline__ float8 widen(uint4 v) {
+  const float2 a = unpack_bf16x2(v.x), b = unpack_bf16x2(v.y), c = unpack_bf16x2(v.z), d = unpack_bf16x2(v.w);
+  return {make_float4(a.x, a.y, b.x, b.y), make_float4(c.x, c.y, d.x, d.y)};
+}
+__device__ __forceinline__ float4 widen(float4 v) { return v; }
+__device__ __forceinline__ float4 widen(uint2 v) {
+  const float2 a = unpack_bf16x2(v.x), b = unpack_bf16x2(v.y);
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ float8 load8(const __nv_bfloat16* p) { return widen(*reinterpret_cast<const uint4*>(p)); }
+// As stored, for loads that are requested together before the first is used.
+__device__ __forceinline__ float4 raw4(const float* p) { return load4(p); }
+__device__ __forceinline__ uint2 raw4(const __nv_bfloat16* p) { return *reinterpret_cast<const uint2*>(p); }
+__device__ __forceinline__ float8 raw8(const float* p) { return load8(p); }
+__device__ __forceinline__ uint4 raw8(const __nv_bfloat16* p) { return *reinterpret_cast<const uint4*>(p); }
+__device__ __forceinline__ void store8(float* p, float8 v) { store4(p, v.lo); store4(p + 4, v.hi); }
+__device__ __forceinline__ void store8(__nv_bfloat16* p, float8 v) {
+  *reinterpret_cast<uint4*>(p) = make_uint4(pack_bf16x2(v.lo.x, v.lo.y), pack_bf16x2(v.lo.z, v.lo.w), pack_bf16x2(v.hi.x, v.hi.y), pack_bf16x2(v.hi.z, v.hi.w));
+}
 __device__ __forceinline__ float2 load2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ float2 load2(const __nv_bfloat16* p) { return unpack_bf16x2(*reinterpret_cast<const uint32_t*>(p)); }
 __device__ __forceinline__ void store2(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
@@ -22,6 +45,23 @@ __device__ __forceinline__ float load1(const float* p) { return *p; }
 __device__ __forceinline__ float load1(const __nv_bfloat16* p) { return __bfloat162float(*p); }
 
 __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+
+// at(0) + at(1) + ... + at(n - 1), in that order; B + 1 of them are requested together, whatever n is. (An unrolled loop over n leaves what n is over its
+// unrolling to a loop of single loads: with six slabs or experts that was all of them, a round trip to L2 each.)
+template <int B, typename At>
+__device__ __forceinline__ auto sum_in_order(int n, At at) {
+  auto v = at(0);
+  for (int k0 = 1; k0 < n; k0 += B) {
+    decltype(v) a[B];
+#pragma unroll
+    for (int i = 0; i < B; ++i)
+      if (k0 + i < n) a[i] = at(k0 + i);
+#pragma unroll
+    for (int i = 0; i < B; ++i)
+      if (k0 + i < n) v = add4(v, a[i]);
+  }
+  return v;
+}
 
 // Two fp32 numbers in one register pair, for the packed fp32 instructions.
 __device__ __forceinline__ uint64_t pack2(float a, float b) {

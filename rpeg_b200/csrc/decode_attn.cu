@@ -14,7 +14,7 @@
 // Replaces the reference's static-KV decode: Megatron StaticInferenceContext plus per-layer
 // index_select/copy compaction (RPEG/runtime/workers/megatron_worker.py:2585-2598, 2667-2811).
 #include <cmath>
-#include "common.cuh"
+#include "act_io.cuh"
 #include "rpeg_kernels.h"
 
 namespace rpeg {
@@ -121,14 +121,12 @@ rope_kv_append_partials_kernel(const float* __restrict__ parts, int splits, long
   constexpr int half = HD / 2;
   const int i = lane * 2;
   // lane owns elements (i, i+1) and their rotation partners (i+half, i+half+1)
-  float lo0 = 0.f, lo1 = 0.f, hi0 = 0.f, hi1 = 0.f;
   const size_t off = static_cast<size_t>(t) * ld + col;
-  for (int s = 0; s < splits; ++s) {
-    const float2 a = *reinterpret_cast<const float2*>(parts + s * stride + off + i);
-    const float2 b = *reinterpret_cast<const float2*>(parts + s * stride + off + i + half);
-    lo0 += a.x; lo1 += a.y; hi0 += b.x; hi1 += b.y;
-  }
-  uint32_t lo = pack_bf16x2(lo0, lo1), hi = pack_bf16x2(hi0, hi1);
+  const float4 x = sum_in_order<8>(splits, [&](int s) {
+    const float2 a = load2(parts + s * stride + off + i), b = load2(parts + s * stride + off + i + half);
+    return make_float4(a.x, a.y, b.x, b.y);
+  });
+  uint32_t lo = pack_bf16x2(x.x, x.y), hi = pack_bf16x2(x.z, x.w);
   if (job < H + Hkv) {
     float2 a = unpack_bf16x2(lo), b = unpack_bf16x2(hi);
     if constexpr (NORM) {                    // rounded where headnorm_fwd_kernel rounds

@@ -9,7 +9,7 @@
 //
 // The reference keeps this state in Python per generation call and compacts KV rows on the host
 // side after every EOS (RPEG/runtime/workers/megatron_worker.py:2463-2598).
-#include "common.cuh"
+#include "act_io.cuh"
 #include "decode_state.cuh"
 #include "rpeg_kernels.h"
 
@@ -86,11 +86,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, __nv_bfloat
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= static_cast<long long>(M) * nv) return;
   const int m = static_cast<int>(idx / nv), j = static_cast<int>(idx % nv);
-  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int s = 0; s < splits; ++s) {
-    const float4 p = reinterpret_cast<const float4*>(part + (static_cast<size_t>(s) * M + m) * N)[j];
-    a.x += p.x; a.y += p.y; a.z += p.z; a.w += p.w;
-  }
+  const float4 a = sum_in_order<8>(splits, [&](int s) { return load4(part + (static_cast<size_t>(s) * M + m) * N + j * 4); });
   uint2 o;
   o.x = pack_bf16x2(a.x, a.y);
   o.y = pack_bf16x2(a.z, a.w);

@@ -34,10 +34,7 @@ __device__ __forceinline__ float4 read_projection(const Projection& s, int t, in
   const size_t off = static_cast<size_t>(t) * s.ld + col;
   if constexpr (PARTIALS) {
     const float* p = static_cast<const float*>(s.p) + off;
-    float4 a = load4(p);
-#pragma unroll 8
-    for (int k = 1; k < s.splits; ++k) a = add4(a, load4(p + k * s.stride));
-    return a;
+    return sum_in_order<8>(s.splits, [&](int k) { return load4(p + k * s.stride); });
   } else {
     return load4(static_cast<const T*>(s.p) + off);
   }

@@ -390,20 +390,32 @@ latent_merge_kernel(const float* __restrict__ partial, const float2* __restrict_
   const size_t at = blockIdx.x;
   const float sl = sink != nullptr ? sink[blockIdx.x % H] * 1.4426950408889634f : -INFINITY;
   const float2* w = ml + at * nsplit;
+  const int lane = threadIdx.x & 31;
+  // a split per lane; the sums themselves are requested in eights, before what they weigh is known
   float gm = sl;
-  for (int s = 0; s < nsplit; ++s) gm = fmaxf(gm, w[s].x);
-  float gl = sl == -INFINITY ? 0.f : exp2f(sl - gm);
-  for (int s = 0; s < nsplit; ++s) gl += w[s].x == -INFINITY ? 0.f : w[s].y * exp2f(w[s].x - gm);
+  for (int s = lane; s < nsplit; s += 32) gm = fmaxf(gm, w[s].x);
+  gm = warp_max(gm);
+  float gl = 0.f;
+  for (int s = lane; s < nsplit; s += 32) gl += w[s].x == -INFINITY ? 0.f : w[s].y * exp2f(w[s].x - gm);
+  gl = warp_sum(gl) + (sl == -INFINITY ? 0.f : exp2f(sl - gm));
   const float inv = gl > 0.f ? 1.f / gl : 0.f;
   for (int d = threadIdx.x * 4; d < rank_p; d += 512) {
     float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-    for (int s = 0; s < nsplit; ++s) {
-      const float2 m = w[s];
-      if (m.x == -INFINITY) continue;
-      const float f = exp2f(m.x - gm) * inv;
-      const float4 v = load4(partial + (at * nsplit + s) * rank_p + d);
-      r.x = fmaf(v.x, f, r.x); r.y = fmaf(v.y, f, r.y); r.z = fmaf(v.z, f, r.z); r.w = fmaf(v.w, f, r.w);
+    for (int s0 = 0; s0 < nsplit; s0 += 8) {
+      float4 v[8];
+      float m[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (s0 + i < nsplit) {
+          v[i] = load4(partial + (at * nsplit + s0 + i) * rank_p + d);
+          m[i] = w[s0 + i].x;
+        }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (s0 + i < nsplit && m[i] != -INFINITY) {
+          const float f = exp2f(m[i] - gm) * inv;
+          r.x = fmaf(v[i].x, f, r.x); r.y = fmaf(v[i].y, f, r.y); r.z = fmaf(v[i].z, f, r.z); r.w = fmaf(v[i].w, f, r.w);
+        }
     }
     store4(out + at * rank_p + d, r);
   }

@@ -52,18 +52,26 @@ moe_route_kernel(const float* __restrict__ logits, int splits, long long stride,
   int* pick = reinterpret_cast<int*>(gs + n_groups);
   const float* lr = logits + static_cast<size_t>(t) * ld;
   float mx = -INFINITY;
-  for (int e = lane; e < E; e += 32) {
-    float z = lr[e];
-    for (int s0 = 1; s0 < splits; s0 += 16) {              // 16 slabs in flight
-      float a[16];
+  for (int e = lane; e < E; e += 64) {                     // two experts a lane, 16 slabs of each in flight
+    const bool two = e + 32 < E;
+    float z = lr[e], z2 = two ? lr[e + 32] : 0.f;
+    for (int s0 = 1; s0 < splits; s0 += 16) {
+      float a[16], a2[16];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) a[i] = s0 + i < splits ? lr[(s0 + i) * stride + e] : 0.f;
+      for (int i = 0; i < 16; ++i) {
+        a[i] = s0 + i < splits ? lr[(s0 + i) * stride + e] : 0.f;
+        a2[i] = two && s0 + i < splits ? lr[(s0 + i) * stride + e + 32] : 0.f;
+      }
 #pragma unroll
       for (int i = 0; i < 16; ++i)
-        if (s0 + i < splits) z += a[i];
+        if (s0 + i < splits) { z += a[i]; z2 += a2[i]; }
     }
     sc[e] = z;
     mx = fmaxf(mx, z);
+    if (two) {
+      sc[e + 32] = z2;
+      mx = fmaxf(mx, z2);
+    }
   }
   if (sigmoid) {
     for (int e = lane; e < E; e += 32) sc[e] = sigmoidf(sc[e]);

@@ -22,18 +22,24 @@ template <typename T, int SRC>
 __device__ __forceinline__ float4 norm_source(const NormSource& s, const int* choice_row, const float* choice_w, int row, int rows, int c) {
   if constexpr (SRC == NSRC_PARTIALS) {
     const float* p = static_cast<const float*>(s.p) + static_cast<size_t>(row) * s.ld + c;
-    float4 v = load4(p);
-#pragma unroll 8
-    for (int k = 1; k < s.splits; ++k) v = add4(v, load4(p + k * s.stride));
-    return v;
+    return sum_in_order<8>(s.splits, [&](int k) { return load4(p + k * s.stride); });
   } else if constexpr (SRC == NSRC_MOE) {
     const T* y = static_cast<const T*>(s.p) + c;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-    for (int k = 0; k < s.top + s.n_shared; ++k) {
-      const float w = choice_w[k];
-      const float4 e = load4(y + static_cast<size_t>(choice_row[k]) * s.ld);
-      v.x = fmaf(w, e.x, v.x); v.y = fmaf(w, e.y, v.y); v.z = fmaf(w, e.z, v.z); v.w = fmaf(w, e.w, v.w);
+    const int n = s.top + s.n_shared;
+    constexpr int B = sizeof(T) == 2 ? 10 : 5;
+    for (int k0 = 0; k0 < n; k0 += B) {              // B rows in flight, whatever n is
+      decltype(raw4(y)) a[B];
+#pragma unroll
+      for (int i = 0; i < B; ++i)
+        if (k0 + i < n) a[i] = raw4(y + static_cast<size_t>(choice_row[k0 + i]) * s.ld);
+#pragma unroll
+      for (int i = 0; i < B; ++i)
+        if (k0 + i < n) {
+          const float w = choice_w[k0 + i];
+          const float4 e = widen(a[i]);
+          v.x = fmaf(w, e.x, v.x); v.y = fmaf(w, e.y, v.y); v.z = fmaf(w, e.z, v.z); v.w = fmaf(w, e.w, v.w);
+        }
     }
     return v;
   } else if constexpr (SRC == NSRC_EMBED) {
@@ -42,6 +48,34 @@ __device__ __forceinline__ float4 norm_source(const NormSource& s, const int* ch
     return load4(static_cast<const float*>(s.p) + static_cast<size_t>(row) * s.ld + c);
   } else {
     return load4(static_cast<const T*>(s.p) + static_cast<size_t>(row) * s.ld + c);
+  }
+}
+
+// Eight columns of an activation or of expert rows, of which B are requested together.
+template <typename T, int SRC, int B = 1>
+__device__ __forceinline__ float8 norm_source8(const NormSource& s, const int* choice_row, const float* choice_w, int row, int c) {
+  const T* y = static_cast<const T*>(s.p) + c;
+  if constexpr (SRC == NSRC_MOE) {
+    float8 v = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+    const int n = s.top + s.n_shared;
+    for (int k0 = 0; k0 < n; k0 += B) {
+      decltype(raw8(y)) a[B];
+#pragma unroll
+      for (int i = 0; i < B; ++i)
+        if (k0 + i < n) a[i] = raw8(y + static_cast<size_t>(choice_row[k0 + i]) * s.ld);
+#pragma unroll
+      for (int i = 0; i < B; ++i)
+        if (k0 + i < n) {
+          const float w = choice_w[k0 + i];
+          const float8 e = widen(a[i]);
+          v.lo.x = fmaf(w, e.lo.x, v.lo.x); v.lo.y = fmaf(w, e.lo.y, v.lo.y); v.lo.z = fmaf(w, e.lo.z, v.lo.z); v.lo.w = fmaf(w, e.lo.w, v.lo.w);
+          v.hi.x = fmaf(w, e.hi.x, v.hi.x); v.hi.y = fmaf(w, e.hi.y, v.hi.y); v.hi.z = fmaf(w, e.hi.z, v.hi.z); v.hi.w = fmaf(w, e.hi.w, v.hi.w);
+        }
+    }
+    return v;
+  } else {
+    static_assert(SRC == NSRC_ACT, "activations and expert rows");
+    return load8(y + static_cast<size_t>(row) * s.ld);
   }
 }
 

@@ -42,10 +42,7 @@ rotary_append_kernel(const void* __restrict__ src_v, int splits, long long strid
     const size_t off = static_cast<size_t>(t) * ld + col;
     if constexpr (PARTIALS) {
       const float* s = static_cast<const float*>(src_v) + off;
-      float4 a = load4(s);
-#pragma unroll 8
-      for (int k = 1; k < splits; ++k) a = add4(a, load4(s + k * stride));
-      return a;
+      return sum_in_order<8>(splits, [&](int k) { return load4(s + k * stride); });
     } else {
       return load4(static_cast<const T*>(src_v) + off);
     }

@@ -493,3 +493,35 @@ def test_paged_decode_attn_many_rows(cuda_device, rows, h, hkv, pages):
         w = (torch.einsum("hd,hkd->hk", q[i, :h * hd].double().view(h, hd), kk) * hd ** -0.5).softmax(-1)
         assert _rel(out[i], torch.einsum("hk,hkd->hd", w, vv).reshape(-1)) < 2 ** -8
     assert _rel(out, row) < 2 ** -8                               # both round the same sums to bf16
+
+
+# rows of prompts: eight columns a thread, gathers in batches of 8 and 6 (4 and 3 in fp32): fewer experts than a batch, one more, two batches; ragged ends of a row
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,d,top,shared", [(297, 1000, 1, 0), (300, 2048, 7, 0), (331, 1036, 6, 3), (297, 8192, 2, 1)])
+def test_expert_rows_of_prompts(cuda_device, dtype, rows, d, top, shared):
+    g = torch.Generator(device=cuda_device).manual_seed(d)
+    f32 = dict(generator=g, device=cuda_device)
+    dp = -(-d // 8) * 8
+    pad = lambda t: torch.nn.functional.pad(t, (0, dp - d)).contiguous()
+    out = pad(torch.randn(rows * (top + shared), d, **f32)).to(dtype)
+    row_of = torch.randperm(rows * top, generator=g, device=cuda_device).int().view(rows, top)
+    wts = torch.rand(rows, top, **f32)
+    w, w2, b, a = (pad(torch.randn(*s, d, **f32)).to(dtype) for s in ((), (), (), (rows,)))
+    x0 = pad(torch.randn(rows, d, **f32))
+    src = K.MoEOutput(out, row_of, wts, shared)
+    mix = (out[row_of.long()].double() * wts[..., None].double()).sum(1)
+    for s in range(shared):
+        mix += out[rows * top + s * rows: rows * top + (s + 1) * rows].double()
+    tol = F32 if dtype == torch.float32 else 2 ** -8                   # a bf16 result is rounded once
+    norm = lambda t, v: t * torch.rsqrt((t * t).sum(-1, keepdim=True) / d + 1e-3) * v.double()
+    x = x0.clone()
+    y = K.residual_norm(src, w, 1e-3, d, x=x, zero_centered=False)
+    want = x0.double() + norm(mix, w)
+    assert _rel(x, want) < F32 and _rel(y, want) < tol
+    x = x0.clone()
+    assert _rel(K.residual_norm(src, w, 1e-3, d, x=x, w2=w2, zero_centered=False), norm(want, w2)) < tol and _rel(x, want) < F32
+    if shared == 0:
+        x = x0.clone()
+        y = K.stream_update(a, src, torch.tensor(0.3, device=cuda_device), w, b, x)
+        want = x0.double() + a.double() + mix
+        assert _rel(x, want) < F32 and _rel(y, torch.tanh(0.3 * want) * w.double() + b.double()) < tol
