@@ -12,6 +12,10 @@
 // P stays fp32: it enters the product as three bf16 parts (8 + 8 + 8 bits, exact). Columns a block is not for are neither scored nor added to, so
 // what one row holds (infinities, NaN) never reaches another.
 //
+// Rows may see no more than the window of keys that they are in (windows are whole pages), and a sink per head may join the denominator: the served
+// decoders' rows (window_attn.cu has the general kernel; 64 rows, 32 heads, 8 KV heads, 80 to 200 keys: 14 us, there 20; 8 rows of up to 1000 13, there
+// 22).
+//
 // Bound by the bytes of the pages; the row kernel (decode_attn.cu) reads the shared ones once per row, from L2.
 #include <cmath>
 #include "pair.cuh"
@@ -52,25 +56,38 @@ __device__ __forceinline__ uint32_t take_bf16x2(float& a, float& b) {
   return __byte_perm(x, y, 0x7632);
 }
 
+// What a row sees: keys [first, n) of page-table row slot[row], n = lens[row] (or pos[row] + 1), first = the start of n - 1's window (0: no windows).
+struct PackedRows {
+  const int* lens;
+  const int* pos;
+  const int* slot;            // null: row
+  int window;
+  const float* sink;          // [H] or null
+};
+
 template <int G>
 __global__ void __launch_bounds__(DP_THREADS, 3)
 paged_decode_attn_packed_kernel(const __nv_bfloat16* __restrict__ q, int ldq, int q_col0, const __nv_bfloat16* __restrict__ kcache,
                                 const __nv_bfloat16* __restrict__ vcache, const int* __restrict__ page_table, int max_pages,
-                                const int* __restrict__ seq_lens, __nv_bfloat16* __restrict__ out, int B, int H, int Hkv, int nsplit,
-                                float scale_log2) {
+                                const PackedRows seen, __nv_bfloat16* __restrict__ out, int B, int H, int Hkv, int nsplit, float scale_log2) {
   griddep_launch();
   griddep_wait();   // may have been scheduled under the previous kernel's tail: nothing is read or written before this
   __shared__ int2 list[DP_LIST];                             // first cache row of a block; its first key | columns << 24 | keys - 1
-  __shared__ int lens_s[DP_COLS], warp_total[DP_WARPS];
+  __shared__ int lens_s[DP_COLS], first_s[DP_COLS], warp_total[DP_WARPS];     // keys and first page of every row
   __shared__ __align__(8) float2 sum_ml[DP_COLS];             // this split's maxima and sums
   __shared__ float red_m[DP_WARPS][DP_COLS], red_l[DP_WARPS][DP_COLS];
   __shared__ __align__(16) float red_o[DP_WARPS][DP_COLS][DP_HD];
   constexpr int rows = DP_COLS / G;
   const int hk = blockIdx.x, row0 = blockIdx.y * rows, split = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  if (tid < DP_COLS) lens_s[tid] = tid < rows && row0 + tid < B ? seq_lens[row0 + tid] : 0;
+  if (tid < DP_COLS) {
+    const int n = tid < rows && row0 + tid < B ? (seen.lens != nullptr ? seen.lens[row0 + tid] : seen.pos[row0 + tid] + 1) : 0;
+    lens_s[tid] = n;
+    first_s[tid] = seen.window > 0 && n > 0 ? (n - 1) / seen.window * seen.window / DP_PAGE : 0;
+  }
   const int pr = tid & 7, pi = tid >> 3;                     // this thread's row and page in a listing
-  const int* table = page_table + static_cast<size_t>(min(row0 + pr, B - 1)) * max_pages;
+  const int trow = min(row0 + pr, B - 1);
+  const int* table = page_table + static_cast<size_t>(seen.slot != nullptr ? seen.slot[trow] : trow) * max_pages;
   int pages[2];
 #pragma unroll
   for (int i = 0; i < 2; ++i) pages[i] = pr < rows && pi + 16 * i < max_pages ? table[pi + 16 * i] : 0;
@@ -87,25 +104,26 @@ paged_decode_attn_packed_kernel(const __nv_bfloat16* __restrict__ q, int ldq, in
   }
   __syncthreads();
   const int len0 = lens_s[2 * t / G], len1 = lens_s[(2 * t + 1) / G];     // of this lane's columns 2t, 2t + 1
-  int longest = 0, live = 0;
+  int longest = 0, live = 0, w_first = max_pages;
 #pragma unroll
   for (int c = 0; c < DP_COLS; ++c) {
     const int n = lens_s[c / G];
     longest = max(longest, n);
     live |= (n > 0 ? 1 : 0) << c;
+    if (n > 0) w_first = min(w_first, first_s[c / G]);
   }
   const int n_pages = min(max_pages, (longest + DP_PAGE - 1) / DP_PAGE);
 
   float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
   float acc[8][4] = {};                                      // [i]: dimensions 8g + i (columns 2t, 2t + 1) and 64 + 8g + i
-  for (int w0 = 0; w0 < n_pages; w0 += DP_WINDOW) {
+  for (int w0 = w_first; w0 < n_pages; w0 += DP_WINDOW) {
     // ---- list the window's blocks
     int count[2], mask[2], keys[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int page = w0 + pi + 16 * i, left = lens_s[pr] - page * DP_PAGE;
       if (w0 > 0) pages[i] = pr < rows && page < n_pages ? table[page] : 0;
-      const int own = pr < rows && page < n_pages ? max(0, min(left, DP_PAGE)) : 0;      // keys of this page that the row sees
+      const int own = pr < rows && page < n_pages && page >= first_s[pr] ? max(0, min(left, DP_PAGE)) : 0;      // keys of this page that the row sees
       int most = own, cols = 0;
       bool first = own > 0;
 #pragma unroll
@@ -279,14 +297,20 @@ paged_decode_attn_packed_kernel(const __nv_bfloat16* __restrict__ q, int ldq, in
 #pragma unroll
     for (int i = 0; i < 8; ++i) o[i] += red_o[w][col][d0 + i] * f;
   }
-  auto store = [&](const float (&v)[8], float l) {
+  auto store = [&](float (&v)[8], float m, float l) {
+    if (seen.sink != nullptr) {
+      const float sl = seen.sink[hk * G + col % G] * 1.4426950408889634f, nm = fmaxf(m, sl), f = m == -INFINITY ? 0.f : exp2f(m - nm);
+      l = l * f + exp2f(sl - nm);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] *= f;
+    }
     uint32_t u[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) u[i] = l > 0.f ? pack_bf16x2(v[2 * i] / l, v[2 * i + 1] / l) : 0u;
     *reinterpret_cast<uint4*>(out + (static_cast<size_t>(row) * H + hk * G + col % G) * DP_HD + d0) = make_uint4(u[0], u[1], u[2], u[3]);
   };
   if (nsplit == 1) {
-    if (row < B) store(o, gl);
+    if (row < B) store(o, gm, gl);
     return;
   }
   // every (column, eight dimensions) was read by the thread that now rewrites it; the splits share the merge out among themselves
@@ -313,7 +337,7 @@ paged_decode_attn_packed_kernel(const __nv_bfloat16* __restrict__ q, int ldq, in
 #pragma unroll
       for (int i = 0; i < 8; ++i) o[i] = o[i] * f0 + e[i] * f;
     }
-    store(o, gl);
+    store(o, gm, gl);
   }
   __syncwarp();
   cluster_sync_all();                                        // nobody's shared memory goes while another reads it
@@ -323,12 +347,14 @@ paged_decode_attn_packed_kernel(const __nv_bfloat16* __restrict__ q, int ldq, in
 
 using namespace rpeg;
 
-// rpeg_paged_decode_attn for rows that may alias pages, without scratch. H / Hkv must divide 8; at most eight splits.
+// rpeg_paged_decode_attn for rows that may alias pages, without scratch. H / Hkv must divide 8; at most eight splits. seq_lens null: pos + 1; slot null:
+// row t has page-table row t; window: whole pages, or 0; sink [H] or null.
 extern "C" int rpeg_paged_decode_attn_packed(const void* q, int ldq, int q_col0, const void* kcache, const void* vcache, const int* page_table,
-                                             int max_pages, const int* seq_lens, void* out, int B, int H, int Hkv, int hd, int nsplit, float scale,
-                                             void* stream) {
+                                             int max_pages, const int* seq_lens, const int* pos, const int* slot, int window, const float* sink,
+                                             void* out, int B, int H, int Hkv, int hd, int nsplit, float scale, void* stream) {
   if (hd != DP_HD || Hkv <= 0 || H % Hkv != 0 || H / Hkv > DP_COLS || DP_COLS % (H / Hkv) != 0) return -2;
   if (nsplit < 1 || nsplit > 8) return -3;
+  if (window < 0 || window % DP_PAGE != 0 || (seq_lens == nullptr && pos == nullptr)) return -4;
   if ((ldq | q_col0) & 7) return -5;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache) | reinterpret_cast<uintptr_t>(out)) &
       15) return -1;
@@ -350,6 +376,7 @@ extern "C" int rpeg_paged_decode_attn_packed(const void* q, int ldq, int q_col0,
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<const __nv_bfloat16*>(q), ldq, q_col0, static_cast<const __nv_bfloat16*>(kcache),
-                            static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages, seq_lens, static_cast<__nv_bfloat16*>(out), B, H, Hkv,
+                            static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages, PackedRows{seq_lens, pos, slot, window, sink},
+                            static_cast<__nv_bfloat16*>(out), B, H, Hkv,
                             nsplit, scale * 1.4426950408889634f) == cudaSuccess ? 0 : -21;
 }

@@ -144,7 +144,7 @@ class DulisunLayout(FlatLayout):
 class DulisunModel(ServedDecoder):
     """Weights and kernels of one model on one GPU."""
 
-    KERNEL_SOURCES = ("gemm.cu", "gemm_pair.cu", "gemm_skinny.cu", "generate.cu", "loss.cu", "residual_norm.cu", "window_attn.cu", "window_prefill.cu", "moe.cu", "moe_pair.cu", "gemm_f32.cu")
+    KERNEL_SOURCES = ("gemm.cu", "gemm_pair.cu", "gemm_skinny.cu", "generate.cu", "loss.cu", "residual_norm.cu", "window_attn.cu", "decode_attn_packed.cu", "window_prefill.cu", "moe.cu", "moe_pair.cu", "gemm_f32.cu")
 
     def __init__(self, cfg: DulisunConfig, device, *, dtype: torch.dtype = torch.bfloat16, seed: Optional[int] = 0,
                  trainable: bool = False):

@@ -593,8 +593,8 @@ def paged_decode_attn(q, q_col0, kcache, vcache, page_table, seq_lens, n_heads, 
         if 8 % (n_heads // n_kv_heads) == 0 and aligned and B <= 8192 and page_table.shape[1] <= 1 << 18:
             nsplit = packed_decode_splits(B, n_heads, n_kv_heads, page_table.shape[1])
             check(lib().rpeg_paged_decode_attn_packed(q.data_ptr(), q.stride(0), q_col0, kcache.data_ptr(), vcache.data_ptr(),
-                                                      page_table.data_ptr(), page_table.stride(0), seq_lens.data_ptr(), out.data_ptr(), B, n_heads,
-                                                      n_kv_heads, head_dim, nsplit, scale, _stream()), "rpeg_paged_decode_attn_packed")
+                                                      page_table.data_ptr(), page_table.stride(0), seq_lens.data_ptr(), None, None, 0, None, out.data_ptr(),
+                                                      B, n_heads, n_kv_heads, head_dim, nsplit, scale, _stream()), "rpeg_paged_decode_attn_packed")
             return out
     if groups is not None:
         group_rows, group_shared, row_key0 = groups
@@ -819,6 +819,16 @@ def rows_attn(q: torch.Tensor, kcache, vcache, page_table, slot, pos, n_heads: i
     if nsplit > 1 and (scratch is None or scratch.numel() < rows_attn_scratch(rows, n_heads, dp, nsplit) or arrive is None or arrive.numel() < rows * n_heads):
         raise ValueError("rows_attn: split attention needs scratch and arrival counters")
     out = torch.empty((rows, n_heads * dp), dtype=q.dtype, device=q.device)
+    # Four or eight query heads a KV head of 128: eight columns on the tensor cores (us, 32 heads, 8 KV heads, keys up to 200 / 1000, here and there: 1 row
+    # 11.2 / 10.1 and 5.1 / 6.5; 8 rows 13.7 / 21.8 and 7.7 / 12.9; 64 rows 20.3 / 63 and 14.4 / 47.5; 256 rows 55.3 and 39.0; level only at 64 keys).
+    if (q.dtype == torch.bfloat16 and dp == 128 and n_heads in (4 * n_kv, 8 * n_kv) and window % KV_PAGE == 0 and 0 < rows <= 65535 and
+            (q.data_ptr() | kcache.data_ptr() | vcache.data_ptr()) % 16 == 0 and q.stride(0) % 8 == 0 and page_table.shape[1] <= 1 << 18):
+        pages = min(page_table.shape[1], window // KV_PAGE) if window else page_table.shape[1]
+        check(lib().rpeg_paged_decode_attn_packed(q.data_ptr(), q.stride(0), 0, kcache.data_ptr(), vcache.data_ptr(), page_table.data_ptr(),
+                                                  page_table.stride(0), _ptr(lens), pos.data_ptr(), slot.data_ptr(), window, _ptr(sink), out.data_ptr(),
+                                                  rows, n_heads, n_kv, dp, packed_decode_splits(rows, n_heads, n_kv, pages), scale, _stream()),
+              "rpeg_paged_decode_attn_packed")
+        return out
     check(lib().rpeg_rows_attn(q.data_ptr(), q.stride(0), kcache.data_ptr(), vcache.data_ptr(), page_table.data_ptr(), page_table.stride(0),
                                slot.data_ptr(), pos.data_ptr(), _ptr(lens), _ptr(sink), out.data_ptr(), out.stride(0), _ptr(scratch), _ptr(arrive),
                                rows, n_heads, n_kv, dp, window, nsplit, scale, int(q.dtype == torch.float32), status_word(q.device).data_ptr(),

@@ -525,3 +525,31 @@ def test_expert_rows_of_prompts(cuda_device, dtype, rows, d, top, shared):
         y = K.stream_update(a, src, torch.tensor(0.3, device=cuda_device), w, b, x)
         want = x0.double() + a.double() + mix
         assert _rel(x, want) < F32 and _rel(y, torch.tanh(0.3 * want) * w.double() + b.double()) < tol
+
+
+# the tensor-core kernel for a served decoder's rows: windows of one and two pages and none, a sink, rows of one prompt, lengths or positions, splits
+@pytest.mark.parametrize("window,sink,split", [(0, False, 1), (64, True, 1), (128, False, 3), (0, True, 8)])
+@pytest.mark.parametrize("h,hkv", [(4, 1), (16, 2)])
+def test_rows_attn_grouped_heads(cuda_device, monkeypatch, h, hkv, window, sink, split):
+    hd, dev = 128, cuda_device
+    monkeypatch.setattr(K, "packed_decode_splits", lambda *a: split)
+    g = torch.Generator(device=dev).manual_seed(window + h)
+    lens = [1, 0, 64, 65, 128, 129, 300, 301, 2200]
+    slot = torch.tensor([3, 0, 5, 1, 2, 4, 6, 6, 7], dtype=torch.int32, device=dev)
+    table = torch.randperm(8 * 35, generator=g, device=dev).int().view(8, 35)
+    k, v = (torch.randn(8 * 35, hkv, 64, hd, generator=g, device=dev).bfloat16() for _ in range(2))
+    q = torch.randn(len(lens), h * hd, generator=g, device=dev).bfloat16()
+    sk = torch.randn(h, generator=g, device=dev) if sink else None
+    n = torch.tensor(lens, dtype=torch.int32, device=dev)
+    kw = dict(window=window, scale=0.11, sink=sk)
+    got = K.rows_attn(q, k, v, table, slot, n - 1, h, lens=n, **kw)
+    by_pos = K.rows_attn(q[2:], k, v, table, slot[2:], n[2:] - 1, h, **kw)
+    assert split > 1 or torch.equal(by_pos, got[2:])
+    for i, l in enumerate(lens):
+        lo = (l - 1) // window * window if window and l else 0
+        kk, vv = (t[table[slot[i]].long()].transpose(0, 1).reshape(hkv, -1, hd)[:, lo:l].double().repeat_interleave(h // hkv, 0) for t in (k, v))
+        s = torch.einsum("hd,hkd->hk", q[i].double().view(h, hd), kk) * 0.11
+        w = torch.cat([s, sk.double()[:, None]], 1).softmax(-1)[:, :-1] if sink else s.softmax(-1)
+        want = torch.einsum("hk,hkd->hd", w, vv).reshape(-1)
+        assert bool((got[i] == 0).all()) if l == 0 else _rel(got[i], want) < 2 ** -8
+        assert i < 2 or _rel(by_pos[i - 2], want) < 2 ** -8
