@@ -7,7 +7,9 @@
 // on fragments that are loaded straight from the pages: a lane's 16-byte chunks of K are two k steps each (the order of the head dimensions inside
 // a step is free, Q has the same), V's keys 2t, 2t + 1, 2t + 8, 2t + 9 are paired by byte permutes, P^T turns by movmatrix. Every warp keeps its own
 // softmax state for the eight columns; the four are merged at the end. The splits of
-// an item are a cluster and are merged through each other's shared memory: no scratch, and no counters that launches on two streams would share.
+// an item are a cluster and are merged through each other's shared memory: no scratch, and no counters that launches on two streams would share. Where the
+// items fill all SMs once or more, only those of the last wave are split (256 rows of 512 shared and 48 own keys, 32 heads: 2.3 waves, 74 us; all whole
+// 80).
 //
 // P stays fp32: it enters the product as three bf16 parts (8 + 8 + 8 bits, exact). Columns a block is not for are neither scored nor added to, so
 // what one row holds (infinities, NaN) never reaches another.
@@ -69,7 +71,7 @@ template <int G>
 __global__ void __launch_bounds__(DP_THREADS, 3)
 paged_decode_attn_packed_kernel(const __nv_bfloat16* __restrict__ q, int ldq, int q_col0, const __nv_bfloat16* __restrict__ kcache,
                                 const __nv_bfloat16* __restrict__ vcache, const int* __restrict__ page_table, int max_pages,
-                                const PackedRows seen, __nv_bfloat16* __restrict__ out, int B, int H, int Hkv, int nsplit, float scale_log2) {
+                                const PackedRows seen, __nv_bfloat16* __restrict__ out, int B, int H, int Hkv, int cluster, int whole, float scale_log2) {
   griddep_launch();
   griddep_wait();   // may have been scheduled under the previous kernel's tail: nothing is read or written before this
   __shared__ int2 list[DP_LIST];                             // first cache row of a block; its first key | columns << 24 | keys - 1
@@ -78,7 +80,11 @@ paged_decode_attn_packed_kernel(const __nv_bfloat16* __restrict__ q, int ldq, in
   __shared__ float red_m[DP_WARPS][DP_COLS], red_l[DP_WARPS][DP_COLS];
   __shared__ __align__(16) float red_o[DP_WARPS][DP_COLS][DP_HD];
   constexpr int rows = DP_COLS / G;
-  const int hk = blockIdx.x, row0 = blockIdx.y * rows, split = blockIdx.z;
+  // Clusters below `whole` take an item a CTA, the ones behind an item each, in as many splits as they have CTAs.
+  const int cl = blockIdx.x / cluster, rank = blockIdx.x - cl * cluster;
+  const bool shared = cl * cluster >= whole;
+  const int item = shared ? whole + cl - whole / cluster : cl * cluster + rank, nsplit = shared ? cluster : 1, split = shared ? rank : 0;
+  const int hk = item % Hkv, row0 = item / Hkv * rows;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   if (tid < DP_COLS) {
     const int n = tid < rows && row0 + tid < B ? (seen.lens != nullptr ? seen.lens[row0 + tid] : seen.pos[row0 + tid] + 1) : 0;
@@ -347,11 +353,13 @@ paged_decode_attn_packed_kernel(const __nv_bfloat16* __restrict__ q, int ldq, in
 
 using namespace rpeg;
 
-// rpeg_paged_decode_attn for rows that may alias pages, without scratch. H / Hkv must divide 8; at most eight splits. seq_lens null: pos + 1; slot null:
+// rpeg_paged_decode_attn for rows that may alias pages, without scratch. H / Hkv must divide 8; at most eight splits, for the
+// items (eight columns of a KV head) from `whole`, a multiple of nsplit, on. seq_lens null: pos + 1; slot null:
 // row t has page-table row t; window: whole pages, or 0; sink [H] or null.
 extern "C" int rpeg_paged_decode_attn_packed(const void* q, int ldq, int q_col0, const void* kcache, const void* vcache, const int* page_table,
                                              int max_pages, const int* seq_lens, const int* pos, const int* slot, int window, const float* sink,
-                                             void* out, int B, int H, int Hkv, int hd, int nsplit, float scale, void* stream) {
+                                             void* out, int B, int H, int Hkv, int hd, int nsplit, int whole, float scale,
+                                             void* stream) {
   if (hd != DP_HD || Hkv <= 0 || H % Hkv != 0 || H / Hkv > DP_COLS || DP_COLS % (H / Hkv) != 0) return -2;
   if (nsplit < 1 || nsplit > 8) return -3;
   if (window < 0 || window % DP_PAGE != 0 || (seq_lens == nullptr && pos == nullptr)) return -4;
@@ -361,16 +369,17 @@ extern "C" int rpeg_paged_decode_attn_packed(const void* q, int ldq, int q_col0,
   if (max_pages < 1 || max_pages > (1 << 24) / DP_PAGE) return -6;         // a block's first key has 24 bits
   if (B <= 0) return 0;
   const int rows = DP_COLS / (H / Hkv), items = (B + rows - 1) / rows;
-  if (items > 65535) return -7;
+  const long long all = static_cast<long long>(items) * Hkv;
+  if (whole < 0 || whole > all || whole % nsplit != 0 || (all - whole) * nsplit + whole > 0x7fffffffll) return -7;
   auto kern = H == Hkv ? paged_decode_attn_packed_kernel<1>
               : H == 2 * Hkv ? paged_decode_attn_packed_kernel<2> : H == 4 * Hkv ? paged_decode_attn_packed_kernel<4> : paged_decode_attn_packed_kernel<8>;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim = {1, 1, static_cast<unsigned>(nsplit)};
+  attr[0].val.clusterDim = {static_cast<unsigned>(nsplit), 1, 1};
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(Hkv, items, nsplit);
+  cfg.gridDim = dim3(static_cast<unsigned>((all - whole) * nsplit + whole));
   cfg.blockDim = dim3(DP_THREADS);
   cfg.stream = reinterpret_cast<cudaStream_t>(stream);
   cfg.attrs = attr;
@@ -378,5 +387,5 @@ extern "C" int rpeg_paged_decode_attn_packed(const void* q, int ldq, int q_col0,
   return cudaLaunchKernelEx(&cfg, kern, static_cast<const __nv_bfloat16*>(q), ldq, q_col0, static_cast<const __nv_bfloat16*>(kcache),
                             static_cast<const __nv_bfloat16*>(vcache), page_table, max_pages, PackedRows{seq_lens, pos, slot, window, sink},
                             static_cast<__nv_bfloat16*>(out), B, H, Hkv,
-                            nsplit, scale * 1.4426950408889634f) == cudaSuccess ? 0 : -21;
+                            nsplit, whole, scale * 1.4426950408889634f) == cudaSuccess ? 0 : -21;
 }

@@ -140,8 +140,8 @@ int rpeg_paged_decode_attn(const void* q, int ldq, int q_col0, const void* kcach
 // Same, for rows that alias pages (decode_attn_packed.cu): what neighbouring rows share is read once. H / Hkv divides 8.
 int rpeg_paged_decode_attn_packed(const void* q, int ldq, int q_col0, const void* kcache, const void* vcache,
                                   const int* page_table, int max_pages, const int* seq_lens, const int* pos, const int* slot,
-                                  int window, const float* sink, void* out, int B, int H, int Hkv, int hd, int nsplit, float scale,
-                                  void* stream);
+                                  int window, const float* sink, void* out, int B, int H, int Hkv, int hd, int nsplit, int whole,
+                                  float scale, void* stream);
 // Same, for batches whose rows share their first keys in groups (page-table aliasing): group_rows [B, 8], group_shared [B],
 // row_key0 [B]; scratch sized for nsplit + 1 partials.
 int rpeg_paged_decode_attn_grouped(const void* q, int ldq, int q_col0, const void* kcache, const void* vcache,

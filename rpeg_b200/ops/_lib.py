@@ -66,7 +66,7 @@ _SIGNATURES = {
     "rpeg_paged_decode_attn": [P, I, I, P, P, P, I, P, P, P, I, I, I, I, I, F, P],
     "rpeg_embed_rmsnorm_fwd": [P, P, P, P, P, I, I, F, P],
     "rpeg_sample_step": [P, I, I, I, I, F, I, c_ulonglong, P, P, P, P, P, P, P, P, P, P, I, I, P, P, P, P],
-    "rpeg_paged_decode_attn_packed": [P, I, I, P, P, P, I, P, P, P, I, P, P, I, I, I, I, I, F, P],
+    "rpeg_paged_decode_attn_packed": [P, I, I, P, P, P, I, P, P, P, I, P, P, I, I, I, I, I, I, F, P],
     "rpeg_paged_decode_attn_grouped": [P, I, I, P, P, P, I, P, P, P, I, I, I, I, I, F, P, P, P, P],
     "rpeg_tp_allreduce_rmsnorm": [P, P, I, I, LL, P, P, LL, LL, I, I, F, LL, P, c_ulonglong, P, P],
     "rpeg_tp_allgather_cols": [P, P, I, I, LL, I, I, I, LL, P, c_ulonglong, P, P],

@@ -548,12 +548,19 @@ def decode_scratch_numel(B: int, H: int, nsplit: int) -> int:
 ALIASED = "aliased"
 
 
-def packed_decode_splits(B: int, n_heads: int, n_kv_heads: int, pages: int) -> int:
-    """Splits of the kernel for aliased rows: three CTAs an SM, twice as many where rows of one query head a KV head may be long (their last wave
-    weighs more: 64 rows of 1000 to 2000 keys 311 us whole, 245 in three; 256 rows of 512 + 30 keys 79 whole, 92 in two; 48 rows of 400 to 1000
-    keys, 32 heads, 8 KV heads 31.0 in two, 36.2 in four)."""
-    ctas = -(-B // (8 * n_kv_heads // n_heads)) * n_kv_heads
-    return max(1, min(8, 444 // ctas, pages // 2)) if pages < 24 or n_heads > n_kv_heads else max(2, min(8, 888 // ctas))
+def packed_decode_splits(B: int, n_heads: int, n_kv_heads: int, pages: int) -> tuple[int, int]:
+    """``(splits, whole)`` of the kernel for aliased rows: three CTAs an SM take the items (eight columns of a KV head), and items that are few are split among
+    them. Rows of one query head a KV head that may be long are split twice as finely (their last wave weighs more: 64 rows of 1000 to 2000 keys 311 us
+    whole, 245 in three; but 48 rows of 400 to 1000 keys, 32 heads, 8 KV heads 31.0 in two, 36.2 in four). Behind a full wave or more, the items of
+    a last one that is at most half full go in two, unless rows are short (256 rows of 512 shared and 48 own keys, 32 heads, 2.3 waves: 79.5 us all
+    ``whole``, 74.2 so, 81.0 in three, 90.8 all in two; 128 rows up to 300 keys, 8 KV heads 31.9 and 29.3, up to 100 keys 16.5 and 16.9; 1.7 waves 37.6 and 43.2)."""
+    items, slots = -(-B // (8 * n_kv_heads // n_heads)) * n_kv_heads, 444
+    last = items % slots or slots
+    if items > slots and 2 * last <= slots and pages >= 5:
+        return 2, (items - last) // 2 * 2
+    if pages >= 24 and n_heads == n_kv_heads:
+        return max(2, min(8, 2 * slots // items)), 0
+    return max(1, min(8, slots // items, pages // 2)), 0
 
 
 #: From this many (row, head) pairs on, the kernel for aliased rows is the faster one for four or eight query heads a KV head, pages shared or not: it
@@ -591,10 +598,10 @@ def paged_decode_attn(q, q_col0, kcache, vcache, page_table, seq_lens, n_heads, 
         groups = None
         aligned = (q.data_ptr() | kcache.data_ptr() | vcache.data_ptr() | out.data_ptr()) % 16 == 0 and (q.stride(0) | q_col0) % 8 == 0
         if 8 % (n_heads // n_kv_heads) == 0 and aligned and B <= 8192 and page_table.shape[1] <= 1 << 18:
-            nsplit = packed_decode_splits(B, n_heads, n_kv_heads, page_table.shape[1])
+            nsplit, whole = packed_decode_splits(B, n_heads, n_kv_heads, page_table.shape[1])
             check(lib().rpeg_paged_decode_attn_packed(q.data_ptr(), q.stride(0), q_col0, kcache.data_ptr(), vcache.data_ptr(),
                                                       page_table.data_ptr(), page_table.stride(0), seq_lens.data_ptr(), None, None, 0, None, out.data_ptr(),
-                                                      B, n_heads, n_kv_heads, head_dim, nsplit, scale, _stream()), "rpeg_paged_decode_attn_packed")
+                                                      B, n_heads, n_kv_heads, head_dim, nsplit, whole, scale, _stream()), "rpeg_paged_decode_attn_packed")
             return out
     if groups is not None:
         group_rows, group_shared, row_key0 = groups
@@ -826,7 +833,7 @@ def rows_attn(q: torch.Tensor, kcache, vcache, page_table, slot, pos, n_heads: i
         pages = min(page_table.shape[1], window // KV_PAGE) if window else page_table.shape[1]
         check(lib().rpeg_paged_decode_attn_packed(q.data_ptr(), q.stride(0), 0, kcache.data_ptr(), vcache.data_ptr(), page_table.data_ptr(),
                                                   page_table.stride(0), _ptr(lens), pos.data_ptr(), slot.data_ptr(), window, _ptr(sink), out.data_ptr(),
-                                                  rows, n_heads, n_kv, dp, packed_decode_splits(rows, n_heads, n_kv, pages), scale, _stream()),
+                                                  rows, n_heads, n_kv, dp, *packed_decode_splits(rows, n_heads, n_kv, pages), scale, _stream()),
               "rpeg_paged_decode_attn_packed")
         return out
     check(lib().rpeg_rows_attn(q.data_ptr(), q.stride(0), kcache.data_ptr(), vcache.data_ptr(), page_table.data_ptr(), page_table.stride(0),

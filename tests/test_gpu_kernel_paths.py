@@ -318,7 +318,7 @@ def test_sample_rows(cuda_device, dtype, rows, vocab, shift):
 
 # 11 rows: groups that share one, two or 33 pages (a second listing of 32), a row of its own, an empty one; eight columns of 8, 4, 2 and 1 rows
 @pytest.mark.parametrize("h,hkv", [(3, 3), (4, 2), (8, 2), (8, 1)])
-@pytest.mark.parametrize("split", [1, 3, 8])
+@pytest.mark.parametrize("split", [(1, 0), (3, 0), (8, 0), (1, 1), (2, 2)])
 def test_paged_decode_attn_aliased_rows(cuda_device, monkeypatch, h, hkv, split):
     hd, dev = 128, cuda_device
     monkeypatch.setattr(K, "packed_decode_splits", lambda *a: split)
@@ -474,7 +474,7 @@ def test_rope_append_partials_normalises_heads(cuda_device, rows, splits, h, hkv
 
 
 # eight columns of two rows and of one; the last group of rows is not full; whole and in splits; room for long rows
-@pytest.mark.parametrize("rows,h,hkv,pages", [(193, 8, 2, 3), (49, 32, 8, 6), (48, 32, 4, 30)])
+@pytest.mark.parametrize("rows,h,hkv,pages", [(193, 8, 2, 3), (49, 32, 8, 6), (48, 32, 4, 30), (112, 32, 8, 6)])
 def test_paged_decode_attn_many_rows(cuda_device, rows, h, hkv, pages):
     hd, dev = 128, cuda_device
     assert rows * h >= K.PACKED_MIN_HEADS
@@ -528,7 +528,7 @@ def test_expert_rows_of_prompts(cuda_device, dtype, rows, d, top, shared):
 
 
 # the tensor-core kernel for a served decoder's rows: windows of one and two pages and none, a sink, rows of one prompt, lengths or positions, splits
-@pytest.mark.parametrize("window,sink,split", [(0, False, 1), (64, True, 1), (128, False, 3), (0, True, 8)])
+@pytest.mark.parametrize("window,sink,split", [(0, False, (1, 0)), (64, True, (1, 0)), (128, False, (3, 0)), (0, True, (8, 0)), (64, False, (2, 2))])
 @pytest.mark.parametrize("h,hkv", [(4, 1), (16, 2)])
 def test_rows_attn_grouped_heads(cuda_device, monkeypatch, h, hkv, window, sink, split):
     hd, dev = 128, cuda_device
@@ -544,7 +544,7 @@ def test_rows_attn_grouped_heads(cuda_device, monkeypatch, h, hkv, window, sink,
     kw = dict(window=window, scale=0.11, sink=sk)
     got = K.rows_attn(q, k, v, table, slot, n - 1, h, lens=n, **kw)
     by_pos = K.rows_attn(q[2:], k, v, table, slot[2:], n[2:] - 1, h, **kw)
-    assert split > 1 or torch.equal(by_pos, got[2:])
+    assert split[0] > 1 or torch.equal(by_pos, got[2:])
     for i, l in enumerate(lens):
         lo = (l - 1) // window * window if window and l else 0
         kk, vv = (t[table[slot[i]].long()].transpose(0, 1).reshape(hkv, -1, hd)[:, lo:l].double().repeat_interleave(h // hkv, 0) for t in (k, v))
