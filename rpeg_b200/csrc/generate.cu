@@ -41,8 +41,8 @@ __global__ void decode_advance_kernel(const int* __restrict__ sampled, const flo
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s == 0 && step_counter != nullptr) step_counter[0] += 1;
   if (s >= n_slots || !active[s]) return;
-  advance_row(DecodeState{nullptr, token, pos, seq_len, active, gen_count, out_tok, out_lp, max_new, eos, n_finished, nullptr, nullptr}, s, sampled[s],
-              sampled_lp[s]);
+  const DecodeState st{nullptr, token, pos, seq_len, active, gen_count, out_tok, out_lp, max_new, eos, n_finished, nullptr, nullptr};
+  advance_row(st, row_state(st, s), s, sampled[s], sampled_lp[s]);
 }
 
 // out[i, :] = x[rows[i], :]   (bf16 rows, 16-byte vectors)

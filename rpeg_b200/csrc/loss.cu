@@ -9,7 +9,7 @@
 // RPEG/runtime/ppo_math.py:14-92, the loss tuples are megatron_worker.py:4264-4274 (DPO),
 // :4361-4387 (GRPO), :4388-4417 (PPO actor), :4650 (critic), group advantages :4418, and the
 // sampler is megatron_worker.py:83-123.
-#include "common.cuh"
+#include "pair.cuh"
 #include "decode_state.cuh"
 #include "rpeg_kernels.h"
 
@@ -386,6 +386,9 @@ __device__ __forceinline__ float logit_at(const float* p) { return *p; }
 
 // One CTA per row; a decode step waits for it. Eight logits a turn: their maximum first, so that their exponentials do not wait for one
 // another (one at a time in 256 threads: 32000 bf16 logits 8.2 us greedy and 18.6 us with noise, now 4.9 and 9.8; 256 rows 54 us with noise, now 20).
+// `parts` CTAs a row, a cluster: where rows are few, one SM's loads and exponentials are what the step waits for. Each takes every parts-th turn, the
+// first one merges (bf16 logits in a decode step, in one and so: one row of 32000 6.8 and 6.3 us greedy, 12.1 and 8.9 with noise; 16 rows of 151936
+// 16.5 and 9.1, 41.0 and 15.4).
 // THREADS: 1024, or 256 below 8192 logits, which are at most four turns of them (256 rows of 1000: 4.9 us with 1024, 3.1 with 256).
 // STEP: the bookkeeping of a decode step around the choice (generate.cu: the forced token before it, the row's state behind it), which were launches of
 // their own; the last CTA advances the step counter, which is the others' noise.
@@ -393,21 +396,26 @@ template <typename T, int THREADS, bool STEP>
 __global__ void __launch_bounds__(THREADS)
 sample_kernel(const T* __restrict__ logits, int V, int ld, float inv_temp, int greedy,
               unsigned long long seed, const unsigned long long* seed_offset,
-              const int* __restrict__ forced, int* __restrict__ token_out, float* __restrict__ logp_out, const DecodeState st) {
+              const int* __restrict__ forced, int* __restrict__ token_out, float* __restrict__ logp_out, const DecodeState st, int parts) {
   griddep_launch();
   griddep_wait();   // may have been scheduled under the previous kernel's tail: nothing is read or written before this
-  __shared__ float sm_m[32], sm_s[32], sm_best[32];
+  __shared__ float sm_m[32], sm_s[32], sm_best[32], sm_x[32];
   __shared__ int sm_idx[32];
-  const int row = blockIdx.x;
+  __shared__ __align__(16) float4 part_sums;           // maximum, sum, best key, its logit
+  __shared__ int part_idx;
+  const int row = blockIdx.x / parts, rank = blockIdx.x - row * parts;
+  RowState before{};
+  if constexpr (STEP)
+    if (threadIdx.x == 0 && rank == 0) before = row_state(st, row);
   // a device-resident offset (e.g. a step counter) keeps replays of a captured graph from reusing noise
   if (seed_offset != nullptr) seed += seed_offset[0] * 0xD1B54A32D192ED03ull;
   const T* lr = logits + static_cast<size_t>(row) * ld;
-  float m = -INFINITY, s = 0.f, best = -INFINITY;
-  int best_i = 0;
+  float m = -INFINITY, s = 0.f, best = -INFINITY, best_x = 0.f;
+  int best_i = rank == 0 ? 0 : 0x7fffffff;
   auto pick = [&](int i, float x) {
     float key = x;
     if (!greedy) key += -__logf(-__logf(hash_uniform(seed, row, i)));
-    if (key > best || (key == best && i < best_i)) { best = key; best_i = i; }
+    if (key > best || (key == best && i < best_i)) { best = key; best_i = i; best_x = x; }
   };
   auto take = [&](int i, float raw) {
     const float x = raw * inv_temp;
@@ -437,7 +445,7 @@ sample_kernel(const T* __restrict__ logits, int V, int ld, float inv_temp, int g
     const uint4* lv = reinterpret_cast<const uint4*>(lr);
     const int nvec = V >> 3;
 #pragma unroll 2
-    for (int j = threadIdx.x; j < nvec; j += THREADS) {
+    for (int j = rank * THREADS + threadIdx.x; j < nvec; j += THREADS * parts) {
       float x[8];
       if constexpr (PER == 8) {
         const uint4 a = lv[j];
@@ -456,43 +464,67 @@ sample_kernel(const T* __restrict__ logits, int V, int ld, float inv_temp, int g
       }
       take8(j * 8, x);
     }
-    for (int i = (nvec << 3) + threadIdx.x; i < V; i += THREADS) take(i, logit_at(lr + i));
+    for (int i = (nvec << 3) + rank * THREADS + threadIdx.x; i < V; i += THREADS * parts) take(i, logit_at(lr + i));
   } else {
-    for (int i = threadIdx.x; i < V; i += THREADS) take(i, logit_at(lr + i));
+    for (int i = rank * THREADS + threadIdx.x; i < V; i += THREADS * parts) take(i, logit_at(lr + i));
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto better = [&](float b2, int i2, float x2) {
+    if (b2 > best || (b2 == best && i2 < best_i)) { best = b2; best_i = i2; best_x = x2; }
+  };
   auto best_of_warp = [&]() {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-      const float b2 = __shfl_xor_sync(0xffffffffu, best, o);
-      const int i2 = __shfl_xor_sync(0xffffffffu, best_i, o);
-      if (b2 > best || (b2 == best && i2 < best_i)) { best = b2; best_i = i2; }
+      const float b2 = __shfl_xor_sync(0xffffffffu, best, o), x2 = __shfl_xor_sync(0xffffffffu, best_x, o);
+      better(b2, __shfl_xor_sync(0xffffffffu, best_i, o), x2);
     }
   };
   best_of_warp();
-  if (lane == 0) { sm_best[warp] = best; sm_idx[warp] = best_i; }
+  if (lane == 0) { sm_best[warp] = best; sm_idx[warp] = best_i; sm_x[warp] = best_x; }
   block_lse(m, s, sm_m, sm_s);  // contains __syncthreads
   if (warp == 0) {
     best = lane < THREADS / 32 ? sm_best[lane] : -INFINITY;
     best_i = lane < THREADS / 32 ? sm_idx[lane] : 0x7fffffff;
+    best_x = lane < THREADS / 32 ? sm_x[lane] : 0.f;
     best_of_warp();
     if (lane == 0) {
-      if constexpr (STEP) {
-        best_i = forced_token(st, row, best_i);
-      } else {
-        if (forced != nullptr && forced[row] >= 0) best_i = forced[row];
+      part_sums = make_float4(m, s, best, best_x);
+      part_idx = best_i;
+    }
+  }
+  if (parts > 1) {
+    __syncwarp();
+    cluster_sync_all();
+    if (rank == 0 && threadIdx.x == 0)
+      for (int r = 1; r < parts; ++r) {
+        float4 o;
+        int oi;
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w) : "r"(cluster_addr(&part_sums, r)) : "memory");
+        asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(oi) : "r"(cluster_addr(&part_idx, r)) : "memory");
+        online_merge(m, s, o.x, o.y);
+        better(o.z, oi, o.w);
       }
-      const float lp = logit_at(lr + best_i) * inv_temp - (m + __logf(s));
-      token_out[row] = best_i;
-      logp_out[row] = lp;
-      if constexpr (STEP) {
-        advance_row(st, row, best_i, lp);
-        __threadfence();
-        if (atomicAdd(st.arrived, 1) == static_cast<int>(gridDim.x) - 1) {
-          *st.arrived = 0;
-          *st.step_counter += 1;
-        }
-      }
+    __syncwarp();
+    cluster_sync_all();                                // nobody's shared memory goes while it is read
+    if (rank != 0) return;
+  }
+  if (threadIdx.x != 0) return;
+  const int chosen = best_i;
+  if constexpr (STEP) {
+    best_i = forced_token(st, before, best_i);
+  } else {
+    if (forced != nullptr && forced[row] >= 0) best_i = forced[row];
+  }
+  const float x = best_i == chosen && best > -INFINITY ? best_x : logit_at(lr + best_i) * inv_temp;
+  const float lp = x - (m + __logf(s));
+  token_out[row] = best_i;
+  logp_out[row] = lp;
+  if constexpr (STEP) {
+    advance_row(st, before, row, best_i, lp);
+    __threadfence();
+    if (atomicAdd(st.arrived, 1) == static_cast<int>(gridDim.x) / parts - 1) {
+      *st.arrived = 0;
+      *st.step_counter += 1;
     }
   }
 }
@@ -712,22 +744,39 @@ extern "C" int rpeg_group_advantage(const float* rewards, float* out, int G, int
   group_advantage_kernel<<<(G + 63) / 64, 64, 0, STREAM(stream)>>>(rewards, out, G, K);
   return LAUNCH_OK();
 }
+template <typename T, bool STEP>
+static int launch_sample_rows(const void* logits, int B, int V, int ld, float temperature, int greedy, unsigned long long seed,
+                              const unsigned long long* seed_offset, const int* forced, int* token_out, float* logp_out, const DecodeState& st,
+                              void* stream) {
+  const bool few = V < 8192;
+  // CTAs of a row: while a turn is left for each, and they fit an SM each beside what parts of the chip cannot take a cluster (151936 logits, greedy:
+  // 16 rows 16.5 us in one, 13.1 in eight; 32 rows 17.2 and 19.1 in four; 64 rows 17.3 and 16.6 in two; 74 rows 17.4 and 23.0 in two)
+  int parts = 1;
+  while (!few && parts < 8 && static_cast<long long>(B) * parts * 2 <= (parts == 1 ? 128 : 64) && V >= parts * 2 * 1024 * 8) parts *= 2;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim = {static_cast<unsigned>(parts), 1, 1};
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(B) * parts);
+  cfg.blockDim = dim3(few ? 256 : 1024);
+  cfg.stream = STREAM(stream);
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, few ? sample_kernel<T, 256, STEP> : sample_kernel<T, 1024, STEP>, static_cast<const T*>(logits), V, ld,
+                            1.f / temperature, greedy, seed, seed_offset, forced, token_out, logp_out, st, parts) == cudaSuccess ? 0 : -21;
+}
 template <typename T>
 static int launch_sample(const void* logits, int B, int V, int ld, float temperature, int greedy, unsigned long long seed,
                          const unsigned long long* seed_offset, const int* forced, int* token_out, float* logp_out, void* stream) {
   if (B <= 0) return 0;
-  const bool few = V < 8192;
-  launch_pdl(few ? sample_kernel<T, 256, false> : sample_kernel<T, 1024, false>, dim3(B), dim3(few ? 256 : 1024), 0, STREAM(stream), static_cast<const T*>(logits), V, ld,
-             1.f / temperature, greedy, seed, seed_offset, forced, token_out, logp_out, DecodeState{});
-  return LAUNCH_OK();
+  return launch_sample_rows<T, false>(logits, B, V, ld, temperature, greedy, seed, seed_offset, forced, token_out, logp_out, DecodeState{}, stream);
 }
 template <typename T>
 static int launch_sample_step(const void* logits, int B, int V, int ld, float temperature, int greedy, unsigned long long seed, int* token_out,
                               float* logp_out, const DecodeState& st, void* stream) {
-  const bool few = V < 8192;
-  launch_pdl(few ? sample_kernel<T, 256, true> : sample_kernel<T, 1024, true>, dim3(B), dim3(few ? 256 : 1024), 0, STREAM(stream), static_cast<const T*>(logits), V, ld,
-             1.f / temperature, greedy, seed, st.step_counter, nullptr, token_out, logp_out, st);
-  return LAUNCH_OK();
+  return launch_sample_rows<T, true>(logits, B, V, ld, temperature, greedy, seed, st.step_counter, nullptr, token_out, logp_out, st, stream);
 }
 template <typename T>
 static int launch_sample_filtered(const void* logits, int B, int V, int ld, float temperature, int top_k, float top_p,

@@ -396,7 +396,7 @@ def test_moe_gemm_few_rows(cuda_device, t, e, top, shared, n, k, act):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("rows,vocab", [(1, 1003), (5, 8192), (37, 640)])
+@pytest.mark.parametrize("rows,vocab", [(1, 1003), (5, 8192), (37, 640), (3, 40000), (9, 70000)])
 @pytest.mark.parametrize("greedy", [True, False])
 def test_sample_step_is_prepare_sample_advance(cuda_device, dtype, rows, vocab, greedy):
     dev, g = cuda_device, torch.Generator(device=cuda_device).manual_seed(rows)
@@ -553,3 +553,9 @@ def test_rows_attn_grouped_heads(cuda_device, monkeypatch, h, hkv, window, sink,
         want = torch.einsum("hk,hkd->hd", w, vv).reshape(-1)
         assert bool((got[i] == 0).all()) if l == 0 else _rel(got[i], want) < 2 ** -8
         assert i < 2 or _rel(by_pos[i - 2], want) < 2 ** -8
+
+
+# rows of two, four and eight CTAs, with a tail of less than eight logits, unaligned, and one CTA more than the rule for two allows
+@pytest.mark.parametrize("rows,vocab,shift", [(64, 16384, 0), (65, 16387, 0), (16, 32771, 1), (8, 65541, 0), (2, 65536, 3)])
+def test_sample_rows_in_parts(cuda_device, rows, vocab, shift):
+    test_sample_rows(cuda_device, torch.bfloat16, rows, vocab, shift)
