@@ -148,11 +148,12 @@ extern "C" int rpeg_splitk_reduce(const float* part, void* out, int M, int N, in
 
 // Switch programmatic dependent launches on or off for the kernels launched from now on (a CUDA graph keeps what was
 // in force while it was captured). The environment's RPEG_PDL=0 wins. 2: what follows on this thread is a chain whose first kernel waits before it
-// lets others start (see pdl_chain()).
-extern "C" void rpeg_set_pdl(int on) {
-  pdl_enabled();
+// lets others start (see pdl_chain()). Returns what was in force.
+extern "C" int rpeg_set_pdl(int on) {
+  const int was = pdl_enabled();
   pdl_chain() = on == 2;
   int& v = pdl_state();
   if (v != 2) v = on ? 1 : 0;
+  return was;
 }
 

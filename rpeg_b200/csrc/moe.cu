@@ -443,9 +443,10 @@ extern "C" int rpeg_moe_dispatch(const void* x, int dp, const int* ids, const in
 
 // A [a_rows_total, K]: routed rows (and the always-on ones unless X is given); X [seg_rows, K] or null; B [(n_routed +
 // n_shared) * N, K] (2 N rows per segment for FF_SWIGLU); C rows as A's segments. `choices` = routed rows in total (seg_rows * top), for the grid size.
+// `spare`: SMs that a product of few rows leaves to kernels of another stream.
 extern "C" int rpeg_moe_gemm(const void* A, long long a_rows_total, const void* X, const void* B, void* C, const int* seg_off, int n_routed,
                              int n_shared, int seg_rows, long long choices, int N, int K, int lda, int ldx, int ldb, int ldc, int act,
-                             int bn_hint, int* status, void* stream) {
+                             int bn_hint, int spare, int* status, void* stream) {
   if (seg_rows <= 0 || N <= 0 || K <= 0) return 0;
   const int S = n_routed + n_shared;
   if (S < 1 || S > MOE_MAX_SEGMENTS) return -3;
@@ -465,8 +466,9 @@ extern "C" int rpeg_moe_gemm(const void* A, long long a_rows_total, const void* 
   int bn = bn_hint;
   if (bn == 0 && seg_rows <= (act == FF_SWIGLU ? 128 : 64) && (act != FF_SWIGLU || (N & 15) == 0)) {
     const long long items = (active + n_shared) * (act == FF_SWIGLU ? (N + 63) / 64 : (N + 127) / 128);
+    const int sms = spare > 0 && spare < num_sms ? num_sms - spare : num_sms;
     return skinny_experts(A, a_rows_total, X, B, C, seg_off, n_routed, n_shared, seg_rows, N, K, lda, ldx, ldb, ldc, act,
-                          static_cast<int>(items < num_sms ? items : num_sms), status, STREAM(stream));
+                          static_cast<int>(items < sms ? items : sms), status, STREAM(stream));
   }
   if (bn == 0) {
     // Prompts: pairs of CTAs with tiles as high as a segment's rows ask for (moe_pair.cu), once experts have about 160 rows and there are six

@@ -105,7 +105,7 @@ int rpeg_scatter_rows_by_index(const void* src, long long n, long long row_bytes
 // Version words of pushed data: release-store `version` into word `word` of every destination flag array after
 // the copies queued before it; poll flags[0..n) >= min_version with a bound (result[0] = 1 reached, 0 not yet).
 // Programmatic dependent launches on/off for subsequent launches (graphs keep the setting of their capture).
-void rpeg_set_pdl(int on);
+int rpeg_set_pdl(int on);
 int rpeg_publish_version(void* const* flag_arrays, int n_dst, int word, unsigned version, void* stream);
 int rpeg_wait_flags(const unsigned* flags, int n, unsigned min_version, unsigned long long timeout_ns, int* result,
                     void* stream);
@@ -204,7 +204,7 @@ int rpeg_moe_dispatch(const void* x, int dp, const int* ids, const int* ticket, 
                       int top, void* xs, int* row_of, int* seg_off, int f32, void* stream);
 int rpeg_moe_gemm(const void* A, long long a_rows_total, const void* X, const void* B, void* C, const int* seg_off, int n_routed,
                   int n_shared, int seg_rows, long long choices, int N, int K, int lda, int ldx, int ldb, int ldc, int act,
-                  int bn_hint, int* status, void* stream);
+                  int bn_hint, int spare, int* status, void* stream);
 
 // ---- gemm_f32.cu: fp32 matrix products on the CUDA cores
 int rpeg_gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, int lda, int ldb, int ldc, void* stream);

@@ -24,6 +24,7 @@ This family is served (generation, log-probs); it has no backward pass here.
 """
 from __future__ import annotations
 
+import contextlib
 import math
 from dataclasses import dataclass
 from typing import Dict, Iterable, List, Optional, Tuple, Union
@@ -235,6 +236,11 @@ class ZafopelModel(ServedDecoder):
     """Weights and kernels of one model on one GPU."""
 
     prefill_spans = True
+    # Up to this many rows the two branches of a decode step's layer run side by side (4 layers, 32 tokens after 300 to 600: 1 row 15.1 -> 12.7 ms, 8 rows 29.3
+    # -> 26.9, 16 rows 35.9 -> 33.5, 64 rows 54.6 -> 52.9; 96 rows and more level), and the experts leave that many SMs to the attention (8 rows: 27.9 ms with
+    # none, 27.5 with 12, 27.0 with 20, 27.4 with 32, 28.2 with 44).
+    SPARE_SMS = 20
+    SIDE_MAX_ROWS = 64
     KERNEL_SOURCES = ("gemm.cu", "gemm_pair.cu", "gemm_skinny.cu", "generate.cu", "loss.cu", "stream_update.cu", "latent.cu", "latent_decode.cu", "latent_prefill.cu", "head_gemm.cu",
                       "moe.cu", "moe_pair.cu", "gemm_f32.cu")
 
@@ -246,6 +252,7 @@ class ZafopelModel(ServedDecoder):
         self.alpha = torch.ones(cfg.n_layers + 1, **f32)           # per layer, then the last norm's
         self.max_experts = max([l.mlp.experts for l in cfg.layers if isinstance(l.mlp, InputScaledMixture)], default=1)
         self._split: Dict[Tuple[int, int], torch.Tensor] = {}
+        self._side: Optional[torch.cuda.Stream] = None
         if seed is not None:
             self.init_weights(seed)
 
@@ -404,19 +411,24 @@ class ZafopelModel(ServedDecoder):
         out = torch.empty((T, m.heads, m.vdim_p), **bf)
         return K.head_gemm(avg, uv, out).view(T, -1)
 
-    def _feed_forward(self, i: int, h: torch.Tensor, first, counts: torch.Tensor, decode: bool):
+    def _feed_forward(self, i: int, h: torch.Tensor, first, counts: torch.Tensor, decode: bool, held: Optional[list] = None):
         """What the feed-forward adds to the stream, as a source of ``stream_update``. ``first``: a mixture's router logits, or a dense one's
-        activation (None: not computed yet)."""
+        activation (None: not computed yet). ``held``: gets what a mixture's kernels, launched on a stream that has just waited for another one's event, work
+        on; they leave some SMs to that one."""
         p, e = self.p, self.cfg.layers[i].mlp
         if e is None:
             return None
         if isinstance(e, DenseFF):
             act = K.ff_first(h, self._ff_rows(i), "relu2") if first is None else first
             return self._lin(act, p[f"l{i}.w_down"], decode, ws=1)
-        ids, wts, ticket = K.moe_route(first, e.experts, e.top, counts, sigmoid=True)
+        with contextlib.nullcontext() if held is None else K.plain_order():
+            ids, wts, ticket = K.moe_route(first, e.experts, e.top, counts, sigmoid=True)
+        spare = 0 if held is None else self.SPARE_SMS
         r = K.moe_dispatch(h, ids, wts, ticket, counts, e.experts, weigh_inputs=True)
-        act = K.moe_gemm(r.x_sorted, p[f"l{i}.w_gate_up"], r, e.experts, 0, act="swiglu")
-        return K.MoEOutput(K.moe_gemm(act, p[f"l{i}.w_down"], r, e.experts, 0), r.row_of, r.weights, 0)
+        act = K.moe_gemm(r.x_sorted, p[f"l{i}.w_gate_up"], r, e.experts, 0, act="swiglu", spare=spare)
+        if held is not None:
+            held += [h, first, wts, ticket, r, act]
+        return K.MoEOutput(K.moe_gemm(act, p[f"l{i}.w_down"], r, e.experts, 0, spare=spare), r.row_of, r.weights, 0)
 
     def _run(self, tokens, pos, slot, page_table, kcache, decode: bool, form, attend, trace=None) -> torch.Tensor:
         """All layers on ``T`` tokens. ``form(layer)`` gives the way of a layer's attention. Returns the hidden rows the logits are taken from,
@@ -447,10 +459,25 @@ class ZafopelModel(ServedDecoder):
                 if isinstance(e, InputScaledMixture):
                     first = self._lin(h, w_in[n_attn:], False, f32_out=True)
             own = i if m.kv_from is None else m.kv_from
-            o = self._attention(i, h, proj, pos, slot, page_table, kcache[own], decode, form(i, m) if form else None, attend, ff_act)
-            ff = self._feed_forward(i, h, first, counts[i], decode)
-            o = self._lin(o, p[f"l{i}.wo"], decode)
-            h = update(o, ff, i + 1)
+            cache, formed = kcache[own], form(i, m) if form else None
+            if decode and isinstance(e, InputScaledMixture) and T <= self.SIDE_MAX_ROWS:
+                # The two branches of a decode step's layer run side by side: the experts stream their weights on all SMs but a few, on which the chain of
+                # small kernels of the attention is through before they are. `held`: nothing of theirs is given back before this stream has waited.
+                side, here, held = self._side_stream(), torch.cuda.current_stream(self.device), []
+                side.wait_event(here.record_event())
+                with K.launching_on(side):
+                    ff = self._feed_forward(i, h, first, counts[i], True, held)
+                    through = side.record_event()
+                o = self._attention(i, h, proj, pos, slot, page_table, cache, True, formed, attend, ff_act)
+                o = self._lin(o, p[f"l{i}.wo"], True, ws=1)           # the router may still be reading the other workspace
+                here.wait_event(through)
+                with K.plain_order():
+                    h = update(o, ff, i + 1)
+            else:
+                o = self._attention(i, h, proj, pos, slot, page_table, cache, decode, formed, attend, ff_act)
+                ff = self._feed_forward(i, h, first, counts[i], decode)
+                o = self._lin(o, p[f"l{i}.wo"], decode)
+                h = update(o, ff, i + 1)
             if trace is not None:
                 trace.append(x[:, : cfg.width].clone())
         return h
@@ -479,6 +506,12 @@ class ZafopelModel(ServedDecoder):
         if not self.f32 and m.scale > 0 and K.latent_decode_fits(m.rank_p, m.row_width):
             return K.latent_decode(q, cache, m.rank_p, page_table, slot, pos, nsplit=nsplit, scratch=scratch, **kw)
         return K.latent_attn_rows(q, cache, m.rank_p, page_table, slot, pos, **kw)
+
+    def _side_stream(self) -> torch.cuda.Stream:
+        """The stream of a decode step's experts; like the workspaces, it is for one step at a time."""
+        if self._side is None:
+            self._side = torch.cuda.Stream(device=self.device)
+        return self._side
 
     def _nsplit(self, m: LatentMixer, rows: int, table_pages: int) -> int:
         """Splits of a decode row's pages: the fewest page times over all waves of CTAs, where a CTA costs about four pages on

@@ -93,7 +93,7 @@ _SIGNATURES = {
     "rpeg_window_prefill": [P, I, P, P, LL, P, I, P, P, P, P, P, I, I, I, I, I, I, I, I, F, P, P],
     "rpeg_moe_route": [P, I, LL, I, I, I, I, I, I, I, I, P, P, P, P, P],
     "rpeg_moe_dispatch": [P, I, P, P, P, P, I, I, I, P, P, P, I, P],
-    "rpeg_moe_gemm": [P, LL, P, P, P, P, I, I, I, LL, I, I, I, I, I, I, I, I, P, P],
+    "rpeg_moe_gemm": [P, LL, P, P, P, P, I, I, I, LL, I, I, I, I, I, I, I, I, I, P, P],
     "rpeg_moe_gemm_f32": [P, P, P, P, P, I, I, I, I, I, I, I, I, I, P],
     "rpeg_gemm_f32": [P, P, P, I, I, I, I, I, I, P],
     "rpeg_gemm_f32_batched": [P, P, P, I, I, I, I, I, I, LL, LL, LL, I, I, P],

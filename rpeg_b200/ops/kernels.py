@@ -9,7 +9,9 @@ validate the index VALUES held by tensor arguments before the launch (``ops/chec
 from __future__ import annotations
 
 import ctypes
+import contextlib
 import math
+import threading
 
 import torch
 
@@ -25,8 +27,23 @@ class KernelWaitTimeout(RuntimeError):
     """A bounded device-side wait (mbarrier or peer flag) ran out; the kernel returned early."""
 
 
+_launch = threading.local()
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    other = getattr(_launch, "stream", None)
+    return (torch.cuda.current_stream() if other is None else other).cuda_stream
+
+
+@contextlib.contextmanager
+def launching_on(stream: torch.cuda.Stream):
+    """Calls of this thread inside launch on ``stream`` but allocate on the current one: keep what they return and what it was made from until the current
+    stream has waited for ``stream``, and nothing more needs to be told to the allocator."""
+    was, _launch.stream = getattr(_launch, "stream", None), stream
+    try:
+        yield
+    finally:
+        _launch.stream = was
 
 
 def _ptr(t: torch.Tensor | None) -> int | None:
@@ -142,6 +159,17 @@ def set_pdl(on: bool, chain: bool = False) -> None:
     """Programmatic dependent launches for the kernels launched from now on (a captured graph keeps its setting). ``chain``: what this thread launches
     next is a decode step, whose products may request weights before the kernel in front of them is through."""
     lib().rpeg_set_pdl(2 if on and chain else int(bool(on)))
+
+
+@contextlib.contextmanager
+def plain_order():
+    """Launches inside start when everything that they depend on is through: a kernel whose stream has just waited for an event of another one is not a
+    programmatic dependent."""
+    was = lib().rpeg_set_pdl(0)
+    try:
+        yield
+    finally:
+        lib().rpeg_set_pdl(was)
 
 
 def publish_version(flag_ptrs, word: int, version: int) -> None:
@@ -914,9 +942,10 @@ FF_ACTS = {"none": 0, "gelu": 1, "swiglu": 2, "relu2": 3}
 
 
 def moe_gemm(a: torch.Tensor, b: torch.Tensor, r: MoERouting, n_experts: int, n_shared: int, *, shared_x: torch.Tensor | None = None,
-             act: str = "none", bn: int = 0) -> torch.Tensor:
+             act: str = "none", bn: int = 0, spare: int = 0) -> torch.Tensor:
     """``C[rows of segment s] = act(a[rows of s] @ b[s].T)`` over the experts' segments; ``b [E + n_shared, N, K]``. ``act``: none, gelu,
-    relu2 (squared relu) or swiglu (``b [E + n_shared, 2 N, K]``, gate rows first: ``silu(gate) * up``). The always-on segments take their rows from ``shared_x [T, K]`` (tokens in order) or, without it, from ``a`` behind the routed rows."""
+    relu2 (squared relu) or swiglu (``b [E + n_shared, 2 N, K]``, gate rows first: ``silu(gate) * up``). The always-on segments take their rows from ``shared_x [T, K]`` (tokens in order) or, without it, from ``a`` behind the routed rows.
+    ``spare``: SMs that a product of few rows leaves to what another stream launches beside it."""
     T, top = r.row_of.shape
     S, N, Kd = b.shape
     code = FF_ACTS[act]
@@ -935,7 +964,7 @@ def moe_gemm(a: torch.Tensor, b: torch.Tensor, r: MoERouting, n_experts: int, n_
         return c
     _req(a, torch.bfloat16, "a")
     check(lib().rpeg_moe_gemm(a.data_ptr(), a.shape[0], _ptr(shared_x), b.data_ptr(), c.data_ptr(), r.seg_off.data_ptr(), n_experts, n_shared, T,
-                              T * top, N, Kd, a.stride(0), 0 if shared_x is None else shared_x.stride(0), Kd, c.stride(0), code, bn,
+                              T * top, N, Kd, a.stride(0), 0 if shared_x is None else shared_x.stride(0), Kd, c.stride(0), code, bn, spare,
                               status_word(a.device).data_ptr(), _stream()), "rpeg_moe_gemm")
     return c
 

@@ -559,3 +559,23 @@ def test_rows_attn_grouped_heads(cuda_device, monkeypatch, h, hkv, window, sink,
 @pytest.mark.parametrize("rows,vocab,shift", [(64, 16384, 0), (65, 16387, 0), (16, 32771, 1), (8, 65541, 0), (2, 65536, 3)])
 def test_sample_rows_in_parts(cuda_device, rows, vocab, shift):
     test_sample_rows(cuda_device, torch.bfloat16, rows, vocab, shift)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("graphs", [True, False])
+def test_branches_of_a_step_side_by_side(cuda_device, monkeypatch, dtype, graphs):
+    """Attention and experts of a layer on two streams give what one after the other gives, bit for bit, step after step."""
+    from rpeg_b200.engine.generation import Generator
+    from rpeg_b200.models.zafopel import InputScaledMixture, LatentMixer, ParallelLayer, ZafopelConfig, ZafopelModel
+    common = dict(heads=4, dim=128, rot_dim=64, vdim=128, kv_rank=512, scale=192 ** -0.5)
+    mixers = (LatentMixer(**common, q_rank=256, sink=True), LatentMixer(**common, window=64))
+    layers = tuple(ParallelLayer(m, InputScaledMixture(16, 3, 512)) for m in mixers * 3)
+    model = ZafopelModel(ZafopelConfig(1024, 4096, layers, max_pos=512), cuda_device, dtype=dtype, seed=3)
+    prompts = [torch.randint(3, 4096, (n,), device=cuda_device, dtype=torch.int32) for n in (70, 5, 33, 1, 64, 40)]
+    out = []
+    for rows in (0, 64, 64, 64):
+        monkeypatch.setattr(ZafopelModel, "SIDE_MAX_ROWS", rows)
+        gen = Generator(model, max_slots=6, max_seq_len=128, kv_budget_bytes=1e9, eos_id=1, use_graphs=graphs)
+        out.append(gen.generate(prompts, 40, greedy=True))
+    for r in out[1:]:
+        assert torch.equal(r.tokens, out[0].tokens) and torch.equal(r.logprobs, out[0].logprobs)
