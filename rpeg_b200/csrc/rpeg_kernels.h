@@ -90,7 +90,7 @@ int rpeg_head_gemv_bwd(const void* h, const void* w, const float* dout, void* dh
 // ---- optim.cu
 int rpeg_adamw(float* p32, float* m, float* v, const float* grad, void* w16, long long n, float lr, float beta1,
                float beta2, float eps, float wd, int step, float grad_scale, const float* sumsq, int n_partials,
-               float max_norm, void* stream);
+               float max_norm, int* status, void* stream);
 int rpeg_sumsq(const float* x, long long n, float* out, void* stream);
 int rpeg_flag_barrier(void* const* pads, int rank, int world, int slot, unsigned epoch, const float* payload_in,
                       float* payload_out, unsigned long long timeout_ns, int* status, void* stream);

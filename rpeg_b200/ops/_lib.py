@@ -44,7 +44,7 @@ _SIGNATURES = {
     "rpeg_sample": [P, I, I, I, F, I, c_ulonglong, P, P, P, P, P],
     "rpeg_head_gemv": [P, P, P, P, I, I, P],
     "rpeg_head_gemv_bwd": [P, P, P, P, P, P, I, I, P],
-    "rpeg_adamw": [P, P, P, P, P, LL, F, F, F, F, F, I, F, P, I, F, P],
+    "rpeg_adamw": [P, P, P, P, P, LL, F, F, F, F, F, I, F, P, I, F, P, P],
     "rpeg_sumsq": [P, LL, P, P],
     "rpeg_flag_barrier": [P, I, I, I, c_uint, P, P, c_ulonglong, P, P],
     "rpeg_dp_reduce_norm": [P, I, LL, LL, F, P, P, P],

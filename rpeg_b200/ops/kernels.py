@@ -460,7 +460,7 @@ def adamw_(p32, m, v, grad, w16, *, lr, beta1=0.9, beta2=0.999, eps=1e-8, wd=0.0
     n = p32.numel()
     check(lib().rpeg_adamw(p32.data_ptr(), m.data_ptr(), v.data_ptr(), grad.data_ptr(), w16.data_ptr(), n, lr,
                            beta1, beta2, eps, wd, step, grad_scale, _ptr(sumsq),
-                           0 if sumsq is None else sumsq.numel(), max_norm, _stream()), "rpeg_adamw")
+                           0 if sumsq is None else sumsq.numel(), max_norm, status_word(p32.device).data_ptr(), _stream()), "rpeg_adamw")
 
 
 def sumsq(x: torch.Tensor, out: torch.Tensor) -> None:

@@ -579,3 +579,22 @@ def test_branches_of_a_step_side_by_side(cuda_device, monkeypatch, dtype, graphs
         out.append(gen.generate(prompts, 40, greedy=True))
     for r in out[1:]:
         assert torch.equal(r.tokens, out[0].tokens) and torch.equal(r.logprobs, out[0].logprobs)
+
+
+# whole tiles; a remainder; the last run of tiles not full; one word less than the rule for tiles
+@pytest.mark.parametrize("n", [148 * 4 * 4096, 148 * 4 * 4096 + 4 * 1023, 5_000_000, 148 * 4 * 4096 - 4])
+def test_adamw_tiles(cuda_device, n):
+    """Whole models go through shared memory in tiles; the copy of the weights 8 bytes off keeps the kernel for any size: bit for bit the same."""
+    g = torch.Generator(device=cuda_device).manual_seed(n)
+    p0, m0, grad = (torch.randn(n, generator=g, device=cuda_device) for _ in range(3))
+    v0 = torch.rand(n, generator=g, device=cuda_device)
+    ss = torch.full((1,), 9.0, device=cuda_device)
+    out = []
+    for shift in (0, 4):
+        p, m, v, w = p0.clone(), m0.clone(), v0.clone(), torch.empty(n + 4, device=cuda_device, dtype=torch.bfloat16)[shift:shift + n]
+        for step in (1, 2):
+            K.adamw_(p, m, v, grad, w, lr=1e-2, beta1=0.9, beta2=0.95, eps=1e-8, wd=0.1, step=step, grad_scale=0.5, sumsq=ss, max_norm=1.0)
+        out.append((p, m, v, w))
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
+    assert torch.equal(out[0][3], out[0][0].bfloat16())
