@@ -28,9 +28,9 @@ constexpr int PG_STAGING = 4 * 2 * 4096;
 constexpr int PG_A_BYTES = PG_BM * PG_BK * 2;
 constexpr int PG_STAGE_BYTES = PG_A_BYTES + 128 * PG_BK * 2;     // up to 128 columns of B per CTA
 // Stages: six, or five for the partial sums of a decode step (see gemm_skinny.cu on the shared memory of chained kernels).
-constexpr int pair_stages(int epi) { return epi == 1 ? 5 : 6; }
-constexpr int pair_smem(int epi) { return 1024 + pair_stages(epi) * PG_STAGE_BYTES + PG_STAGING + 512; }
-static_assert(pair_smem(0) <= 227 * 1024 && pair_smem(1) <= 196 * 1024, "shared memory");
+constexpr int pair_stages(int epi, bool chain) { return epi == 1 && chain ? 5 : 6; }
+constexpr int pair_smem(int epi, bool chain) { return 1024 + pair_stages(epi, chain) * PG_STAGE_BYTES + PG_STAGING + 512; }
+static_assert(pair_smem(0, false) <= 227 * 1024 && pair_smem(1, true) <= 196 * 1024, "shared memory");
 
 // Work of a launch: tiles of 256 rows x `bn` accumulator columns, each cut into `splits` pieces of `kb_per` K blocks (splits > 1: every piece
 // stores its own sums, `PG_F32` only).
@@ -41,11 +41,14 @@ struct PairWork {
 
 enum { PG_BF16 = 0, PG_F32 = 1, PG_F32_ADD = 2, PG_SWIGLU = 3 };
 
-template <int EPI, bool A_MN, bool B_MN>
+// CHAIN: a product of a decode step, whose weights one row tile reads: they are the first that L2 gives up, and the first of them may be requested before
+// the wait for the kernel in front. (In the one loop for both, a test per K block and B in front of A cost large products 1 to 5 %: 8192 x 12288 x 4096,
+// weight gradient 602 -> 625 us.)
+template <int EPI, bool A_MN, bool B_MN, bool CHAIN>
 __global__ void __launch_bounds__(PG_THREADS, 1) __cluster_dims__(2, 1, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                  const __grid_constant__ CUtensorMap tmap_c, const PairWork pw, int* status) {
-  constexpr int STAGES = pair_stages(EPI);
+  constexpr int STAGES = pair_stages(EPI, CHAIN);
   const int M = pw.M, N = pw.N, BN = pw.bn;
   const int TN = EPI == PG_SWIGLU ? BN / 2 : BN;           // output columns per tile
   extern __shared__ uint8_t smem_raw[];
@@ -93,7 +96,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   griddep_launch();
-  if (warp != 0) griddep_wait();        // returns at once unless this grid was launched as a programmatic dependent; the producer waits further down
+  if (!CHAIN || warp != 0) griddep_wait();      // returns at once unless this grid was launched as a programmatic dependent; a chain's producer waits below
 
   // Item order: groups of eight row tiles sweep N together, so that their rows of A stay in L2; the pieces of a tile follow each other.
   struct Item { int tm, tn, split, kb0, kb1; };
@@ -110,42 +113,49 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
   if (warp == 0) {
     if (lane == 0) {
-      const uint64_t policy = l2_policy(m_tiles == 1 && (EPI == PG_F32 || pw.pdl != 0));      // decode: weights that one row tile reads
-      auto load_b = [&](const Item& it, int stage, int kb) {
-        uint8_t* sb = smem + stage * PG_STAGE_BYTES + PG_A_BYTES;
-        // swiglu: the even CTA holds the gate rows of the tile's columns, the odd one the up rows (N = f rows further on)
-        const int n0 = EPI == PG_SWIGLU ? it.tn * TN + static_cast<int>(rank) * N : it.tn * TN + static_cast<int>(rank) * (BN / 2);
-        if (rank == 0) mbar_expect_tx(&full_bar[stage], stage_tx);
-        const uint32_t bar = cluster_addr(&full_bar[stage], 0);
-        if constexpr (!B_MN) {
-          tma_load_2d_pair_hint(sb, &tmap_b, bar, kb * PG_BK, n0, policy);
-        } else {
-          for (int c = 0; c * 64 < BN / 2; ++c) tma_load_2d_pair(sb + c * (64 * PG_BK * 2), &tmap_b, bar, n0 + c * 64, kb * PG_BK);
+      static_assert(!CHAIN || (!A_MN && !B_MN), "decode");
+      const uint64_t policy = l2_policy(m_tiles == 1);
+      int ahead = 0;                    // K blocks of the first item whose weights are under way
+      if constexpr (CHAIN) {
+        if (pw.pdl == 2 && first < num_items) {
+          const Item it = item(first);
+          for (int kb = it.kb0; kb < it.kb1 && ahead < STAGES; ++kb, ++ahead) {
+            if (rank == 0) mbar_expect_tx(&full_bar[ahead], stage_tx);
+            tma_load_2d_pair_hint(smem + ahead * PG_STAGE_BYTES + PG_A_BYTES, &tmap_b, cluster_addr(&full_bar[ahead], 0), kb * PG_BK,
+                                  it.tn * TN + static_cast<int>(rank) * (BN / 2), policy);
+          }
         }
-      };
-      int ahead = 0;
-      if (pw.pdl == 2 && first < num_items) {
-        const Item it = item(first);
-        for (int kb = it.kb0; kb < it.kb1 && ahead < STAGES; ++kb) load_b(it, ahead++, kb);
+        griddep_wait();
       }
-      griddep_wait();
-      int stage = 0, i = 0;
+      int stage = 0;
       uint32_t phase = 0;
       for (int w = first; w < num_items; w += step) {
         const Item it = item(w);
         const int m0 = it.tm * 2 * PG_BM + static_cast<int>(rank) * PG_BM;
-        for (int kb = it.kb0; kb < it.kb1; ++kb, ++i) {
-          if (i >= ahead) {
-            if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, status, 160)) goto producer_done;
-            load_b(it, stage, kb);
-          }
+        // swiglu: the even CTA holds the gate rows of the tile's columns, the odd one the up rows (N = f rows further on)
+        const int n0 = EPI == PG_SWIGLU ? it.tn * TN + static_cast<int>(rank) * N : it.tn * TN + static_cast<int>(rank) * (BN / 2);
+        for (int kb = it.kb0; kb < it.kb1; ++kb) {
+          const bool started = CHAIN && ahead > 0;
+          if (!started && !mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, status, 160)) goto producer_done;
           uint8_t* sa = smem + stage * PG_STAGE_BYTES;
+          uint8_t* sb = sa + PG_A_BYTES;
+          if (rank == 0 && !started) mbar_expect_tx(&full_bar[stage], stage_tx);
           const uint32_t bar = cluster_addr(&full_bar[stage], 0);
+          if constexpr (CHAIN) {
+            if (!started) tma_load_2d_pair_hint(sb, &tmap_b, bar, kb * PG_BK, n0, policy);
+            ahead -= started ? 1 : 0;
+          }
           if constexpr (!A_MN) {
             tma_load_2d_pair(sa, &tmap_a, bar, kb * PG_BK, m0);
           } else {
 #pragma unroll
             for (int c = 0; c < PG_BM / 64; ++c) tma_load_2d_pair(sa + c * (64 * PG_BK * 2), &tmap_a, bar, m0 + c * 64, kb * PG_BK);
+          }
+          if constexpr (CHAIN) {
+          } else if constexpr (!B_MN) {
+            tma_load_2d_pair(sb, &tmap_b, bar, kb * PG_BK, n0);
+          } else {
+            for (int c = 0; c * 64 < BN / 2; ++c) tma_load_2d_pair(sb + c * (64 * PG_BK * 2), &tmap_b, bar, n0 + c * 64, kb * PG_BK);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
@@ -284,13 +294,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   }
 }
 
-template <int EPI, bool A_MN, bool B_MN>
-static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const PairWork& pw, int num_sms, int* status,
+template <int EPI, bool A_MN, bool B_MN, bool CHAIN>
+static int launch_pair_kernel(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const PairWork& pw, int num_sms, int* status,
                        cudaStream_t stream) {
-  auto kern = gemm_pair_kernel<EPI, A_MN, B_MN>;
+  auto kern = gemm_pair_kernel<EPI, A_MN, B_MN, CHAIN>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_smem(EPI)) != cudaSuccess) return -20;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_smem(EPI, CHAIN)) != cudaSuccess) return -20;
     configured = true;
   }
   const int tn = EPI == PG_SWIGLU ? pw.bn / 2 : pw.bn;
@@ -299,7 +309,7 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs);
   cfg.blockDim = dim3(PG_THREADS);
-  cfg.dynamicSmemBytes = pair_smem(EPI);
+  cfg.dynamicSmemBytes = pair_smem(EPI, CHAIN);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -307,6 +317,14 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
   cfg.attrs = attr;
   cfg.numAttrs = pw.pdl ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, pw, status) == cudaSuccess ? 0 : -21;
+}
+
+template <int EPI, bool A_MN, bool B_MN>
+static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const PairWork& pw, int num_sms, int* status,
+                       cudaStream_t stream) {
+  if constexpr (!A_MN && !B_MN && (EPI == PG_BF16 || EPI == PG_F32))
+    if (pw.pdl != 0) return launch_pair_kernel<EPI, A_MN, B_MN, true>(ta, tb, tc, pw, num_sms, status, stream);
+  return launch_pair_kernel<EPI, A_MN, B_MN, false>(ta, tb, tc, pw, num_sms, status, stream);
 }
 
 template <int EPI>

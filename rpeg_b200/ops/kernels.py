@@ -27,11 +27,15 @@ class KernelWaitTimeout(RuntimeError):
     """A bounded device-side wait (mbarrier or peer flag) ran out; the kernel returned early."""
 
 
-_launch = threading.local()
+class _Launch(threading.local):
+    stream = None              # where this thread launches instead of on its current stream
+
+
+_launch = _Launch()
 
 
 def _stream() -> int:
-    other = getattr(_launch, "stream", None)
+    other = _launch.stream
     return (torch.cuda.current_stream() if other is None else other).cuda_stream
 
 
@@ -39,7 +43,7 @@ def _stream() -> int:
 def launching_on(stream: torch.cuda.Stream):
     """Calls of this thread inside launch on ``stream`` but allocate on the current one: keep what they return and what it was made from until the current
     stream has waited for ``stream``, and nothing more needs to be told to the allocator."""
-    was, _launch.stream = getattr(_launch, "stream", None), stream
+    was, _launch.stream = _launch.stream, stream
     try:
         yield
     finally:
