@@ -95,7 +95,7 @@ rope_kv_append_kernel(__nv_bfloat16* __restrict__ qkv, int ld, int q_col0, int k
 // attention kernel reads, k and v into the paged cache. NORM replaces a reduction, two norms and a rotation of their own
 // (Qwen3-8B, 4
 // layers, a step of 128 rows, with the other products' partial sums added up by their readers too: 0.98 -> 0.80 ms).
-template <bool NORM>
+template <bool NORM, int BATCH>
 __global__ void __launch_bounds__(256)
 rope_kv_append_partials_kernel(const float* __restrict__ parts, int splits, long long stride, __nv_bfloat16* __restrict__ qkv,
                                int ld, int q_col0, int k_col0, int v_col0, const int* __restrict__ seq_id,
@@ -122,7 +122,7 @@ rope_kv_append_partials_kernel(const float* __restrict__ parts, int splits, long
   const int i = lane * 2;
   // lane owns elements (i, i+1) and their rotation partners (i+half, i+half+1)
   const size_t off = static_cast<size_t>(t) * ld + col;
-  const float4 x = sum_in_order<8>(splits, [&](int s) {
+  const float4 x = sum_in_order<BATCH>(splits, [&](int s) {
     const float2 a = load2(parts + s * stride + off + i), b = load2(parts + s * stride + off + i + half);
     return make_float4(a.x, a.y, b.x, b.y);
   });
@@ -892,7 +892,9 @@ extern "C" int rpeg_rope_kv_append_partials(const float* parts, int splits, long
   if ((q_norm == nullptr) != (k_norm == nullptr)) return -4;
   const long long threads = static_cast<long long>(T) * (H + 2 * Hkv) * 32;
   if (threads <= 0) return 0;
-  auto kern = q_norm != nullptr ? rope_kv_append_partials_kernel<true> : rope_kv_append_partials_kernel<false>;
+  const bool few = T <= FEW_ROWS / 2;          // 32 heads: at 64 rows the loop is ahead already (3.04 and 3.38 us of two slabs)
+  auto kern = q_norm != nullptr ? (few ? rope_kv_append_partials_kernel<true, 4> : rope_kv_append_partials_kernel<true, 0>)
+                                : (few ? rope_kv_append_partials_kernel<false, 4> : rope_kv_append_partials_kernel<false, 0>);
   launch_pdl(kern, dim3(static_cast<unsigned>((threads + 255) / 256)), dim3(256), 0, STREAM(stream),
       parts, splits, stride, static_cast<__nv_bfloat16*>(qkv), ld, q_col0, k_col0, v_col0, seq_id, pos, cos_t, sin_t, page_table,
       max_pages, static_cast<__nv_bfloat16*>(kcache), static_cast<__nv_bfloat16*>(vcache), T, H, Hkv,

@@ -86,7 +86,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, __nv_bfloat
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= static_cast<long long>(M) * nv) return;
   const int m = static_cast<int>(idx / nv), j = static_cast<int>(idx % nv);
-  const float4 a = sum_in_order<8>(splits, [&](int s) { return load4(part + (static_cast<size_t>(s) * M + m) * N + j * 4); });
+  const float4 a = sum_in_order<0>(splits, [&](int s) { return load4(part + (static_cast<size_t>(s) * M + m) * N + j * 4); });
   uint2 o;
   o.x = pack_bf16x2(a.x, a.y);
   o.y = pack_bf16x2(a.z, a.w);

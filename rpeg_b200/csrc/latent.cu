@@ -29,12 +29,12 @@ struct Projection {
   int ld;
 };
 
-template <typename T, bool PARTIALS>
+template <typename T, int PARTIALS>
 __device__ __forceinline__ float4 read_projection(const Projection& s, int t, int col) {
   const size_t off = static_cast<size_t>(t) * s.ld + col;
   if constexpr (PARTIALS) {
     const float* p = static_cast<const float*>(s.p) + off;
-    return sum_in_order<8>(s.splits, [&](int k) { return load4(p + k * s.stride); });
+    return sum_in_order<PARTIALS == 2 ? 4 : 0>(s.splits, [&](int k) { return load4(p + k * s.stride); });
   } else {
     return load4(static_cast<const T*>(s.p) + off);
   }
@@ -73,7 +73,7 @@ __device__ __forceinline__ float4 rotate_pairs(float4 u, const LatentRows& a, in
 }
 
 // The first blocks normalise (one per token and segment), the others do what is elementwise (four columns per thread).
-template <typename T, bool PARTIALS>
+template <typename T, int PARTIALS>
 __global__ void __launch_bounds__(512)
 latent_rows_kernel(const LatentRows a, int norm_blocks, int items) {
   griddep_launch();
@@ -327,9 +327,10 @@ extern "C" int rpeg_latent_rows(const void* src, int splits, long long stride, i
 #define RPEG_LR(T_, P_)                                                                                                                      \
   return launch_pdl(latent_rows_kernel<T_, P_>, dim3(static_cast<unsigned>(blocks)), dim3(threads), smem, STREAM(stream), a,                 \
                     static_cast<int>(norm_blocks), items) == cudaSuccess ? 0 : -21;
-  if (f32) { RPEG_LR(float, false) }
-  if (splits > 0) { RPEG_LR(__nv_bfloat16, true) }
-  RPEG_LR(__nv_bfloat16, false)
+  if (f32) { RPEG_LR(float, 0) }
+  if (splits > 0 && rows <= FEW_ROWS) { RPEG_LR(__nv_bfloat16, 2) }
+  if (splits > 0) { RPEG_LR(__nv_bfloat16, 1) }
+  RPEG_LR(__nv_bfloat16, 0)
 #undef RPEG_LR
 }
 

@@ -34,7 +34,7 @@ __device__ __forceinline__ float4 weigh4(float4 v, float r, float w_add, float4 
 
 // NV > 0: a thread keeps NV groups of 4 columns in registers, together with their weights and (for an update) the stream's
 // old values, all requested before the first sum. NV = 0: rows of any width, held in shared memory.
-template <typename T, int SRC, int NV>
+template <typename T, int SRC, int NV, bool FEW>
 __global__ void __launch_bounds__(NV == 4 ? 512 : 1024)
 residual_norm_kernel(const NormSource src, const T* __restrict__ w, const T* __restrict__ w2, float* x, T* __restrict__ y,
                      int rows, int d, int dp, float eps, float w_add, int add) {
@@ -74,7 +74,7 @@ residual_norm_kernel(const NormSource src, const T* __restrict__ w, const T* __r
       v[j] = old[j] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (c < dp) {
         if (add) old[j] = load4(xr + c);
-        v[j] = norm_source<T, SRC>(src, choice_row, choice_w, row, rows, c);
+        v[j] = norm_source<T, SRC, FEW>(src, choice_row, choice_w, row, rows, c);
       }
       ss += dot4(v[j]);
     }
@@ -103,7 +103,7 @@ residual_norm_kernel(const NormSource src, const T* __restrict__ w, const T* __r
   } else {
     float ss = 0.f;
     for (int c = threadIdx.x * 4; c < dp; c += blockDim.x * 4) {
-      const float4 v = norm_source<T, SRC>(src, choice_row, choice_w, row, rows, c);
+      const float4 v = norm_source<T, SRC, FEW>(src, choice_row, choice_w, row, rows, c);
       store4(rowbuf + c, v);
       ss += dot4(v);
     }
@@ -203,7 +203,8 @@ static int launch_residual_norm_src(const NormSource& src, const T* w, const T* 
   if (smem > 220 * 1024) return -2;
 #define RPEG_NORM_NV(NV_)                                                                                                       \
   {                                                                                                                             \
-    auto kern = residual_norm_kernel<T, SRC, NV_>;                                                                              \
+    constexpr bool SUMS = SRC == NSRC_MOE || SRC == NSRC_PARTIALS;                                                              \
+    auto kern = SUMS && rows > FEW_ROWS ? residual_norm_kernel<T, SRC, NV_, !SUMS> : residual_norm_kernel<T, SRC, NV_, true>;   \
     if (smem > 48 * 1024 &&                                                                                                     \
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)         \
       return -20;                                                                                                               \

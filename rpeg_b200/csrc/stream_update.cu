@@ -14,7 +14,7 @@ namespace rpeg {
 constexpr int SU_THREADS = 128;
 enum { SU_NONE = -1 };
 
-template <typename T, int SRC_A, int SRC_B>
+template <typename T, int SRC_A, int SRC_B, bool FEW>
 __global__ void __launch_bounds__(SU_THREADS)
 stream_update_kernel(const NormSource a, const NormSource b, const float* __restrict__ alpha, const T* __restrict__ w,
                      const T* __restrict__ bias, float* __restrict__ x, T* __restrict__ y, int rows, int dp) {
@@ -38,8 +38,8 @@ stream_update_kernel(const NormSource a, const NormSource b, const float* __rest
   }
   if (!live) return;
   float* xr = x + static_cast<size_t>(row) * dp + c;
-  float4 v = norm_source<T, SRC_A>(a, nullptr, nullptr, row, rows, c);
-  if constexpr (SRC_B != SU_NONE) v = add4(v, norm_source<T, SRC_B>(b, choice_row, choice_w, row, rows, c));
+  float4 v = norm_source<T, SRC_A, FEW>(a, nullptr, nullptr, row, rows, c);
+  if constexpr (SRC_B != SU_NONE) v = add4(v, norm_source<T, SRC_B, FEW>(b, choice_row, choice_w, row, rows, c));
   if constexpr (SRC_A != NSRC_EMBED) v = add4(load4(xr), v);
   store4(xr, v);
   store4(y + static_cast<size_t>(row) * dp + c,
@@ -94,7 +94,8 @@ static int launch_stream_update(const NormSource& a, const NormSource& b, const 
       return launch_pdl(stream_update_rows_kernel<T>, dim3(rows * runs), dim3(SU_THREADS), smem, stream, a, b, alpha, static_cast<const T*>(w),
                         static_cast<const T*>(bias), x, static_cast<T*>(y), rows, dp, runs) == cudaSuccess ? 0 : -21;
   }
-  return launch_pdl(stream_update_kernel<T, SRC_A, SRC_B>, grid, dim3(SU_THREADS), smem, stream, a, b, alpha, static_cast<const T*>(w),
+  auto kern = rows <= FEW_ROWS ? stream_update_kernel<T, SRC_A, SRC_B, true> : stream_update_kernel<T, SRC_A, SRC_B, false>;
+  return launch_pdl(kern, grid, dim3(SU_THREADS), smem, stream, a, b, alpha, static_cast<const T*>(w),
                     static_cast<const T*>(bias), x, static_cast<T*>(y), rows, dp) == cudaSuccess ? 0 : -21;
 }
 

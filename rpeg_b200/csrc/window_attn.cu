@@ -22,7 +22,7 @@ constexpr int WPAGE = RPEG_KV_PAGE;
 // One warp per HPW heads of a token (query heads, then KV heads). A lane owns runs of 4 elements, i.e. whole pairs
 // (2i, 2i + 1), so the rotation is local; a rotation keeps the sum of squares, so the norm is known before it. Prompts take
 // four heads per warp (the angles are read once for all of them), decode one (more warps for few tokens).
-template <typename T, bool PARTIALS, int HPW>
+template <typename T, int PARTIALS, int HPW>       // PARTIALS: 0 an activation, 1 slabs of many rows, 2 of few
 __global__ void __launch_bounds__(256)
 rotary_append_kernel(const void* __restrict__ src_v, int splits, long long stride, int ld, int q_col0, int k_col0, int v_col0,
                      const int* __restrict__ slot, const int* __restrict__ pos, const float* __restrict__ cos_t,
@@ -42,7 +42,7 @@ rotary_append_kernel(const void* __restrict__ src_v, int splits, long long strid
     const size_t off = static_cast<size_t>(t) * ld + col;
     if constexpr (PARTIALS) {
       const float* s = static_cast<const float*>(src_v) + off;
-      return sum_in_order<8>(splits, [&](int k) { return load4(s + k * stride); });
+      return sum_in_order<PARTIALS == 2 ? 4 : 0>(splits, [&](int k) { return load4(s + k * stride); });
     } else {
       return load4(static_cast<const T*>(src_v) + off);
     }
@@ -452,10 +452,11 @@ extern "C" int rpeg_rotary_append(const void* src, int splits, long long stride,
   return launch_pdl(rotary_append_kernel<T_, P_, H_>, grid, dim3(256), 0, STREAM(stream), src, splits, stride, ld, q_col0, k_col0, v_col0, \
                     slot, pos, cos_t, sin_t, page_table, max_pages, static_cast<T_*>(q_out), ldq, static_cast<T_*>(kcache),            \
                     static_cast<T_*>(vcache), rows, H, Hkv, dim, dp, rot_dims, do_norm, eps) == cudaSuccess ? 0 : -21;
-  if (f32) { RPEG_RA(float, false, 1) }
-  if (splits > 0) { RPEG_RA(__nv_bfloat16, true, 1) }
-  if (hpw == 4) { RPEG_RA(__nv_bfloat16, false, 4) }
-  RPEG_RA(__nv_bfloat16, false, 1)
+  if (f32) { RPEG_RA(float, 0, 1) }
+  if (splits > 0 && rows <= FEW_ROWS) { RPEG_RA(__nv_bfloat16, 2, 1) }
+  if (splits > 0) { RPEG_RA(__nv_bfloat16, 1, 1) }
+  if (hpw == 4) { RPEG_RA(__nv_bfloat16, 0, 4) }
+  RPEG_RA(__nv_bfloat16, 0, 1)
 #undef RPEG_RA
 }
 
